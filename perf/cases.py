@@ -257,3 +257,48 @@ def tolerance(case):
         # e4m3 numbers may then become the other one, 1/16 away at most
         return {"rel": 6.6e-3, "max": 7e-2}
     return {"rel": 6.6e-3, "max": 1.6e-2}
+
+
+def _quantized(x, block):
+    """x[R, K] as e4m3 values with one scale per `block` of K (the largest value of a block becomes 448), in 64 bits.
+    The scales are arbitrary fp32 numbers for blocks of 128 and powers of two (MXFP8) for blocks of 32."""
+    r, k = x.shape
+    g = x.float().view(r, k // block, block)
+    scale = g.abs().amax(-1, keepdim=True).clamp_min(2.0 ** -100) * (1.0 / 448.0)
+    if block == 32:
+        scale = torch.exp2(torch.ceil(torch.log2(scale)))
+    return ((g * (1.0 / scale)).to(torch.float8_e4m3fn).double() * scale.double()).view(r, k)
+
+
+def exact(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kind = case["kind"]
+    if kind == "rpc":
+        return [_view(case, DTYPES[case["dtype"]], gen).double() for _ in range(case["calls"])]
+    if kind == "push":
+        x = _view(case, DTYPES[case["src"]], gen)
+        if case["src"] == "u8":
+            return x
+        return {"none": lambda v: v, "add": lambda v: v + 0.5, "mul": lambda v: v * 0.5}[case["op"]](x.double())
+    if kind == "gemm":
+        m, n, k, fmt = case["m"], case["n"], case["k"], case["fmt"]
+        x = torch.randn(m, k, device="cuda", generator=gen)
+        if case["via"] == "call":
+            gen = torch.Generator(device="cuda").manual_seed(4321)
+        w = torch.randn(k, n, device="cuda", generator=gen) * 0.02
+        if case["via"] == "call" or fmt == "bf16":
+            w = w.to(torch.bfloat16).float()
+        if fmt == "bf16":
+            return x.to(torch.bfloat16).double() @ w.double()
+        if fmt == "mxfp8":
+            return _quantized(x, 32) @ _quantized(w.t(), 32).t()
+        # weights: one scale per 128 x 128 block
+        blocks = w.t().reshape(n // 128, 128, k // 128, 128).transpose(1, 2).reshape(-1, 128 * 128)
+        w_t = _quantized(blocks, 128 * 128).view(n // 128, k // 128, 128, 128).transpose(1, 2).reshape(n, k)
+        return _quantized(x, 128) @ w_t.t()
+    t, topk, experts = case["tokens"], case["topk"], case["experts"]
+    x = torch.randn(t, case["hidden"], device="cuda", generator=gen).to(torch.bfloat16)
+    gates = torch.softmax(torch.randn(t, experts, device="cuda", generator=gen), dim=-1).topk(topk, dim=-1)
+    # an identity expert: every one of a token's copies comes back as its (quantised) row
+    rows = _quantized(x, 128) if case["fp8"] else x.double()
+    return rows * gates.values.double().sum(-1, keepdim=True)
