@@ -72,6 +72,7 @@ __device__ __forceinline__ bool cta_wait_arrival(const eux_xfer_desc& d) {
 // skip its share of the copy) while the last one to arrive succeeded. The scratch word counts arrivals
 // in its low 31 bits; a CTA that failed sets the top bit before it counts itself.
 __device__ __forceinline__ void cta_publish(const eux_xfer_desc& d, uint32_t* counter, bool ok) {
+  if (!d.flag && !d.flag2) return;  // nobody is told: the end of the launch is enough
   __syncthreads();
   if (threadIdx.x != 0) return;
   __threadfence_system();
@@ -302,39 +303,250 @@ __global__ void __launch_bounds__(kXferThreads) xfer_rpc_step_kernel(RpcStepArgs
   }
 }
 
-// Strided gather (and the catch-all for unaligned bases): one element per step.
-__global__ void __launch_bounds__(kXferThreads) xfer_strided_kernel(XferArgs a) {
+// ---- gathers ---------------------------------------------------------------------------------------
+// What the layout is, eux_xfer_launch finds out on the host (size-1 dimensions dropped, dimensions that are
+// contiguous with one another merged) and picks one of two kernels:
+//   * xfer_gather_kernel: the elements of the innermost dimension are next to one another in the source (row
+//     slices, permuted outer dimensions, dense tensors at any offset), or no dimension has stride 1;
+//   * xfer_tile_kernel: some other dimension has stride 1 (transposes): tiles through shared memory.
+
+__device__ __forceinline__ uint64_t div_u64(uint64_t a, uint64_t b) {
+  if (((a | b) >> 32) == 0) return (uint32_t)a / (uint32_t)b;  // most tensors; a 64-bit division costs several times as much
+  return a / b;
+}
+
+// NB bytes from any address, as aligned 16-byte loads of just the granules that hold them, and a byte shift.
+template <int NB>
+__device__ __forceinline__ void load_span(const unsigned char* p, uint32_t (&out)[NB / 4]) {
+  constexpr int NW = NB / 4;
+  constexpr int NL = (NB + 15) / 16;  // granules when aligned; one more otherwise
+  const uint32_t off = (uint32_t)(uintptr_t)p & 15u;
+  const uint4* base = reinterpret_cast<const uint4*>(p - off);
+  uint32_t w[4 * (NL + 1)];
+#pragma unroll
+  for (int i = 0; i <= NL; ++i) {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (i < NL ? true : off + NB > 16 * NL) v = base[i];
+    w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+  }
+#pragma unroll
+  for (int i = 0; i < NW + 2; ++i) w[i] = (off & 8u) ? (i + 2 < 4 * (NL + 1) ? w[i + 2] : 0u) : w[i];
+#pragma unroll
+  for (int i = 0; i < NW + 1; ++i) w[i] = (off & 4u) ? w[i + 1] : w[i];
+  const uint32_t sh = (off & 3u) * 8u;
+#pragma unroll
+  for (int i = 0; i < NW; ++i) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
+}
+
+// One element of the source as one of the destination: the bits themselves (RAW), or handler and cast.
+template <typename S, typename D, bool RAW>
+struct Convert;
+template <typename S, typename D>
+struct Convert<S, D, true> {
+  static __device__ __forceinline__ D one(S v, int, float) { return v; }
+};
+template <typename S, typename D>
+struct Convert<S, D, false> {
+  static __device__ __forceinline__ D one(S v, int op, float arg) { return Elem<D>::from(apply_op(Elem<S>::to(v), op, arg)); }
+};
+
+// Offset in the source, in elements, of the row (every dimension but the innermost) and the column of element e.
+__device__ __forceinline__ int64_t gather_row(const eux_xfer_desc& d, uint64_t e, uint64_t& col) {
+  const int last = d.ndim - 1;
+  uint64_t rem = div_u64(e, (uint64_t)d.shape[last]);
+  col = e - rem * (uint64_t)d.shape[last];
+  int64_t off = 0;
+  for (int k = last - 1; k >= 0; --k) {
+    const uint64_t q = div_u64(rem, (uint64_t)d.shape[k]);
+    off += (int64_t)(rem - q * (uint64_t)d.shape[k]) * d.stride[k];
+    rem = q;
+  }
+  return off;
+}
+
+// A thread makes 16 (8 for a narrowing cast to one byte, 32 for one to fp32) aligned bytes of the destination per
+// step: one index computation for them, one or two aligned loads when they lie in one row of the source, single
+// elements when they straddle rows or the innermost stride is not 1. Bound by DRAM.
+template <typename S, typename D, bool RAW>
+__global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_constant__ XferArgs a) {
   const eux_xfer_desc& d = a.d;
   bool ok = cta_wait_arrival(d);
   if (ok) {
+    constexpr int V = RAW ? 16 / (int)sizeof(D) : 8;
+    constexpr int DB = V * (int)sizeof(D);
+    constexpr int SB = V * (int)sizeof(S);
+    constexpr int VEC = DB >= 16 ? 16 : 8;
+    const S* src = reinterpret_cast<const S*>(d.src);
+    D* dst = reinterpret_cast<D*>(d.dst);
+    const uint64_t n = d.n_elems;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
-    const bool raw = (d.src_dtype == d.dst_dtype && d.op == EUX_OP_NONE) || d.src_dtype == EUX_DT_BYTES;
-    const int esz = dtype_size(d.src_dtype);
-    for (uint64_t e = tid; e < d.n_elems; e += nthreads) {
-      uint64_t rem = e;
-      int64_t off = 0;
-      if (d.ndim == 0) {
-        off = (int64_t)e;
+    const uint64_t cols = (uint64_t)d.shape[d.ndim - 1];
+    const int64_t inner = d.stride[d.ndim - 1];
+    const int op = d.op;
+    const float arg = d.op_arg;
+    uint64_t lead = ((VEC - ((uintptr_t)dst & (VEC - 1))) & (VEC - 1)) / sizeof(D);  // elements in front of the first aligned vector
+    if (lead > n) lead = n;
+    const uint64_t chunks = (n - lead) / V;
+    for (uint64_t i = tid; i < chunks; i += nthreads) {
+      const uint64_t e = lead + i * V;
+      uint64_t c;
+      int64_t row = gather_row(d, e, c);
+      alignas(16) D out[V];
+      if (inner == 1 && c + V <= cols) {
+        alignas(16) uint32_t w[SB / 4];
+        load_span<SB>(reinterpret_cast<const unsigned char*>(src + row + (int64_t)c), w);
+        const S* sv = reinterpret_cast<const S*>(w);
+#pragma unroll
+        for (int k = 0; k < V; ++k) out[k] = Convert<S, D, RAW>::one(sv[k], op, arg);
       } else {
-        for (int k = d.ndim - 1; k >= 0; --k) {
-          uint64_t q = rem / (uint64_t)d.shape[k];
-          off += (int64_t)(rem - q * (uint64_t)d.shape[k]) * d.stride[k];
-          rem = q;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          if (c >= cols) row = gather_row(d, e + k, c);
+          out[k] = Convert<S, D, RAW>::one(src[row + (int64_t)c * inner], op, arg);
+          ++c;
         }
       }
-      if (raw) {
-        const unsigned char* s = reinterpret_cast<const unsigned char*>(d.src) + off * esz;
-        unsigned char* t = reinterpret_cast<unsigned char*>(d.dst) + e * esz;
-        if (esz == 4) *reinterpret_cast<uint32_t*>(t) = *reinterpret_cast<const uint32_t*>(s);
-        else if (esz == 2) *reinterpret_cast<uint16_t*>(t) = *reinterpret_cast<const uint16_t*>(s);
-        else *t = *s;
-      } else {
-        store_from_float(d.dst, e, d.dst_dtype, apply_op(load_as_float(d.src, (uint64_t)off, d.src_dtype), d.op, d.op_arg));
-      }
+#pragma unroll
+      for (int k = 0; k < DB / VEC; ++k)
+        reinterpret_cast<typename PackT<VEC>::type*>(dst + e)[k] = reinterpret_cast<typename PackT<VEC>::type*>(out)[k];
+    }
+    const uint64_t tail = lead + chunks * V;  // single elements in front of the vectors and behind them
+    for (uint64_t i = tid; i < lead + (n - tail); i += nthreads) {
+      const uint64_t e = i < lead ? i : tail + (i - lead);
+      uint64_t c;
+      const int64_t row = gather_row(d, e, c);
+      dst[e] = Convert<S, D, RAW>::one(src[row + (int64_t)c * inner], op, arg);
     }
   }
   cta_publish(d, a.counter, ok);
+}
+
+// Transposes. A tile is `tp` steps of the dimension with stride 1 in the source (P) times `tq` of the innermost
+// dimension (Q): it is read along P, with 16-byte loads where the rows' alignment allows them (VECTOR) and element
+// by element otherwise, converted, and kept in shared memory as words of G = 4 / sizeof(D) neighbours along Q, so
+// that 1- and 2-byte elements are transposed within registers and shared memory only ever moves whole words. The
+// row pitch is odd, so reads and writes meet at most two-way bank conflicts. Rows of Q leave as 16-byte stores, or
+// element by element where the destination's rows are not 16-byte aligned.
+constexpr int kTileThreads = 256;
+constexpr int kTileWords = 64 * 33;  // 64 steps of P, 32 words (128 bytes) of Q, one word of padding
+struct TileArgs {
+  XferArgs x;
+  int64_t batch_src[EUX_MAX_DIMS], batch_dst[EUX_MAX_DIMS];  // strides of the other dimensions, in elements
+  uint32_t batch_shape[EUX_MAX_DIMS];
+  int64_t q_src, p_dst;  // strides, in elements
+  uint32_t n_batch, np, nq, tp, tq, tiles_p, tiles_q;
+  uint32_t pitch;  // words
+  uint32_t vector_store;
+  uint64_t tiles;
+};
+
+template <typename S, typename D, bool RAW, bool VECTOR>
+__global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_constant__ TileArgs t) {
+  __shared__ uint32_t sm[kTileWords];
+  const eux_xfer_desc& d = t.x.d;
+  const bool ok = cta_wait_arrival(d);
+  if (ok) {
+    constexpr int G = 4 / (int)sizeof(D);
+    constexpr int VP = VECTOR ? 16 / (int)sizeof(S) : 1;
+    const int op = d.op;
+    const float arg = d.op_arg;
+    const uint32_t pitch = t.pitch;
+    for (uint64_t tile = blockIdx.x; tile < t.tiles; tile += gridDim.x) {
+      // neighbouring tiles along P first: they share the source's lines where rows are not aligned to lines
+      uint64_t r = div_u64(tile, t.tiles_p);
+      const uint32_t p0 = (uint32_t)(tile - r * t.tiles_p) * t.tp;
+      uint64_t b = div_u64(r, t.tiles_q);
+      const uint32_t q0 = (uint32_t)(r - b * t.tiles_q) * t.tq;
+      int64_t so = (int64_t)p0 + (int64_t)q0 * t.q_src;
+      int64_t dof = (int64_t)p0 * t.p_dst + (int64_t)q0;
+      for (int k = (int)t.n_batch - 1; k >= 0; --k) {
+        const uint64_t bq = div_u64(b, t.batch_shape[k]);
+        const int64_t ix = (int64_t)(b - bq * t.batch_shape[k]);
+        so += ix * t.batch_src[k];
+        dof += ix * t.batch_dst[k];
+        b = bq;
+      }
+      const S* src = reinterpret_cast<const S*>(d.src) + so;
+      D* dst = reinterpret_cast<D*>(d.dst) + dof;
+      const uint32_t pn = min(t.tp, t.np - p0), qn = min(t.tq, t.nq - q0);
+
+      // read: a unit is VP steps of P by G of Q; the unit index is kept split so that no step divides
+      const uint32_t pu = (pn + VP - 1) / VP, qw = (qn + G - 1) / G;
+      {
+        const uint32_t dq = kTileThreads / pu, dp = kTileThreads - dq * pu;
+        uint32_t iq = threadIdx.x / pu, ip = threadIdx.x - iq * pu;
+#pragma unroll 4
+        while (iq < qw) {
+          const uint32_t p = ip * VP;
+          alignas(16) S v[G][VP];
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            const uint32_t q = iq * G + g;
+            const S* s = src + (int64_t)q * t.q_src + p;
+            if (VECTOR && q < qn && p + VP <= pn) {
+              *reinterpret_cast<uint4*>(v[g]) = *reinterpret_cast<const uint4*>(s);
+            } else {
+#pragma unroll
+              for (int i = 0; i < VP; ++i) {
+                if (q < qn && p + i < pn) v[g][i] = s[i];
+                else memset(&v[g][i], 0, sizeof(S));
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < VP; ++i) {
+            uint32_t word;
+            alignas(4) D o[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) o[g] = Convert<S, D, RAW>::one(v[g][i], op, arg);
+            memcpy(&word, o, 4);
+            if (p + i < pn) sm[(p + i) * pitch + iq] = word;
+          }
+          ip += dp;
+          iq += dq;
+          if (ip >= pu) ip -= pu, ++iq;
+        }
+      }
+      __syncthreads();
+
+      // write
+      if (t.vector_store) {
+        constexpr uint32_t E = 16 / sizeof(D);
+        const uint32_t vr = (qn + E - 1) / E;
+        const uint32_t dr = kTileThreads / vr, dv = kTileThreads - dr * vr;
+        uint32_t row = threadIdx.x / vr, v = threadIdx.x - row * vr;
+        while (row < pn) {
+          const uint32_t* w = sm + row * pitch + v * 4;
+          D* out = dst + (int64_t)row * t.p_dst + v * E;
+          if (v * E + E <= qn) {
+            *reinterpret_cast<uint4*>(out) = make_uint4(w[0], w[1], w[2], w[3]);
+          } else {
+            for (uint32_t i = 0; v * E + i < qn; ++i) {
+              const uint32_t word = w[i / G] >> (8 * sizeof(D) * (i % G));
+              memcpy(out + i, &word, sizeof(D));
+            }
+          }
+          row += dr;
+          v += dv;
+          if (v >= vr) v -= vr, ++row;
+        }
+      } else {
+        const uint32_t dr = kTileThreads / qn, dq = kTileThreads - dr * qn;
+        uint32_t row = threadIdx.x / qn, q = threadIdx.x - row * qn;
+#pragma unroll 4
+        while (row < pn) {
+          const uint32_t word = sm[row * pitch + q / G] >> (8 * sizeof(D) * (q % G));
+          memcpy(dst + (int64_t)row * t.p_dst + q, &word, sizeof(D));
+          row += dr;
+          q += dq;
+          if (q >= qn) q -= qn, ++row;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  cta_publish(d, t.x.counter, ok);
 }
 
 // One CTA per descriptor; meant for many small messages per launch.
@@ -496,6 +708,101 @@ static int launch_typed(const XferArgs& a, int grid, cudaStream_t st) {
   return 0;
 }
 
+// The layout with as few dimensions as describe it. False: it describes nothing (a size below 1, or a size that
+// does not multiply up to the number of elements): the caller's own words are then followed as they stand.
+static bool collapse(eux_xfer_desc& d) {
+  uint64_t prod = 1;
+  for (int i = 0; i < d.ndim; ++i) {
+    if (d.shape[i] < 1 || __builtin_mul_overflow(prod, (uint64_t)d.shape[i], &prod)) return false;
+  }
+  if (prod != d.n_elems || prod >> 62) return false;
+  int nd = 0;
+  for (int i = 0; i < d.ndim; ++i) {
+    if (d.shape[i] == 1) continue;
+    int64_t span;
+    if (nd > 0 && !__builtin_mul_overflow(d.shape[i], d.stride[i], &span) && d.stride[nd - 1] == span) {
+      d.shape[nd - 1] *= d.shape[i];  // the outer one steps over the whole of the inner one: one dimension
+      d.stride[nd - 1] = d.stride[i];
+    } else {
+      d.shape[nd] = d.shape[i];
+      d.stride[nd] = d.stride[i];
+      ++nd;
+    }
+  }
+  d.ndim = nd;
+  if (nd == 0 || (nd == 1 && d.stride[0] == 1)) d.ndim = 0;
+  return true;
+}
+
+template <typename S, typename D, bool RAW>
+static void launch_gather(const XferArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
+  if (!t) xfer_gather_kernel<S, D, RAW><<<grid, kXferThreads, 0, st>>>(a);
+  else if (vector) xfer_tile_kernel<S, D, RAW, true><<<grid, kTileThreads, 0, st>>>(*t);
+  else xfer_tile_kernel<S, D, RAW, false><<<grid, kTileThreads, 0, st>>>(*t);
+}
+template <typename S>
+static int launch_gather_from(const XferArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
+  switch (a.d.dst_dtype) {
+    case EUX_DT_F32: launch_gather<S, float, false>(a, t, vector, grid, st); break;
+    case EUX_DT_F16: launch_gather<S, __half, false>(a, t, vector, grid, st); break;
+    case EUX_DT_BF16: launch_gather<S, __nv_bfloat16, false>(a, t, vector, grid, st); break;
+    case EUX_DT_F8E4M3: launch_gather<S, __nv_fp8_e4m3, false>(a, t, vector, grid, st); break;
+    default: return EUX_ERR_BAD_ARG;
+  }
+  return 0;
+}
+
+// Fills `t` when the layout is a transpose the tile kernel takes: the innermost dimension is strided and another one
+// has stride 1. (Without such a dimension every element has a line of its own and tiles would gain nothing.)
+static bool plan_tiles(const eux_xfer_desc& d, TileArgs& t, bool& vector) {
+  const int last = d.ndim - 1;
+  if (d.ndim < 2 || d.stride[last] == 1) return false;
+  int p = -1;
+  for (int k = 0; k < last; ++k)
+    if (d.stride[k] == 1) p = k;
+  if (p < 0) return false;
+  for (int k = 0; k < d.ndim; ++k)
+    if (d.shape[k] > 0x7fffffff) return false;
+  const int ssz = dtype_size(d.src_dtype), dsz = dtype_size(d.dst_dtype), g = 4 / dsz;
+  t.np = (uint32_t)d.shape[p], t.nq = (uint32_t)d.shape[last];
+  t.q_src = d.stride[last];
+  bool store16 = ((uintptr_t)d.dst & 15u) == 0;
+  vector = (((uintptr_t)d.src | (uint64_t)(t.q_src * ssz)) & 15u) == 0;
+  uint64_t inner = 1, batch = 1;
+  int64_t dst_stride[EUX_MAX_DIMS];
+  for (int k = last; k >= 0; --k) {
+    dst_stride[k] = (int64_t)inner;
+    inner *= (uint64_t)d.shape[k];
+  }
+  t.n_batch = 0;
+  for (int k = 0; k < last; ++k) {
+    if ((dst_stride[k] * dsz) & 15) store16 = false;
+    if (k == p) continue;
+    if ((d.stride[k] * ssz) & 15) vector = false;
+    t.batch_src[t.n_batch] = d.stride[k], t.batch_dst[t.n_batch] = dst_stride[k];
+    t.batch_shape[t.n_batch++] = (uint32_t)d.shape[k];
+    batch *= (uint64_t)d.shape[k];
+  }
+  t.p_dst = dst_stride[p];
+  // 64 steps of P by 128 bytes of Q; where one of the two is shorter the tile is as much longer in the other
+  uint32_t qw_all = (t.nq + g - 1) / g, qw = 32, tp = 64;
+  if (t.np < 64) {
+    tp = t.np;
+    qw = (uint32_t)(kTileWords / tp - 1) & ~3u;
+    if (qw > qw_all) qw = qw_all;
+  } else if (qw_all < 32) {
+    qw = qw_all;
+    tp = ((uint32_t)kTileWords / (qw | 1u)) & ~15u;  // whole vectors of P
+    if (tp > t.np) tp = t.np;
+  }
+  t.pitch = qw | 1u;
+  t.tp = tp, t.tq = qw * g < t.nq ? qw * g : t.nq;
+  t.tiles_p = (t.np + tp - 1) / tp, t.tiles_q = (t.nq + t.tq - 1) / t.tq;
+  t.tiles = batch * t.tiles_p * t.tiles_q;
+  t.vector_store = store16;
+  return true;
+}
+
 }  // namespace eux
 
 using namespace eux;
@@ -508,21 +815,21 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
   const int sms = num_sms();
   const bool ctas_given = max_ctas > 0;
   if (!ctas_given) max_ctas = 2 * sms;
-  const uint64_t src_bytes = d->n_elems * (uint64_t)dtype_size(d->src_dtype);
   const bool raw = d->src_dtype == d->dst_dtype && d->op == EUX_OP_NONE;
+  const bool whole = collapse(a.d);
+  const int ssz = dtype_size(d->src_dtype), dsz = dtype_size(d->dst_dtype);
   const uintptr_t al = ((uintptr_t)d->src) | ((uintptr_t)d->dst);
+  auto limit = [&](uint64_t want) { return (int)(want < 1 ? 1 : (want > (uint64_t)max_ctas ? max_ctas : want)); };
   int grid;
-  if (d->ndim == 0 && raw && (al & 15u) == 0) {
+  if (a.d.ndim == 0 && raw && (al & 15u) == 0) {
     // 64 B per thread per step, one CTA per SM; small messages stay on one CTA (no counter traffic)
     if (!ctas_given) max_ctas = sms;
-    uint64_t want = (src_bytes + (uint64_t)kXferThreads * 64 - 1) / ((uint64_t)kXferThreads * 64);
-    grid = (int)(want < 1 ? 1 : (want > (uint64_t)max_ctas ? max_ctas : want));
+    grid = limit((d->n_elems * (uint64_t)ssz + (uint64_t)kXferThreads * 64 - 1) / ((uint64_t)kXferThreads * 64));
     if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
     if ((al & 31u) == 0) xfer_bytes_kernel<true><<<grid, kXferThreads, 0, st>>>(a);
     else xfer_bytes_kernel<false><<<grid, kXferThreads, 0, st>>>(a);
-  } else if (d->ndim == 0 && d->src_dtype != EUX_DT_BYTES && (al & 15u) == 0) {
-    uint64_t want = (d->n_elems / 8 + kXferThreads - 1) / kXferThreads;
-    grid = (int)(want < 1 ? 1 : (want > (uint64_t)max_ctas ? max_ctas : want));
+  } else if (a.d.ndim == 0 && d->src_dtype != EUX_DT_BYTES && (al & 15u) == 0) {
+    grid = limit((d->n_elems / 8 + kXferThreads - 1) / kXferThreads);
     if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
     int rc = 0;
     switch (d->src_dtype) {
@@ -534,10 +841,43 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     }
     if (rc) return rc;
   } else {
-    uint64_t want = (d->n_elems + kXferThreads * 4 - 1) / (kXferThreads * 4);
-    grid = (int)(want < 1 ? 1 : (want > (uint64_t)max_ctas ? max_ctas : want));
+    bool as_bytes = false;
+    if (a.d.ndim == 0) {  // dense, but not on a 16-byte boundary: one row
+      as_bytes = raw;
+      if (as_bytes) a.d.n_elems *= (uint64_t)ssz;
+      a.d.ndim = 1;
+      a.d.shape[0] = a.d.n_elems ? (int64_t)a.d.n_elems : 1;
+      a.d.stride[0] = 1;
+    }
+    if (!as_bytes && (((uintptr_t)d->src % ssz) || ((uintptr_t)d->dst % dsz))) return EUX_ERR_BAD_ARG;  // would fault
+    for (int k = 0; k < a.d.ndim; ++k)
+      if (a.d.shape[k] < 1 && a.d.n_elems) return EUX_ERR_BAD_ARG;
+    TileArgs t;
+    bool vector = false;
+    const bool tiled = whole && !as_bytes && plan_tiles(a.d, t, vector);
+    if (tiled) t.x = a;
+    // Eight tile CTAs (256 threads) and four gather CTAs (512) fill an SM's threads.
+    if (!ctas_given) max_ctas = (tiled ? 8 : 4) * sms;
+    const uint64_t per_cta = (uint64_t)kXferThreads * (raw ? 16 / (as_bytes ? 1 : dsz) : 8);
+    grid = limit(tiled ? t.tiles : (a.d.n_elems + per_cta - 1) / per_cta);
     if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
-    xfer_strided_kernel<<<grid, kXferThreads, 0, st>>>(a);
+    const TileArgs* tp = tiled ? &t : nullptr;
+    int rc = 0;
+    if (raw) {
+      const int esz = as_bytes ? 1 : ssz;
+      if (esz == 4) launch_gather<uint32_t, uint32_t, true>(a, tp, vector, grid, st);
+      else if (esz == 2) launch_gather<uint16_t, uint16_t, true>(a, tp, vector, grid, st);
+      else launch_gather<uint8_t, uint8_t, true>(a, tp, vector, grid, st);
+    } else {
+      switch (d->src_dtype) {
+        case EUX_DT_F32: rc = launch_gather_from<float>(a, tp, vector, grid, st); break;
+        case EUX_DT_F16: rc = launch_gather_from<__half>(a, tp, vector, grid, st); break;
+        case EUX_DT_BF16: rc = launch_gather_from<__nv_bfloat16>(a, tp, vector, grid, st); break;
+        case EUX_DT_F8E4M3: rc = launch_gather_from<__nv_fp8_e4m3>(a, tp, vector, grid, st); break;
+        default: rc = EUX_ERR_BAD_ARG;
+      }
+    }
+    if (rc) return rc;
   }
   return (int)cudaGetLastError();
 }
@@ -716,6 +1056,13 @@ int preload_one(K kernel) {
   cudaFuncAttributes attr;
   return (int)cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(kernel));
 }
+template <typename S, typename D, bool RAW>
+int preload_gather() {
+  int rc = preload_one(xfer_gather_kernel<S, D, RAW>);
+  if (!rc) rc = preload_one(xfer_tile_kernel<S, D, RAW, true>);
+  if (!rc) rc = preload_one(xfer_tile_kernel<S, D, RAW, false>);
+  return rc;
+}
 template <typename S>
 int preload_typed() {
   int rc = preload_one(xfer_typed_kernel<S, float>);
@@ -723,6 +1070,10 @@ int preload_typed() {
   if (!rc) rc = preload_one(xfer_typed_kernel<S, __nv_bfloat16>);
   if (!rc) rc = preload_one(xfer_typed_kernel<S, __nv_fp8_e4m3>);
   if (!rc) rc = preload_one(xfer_rpc_step_kernel<S>);
+  if (!rc) rc = preload_gather<S, float, false>();
+  if (!rc) rc = preload_gather<S, __half, false>();
+  if (!rc) rc = preload_gather<S, __nv_bfloat16, false>();
+  if (!rc) rc = preload_gather<S, __nv_fp8_e4m3, false>();
   return rc;
 }
 }  // namespace
@@ -731,7 +1082,9 @@ extern "C" int eux_xfer_preload(void) {
   int rc = preload_one(xfer_bytes_kernel<true>);
   if (!rc) rc = preload_one(xfer_bytes_kernel<false>);
   if (!rc) rc = preload_one(xfer_bulk_kernel);
-  if (!rc) rc = preload_one(xfer_strided_kernel);
+  if (!rc) rc = preload_gather<uint8_t, uint8_t, true>();
+  if (!rc) rc = preload_gather<uint16_t, uint16_t, true>();
+  if (!rc) rc = preload_gather<uint32_t, uint32_t, true>();
   if (!rc) rc = preload_one(xfer_batch_kernel);
   if (!rc) rc = preload_one(pingpong_kernel);
   if (!rc) rc = preload_one(xfer_pull_batch_kernel);

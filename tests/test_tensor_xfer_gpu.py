@@ -62,6 +62,62 @@ def test_strided_gather(cuda_device):
         assert torch.equal(raw, view.contiguous().view(-1))
 
 
+def _views(dtype, dev):
+    """Layouts at the edges of the gather and tile kernels, as (name, view): tile remainders, rows of a few elements,
+    odd offsets and pitches, several dimensions in any order, broadcast and stepped ones."""
+    def t(*shape):
+        x = torch.randn(shape, device=dev) * 2
+        return (x * 40).to(torch.uint8) if dtype == torch.uint8 else x.to(dtype)
+    yield "offset", t(4099)[3:].view(8, 512)
+    yield "rows", t(37, 200)[:, :150]
+    yield "rows of 3", t(300, 5)[:, 1:4]
+    yield "rows aligned", t(50, 256)[:, 128:]
+    yield "transposed", t(129, 67).t()
+    yield "transposed aligned", t(256, 192).t()
+    yield "transposed wide", t(4096, 3).t()
+    yield "transposed wide 2", t(5000, 2).t()
+    yield "transposed tall", t(3, 4111).t()
+    yield "transposed tall 2", t(2, 8192).t()
+    yield "transposed offset", t(80, 131)[5:, 3:].t()
+    yield "heads", t(2, 33, 4, 64).transpose(1, 2)
+    yield "heads transposed", t(2, 33, 4, 65).permute(0, 2, 3, 1)
+    yield "reversed", t(5, 6, 7, 72).permute(3, 2, 1, 0)
+    yield "rotated", t(65, 3, 130).permute(2, 0, 1)
+    yield "broadcast inner", t(70, 1).expand(70, 40)
+    yield "broadcast outer", t(1, 90).expand(40, 90)
+    yield "broadcast transposed", t(3, 1, 90).expand(3, 40, 90).transpose(1, 2)
+    yield "stepped", t(40, 200)[:, ::3]
+    yield "stepped transposed", t(130, 140).t()[::2]
+    yield "size 1", t(7, 1, 9, 1, 1).permute(2, 1, 0, 4, 3)
+
+
+@pytest.mark.parametrize("src_dtype,dst_dtype,op", [(torch.uint8, torch.uint8, 0), (torch.float16, torch.float16, 0),
+                                                    (torch.float32, torch.float32, 0), (torch.float32, torch.bfloat16, 0),
+                                                    (torch.bfloat16, torch.float32, 1), (torch.float32, torch.float8_e4m3fn, 2),
+                                                    (torch.float8_e4m3fn, torch.float16, 0), (torch.bfloat16, torch.bfloat16, 2)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gather_layouts(cuda_device, src_dtype, dst_dtype, op, shift):
+    """Every layout, into a destination on and off a 16-byte boundary, with the elements around it left alone. One
+    handler operation in fp32 and one rounding: the results are equal."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    flag = _flag(cuda_device)
+    for i, (name, view) in enumerate(_views(src_dtype, cuda_device)):
+        n = view.numel()
+        if src_dtype == torch.uint8:
+            ref = view.contiguous().view(-1)
+            buf = torch.full((n + 40,), 9, dtype=dst_dtype, device=cuda_device)
+        else:
+            f = view.contiguous().view(-1).float()
+            ref = {0: f, 1: f + 0.5, 2: f * 0.5}[op].to(dst_dtype)
+            buf = torch.full((n + 40,), 9.0, device=cuda_device).to(dst_dtype)
+        dst = buf[16 + shift:16 + shift + n]
+        tx.push(view, dst, op=op, op_arg=0.5, flag_ptr=flag.data_ptr(), flag_value=i + 1)
+        torch.cuda.synchronize()
+        assert torch.equal(dst.float(), ref.float()), name
+        assert bool((buf[:16 + shift].float() == 9).all()) and bool((buf[16 + shift + n:].float() == 9).all()), name
+        assert int(flag[0]) == i + 1, name
+
+
 def test_batch(cuda_device):
     from execution_ucx_b200.ops import tensor_xfer as tx
     g = torch.Generator(device="cpu").manual_seed(3)
