@@ -29,16 +29,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait; returns false (and raises *abort) when the limit passes or another role aborted.
+// Bounded wait; returns false (and raises *abort) when the limit passes or another role aborted. The clock is first
+// read after 256 failed tries: a read of %globaltimer takes longer than most of these waits (a pipeline stage, a
+// partial product), and nearly every wait fails its first try.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort, uint64_t timeout_ns) {
-  if (mbar_try(bar, parity)) return true;
-  const uint64_t limit = timeout_ns ? timeout_ns : 2000000000ull;
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   for (uint32_t it = 0; it < 0x7fffffffu; ++it) {
     if (mbar_try(bar, parity)) return true;
     if ((it & 255u) == 255u) {
       if (*abort) return false;
-      if (globaltimer_ns() - t0 > limit) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > (timeout_ns ? timeout_ns : 2000000000ull)) {
         *abort = 1;
         return false;
       }

@@ -894,14 +894,14 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
         : "memory");
     return ok != 0;
   };
-  if (try_once()) return true;
-  const uint64_t limit = timeout_ns ? timeout_ns : 2000000000ull;
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   for (uint32_t it = 0; it < 0x7fffffffu; ++it) {
     if (try_once()) return true;
     if ((it & 255u) == 255u) {
       if (*abort) return false;
-      if (globaltimer_ns() - t0 > limit) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > (timeout_ns ? timeout_ns : 2000000000ull)) {
         *abort = 1;
         return false;
       }
@@ -912,6 +912,12 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
 }
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// The arrive that hands a TMEM buffer back: what it orders are tcgen05 loads (tcgen05.fence::before_thread_sync in
+// front of it), nothing in memory, so it is not a cluster-scope release. With one, every arrive waited for the
+// warp's outstanding memory operations.
+__device__ __forceinline__ void mbar_arrive_remote_tmem(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // per-CTA tile load of a CTA pair: the bytes land in this CTA, the completion is counted on `bar`, a
 // shared::cluster address (the even CTA's barrier)
@@ -1156,7 +1162,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(map_to_cta(tempty_bar(buf), 0));
+        if (lane == 0) mbar_arrive_remote_tmem(map_to_cta(tempty_bar(buf), 0));
 #pragma unroll
         for (int sl = 0; sl < BN / 64; ++sl, ++slab) {
           const uint32_t sbuf = epi0 + (slab & 1u) * EPI_SLAB_BYTES;
@@ -1201,7 +1207,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         if (sl == BN / 64 - 1) {  // this CTA's half of the accumulator is out of TMEM
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_remote(map_to_cta(tempty_bar(buf), 0));
+          if (lane == 0) mbar_arrive_remote_tmem(map_to_cta(tempty_bar(buf), 0));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         epi_bar_sync(1);
@@ -1227,6 +1233,301 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   const bool ok = s_abort == 0;
   if (!ok && threadIdx.x == 0) {
     set_status(p.status, EUX_ST_TIMEOUT, 22);
+    atomicExch(p.sched + 1, 1u);
+  }
+  finish_cta(p, ok);
+}
+
+// ---------------------------------------------------------------------------
+// Block-scaled fp8 on CTA pairs: the promotion scheme of remote_gemm_fp8_kernel on 256 x 256 tiles. What bounds the
+// 128 x 128 kernel is the operand feed from L2 (about 13 TB/s over all SMs, 46 bytes per SM and cycle): its K-block
+// brings 32 KiB into an SM for 256 cycles of MMA. Here the same 32 KiB serve twice the MMAs. A CTA's 128 x 256 partial
+// product fills half of its TMEM, so two are in flight; each of the eight epilogue warps folds 32 rows by 128 columns
+// into 128 registers (the register file is split unevenly: setmaxnreg). Rows and columns past M and N (both are
+// multiples of 128, a tile is 256) are zero-filled loads, and nothing is stored for them.
+// ---------------------------------------------------------------------------
+constexpr int STAGES8P = 5;
+constexpr int GEMM8P_THREADS = 384;  // warp 0 TMA, warp 1 MMA (even CTA), warps 2 and 3 copy X, warps 4..11 epilogue
+constexpr int STAGE8P_BYTES = A_STAGE_BYTES + B2_STAGE_BYTES;
+constexpr int SCALE8P_K = 8;                                // K-blocks of scales per batch
+constexpr int SCALE8P_FLOATS = 33 * (SCALE8P_K + 1);        // 32 rows of X scales and one of Wt scales, odd pitch
+constexpr size_t GEMM8P_SMEM =
+    (size_t)STAGES8P * STAGE8P_BYTES + 2 * EPI_SLAB_BYTES + 8 * 2 * SCALE8P_FLOATS * sizeof(float) + 1024 + 256;
+// 168 registers per thread at launch; 128 x 96 + 256 x 200 = 63488 of the 384 x 168 = 64512 that the block has
+constexpr int REGS8P_OTHERS = 96, REGS8P_EPILOGUE = 200;
+
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+__device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM8P_THREADS, 1)
+remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                            const __grid_constant__ CUtensorMap map_y, GemmParams p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sA = smem;
+  unsigned char* sB = smem + (size_t)STAGES8P * A_STAGE_BYTES;
+  unsigned char* sEpi = smem + (size_t)STAGES8P * STAGE8P_BYTES;  // one slab per half
+  float* sScale = reinterpret_cast<float*>(sEpi + 2 * EPI_SLAB_BYTES);  // two batches for each epilogue warp
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sScale + 8 * 2 * SCALE8P_FLOATS);
+  // bars: [0,S) full (used in the even CTA), [S,2S) empty, then 2 tmem_full, 2 tmem_empty (even CTA), TILE_RING tile slots
+  __shared__ uint32_t s_tmem_base;
+  __shared__ int s_abort;
+  __shared__ int s_tiles[TILE_RING];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_cta_rank();
+  const bool leader = rank == 0;
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (STAGES8P + s); };
+  auto tfull_bar = [&](int b) { return bar0 + 8u * (2 * STAGES8P + b); };
+  auto tempty_bar = [&](int b) { return bar0 + 8u * (2 * STAGES8P + 2 + b); };
+  auto tile_bar = [&](int i) { return bar0 + 8u * (2 * STAGES8P + 4 + i); };
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < TILE_RING; ++i) mbar_init(tile_bar(i), 1);
+    for (int s = 0; s < STAGES8P; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(tfull_bar(b), 1);
+      mbar_init(tempty_bar(b), 16);  // eight epilogue warps in each CTA of the pair
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                 "r"((uint32_t)TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the partner's barriers exist before anything arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = s_tmem_base;
+
+  const int m_blocks = (p.M + 2 * BM - 1) / (2 * BM), n_blocks = (p.N + BN - 1) / BN;
+  const int total = m_blocks * n_blocks;
+  const int k_blocks = p.K / 128;
+  volatile int* abort = &s_abort;
+  auto next_tile = [&](int it) -> int {
+    if (!mbar_wait_cluster(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
+    return *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
+  };
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS8P_OTHERS));
+    if (warp == 0) {
+      // ---------------- loads: both CTAs, completion counted in the even CTA ----------------
+      if (lane == 0) {
+        int s = 0;
+        uint32_t ph = 0;
+        for (int it = 0;; ++it) {
+          int tile;
+          if (leader) {
+            tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+            const int slot = it & (TILE_RING - 1);
+            s_tiles[slot] = tile;
+            mbar_arrive(tile_bar(slot));
+            st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), 1), (uint32_t)tile);
+            mbar_arrive_remote(map_to_cta(tile_bar(slot), 1));
+          } else {
+            tile = next_tile(it);
+          }
+          if (tile >= total) break;
+          int mb, nb;
+          tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+          const int panel = 2 * mb + (int)rank;  // this CTA's 128 rows (past M for the odd CTA of a last half block)
+          if (p.panel_target > 0 && panel * BM < p.M) {
+            if (!wait_u32_ge_gpu(p.panel_flags + panel, p.panel_target, p.timeout_ns)) {
+              *abort = 1;
+              break;
+            }
+            asm volatile("fence.proxy.async;" ::: "memory");
+          }
+          for (int k = 0; k < k_blocks; ++k) {
+            if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+            const uint32_t full_leader = map_to_cta(full_bar(s), 0);
+            if (leader) mbar_expect_tx(full_bar(s), 2 * STAGE8P_BYTES);
+            tma_load_2d_pair(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_leader, k * 128, panel * BM);
+            tma_load_2d_pair(smem_u32(sB + (size_t)s * B2_STAGE_BYTES), &map_b, full_leader, k * 128, nb * BN + (int)rank * (BN / 2));
+            if (++s == STAGES8P) s = 0, ph ^= 1u;
+          }
+        }
+        if (*abort) {
+          const uint64_t t0 = globaltimer_ns();
+          while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+        }
+      }
+    } else if (warp == 1) {
+      // ---------------- MMA: the even CTA issues for the pair, one partial product per K-block ----------------
+      if (leader && lane == 0) {
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+        int s = 0;
+        uint32_t ph = 0, blk = 0;
+        for (int it = 0;; ++it) {
+          if (next_tile(it) >= total || *abort) break;
+          for (int k = 0; k < k_blocks && !*abort; ++k, ++blk) {
+            const int buf = blk & 1u;
+            if (!mbar_wait(tempty_bar(buf), ((blk >> 1) & 1u) ^ 1u, abort, p.timeout_ns)) break;
+            if (!mbar_wait(full_bar(s), ph, abort, p.timeout_ns)) break;
+            tc_fence_after();
+            const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
+            const uint32_t a0 = smem_u32(sA + (size_t)s * A_STAGE_BYTES);
+            const uint32_t b0 = smem_u32(sB + (size_t)s * B2_STAGE_BYTES);
+#pragma unroll
+            for (int kk = 0; kk < BKB / 32; ++kk)
+              umma_fp8_pair(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)(kk != 0));
+            umma_commit_pair(tfull_bar(buf));
+            umma_commit_pair(map_to_cta(tfull_bar(buf), 1));
+            umma_commit_pair(empty_bar(s));
+            umma_commit_pair(map_to_cta(empty_bar(s), 1));
+            if (++s == STAGES8P) s = 0, ph ^= 1u;
+          }
+        }
+      }
+    } else {
+      // ---------------- warps 2 and 3: X and its scales from the caller's memory into the staging buffer ----------------
+      if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
+    }
+    __syncwarp();
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS8P_EPILOGUE));
+    const int lg = (warp - 4) & 3;     // TMEM lane group
+    const int half = (warp - 4) >> 2;  // which 128 columns of the tile: one block of W's scales
+    const int row_local = lg * 32 + lane;
+    const bool elected = lg == 0 && lane == 0;
+    const uint32_t sbuf = smem_u32(sEpi) + (uint32_t)half * EPI_SLAB_BYTES;
+    const uint32_t tempty0 = map_to_cta(tempty_bar(0), 0);
+    float* my_scales = sScale + (size_t)(warp - 4) * 2 * SCALE8P_FLOATS;
+    uint32_t blk = 0;
+    for (int it = 0;; ++it) {
+      const int tile = next_tile(it);
+      if (epi_vote_any(1 + half, tile >= total)) break;
+      int mb, nb;
+      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+      const int panel = 2 * mb + (int)rank;
+      const int nblk = nb * 2 + half;
+      const bool inside = panel * BM < p.M && nblk * 128 < p.N;  // the same for all threads of a half
+      const float* sx = p.x_scale_stage + (size_t)(panel * BM + lg * 32) * k_blocks;  // of this warp's first row
+      const float* sw = p.w_scale + (size_t)nblk * k_blocks;
+      float acc[128];
+#pragma unroll
+      for (int j = 0; j < 128; ++j) acc[j] = 0.f;
+      bool ok = true;
+      if (p.panel_target > 0 && inside) {  // the scales of pulled rows are there once their panel is reported
+        int arrived = 1;
+        if (lane == 0) arrived = wait_u32_ge_gpu(p.panel_flags + panel, p.panel_target, p.timeout_ns) ? 1 : 0;
+        arrived = __shfl_sync(0xffffffffu, arrived, 0);
+        if (!arrived) {
+          *abort = 1;
+          ok = false;
+        }
+      }
+      // Eight K-blocks of this warp's scales at a time: asynchronous copies into the warp's own buffer, one batch
+      // ahead. (Fetched into registers K-block by K-block, the loads in flight held up the arrive below, which waits
+      // for them: 171 us instead of 85 on 1920 x 4608 x 7168.)
+      auto stage_scales = [&](int batch) {
+        float* buf = my_scales + (batch & 1) * SCALE8P_FLOATS;
+        if (ok && inside) {
+#pragma unroll
+          for (int i = 0; i < SCALE8P_K; ++i) {
+            const int row = i * 4 + (lane >> 3), k = batch * SCALE8P_K + (lane & 7);
+            if (k < k_blocks) cp_async_4(smem_u32(buf + row * (SCALE8P_K + 1) + (lane & 7)), sx + (size_t)row * k_blocks + k);
+          }
+          const int k = batch * SCALE8P_K + lane;
+          if (lane < SCALE8P_K && k < k_blocks) cp_async_4(smem_u32(buf + 32 * (SCALE8P_K + 1) + lane), sw + k);
+        }
+        cp_async_commit();
+      };
+      __syncwarp();
+      stage_scales(0);
+      for (int k = 0; ok && k < k_blocks; ++k, ++blk) {
+        const int j8 = k % SCALE8P_K;
+        if (j8 == 0) {
+          __syncwarp();  // every lane has read the buffer that the next batch goes into
+          stage_scales(k / SCALE8P_K + 1);
+          cp_async_wait_1();
+          __syncwarp();
+        }
+        const int buf = blk & 1u;
+        const uint32_t tph = (blk >> 1) & 1u;
+        if (!mbar_wait(tfull_bar(buf), tph, abort, p.timeout_ns)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const float* sc = my_scales + ((k / SCALE8P_K) & 1) * SCALE8P_FLOATS;
+        const float scale = inside ? sc[lane * (SCALE8P_K + 1) + j8] * sc[32 * (SCALE8P_K + 1) + j8] : 0.f;
+        const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)buf * BN + (uint32_t)half * 128;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tbase + c * 32, r);
+          tmem_ld_wait();
+          if (c == 3) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote_tmem(tempty0 + 8u * buf);  // in registers: the buffer may be overwritten
+          }
+#pragma unroll
+          for (int j = 0; j < 32; j += 2)
+            ffma2(acc[c * 32 + j], acc[c * 32 + j + 1], __uint_as_float(r[j]), __uint_as_float(r[j + 1]), scale);
+        }
+      }
+      if (epi_vote_any(1 + half, !ok)) break;
+      if (!inside) continue;
+#pragma unroll
+      for (int sl = 0; sl < 2; ++sl) {
+        if (elected) bulk_wait_read_0();  // the store before this one has read the slab
+        epi_bar_sync(1 + half);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint4 o;
+          __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            q[j] = __floats2bfloat162_rn(acc[sl * 64 + c * 8 + 2 * j], acc[sl * 64 + c * 8 + 2 * j + 1]);
+          st_shared_u4(sbuf + (uint32_t)row_local * 128u + (uint32_t)((c ^ (row_local & 7)) * 16), o);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        epi_bar_sync(1 + half);
+        if (elected) {
+          tma_store_2d(&map_y, sbuf, nblk * 128 + sl * 64, panel * BM);
+          bulk_commit();
+        }
+      }
+    }
+    if (elected) {
+      bulk_wait_all();
+      asm volatile("fence.proxy.async;" ::: "memory");
+    }
+    __syncwarp();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // neither CTA leaves while the other may still touch its shared memory or TMEM
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
+  }
+  const bool ok = s_abort == 0;
+  if (!ok && threadIdx.x == 0) {
+    set_status(p.status, EUX_ST_TIMEOUT, 23);
     atomicExch(p.sched + 1, 1u);
   }
   finish_cta(p, ok);
@@ -1378,6 +1679,31 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
     }
     return (int)cudaGetLastError();
   }
+  const bool copy_by_warps = pull && (d->flags & EUX_GEMM_FLAG_COPY_WARPS);
+  // Block-scaled fp8 on CTA pairs or on single CTAs: a K-block takes 0.76 us of a pair's 256 x 256 tile and 0.53 us of
+  // a CTA's 128 x 128 tile (1920 x 4608 x 7168: 89 us against 113; 512 x 4096 x 7168, one wave of either: 54 against
+  // 42), so the pairs are taken when they need at most 7 / 10 of the waves. Pulled scales are read through L1, which
+  // is sound while no line holds rows of two panels: their staging buffer starts on a line.
+  const int tiles1 = (d->M / BM) * (d->N / BN8), tiles2 = ((d->M + 2 * BM - 1) / (2 * BM)) * ((d->N + BN - 1) / BN);
+  const int waves1 = (tiles1 + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
+  if (d->fp8 && (!pull || (copy_by_warps && ((uintptr_t)d->x_scale_stage & 127u) == 0)) && waves2 * 10 <= waves1 * 7) {
+    static bool attr8_set[64] = {false};
+    if (!attr8_set[dev]) {
+      cudaError_t e = cudaFuncSetAttribute(remote_gemm_fp8_2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM8P_SMEM);
+      if (e != cudaSuccess) return (int)e;
+      attr8_set[dev] = true;
+    }
+    if (pull) {
+      if (head_arg < 0) p.head_blocks = 2;
+      p.copy_ctas = 0;
+      p.copy_warps = 2 * 2 * (sms / 2);
+      p.panel_target = warp_target(p.copy_warps);
+    }
+    const int pairs = pull ? sms / 2 : (tiles2 < sms / 2 ? tiles2 : sms / 2);
+    // Wt in boxes of 128 rows (`mb`): each CTA of a pair loads its half of a tile's 256
+    remote_gemm_fp8_2cta_kernel<<<2 * pairs, GEMM8P_THREADS, GEMM8P_SMEM, (cudaStream_t)stream>>>(ma, mb, my, p);
+    return (int)cudaGetLastError();
+  }
   const int tiles = (d->M / BM) * (d->N / bn);
   int grid = copy_ctas + (tiles < sms - copy_ctas ? tiles : sms - copy_ctas);
   if (pull && (d->flags & EUX_GEMM_FLAG_COPY_WARPS)) {  // every SM takes part in the copy, with or without a tile
@@ -1452,7 +1778,7 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
 extern "C" int eux_gemm_preload(void) {
   cudaFuncAttributes attr;
   const void* kernels[] = {(const void*)remote_gemm_kernel<false>, (const void*)remote_gemm_fp8_kernel, (const void*)remote_gemm_2cta_kernel<false>,
-                           (const void*)remote_gemm_2cta_kernel<true>};
+                           (const void*)remote_gemm_2cta_kernel<true>, (const void*)remote_gemm_fp8_2cta_kernel};
   for (const void* k : kernels) {
     cudaError_t e = cudaFuncGetAttributes(&attr, k);
     if (e != cudaSuccess) return (int)e;

@@ -59,6 +59,32 @@ def test_block_scaled_fp8_matches_fp32(cuda_device, m, n, k, pull):
         assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(1920, 2688, 128), (1664, 3200, 1152), (3968, 1280, 384)])
+@pytest.mark.parametrize("pull", [False, "warps"])
+def test_block_scaled_fp8_pairs(cuda_device, m, n, k, pull):
+    """More than one wave of 128 x 128 tiles: the kernel on CTA pairs, with half tiles at the end of M and of N, K-blocks
+    that are not whole batches of scales, and every row's scale different. fp32 sums in another order and one rounding to
+    bf16: half a unit in the last of 8 bits of the result, and 1e-5 of the product's scale for the sums."""
+    from execution_ucx_b200.ops import remote_gemm as rg
+    torch.manual_seed(m + n + k)
+    x = torch.randn(m, k, device=cuda_device) * torch.rand(m, 1, device=cuda_device).mul(8).exp2()
+    w = torch.randn(k, n, device=cuda_device) * 0.02
+    g = rg.RemoteGemmFp8(w, m)
+    xq, xs = rg.quantize_rows_1x128(x)
+    buf = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    y = buf[:m]
+    for _ in range(2):
+        y.zero_()
+        g(xq.data_ptr(), xs.data_ptr(), m, y.data_ptr(), x_is_local=not pull)
+        torch.cuda.synchronize()
+        g.check_status()
+        ref = rg.dequantized_reference(xq.double(), xs.double(), g.w_q_t.double(), g.w_scale.double()).double()
+        bound = ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True) + 1e-30
+        assert bool(((y.double() - ref).abs() <= bound).all())
+        assert bool((buf[m] == 7).all())
+        assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+
+
 @pytest.mark.parametrize("pull", [False, True, "warps"])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 768, 1024), (1024, 512, 2048), (5120, 512, 128)])
 def test_bf16_cta_pairs(cuda_device, m, n, k, pull):
