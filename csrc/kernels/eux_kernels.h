@@ -202,7 +202,7 @@ typedef struct eux_gemm_desc {
   int32_t copy_ctas;     /* CTAs that stream X from the peer; 0 when x_stage == x_src */
   int32_t flags;         /* EUX_GEMM_FLAG_* */
 } eux_gemm_desc;
-/* bf16 with M % 256 == 0: tiles of 256 x 256 computed by pairs of CTAs (cta_group::2) */
+/* bf16: tiles of 256 x 256 computed by pairs of CTAs (cta_group::2) where there are enough of them */
 #define EUX_GEMM_FLAG_CTA_PAIRS 1
 /* With a remote X: two spare warps of every CTA copy X (and its scales) beside the GEMM's warps, instead of
    copy_ctas CTAs that copy first and compute afterwards. */

@@ -19,6 +19,7 @@
 // EUX_ST_TIMEOUT in the status word.
 #include <cuda.h>
 
+#include <atomic>
 #include <cstdlib>
 
 #include "eux_bulk.cuh"
@@ -53,6 +54,7 @@ struct GemmParams {
   int head_blocks;  // height of the first tile group in row blocks (0: like the others)
   int copy_warps;   // warps (two per CTA) that copy X beside the GEMM's own warps; 0 when copy CTAs do it
   uint32_t panel_target;  // count at which a panel of X is complete (0: X is local, nothing to wait for)
+  int split;        // CTAs (one cluster) that share the K of a tile
   int done_always;        // publish the done flag after a failed run too (the status word says which it was)
   // block-scaled fp8 only
   const float* x_scale_src;   // [M, K/128], caller's (may be peer)
@@ -108,6 +110,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
 }
@@ -385,7 +396,89 @@ __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   }
 }
 
-template <bool FP8>
+__device__ __forceinline__ uint32_t cluster_cta_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// the address of `addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
+  uint32_t out;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The sum over a cluster whose CTAs have each computed a share of K of one 128 x 256 tile: CTA r owns 256 / split of
+// the columns, every CTA stores its partial sums (fp32) of the other owners' columns into their shared memory, and the
+// owner adds them up in the order of the ranks and writes its part of Y. All pipeline stages are idle by then: the
+// first cluster barrier comes after every CTA's last MMA. All eight warps take part; a thread handles one row.
+// Layout of a part: 16 bytes (four columns) of one row next to the same columns of the next row.
+// `rank` counts the shares of K; the CTA that has another share of the same rows is `stride` cluster ranks per share
+// further on from `first`. (mb, nb): the tile in blocks of 128 rows and 256 columns.
+__device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_base, uint32_t smem0, int mb, int nb, int rank,
+                                          int first, int stride) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lg = warp & 3, side = warp >> 2;
+  const int row = lg * 32 + lane;
+  const int width = BN / p.split, half = width / 2;  // this thread: columns [side * half, +half) of an owner's
+  const uint32_t part_bytes = (uint32_t)width * BM * 4u;
+  const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * half);
+  const uint32_t mine = smem0 + (uint32_t)row * 16u + (uint32_t)(side * half / 4) * (BM * 16u);
+  __syncwarp();
+  cluster_sync_all();
+  for (int d = 1; d < p.split; ++d) {
+    const int owner = (rank + d) % p.split;  // each CTA starts with another one
+    const uint32_t slot = (uint32_t)(rank < owner ? rank : rank - 1);
+    const uint32_t dst = map_to_cta(mine + slot * part_bytes, (uint32_t)(first + owner * stride));
+    for (int c = 0; c < half; c += 16) {
+      uint32_t r[16];
+      tmem_ld16(tbase + (uint32_t)(owner * width + c), r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(c / 4 + q) * (BM * 16u)), "r"(r[4 * q]),
+                     "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
+                     : "memory");
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+  unsigned char* out = p.y + ((size_t)(mb * BM + row) * p.N + (size_t)nb * BN + rank * width + side * half) * 2;
+  for (int c = 0; c < half; c += 16) {
+    uint32_t own[16];
+    tmem_ld16(tbase + (uint32_t)(rank * width + c), own);
+    tmem_ld_wait();
+    float acc[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[j] = 0.f;
+    for (int r = 0; r < p.split; ++r) {
+      const uint32_t src = mine + (uint32_t)(r < rank ? r : r - 1) * part_bytes + (uint32_t)(c / 4) * (BM * 16u);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t v[4] = {own[4 * q], own[4 * q + 1], own[4 * q + 2], own[4 * q + 3]};
+        if (r != rank)
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                       : "r"(src + (uint32_t)q * (BM * 16u))
+                       : "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[4 * q + j] += __uint_as_float(v[j]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint4 o;
+      __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) q[j] = __floats2bfloat162_rn(acc[8 * h + 2 * j], acc[8 * h + 2 * j + 1]);
+      st_u4(out + c * 2 + h * 16, o);
+    }
+  }
+}
+
+template <bool SPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_y, GemmParams p) {
@@ -445,7 +538,10 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   const int m_blocks = p.M / BM, n_blocks = p.N / BN;
   const int total = m_blocks * n_blocks;
-  const int k_iters = p.K * p.elem_bytes / BKB;
+  const int k_all = p.K * p.elem_bytes / BKB;
+  const int rank = SPLIT ? (int)cluster_cta_rank() : 0;
+  const int k_begin = SPLIT ? k_all * rank / p.split : 0;  // this CTA's share of K
+  const int k_iters = (SPLIT ? k_all * (rank + 1) / p.split : k_all) - k_begin;
   const int kelems = BKB / p.elem_bytes;  // elements of K per stage
   volatile int* abort = &s_abort;
   // the next tile as the consumer roles see it: bounded wait on the ring slot, then its content
@@ -460,7 +556,9 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       int s = 0;
       uint32_t ph = 0;
       for (int it = 0;; ++it) {
-        const int tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+        int tile;
+        if (SPLIT) tile = it == 0 ? (int)blockIdx.x / p.split : total;  // one tile per cluster
+        else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
         if (tile >= total) break;
@@ -476,8 +574,8 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int k = 0; k < k_iters; ++k) {
           if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
           mbar_expect_tx(full_bar(s), A_STAGE_BYTES + B_STAGE_BYTES);
-          tma_load_2d(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_bar(s), k * kelems, mb * BM);
-          tma_load_2d(smem_u32(sB + (size_t)s * B_STAGE_BYTES), &map_b, full_bar(s), k * kelems, nb * BN);
+          tma_load_2d(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_bar(s), (k_begin + k) * kelems, mb * BM);
+          tma_load_2d(smem_u32(sB + (size_t)s * B_STAGE_BYTES), &map_b, full_bar(s), (k_begin + k) * kelems, nb * BN);
           if (++s == STAGES) s = 0, ph ^= 1u;
         }
       }
@@ -489,7 +587,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc<FP8, BN>();
+      constexpr uint32_t idesc = make_idesc<false, BN>();
       int s = 0;
       uint32_t ph = 0;
       for (int it = 0;; ++it) {
@@ -506,7 +604,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           const uint32_t b0 = smem_u32(sB + (size_t)s * B_STAGE_BYTES);
 #pragma unroll
           for (int kk = 0; kk < BKB / 32; ++kk) {
-            umma<FP8>(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)((k | kk) != 0));
+            umma<false>(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)((k | kk) != 0));
           }
           umma_commit(empty_bar(s));
           if (++s == STAGES) s = 0, ph ^= 1u;
@@ -535,6 +633,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint32_t tph = (uint32_t)(it >> 1) & 1u;
       const bool got = mbar_wait(tfull_bar(buf), tph, abort, p.timeout_ns);
       if (epi_vote_any(1, !got)) break;  // all four warps or none: the slab barriers below need everyone
+      if (SPLIT) break;  // summed over the cluster below
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)buf * BN;
 #pragma unroll 1
@@ -579,6 +678,14 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   tc_fence_before();
   __syncthreads();
+  if (SPLIT) {
+    tc_fence_after();
+    int mb, nb;
+    tile_coords((int)blockIdx.x / p.split, m_blocks, n_blocks, p.head_blocks, mb, nb);
+    split_sum(p, tmem_base, smem_u32(smem), mb, nb, rank, 0, 1);
+    tc_fence_before();
+    __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
@@ -610,6 +717,66 @@ constexpr int TMEM8_COLS = 512;
 constexpr int TBUF8 = 4;  // partial products in flight: four 128-column TMEM buffers
 constexpr size_t GEMM8_SMEM = (size_t)STAGES8 * (A8_STAGE_BYTES + B8_STAGE_BYTES) + 2 * 16384 /* output slabs */ + 1024 + 256;
 
+// split_sum for the block-scaled fp8 kernel, whose epilogue warps hold their sums in registers: thread (row, half) has
+// the 64 columns of its half of a 128 x 128 tile. Called by the epilogue warps; the others join the two barriers.
+__device__ __forceinline__ void split_sum_regs(const GemmParams& p, const float (&acc)[64], uint32_t smem0, int tile, int m_blocks,
+                                               int n_blocks, int rank, int half, int row) {
+  const int width = 128 / p.split;  // columns per owner: 64, 32 or 16
+  const uint32_t part_bytes = (uint32_t)width * BM * 4u;
+  __syncwarp();
+  cluster_sync_all();
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {  // 16 columns at a time: all of one owner's
+    const int col = half * 64 + g * 16, owner = col / width;
+    if (owner == rank) continue;
+    const uint32_t dst = map_to_cta(smem0 + (uint32_t)(rank < owner ? rank : rank - 1) * part_bytes + (uint32_t)row * 16u +
+                                        (uint32_t)((col - owner * width) / 4) * (BM * 16u),
+                                    (uint32_t)owner);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)q * (BM * 16u)), "f"(acc[g * 16 + 4 * q]),
+                   "f"(acc[g * 16 + 4 * q + 1]), "f"(acc[g * 16 + 4 * q + 2]), "f"(acc[g * 16 + 4 * q + 3])
+                   : "memory");
+  }
+  __syncwarp();
+  cluster_sync_all();
+  int mb, nb;
+  tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const int col = half * 64 + g * 16;
+    if (col / width != rank) continue;
+    float sum[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+    for (int r = 0; r < p.split; ++r) {
+      const uint32_t src = smem0 + (uint32_t)(r < rank ? r : r - 1) * part_bytes + (uint32_t)row * 16u +
+                           (uint32_t)((col - rank * width) / 4) * (BM * 16u);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float v[4] = {acc[g * 16 + 4 * q], acc[g * 16 + 4 * q + 1], acc[g * 16 + 4 * q + 2], acc[g * 16 + 4 * q + 3]};
+        if (r != rank)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                       : "r"(src + (uint32_t)q * (BM * 16u))
+                       : "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[4 * q + j] += v[j];
+      }
+    }
+    unsigned char* out = p.y + ((size_t)(mb * BM + row) * p.N + (size_t)nb * BN8 + col) * 2;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint4 o;
+      __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) q[j] = __floats2bfloat162_rn(sum[8 * h + 2 * j], sum[8 * h + 2 * j + 1]);
+      st_u4(out + h * 16, o);
+    }
+  }
+}
+
+template <bool SPLIT>
 __global__ void __launch_bounds__(GEMM8_THREADS, 1)
 remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_y, GemmParams p) {
@@ -665,7 +832,10 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const uint32_t tmem_base = s_tmem_base;
   const int m_blocks = p.M / BM, n_blocks = p.N / BN8;
   const int total = m_blocks * n_blocks;
-  const int k_blocks = p.K / 128;
+  const int kscales = p.K / 128;
+  const int rank = SPLIT ? (int)cluster_cta_rank() : 0;
+  const int k_begin = SPLIT ? kscales * rank / p.split : 0;  // this CTA's share of K
+  const int k_blocks = (SPLIT ? kscales * (rank + 1) / p.split : kscales) - k_begin;
   volatile int* abort = &s_abort;
   auto next_tile = [&](int it) -> int {
     if (!mbar_wait(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
@@ -677,7 +847,9 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       int s = 0;
       uint32_t ph = 0;
       for (int it = 0;; ++it) {
-        const int tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+        int tile;
+        if (SPLIT) tile = it == 0 ? (int)blockIdx.x / p.split : total;  // one tile per cluster
+        else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
         if (tile >= total) break;
@@ -693,8 +865,8 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         for (int k = 0; k < k_blocks; ++k) {
           if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
           mbar_expect_tx(full_bar(s), A8_STAGE_BYTES + B8_STAGE_BYTES);
-          tma_load_2d(smem_u32(sA + (size_t)s * A8_STAGE_BYTES), &map_a, full_bar(s), k * 128, mb * BM);
-          tma_load_2d(smem_u32(sB + (size_t)s * B8_STAGE_BYTES), &map_b, full_bar(s), k * 128, nb * BN8);
+          tma_load_2d(smem_u32(sA + (size_t)s * A8_STAGE_BYTES), &map_a, full_bar(s), (k_begin + k) * 128, mb * BM);
+          tma_load_2d(smem_u32(sB + (size_t)s * B8_STAGE_BYTES), &map_b, full_bar(s), (k_begin + k) * 128, nb * BN8);
           if (++s == STAGES8) s = 0, ph ^= 1u;
         }
       }
@@ -732,23 +904,28 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   } else if (warp < 4) {
     // warps 2 and 3: X (and its scales) from the caller's memory into the staging buffer
     if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
-  } else {
+  }
+  if (SPLIT && warp < 4) {  // the two barriers of split_sum_regs count every thread of the cluster
+    __syncwarp();
+    cluster_sync_all();
+    cluster_sync_all();
+  }
+  if (warp >= 4) {
     const int lg = (warp - 4) & 3;    // TMEM lane group
     const int half = (warp - 4) >> 2;  // which 64 columns of the tile
     const int row_local = lg * 32 + lane;
     const bool elected = lg == 0 && lane == 0;  // one per half: issues (and owns) that half's TMA stores
     const uint32_t sbuf = smem_u32(sEpi) + (uint32_t)half * EPI_SLAB_BYTES;
     uint32_t blk = 0;
-    const int kscales = p.K / 128;
+    float acc[64];
     for (int it = 0;; ++it) {
       const int tile = next_tile(it);
       if (epi_vote_any(1 + half, tile >= total)) break;  // the four warps of a half leave together
       int mb, nb;
       tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
       const int row = mb * BM + lg * 32 + lane;
-      const float* sx = p.x_scale_stage + (size_t)row * kscales;
-      const float* sw = p.w_scale + (size_t)nb * kscales;
-      float acc[64];
+      const float* sx = p.x_scale_stage + (size_t)row * kscales + k_begin;
+      const float* sw = p.w_scale + (size_t)nb * kscales + k_begin;
 #pragma unroll
       for (int j = 0; j < 64; ++j) acc[j] = 0.f;
       bool ok = true;
@@ -800,6 +977,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         s0 = s1;
         s1 = sx2 * sw2;
       }
+      if (SPLIT) break;  // summed over the cluster below
       if (elected) bulk_wait_read_0();  // the previous tile's store has read this half's slab
       if (epi_vote_any(1 + half, !ok)) break;  // the four warps of a half leave together
 #pragma unroll
@@ -817,6 +995,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         bulk_commit();
       }
     }
+    if (SPLIT) split_sum_regs(p, acc, smem_u32(smem), (int)blockIdx.x / p.split, m_blocks, n_blocks, rank, half, row_local);
     if (elected) {  // Y is complete before this CTA reports
       bulk_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");
@@ -843,7 +1022,8 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // tcgen05.mma.cta_group::2 over both CTAs' shared memory, and each CTA ends up with its 128 rows of
 // the accumulator in its own TMEM. Per CTA and K-step that is 32 KiB of operands instead of 48 KiB,
 // so six stages fit where the one-CTA kernel has four: more bytes in flight against the L2 latency
-// and two thirds of the shared-memory reads per flop. M must be a multiple of 256. With a remote X the first
+// and two thirds of the shared-memory reads per flop. The rows of a last half block (bf16: M is a multiple of 128)
+// are zero-filled loads and are not stored; MX wants M in multiples of 256. With a remote X the first
 // copy_ctas CTAs (whole pairs) copy it before they join, and the even CTA of each pair draws the pair's
 // tiles from the global counter and hands them to its partner through distributed shared memory.
 // All loads are per-CTA loads that signal the even CTA's barrier; no load is broadcast.
@@ -864,20 +1044,6 @@ template <bool MX> struct PairCfg {
 };
 constexpr uint32_t SF_TMEM_COL = 2 * BN - 16;  // 4 columns of X scales, then 8 of Wt scales (MX has one accumulator: 256..511 are free)
 
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// the address of `addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void st_shared_remote_u32(uint32_t cluster_addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
@@ -957,8 +1123,8 @@ __device__ __forceinline__ void umma_mx_pair(uint32_t tmem_c, uint64_t adesc, ui
       : "memory");
 }
 
-template <bool MX>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+template <bool MX, bool SPLIT>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                         const __grid_constant__ CUtensorMap map_y, const __grid_constant__ CUtensorMap map_sfa,
                         const __grid_constant__ CUtensorMap map_sfb, GemmParams p) {
@@ -985,7 +1151,8 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   __shared__ int s_abort;
   __shared__ int s_tiles[TILE_RING];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_cta_rank();
+  const uint32_t rank = cluster_cta_rank() & 1u;  // within the pair
+  const uint32_t even = cluster_cta_rank() & ~1u;  // cluster rank of the pair's even CTA
   const bool leader = rank == 0;
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
@@ -1019,9 +1186,12 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
 
-  const int m_blocks = p.M / (2 * BM), n_blocks = p.N / BN;
+  const int m_blocks = (p.M + 2 * BM - 1) / (2 * BM), n_blocks = p.N / BN;
   const int total = m_blocks * n_blocks;
-  const int k_iters = p.K * p.elem_bytes / BKB;
+  const int k_all = p.K * p.elem_bytes / BKB;
+  const int share = SPLIT ? (int)(even >> 1) : 0;  // this pair's share of K
+  const int k_begin = SPLIT ? k_all * share / p.split : 0;
+  const int k_iters = (SPLIT ? k_all * (share + 1) / p.split : k_all) - k_begin;
   const int kelems = BKB / p.elem_bytes;
   volatile int* abort = &s_abort;
   // The even CTA draws the pair's next tile from the global counter and puts it into both CTAs'
@@ -1039,19 +1209,20 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       for (int it = 0;; ++it) {
         int tile;
         if (leader) {
-          tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+          if (SPLIT) tile = it == 0 ? (int)blockIdx.x / (2 * p.split) : total;  // one tile per cluster
+          else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
           const int slot = it & (TILE_RING - 1);
           s_tiles[slot] = tile;
           mbar_arrive(tile_bar(slot));
-          st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), 1), (uint32_t)tile);
-          mbar_arrive_remote(map_to_cta(tile_bar(slot), 1));
+          st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), even | 1u), (uint32_t)tile);
+          mbar_arrive_remote(map_to_cta(tile_bar(slot), even | 1u));
         } else {
           tile = next_tile(it);
         }
         if (tile >= total) break;
         int mb, nb;
         tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-        if (p.panel_target > 0) {  // this CTA's 128 rows of the 256-row block
+        if (p.panel_target > 0 && (2 * mb + (int)rank) * BM < p.M) {  // this CTA's 128 rows of the 256-row block
           if (!wait_u32_ge_gpu(p.panel_flags + 2 * mb + (int)rank, p.panel_target, p.timeout_ns)) {
             *abort = 1;
             break;
@@ -1060,14 +1231,14 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         }
         for (int k = 0; k < k_iters; ++k) {
           if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-          const uint32_t full_leader = map_to_cta(full_bar(s), 0);
+          const uint32_t full_leader = map_to_cta(full_bar(s), even);
           if (leader) mbar_expect_tx(full_bar(s), 2 * PairCfg<MX>::STAGE_BYTES);
-          tma_load_2d_pair(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_leader, k * kelems, mb * 2 * BM + (int)rank * BM);
-          tma_load_2d_pair(smem_u32(sB + (size_t)s * B2_STAGE_BYTES), &map_b, full_leader, k * kelems, nb * BN + (int)rank * (BN / 2));
+          tma_load_2d_pair(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_leader, (k_begin + k) * kelems, mb * 2 * BM + (int)rank * BM);
+          tma_load_2d_pair(smem_u32(sB + (size_t)s * B2_STAGE_BYTES), &map_b, full_leader, (k_begin + k) * kelems, nb * BN + (int)rank * (BN / 2));
           if (MX) {  // this CTA's X scales of the step, and the whole tile's Wt scales (each CTA needs all 256 in its TMEM)
             const uint32_t sf = smem_u32(sSF + (size_t)s * SF_STAGE_BYTES);
-            tma_load_2d_pair(sf, &map_sfa, full_leader, 0, (mb * 2 + (int)rank) * k_iters + k);
-            tma_load_2d_pair(sf + 512, &map_sfb, full_leader, 0, k * (p.N / 128) + nb * 2);
+            tma_load_2d_pair(sf, &map_sfa, full_leader, 0, (mb * 2 + (int)rank) * k_all + k_begin + k);
+            tma_load_2d_pair(sf + 512, &map_sfb, full_leader, 0, (k_begin + k) * (p.N / 128) + nb * 2);
           }
           if (++s == STAGES2) s = 0, ph ^= 1u;
         }
@@ -1116,11 +1287,11 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
           }
           // the stage is free in both CTAs once these MMAs have read it
           umma_commit_pair(empty_bar(s));
-          umma_commit_pair(map_to_cta(empty_bar(s), 1));
+          umma_commit_pair(map_to_cta(empty_bar(s), even | 1u));
           if (++s == STAGES2) s = 0, ph ^= 1u;
         }
         umma_commit_pair(tfull_bar(buf));
-        umma_commit_pair(map_to_cta(tfull_bar(buf), 1));
+        umma_commit_pair(map_to_cta(tfull_bar(buf), even | 1u));
       }
     }
   } else if (warp < 4) {
@@ -1142,6 +1313,8 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       const uint32_t tph = (uint32_t)(it / NBUF) & 1u;
       const bool got = !*abort && mbar_wait(tfull_bar(buf), tph, abort, p.timeout_ns);
       if (epi_vote_any(1, !got)) break;
+      if (SPLIT) break;  // summed over the cluster below
+      const bool inside = (2 * mb + (int)rank) * BM < p.M;  // the odd CTA of a last half block has no rows to store
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)buf * BN;
       if (MX) {
@@ -1162,7 +1335,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote_tmem(map_to_cta(tempty_bar(buf), 0));
+        if (lane == 0) mbar_arrive_remote_tmem(map_to_cta(tempty_bar(buf), even));
 #pragma unroll
         for (int sl = 0; sl < BN / 64; ++sl, ++slab) {
           const uint32_t sbuf = epi0 + (slab & 1u) * EPI_SLAB_BYTES;
@@ -1176,7 +1349,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           epi_bar_sync(1);
-          if (elected) {
+          if (elected && inside) {
             tma_store_2d(&map_y, sbuf, nb * BN + sl * 64, mb * 2 * BM + (int)rank * BM);
             bulk_commit();
           }
@@ -1207,11 +1380,11 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
         if (sl == BN / 64 - 1) {  // this CTA's half of the accumulator is out of TMEM
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_remote_tmem(map_to_cta(tempty_bar(buf), 0));
+          if (lane == 0) mbar_arrive_remote_tmem(map_to_cta(tempty_bar(buf), even));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         epi_bar_sync(1);
-        if (elected) {
+        if (elected && inside) {
           tma_store_2d(&map_y, sbuf, nb * BN + sl * 64, mb * 2 * BM + (int)rank * BM);
           bulk_commit();
         }
@@ -1225,6 +1398,13 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 
   tc_fence_before();
   __syncthreads();
+  if (SPLIT) {
+    tc_fence_after();
+    int mb, nb;
+    tile_coords((int)blockIdx.x / (2 * p.split), m_blocks, n_blocks, p.head_blocks, mb, nb);
+    split_sum(p, tmem_base, smem_u32(smem), 2 * mb + (int)rank, nb, share, (int)rank, 2);
+    tc_fence_before();
+  }
   cluster_sync_all();  // neither CTA leaves while the other may still touch its shared memory or TMEM
   if (warp == 1) {
     tc_fence_after();
@@ -1270,7 +1450,7 @@ __device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_c, uint64_t adesc, u
       : "memory");
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM8P_THREADS, 1)
+__global__ void __launch_bounds__(GEMM8P_THREADS, 1)
 remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                             const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
@@ -1577,6 +1757,62 @@ static int make_map_sf(CUtensorMap* m, const void* base, uint64_t chunks, uint32
   return r == CUDA_SUCCESS ? 0 : EUX_ERR_BAD_ARG;
 }
 
+// The kernel's shared memory limit, raised before its first launch on a device (threads that race do it twice).
+template <auto KERNEL>
+static cudaError_t allow_smem(int dev, size_t smem) {
+  static std::atomic<bool> done[64];
+  if (done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) done[dev].store(true, std::memory_order_release);
+  return e;
+}
+
+struct ClusterLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  ClusterLaunch(int cluster, int grid, int threads, size_t smem, cudaStream_t st) {
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 1 : 0;
+  }
+};
+
+template <auto KERNEL, typename... Args>
+static int launch_clusters(int dev, int cluster, int grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  if (cudaError_t e = allow_smem<KERNEL>(dev, smem); e != cudaSuccess) return (int)e;
+  ClusterLaunch l(cluster, grid, threads, smem, st);
+  return (int)cudaLaunchKernelEx(&l.cfg, KERNEL, args...);
+}
+
+// Shares of K per tile (1, 2, 4 or 8) for `tiles` clusters of `ctas` CTAs per share: from 24 K steps on, as many as
+// leave eight steps to each while all clusters fit the device at once (asked of the driver, once per device and size).
+template <auto KERNEL>
+static int choose_split(int dev, int threads, size_t smem, int tiles, int ctas, int k_iters) {
+  static std::atomic<int> resident[64][4];  // 1 + the number of clusters
+  int split = 1;
+  for (int i = 1; i < 4 && ctas << i <= 8; ++i) {
+    const int s = 1 << i;
+    if (k_iters < 24 || k_iters < 8 * s) break;
+    int n = resident[dev][i].load(std::memory_order_acquire) - 1;
+    if (n < 0) {
+      n = 0;
+      ClusterLaunch l(ctas * s, ctas * s, threads, smem, nullptr);
+      if (allow_smem<KERNEL>(dev, smem) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, KERNEL, &l.cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      resident[dev][i].store(n + 1, std::memory_order_release);
+    }
+    if (tiles <= n) split = s;
+  }
+  return split;
+}
+
 }  // namespace eux
 
 using namespace eux;
@@ -1624,6 +1860,7 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   // bits 8..15 of the flags: 1 + the height of the first tile group, 0 for the default
   const int head_arg = (int)((d->flags >> 8) & 0xffu) - 1;
   p.copy_warps = 0;
+  p.split = 1;
   p.done_always = (d->flags & EUX_GEMM_FLAG_DONE_ALWAYS) ? 1 : 0;
   p.panel_target = (uint32_t)copy_ctas;
   // copy warps: units of 8 KiB per 128-row panel, plus the units that carry the panel's scales (K * 4 bytes)
@@ -1631,37 +1868,67 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
     return (uint32_t)(((size_t)BM * d->K * eb) >> 13) + (d->fp8 ? (uint32_t)(((size_t)d->K * 4 + 8191) >> 13) : 0u);
   };
   p.head_blocks = !pull ? 0 : head_arg >= 0 ? head_arg : 4;  // of 128 rows: groups of 4, 4, 8, then 8
-  static bool attr_set[64][2] = {{false}};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return EUX_ERR_BAD_ARG;
-  if (!attr_set[dev][d->fp8 ? 1 : 0]) {
-    cudaError_t e = d->fp8 ? cudaFuncSetAttribute(remote_gemm_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM8_SMEM)
-                           : cudaFuncSetAttribute(remote_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set[dev][d->fp8 ? 1 : 0] = true;
-  }
-  // bf16 with M in whole 256-row blocks can run on CTA pairs (bit 0 of the descriptor's flags)
-  const bool want_pairs = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) != 0;
-  if (mx || (want_pairs && !d->fp8 && d->M % (2 * BM) == 0)) {
-    static bool attr2_set[64][2] = {{false}};
-    if (!attr2_set[dev][mx ? 1 : 0]) {
-      cudaError_t e = mx ? cudaFuncSetAttribute(remote_gemm_2cta_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)PairCfg<true>::SMEM)
-                         : cudaFuncSetAttribute(remote_gemm_2cta_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)PairCfg<false>::SMEM);
-      if (e != cudaSuccess) return (int)e;
-      attr2_set[dev][mx ? 1 : 0] = true;
+  const cudaStream_t st = (cudaStream_t)stream;
+  const bool copy_by_warps = pull && (d->flags & EUX_GEMM_FLAG_COPY_WARPS);
+  const int k_iters = d->K * eb / BKB;
+  const int m_pairs = (d->M + 2 * BM - 1) / (2 * BM), n_pairs = (d->N + BN - 1) / BN;
+  const int tiles = (d->M / BM) * (d->N / bn), tiles2 = m_pairs * n_pairs;
+  const int waves = (tiles + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
+  // Few tiles: the K of a tile is shared out over a cluster of CTAs (or CTA pairs), which add their sums up through
+  // distributed shared memory. A K step costs a CTA about half a microsecond, the sum about three: 128 x 8192 x 8192
+  // (32 tiles) takes 49 us with four CTAs per tile and 72 with one, 128 x 512 x 8192 27 with eight and 59 with one;
+  // 384 x 4096 x 1024, sixteen steps, loses 2 us. All clusters have to fit at once: a second wave costs more.
+  if (!pull || copy_by_warps) {
+    if (mx) {
+      const int s = choose_split<remote_gemm_2cta_kernel<true, true>>(dev, GEMM_THREADS, PairCfg<true>::SMEM, tiles2, 2, k_iters);
+      if (s > 1) {
+        CUtensorMap mb2, msa, msb;
+        if (int rc = make_map(&mb2, d->w_t, eb, (uint64_t)d->N, (uint64_t)d->K, BN / 2)) return rc;
+        if (int rc = make_map_sf(&msa, p.x_scale_stage, (uint64_t)(d->M / 128) * (d->K / 128), 1)) return rc;
+        if (int rc = make_map_sf(&msb, d->w_scale, (uint64_t)(d->N / 128) * (d->K / 128), 2)) return rc;
+        p.split = s, p.copy_ctas = 0;
+        p.copy_warps = pull ? 2 * 2 * tiles2 * s : 0;
+        p.panel_target = pull ? warp_target(p.copy_warps) : 0;
+        if (pull && head_arg < 0) p.head_blocks = 2;
+        return launch_clusters<remote_gemm_2cta_kernel<true, true>>(dev, 2 * s, 2 * tiles2 * s, GEMM_THREADS, PairCfg<true>::SMEM, st, ma, mb2,
+                               my, msa, msb, p);
+      }
+    } else {
+      const int s = d->fp8 ? choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters)
+                           : choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, tiles, 1, k_iters);
+      if (s > 1) {
+        p.split = s, p.copy_ctas = 0;
+        p.copy_warps = pull ? 2 * tiles * s : 0;
+        p.panel_target = pull ? warp_target(p.copy_warps) : 0;
+        if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, tiles * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
+        return launch_clusters<remote_gemm_kernel<true>>(dev, s, tiles * s, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
+      }
     }
+  }
+  // bf16 on CTA pairs (bit 0 of the descriptor's flags): a K step of a 256 x 256 tile takes 0.41 us, one of a single
+  // CTA's 128 x 256 tile 0.47, so pairs are taken unless half a tile of padding (M an odd number of 128-row blocks)
+  // costs them a wave or K is short (640 x 8192 x 8192: 98 us against 113, 640 x 4096 x 1024: 25 against 23). CTAs
+  // that copy X before they compute keep to whole tiles.
+  const bool pairs_bf16 = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) && !d->fp8 &&
+                          (d->M % (2 * BM) == 0 || ((!pull || copy_by_warps) && waves2 <= waves && k_iters >= 24));
+  // Block-scaled fp8 on CTA pairs: a K-block takes 0.76 us of a pair's 256 x 256 tile and 0.53 us of a CTA's 128 x 128
+  // tile (1920 x 4608 x 7168: 89 us against 113; 512 x 4096 x 7168, one wave of either: 54 against 42), so the pairs are
+  // taken when they need at most 7 / 10 of the waves and K is not short. Pulled scales are read through L1, which is sound while no line
+  // holds rows of two panels: their staging buffer starts on a line.
+  const bool pairs_fp8 = d->fp8 && !mx && (!pull || (copy_by_warps && ((uintptr_t)d->x_scale_stage & 127u) == 0)) &&
+                         waves2 * 10 <= waves * 7 && k_iters >= 16;
+  if (mx || pairs_bf16 || pairs_fp8) {
     CUtensorMap mb2;  // this CTA's half of a Wt tile: 128 rows
     if (int rc = make_map(&mb2, d->w_t, eb, (uint64_t)d->N, (uint64_t)d->K, BN / 2)) return rc;
-    const int tiles2 = (d->M / (2 * BM)) * (d->N / BN);
     int copy_pairs = pull ? (copy_ctas + 1) / 2 : 0;
     if (copy_pairs > sms / 2 - 1) copy_pairs = sms / 2 - 1;
     p.copy_ctas = 2 * copy_pairs;
     p.panel_target = (uint32_t)p.copy_ctas;
     if (pull && head_arg < 0) p.head_blocks = 2;  // of 256 rows: groups of 2, 2, 4, then 8
-    if (pull && (d->flags & EUX_GEMM_FLAG_COPY_WARPS)) {  // two warps of every CTA copy, no CTA only copies
+    if (copy_by_warps) {  // two warps of every CTA copy, no CTA only copies
       p.copy_ctas = 0;
       p.copy_warps = 2 * 2 * (sms / 2);
       p.panel_target = warp_target(p.copy_warps);
@@ -1669,52 +1936,23 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
     // every pair computes (the copying ones after their transfer), and they all have to be resident:
     // pairs that copy must not wait for a slot behind pairs that wait for their panels
     const int pairs = pull ? sms / 2 : (tiles2 < sms / 2 ? tiles2 : sms / 2);
-    if (mx) {
-      CUtensorMap msa, msb;
-      if (int rc = make_map_sf(&msa, p.x_scale_stage, (uint64_t)(d->M / 128) * (d->K / 128), 1)) return rc;
-      if (int rc = make_map_sf(&msb, d->w_scale, (uint64_t)(d->N / 128) * (d->K / 128), 2)) return rc;
-      remote_gemm_2cta_kernel<true><<<2 * pairs, GEMM_THREADS, PairCfg<true>::SMEM, (cudaStream_t)stream>>>(ma, mb2, my, msa, msb, p);
-    } else {
-      remote_gemm_2cta_kernel<false><<<2 * pairs, GEMM_THREADS, PairCfg<false>::SMEM, (cudaStream_t)stream>>>(ma, mb2, my, ma, ma, p);
-    }
-    return (int)cudaGetLastError();
+    if (pairs_fp8) return launch_clusters<remote_gemm_fp8_2cta_kernel>(dev, 2, 2 * pairs, GEMM8P_THREADS, GEMM8P_SMEM, st, ma, mb2, my, p);
+    if (!mx)
+      return launch_clusters<remote_gemm_2cta_kernel<false, false>>(dev, 2, 2 * pairs, GEMM_THREADS, PairCfg<false>::SMEM, st, ma, mb2, my, ma, ma, p);
+    CUtensorMap msa, msb;
+    if (int rc = make_map_sf(&msa, p.x_scale_stage, (uint64_t)(d->M / 128) * (d->K / 128), 1)) return rc;
+    if (int rc = make_map_sf(&msb, d->w_scale, (uint64_t)(d->N / 128) * (d->K / 128), 2)) return rc;
+    return launch_clusters<remote_gemm_2cta_kernel<true, false>>(dev, 2, 2 * pairs, GEMM_THREADS, PairCfg<true>::SMEM, st, ma, mb2, my, msa, msb, p);
   }
-  const bool copy_by_warps = pull && (d->flags & EUX_GEMM_FLAG_COPY_WARPS);
-  // Block-scaled fp8 on CTA pairs or on single CTAs: a K-block takes 0.76 us of a pair's 256 x 256 tile and 0.53 us of
-  // a CTA's 128 x 128 tile (1920 x 4608 x 7168: 89 us against 113; 512 x 4096 x 7168, one wave of either: 54 against
-  // 42), so the pairs are taken when they need at most 7 / 10 of the waves. Pulled scales are read through L1, which
-  // is sound while no line holds rows of two panels: their staging buffer starts on a line.
-  const int tiles1 = (d->M / BM) * (d->N / BN8), tiles2 = ((d->M + 2 * BM - 1) / (2 * BM)) * ((d->N + BN - 1) / BN);
-  const int waves1 = (tiles1 + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
-  if (d->fp8 && (!pull || (copy_by_warps && ((uintptr_t)d->x_scale_stage & 127u) == 0)) && waves2 * 10 <= waves1 * 7) {
-    static bool attr8_set[64] = {false};
-    if (!attr8_set[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(remote_gemm_fp8_2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM8P_SMEM);
-      if (e != cudaSuccess) return (int)e;
-      attr8_set[dev] = true;
-    }
-    if (pull) {
-      if (head_arg < 0) p.head_blocks = 2;
-      p.copy_ctas = 0;
-      p.copy_warps = 2 * 2 * (sms / 2);
-      p.panel_target = warp_target(p.copy_warps);
-    }
-    const int pairs = pull ? sms / 2 : (tiles2 < sms / 2 ? tiles2 : sms / 2);
-    // Wt in boxes of 128 rows (`mb`): each CTA of a pair loads its half of a tile's 256
-    remote_gemm_fp8_2cta_kernel<<<2 * pairs, GEMM8P_THREADS, GEMM8P_SMEM, (cudaStream_t)stream>>>(ma, mb, my, p);
-    return (int)cudaGetLastError();
-  }
-  const int tiles = (d->M / BM) * (d->N / bn);
   int grid = copy_ctas + (tiles < sms - copy_ctas ? tiles : sms - copy_ctas);
-  if (pull && (d->flags & EUX_GEMM_FLAG_COPY_WARPS)) {  // every SM takes part in the copy, with or without a tile
+  if (copy_by_warps) {  // every SM takes part in the copy, with or without a tile
     grid = sms;
     p.copy_ctas = 0;
     p.copy_warps = 2 * grid;
     p.panel_target = warp_target(p.copy_warps);
   }
-  if (d->fp8) remote_gemm_fp8_kernel<<<grid, GEMM8_THREADS, GEMM8_SMEM, (cudaStream_t)stream>>>(ma, mb, my, p);
-  else remote_gemm_kernel<false><<<grid, GEMM_THREADS, GEMM_SMEM, (cudaStream_t)stream>>>(ma, mb, my, p);
-  return (int)cudaGetLastError();
+  if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<false>>(dev, 1, grid, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
+  return launch_clusters<remote_gemm_kernel<false>>(dev, 1, grid, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -1723,8 +1961,6 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
 // name `g_noalloc_gemm_scratch` is only a stand-in: the address a kernel can use is
 // obtained per device with cudaGetSymbolAddress below.
 // ---------------------------------------------------------------------------
-#include <atomic>
-
 #include "eux_no_alloc.h"
 
 static __device__ __align__(256) uint32_t g_noalloc_gemm_scratch[EUX_NOALLOC_GEMM_SCRATCH_BYTES / 4];
@@ -1777,8 +2013,10 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
 // that loads): a service that launches on behalf of a peer calls this when it is set up.
 extern "C" int eux_gemm_preload(void) {
   cudaFuncAttributes attr;
-  const void* kernels[] = {(const void*)remote_gemm_kernel<false>, (const void*)remote_gemm_fp8_kernel, (const void*)remote_gemm_2cta_kernel<false>,
-                           (const void*)remote_gemm_2cta_kernel<true>, (const void*)remote_gemm_fp8_2cta_kernel};
+  const void* kernels[] = {(const void*)remote_gemm_kernel<false>,           (const void*)remote_gemm_kernel<true>,
+                           (const void*)remote_gemm_fp8_kernel<false>,       (const void*)remote_gemm_fp8_kernel<true>,
+                           (const void*)remote_gemm_2cta_kernel<false, false>, (const void*)remote_gemm_2cta_kernel<true, false>,
+                           (const void*)remote_gemm_2cta_kernel<true, true>, (const void*)remote_gemm_fp8_2cta_kernel};
   for (const void* k : kernels) {
     cudaError_t e = cudaFuncGetAttributes(&attr, k);
     if (e != cudaSuccess) return (int)e;

@@ -40,8 +40,9 @@ class RemoteGemm:
                  copy_warps: Optional[bool] = None) -> None:
         """Y[m,N] (at ``y_ptr``) = X[m,K] (at ``x_ptr``) @ W. Both addresses may be peer memory.
         ``cta_pairs`` selects the kernel that computes 256 x 256 tiles on pairs of CTAs
-        (tcgen05 cta_group::2) whenever ``m`` is a multiple of 256; other shapes, and
-        ``cta_pairs=False``, run the kernel with one CTA per 128 x 256 tile. ``head_blocks``
+        (tcgen05 cta_group::2); shapes that half a tile of padding would cost a wave, and
+        ``cta_pairs=False``, run the kernel with one CTA per 128 x 256 tile. With few tiles a cluster
+        of CTAs shares the K of each (its sums are added up in a fixed order). ``head_blocks``
         overrides the height (in row blocks) of the first group of tiles when X is remote.
         A remote X is copied into the staging buffer by two spare warps of every CTA while the
         other warps compute (``copy_warps``, the default), or, when ``copy_ctas`` > 0 is given, by

@@ -59,7 +59,48 @@ def test_block_scaled_fp8_matches_fp32(cuda_device, m, n, k, pull):
         assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
 
 
-@pytest.mark.parametrize("m,n,k", [(1920, 2688, 128), (1664, 3200, 1152), (3968, 1280, 384)])
+@pytest.mark.parametrize("fmt,m,n,k", [("bf16", 128, 256, 1536), ("bf16", 128, 512, 8192), ("bf16", 384, 2048, 4096 + 64),
+                                       ("bf16", 256, 4096, 1536 + 192), ("bf16", 640, 768, 2048), ("bf16", 1152, 4352, 1600),
+                                       ("fp8_block", 128, 128, 8192), ("fp8_block", 256, 640, 3200), ("fp8_block", 128, 7936, 3328),
+                                       ("mxfp8", 256, 256, 8192), ("mxfp8", 512, 768, 3200), ("mxfp8", 256, 4352, 3200)])
+@pytest.mark.parametrize("pull", [False, True])
+def test_few_tiles(cuda_device, fmt, m, n, k, pull):
+    """Shapes at which a cluster shares the K of a tile (two, four and eight shares, shares of unequal length, and one
+    cluster too many), and odd numbers of 128-row blocks on pairs. fp32 sums in another order (1e-5 of a row's largest
+    result) and one rounding to bf16 (2^-8 of the value)."""
+    from execution_ucx_b200.ops import remote_gemm as rg
+    torch.manual_seed(m + n + k)
+    x = torch.randn(m, k, device=cuda_device)
+    w = torch.randn(k, n, device=cuda_device) * 0.02
+    if fmt == "bf16":
+        g = rg.RemoteGemm(w.to(torch.bfloat16), m)
+        args = [x.to(torch.bfloat16)]
+        ref = args[0].double() @ w.to(torch.bfloat16).double()
+    elif fmt == "fp8_block":
+        g = rg.RemoteGemmFp8(w, m)
+        args = list(rg.quantize_rows_1x128(x))
+        ref = rg.dequantized_reference(args[0], args[1].double(), g.w_q_t, g.w_scale.double())
+    else:
+        g = rg.RemoteGemmMx(w, m)
+        xq, sf = rg.quantize_mx(x)
+        args = [xq, rg.mx_scale_chunks(sf, False)]
+        ref = rg.mx_dequantized_reference(xq.double(), sf.double(), g.w_q_t.double(), g.w_sf.double()).double()
+    buf = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    first = None
+    for _ in range(3):
+        buf[:m].zero_()
+        g(*[a.data_ptr() for a in args], m, buf.data_ptr(), x_is_local=not pull)
+        torch.cuda.synchronize()
+        g.check_status()
+        y = buf[:m].double()
+        assert bool(((y - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
+        assert bool((buf[m] == 7).all())
+        assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+        assert first is None or torch.equal(buf, first)   # the order of the sums is fixed
+        first = buf.clone()
+
+
+@pytest.mark.parametrize("m,n,k", [(1920, 2688, 2048), (1664, 3200, 2176), (3968, 1280, 2432)])
 @pytest.mark.parametrize("pull", [False, "warps"])
 def test_block_scaled_fp8_pairs(cuda_device, m, n, k, pull):
     """More than one wave of 128 x 128 tiles: the kernel on CTA pairs, with half tiles at the end of M and of N, K-blocks
