@@ -350,14 +350,32 @@ struct Convert<S, D, false> {
   static __device__ __forceinline__ D one(S v, int op, float arg) { return Elem<D>::from(apply_op(Elem<S>::to(v), op, arg)); }
 };
 
+// Division of any 32-bit number by one that the host knows: a multiplication and shifts (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", 1994, figure 4.1).
+struct FastDiv {
+  uint32_t m, s1, s2;
+  __device__ __forceinline__ uint32_t operator()(uint32_t a) const {
+    const uint32_t t = __umulhi(a, m);
+    return (t + ((a - t) >> s1)) >> s2;
+  }
+};
+struct GatherArgs {
+  XferArgs x;
+  FastDiv div[EUX_MAX_DIMS];  // by the sizes
+  int small;                  // every size, and the number of elements, fits 32 bits: `div` can be used
+};
+
 // Offset in the source, in elements, of the row (every dimension but the innermost) and the column of element e.
-__device__ __forceinline__ int64_t gather_row(const eux_xfer_desc& d, uint64_t e, uint64_t& col) {
+// (With plain 32-bit divisions a head-major view, four dimensions, was bound by them: 158 us for 16 x 32 x 2048 x 128.)
+__device__ __forceinline__ int64_t gather_row(const GatherArgs& a, uint64_t e, uint64_t& col) {
+  const eux_xfer_desc& d = a.x.d;
   const int last = d.ndim - 1;
-  uint64_t rem = div_u64(e, (uint64_t)d.shape[last]);
+  auto divide = [&](uint64_t v, int k) -> uint64_t { return a.small ? a.div[k]((uint32_t)v) : v / (uint64_t)d.shape[k]; };
+  uint64_t rem = divide(e, last);
   col = e - rem * (uint64_t)d.shape[last];
   int64_t off = 0;
   for (int k = last - 1; k >= 0; --k) {
-    const uint64_t q = div_u64(rem, (uint64_t)d.shape[k]);
+    const uint64_t q = divide(rem, k);
     off += (int64_t)(rem - q * (uint64_t)d.shape[k]) * d.stride[k];
     rem = q;
   }
@@ -365,17 +383,21 @@ __device__ __forceinline__ int64_t gather_row(const eux_xfer_desc& d, uint64_t e
 }
 
 // A thread makes 16 (8 for a narrowing cast to one byte, 32 for one to fp32) aligned bytes of the destination per
-// step: one index computation for them, one or two aligned loads when they lie in one row of the source, single
-// elements when they straddle rows or the innermost stride is not 1. Bound by DRAM.
-template <typename S, typename D, bool RAW>
-__global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_constant__ XferArgs a) {
-  const eux_xfer_desc& d = a.d;
+// chunk, and U chunks per step, whose loads are all in flight together. ALIGNED: every row of the source starts on the
+// load's boundary and is a whole number of chunks long, so a chunk is one aligned load (two for fp32 sources).
+// Otherwise a chunk takes one or two aligned loads when it lies in one row, and single elements when it straddles rows
+// or the innermost stride is not 1. Bound by DRAM and, with rows of a few hundred bytes, by the index computation.
+template <typename S, typename D, bool RAW, bool ALIGNED>
+__global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_constant__ GatherArgs a) {
+  const eux_xfer_desc& d = a.x.d;
   bool ok = cta_wait_arrival(d);
   if (ok) {
     constexpr int V = RAW ? 16 / (int)sizeof(D) : 8;
+    constexpr int U = ALIGNED ? (V * (int)sizeof(S) > 16 ? 2 : 4) : 1;  // two unaligned chunks spill: 59 -> 70 us on 8192 rows of 5461 bf16
     constexpr int DB = V * (int)sizeof(D);
     constexpr int SB = V * (int)sizeof(S);
     constexpr int VEC = DB >= 16 ? 16 : 8;
+    constexpr int SVEC = SB >= 16 ? 16 : 8;
     const S* src = reinterpret_cast<const S*>(d.src);
     D* dst = reinterpret_cast<D*>(d.dst);
     const uint64_t n = d.n_elems;
@@ -385,41 +407,61 @@ __global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_
     const int64_t inner = d.stride[d.ndim - 1];
     const int op = d.op;
     const float arg = d.op_arg;
-    uint64_t lead = ((VEC - ((uintptr_t)dst & (VEC - 1))) & (VEC - 1)) / sizeof(D);  // elements in front of the first aligned vector
+    uint64_t lead = ALIGNED ? 0 : ((VEC - ((uintptr_t)dst & (VEC - 1))) & (VEC - 1)) / sizeof(D);  // elements in front of the first aligned vector
     if (lead > n) lead = n;
     const uint64_t chunks = (n - lead) / V;
-    for (uint64_t i = tid; i < chunks; i += nthreads) {
-      const uint64_t e = lead + i * V;
-      uint64_t c;
-      int64_t row = gather_row(d, e, c);
-      alignas(16) D out[V];
-      if (inner == 1 && c + V <= cols) {
-        alignas(16) uint32_t w[SB / 4];
-        load_span<SB>(reinterpret_cast<const unsigned char*>(src + row + (int64_t)c), w);
-        const S* sv = reinterpret_cast<const S*>(w);
+    for (uint64_t i0 = tid; i0 < chunks; i0 += U * nthreads) {
+      alignas(16) uint32_t w[U][SB / 4];
+      uint64_t c[U];
+      int64_t row[U];
 #pragma unroll
-        for (int k = 0; k < V; ++k) out[k] = Convert<S, D, RAW>::one(sv[k], op, arg);
-      } else {
+      for (int u = 0; u < U; ++u) {
+        const uint64_t i = i0 + u * nthreads;
+        if (i >= chunks) break;
+        row[u] = gather_row(a, lead + i * V, c[u]);
+        const S* s = src + row[u] + (int64_t)c[u];
+        if (ALIGNED) {
 #pragma unroll
-        for (int k = 0; k < V; ++k) {
-          if (c >= cols) row = gather_row(d, e + k, c);
-          out[k] = Convert<S, D, RAW>::one(src[row + (int64_t)c * inner], op, arg);
-          ++c;
+          for (int k = 0; k < SB / SVEC; ++k)
+            reinterpret_cast<typename PackT<SVEC>::type*>(w[u])[k] = reinterpret_cast<const typename PackT<SVEC>::type*>(s)[k];
+        } else if (inner == 1 && c[u] + V <= cols) {
+          load_span<SB>(reinterpret_cast<const unsigned char*>(s), w[u]);
         }
       }
 #pragma unroll
-      for (int k = 0; k < DB / VEC; ++k)
-        reinterpret_cast<typename PackT<VEC>::type*>(dst + e)[k] = reinterpret_cast<typename PackT<VEC>::type*>(out)[k];
+      for (int u = 0; u < U; ++u) {
+        const uint64_t i = i0 + u * nthreads;
+        if (i >= chunks) break;
+        const uint64_t e = lead + i * V;
+        alignas(16) D out[V];
+        if (ALIGNED || (inner == 1 && c[u] + V <= cols)) {
+          const S* sv = reinterpret_cast<const S*>(w[u]);
+#pragma unroll
+          for (int k = 0; k < V; ++k) out[k] = Convert<S, D, RAW>::one(sv[k], op, arg);
+        } else {
+          uint64_t col = c[u];
+          int64_t r = row[u];
+#pragma unroll
+          for (int k = 0; k < V; ++k) {
+            if (col >= cols) r = gather_row(a, e + k, col);
+            out[k] = Convert<S, D, RAW>::one(src[r + (int64_t)col * inner], op, arg);
+            ++col;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < DB / VEC; ++k)
+          reinterpret_cast<typename PackT<VEC>::type*>(dst + e)[k] = reinterpret_cast<typename PackT<VEC>::type*>(out)[k];
+      }
     }
     const uint64_t tail = lead + chunks * V;  // single elements in front of the vectors and behind them
     for (uint64_t i = tid; i < lead + (n - tail); i += nthreads) {
       const uint64_t e = i < lead ? i : tail + (i - lead);
       uint64_t c;
-      const int64_t row = gather_row(d, e, c);
+      const int64_t row = gather_row(a, e, c);
       dst[e] = Convert<S, D, RAW>::one(src[row + (int64_t)c * inner], op, arg);
     }
   }
-  cta_publish(d, a.counter, ok);
+  cta_publish(d, a.x.counter, ok);
 }
 
 // Transposes. A tile is `tp` steps of the dimension with stride 1 in the source (P) times `tq` of the innermost
@@ -428,8 +470,17 @@ __global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_
 // that 1- and 2-byte elements are transposed within registers and shared memory only ever moves whole words. The
 // row pitch is odd, so reads and writes meet at most two-way bank conflicts. Rows of Q leave as 16-byte stores, or
 // element by element where the destination's rows are not 16-byte aligned.
+// The usual tile, TP steps by QW words, has its sizes and trip counts at compile time and all its loads in flight at
+// once; with sizes read at run time throughout, the index arithmetic alone kept the issue slots two thirds busy
+// (8192 x 8192 bf16: 73 us). Tiles at the edges and of other shapes take the general loops.
 constexpr int kTileThreads = 256;
-constexpr int kTileWords = 64 * 33;  // 64 steps of P, 32 words (128 bytes) of Q, one word of padding
+template <typename S>
+constexpr int tile_p() { return sizeof(S) == 1 ? 128 : 64; }  // every thread has a 16-byte load
+// Words of Q: 256 bytes of a destination row where loads are 16 bytes wide (8192 x 8192 bf16: 68 us with 128 bytes, 55
+// with 256), 128 otherwise (8191 x 8193 bytes: 68 us with 128, 94 with 256).
+constexpr int tile_q(bool vector) { return vector ? 64 : 32; }
+constexpr int kNarrowBytes = 24576;
+constexpr int kTileWords = 64 * 33;  // of a tile of any other shape
 struct TileArgs {
   XferArgs x;
   int64_t batch_src[EUX_MAX_DIMS], batch_dst[EUX_MAX_DIMS];  // strides of the other dimensions, in elements
@@ -437,21 +488,34 @@ struct TileArgs {
   int64_t q_src, p_dst;  // strides, in elements
   uint32_t n_batch, np, nq, tp, tq, tiles_p, tiles_q;
   uint32_t pitch;  // words
-  uint32_t vector_store;
+  uint32_t vector_store, narrow;
   uint64_t tiles;
 };
 
+template <typename S, typename D, bool RAW>
+__device__ __forceinline__ uint32_t tile_word(const S* v, int op, float arg) {
+  constexpr int G = 4 / (int)sizeof(D);
+  alignas(4) D o[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) o[g] = Convert<S, D, RAW>::one(v[g], op, arg);
+  uint32_t word;
+  memcpy(&word, o, 4);
+  return word;
+}
+
 template <typename S, typename D, bool RAW, bool VECTOR>
 __global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_constant__ TileArgs t) {
-  __shared__ uint32_t sm[kTileWords];
+  constexpr int G = 4 / (int)sizeof(D);
+  constexpr int VP = VECTOR ? 16 / (int)sizeof(S) : 1;
+  constexpr int TP = tile_p<S>();
+  constexpr int QW = tile_q(VECTOR);  // words of Q in a full tile
+  constexpr uint32_t PITCH = QW + 1;
+  __shared__ uint32_t sm[TP * PITCH > kTileWords ? TP * PITCH : kTileWords];
   const eux_xfer_desc& d = t.x.d;
   const bool ok = cta_wait_arrival(d);
   if (ok) {
-    constexpr int G = 4 / (int)sizeof(D);
-    constexpr int VP = VECTOR ? 16 / (int)sizeof(S) : 1;
     const int op = d.op;
     const float arg = d.op_arg;
-    const uint32_t pitch = t.pitch;
     for (uint64_t tile = blockIdx.x; tile < t.tiles; tile += gridDim.x) {
       // neighbouring tiles along P first: they share the source's lines where rows are not aligned to lines
       uint64_t r = div_u64(tile, t.tiles_p);
@@ -470,48 +534,95 @@ __global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_co
       const S* src = reinterpret_cast<const S*>(d.src) + so;
       D* dst = reinterpret_cast<D*>(d.dst) + dof;
       const uint32_t pn = min(t.tp, t.np - p0), qn = min(t.tq, t.nq - q0);
+      const int64_t q_src = t.q_src;
 
-      // read: a unit is VP steps of P by G of Q; the unit index is kept split so that no step divides
-      const uint32_t pu = (pn + VP - 1) / VP, qw = (qn + G - 1) / G;
-      {
+      // ---- read ----
+      if (pn == TP && qn == QW * G) {
+        constexpr int PU = TP / VP;                    // units along P
+        constexpr int QSTEP = kTileThreads / PU;       // words of Q that one pass of the threads covers
+        constexpr int N = QW / QSTEP;                  // passes
+        constexpr int B = G * VP * (int)sizeof(S) * N <= 64 ? N : (N > 1 && G * VP * (int)sizeof(S) * N / 2 <= 64 ? N / 2 : 1);  // in flight
+        const uint32_t p = (threadIdx.x % PU) * VP, w0 = threadIdx.x / PU;
+        const S* s = src + (int64_t)(w0 * G) * q_src + p;
+#pragma unroll
+        for (int n0 = 0; n0 < N; n0 += B) {
+          alignas(16) S v[B][G][VP];
+#pragma unroll
+          for (int n = 0; n < B; ++n)
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+              const S* e = s + (int64_t)((n0 + n) * QSTEP * G + g) * q_src;
+              if (VECTOR) *reinterpret_cast<uint4*>(v[n][g]) = *reinterpret_cast<const uint4*>(e);
+              else v[n][g][0] = *e;
+            }
+#pragma unroll
+          for (int n = 0; n < B; ++n)
+#pragma unroll
+            for (int i = 0; i < VP; ++i) {
+              S col[G];
+#pragma unroll
+              for (int g = 0; g < G; ++g) col[g] = v[n][g][i];
+              sm[(p + i) * PITCH + w0 + (n0 + n) * QSTEP] = tile_word<S, D, RAW>(col, op, arg);
+            }
+        }
+      } else {
+        // a unit is VP steps of P by G of Q, B of them in flight; unit indexes are kept split so that no step divides
+        constexpr int B = VECTOR ? 1 : 4;
+        const uint32_t pu = (pn + VP - 1) / VP, qw = (qn + G - 1) / G, pitch = t.pitch;
         const uint32_t dq = kTileThreads / pu, dp = kTileThreads - dq * pu;
         uint32_t iq = threadIdx.x / pu, ip = threadIdx.x - iq * pu;
-#pragma unroll 4
         while (iq < qw) {
-          const uint32_t p = ip * VP;
-          alignas(16) S v[G][VP];
+          alignas(16) S v[B][G][VP];
+          uint32_t at[B], steps[B];
 #pragma unroll
-          for (int g = 0; g < G; ++g) {
-            const uint32_t q = iq * G + g;
-            const S* s = src + (int64_t)q * t.q_src + p;
-            if (VECTOR && q < qn && p + VP <= pn) {
-              *reinterpret_cast<uint4*>(v[g]) = *reinterpret_cast<const uint4*>(s);
-            } else {
+          for (int n = 0; n < B; ++n) {
+            const uint32_t p = ip * VP;
+            steps[n] = iq >= qw ? 0 : min((uint32_t)VP, pn - p);
+            at[n] = p * pitch + iq;
+            const S* s = src + (int64_t)(iq * G) * q_src + p;
 #pragma unroll
-              for (int i = 0; i < VP; ++i) {
-                if (q < qn && p + i < pn) v[g][i] = s[i];
-                else memset(&v[g][i], 0, sizeof(S));
+            for (int g = 0; g < G; ++g) {
+              if (VECTOR && iq * G + g < qn && steps[n] == VP) {
+                *reinterpret_cast<uint4*>(v[n][g]) = *reinterpret_cast<const uint4*>(s + g * q_src);
+              } else {
+#pragma unroll
+                for (int i = 0; i < VP; ++i) {
+                  if (iq * G + g < qn && i < (int)steps[n]) v[n][g][i] = s[g * q_src + i];
+                  else memset(&v[n][g][i], 0, sizeof(S));
+                }
               }
             }
+            ip += dp;
+            iq += dq;
+            if (ip >= pu) ip -= pu, ++iq;
           }
 #pragma unroll
-          for (int i = 0; i < VP; ++i) {
-            uint32_t word;
-            alignas(4) D o[G];
+          for (int n = 0; n < B; ++n)
 #pragma unroll
-            for (int g = 0; g < G; ++g) o[g] = Convert<S, D, RAW>::one(v[g][i], op, arg);
-            memcpy(&word, o, 4);
-            if (p + i < pn) sm[(p + i) * pitch + iq] = word;
-          }
-          ip += dp;
-          iq += dq;
-          if (ip >= pu) ip -= pu, ++iq;
+            for (int i = 0; i < VP; ++i) {
+              S col[G];
+#pragma unroll
+              for (int g = 0; g < G; ++g) col[g] = v[n][g][i];
+              if (i < (int)steps[n]) sm[at[n] + i * pitch] = tile_word<S, D, RAW>(col, op, arg);
+            }
         }
       }
       __syncthreads();
 
-      // write
-      if (t.vector_store) {
+      // ---- write ----
+      const uint32_t pitch = t.pitch;
+      if (t.vector_store && pn == TP && qn == QW * G) {
+        constexpr int VR = QW / 4;  // vectors per row
+        constexpr int RSTEP = kTileThreads / VR;
+        const uint32_t v = threadIdx.x % VR, row0 = threadIdx.x / VR;
+        const uint32_t* w = sm + row0 * PITCH + v * 4;
+        D* out = dst + (int64_t)row0 * t.p_dst + v * (16 / sizeof(D));
+#pragma unroll
+        for (int n = 0; n < TP / RSTEP; ++n) {
+          const uint32_t* wn = w + n * RSTEP * PITCH;
+          *reinterpret_cast<uint4*>(out + (int64_t)(n * RSTEP) * t.p_dst) = make_uint4(wn[0], wn[1], wn[2], wn[3]);
+        }
+      } else if (t.vector_store) {
         constexpr uint32_t E = 16 / sizeof(D);
         const uint32_t vr = (qn + E - 1) / E;
         const uint32_t dr = kTileThreads / vr, dv = kTileThreads - dr * vr;
@@ -531,6 +642,17 @@ __global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_co
           v += dv;
           if (v >= vr) v -= vr, ++row;
         }
+      } else if (pn == TP && qn == QW * G) {
+        constexpr int RSTEP = kTileThreads / (QW * G);  // rows that one pass of the threads covers
+        const uint32_t q = threadIdx.x % (QW * G), row0 = threadIdx.x / (QW * G);
+        const uint32_t* w = sm + row0 * PITCH + q / G;
+        const uint32_t shift = 8 * sizeof(D) * (q % G);
+        D* out = dst + (int64_t)row0 * t.p_dst + q;
+#pragma unroll 8
+        for (int n = 0; n < TP / RSTEP; ++n) {
+          const uint32_t word = w[n * RSTEP * PITCH] >> shift;
+          memcpy(out + (int64_t)(n * RSTEP) * t.p_dst, &word, sizeof(D));
+        }
       } else {
         const uint32_t dr = kTileThreads / qn, dq = kTileThreads - dr * qn;
         uint32_t row = threadIdx.x / qn, q = threadIdx.x - row * qn;
@@ -542,6 +664,75 @@ __global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_co
           q += dq;
           if (q >= qn) q -= qn, ++row;
         }
+      }
+      __syncthreads();
+    }
+  }
+  cta_publish(d, t.x.counter, ok);
+}
+
+// Transposes of a dense matrix with few columns (P below 64, rows of the source next to one another): the source of a
+// tile, all of P by `tq` of Q, is one contiguous range. It comes in 16 bytes per thread, whatever its alignment, and is
+// taken apart on the way out: a thread makes 16 bytes of one row of the destination from elements P apart in shared
+// memory. (With element loads, as in the tile kernel, index arithmetic is the bound: 2^24 x 3 bf16 took 119 us.)
+template <typename S, typename D, bool RAW>
+__global__ void __launch_bounds__(kTileThreads) xfer_narrow_kernel(const __grid_constant__ TileArgs t) {
+  __shared__ __align__(16) unsigned char sm[kNarrowBytes];
+  const eux_xfer_desc& d = t.x.d;
+  const bool ok = cta_wait_arrival(d);
+  if (ok) {
+    constexpr uint32_t E = 16 / sizeof(D);
+    const int op = d.op;
+    const float arg = d.op_arg;
+    const uint32_t np = t.np;
+    const S* el = reinterpret_cast<const S*>(sm);
+    for (uint64_t tile = blockIdx.x; tile < t.tiles; tile += gridDim.x) {
+      const uint32_t q0 = (uint32_t)tile * t.tq;
+      const uint32_t qn = min(t.tq, t.nq - q0);
+      const unsigned char* src = reinterpret_cast<const unsigned char*>(reinterpret_cast<const S*>(d.src) + (uint64_t)q0 * np);
+      D* dst = reinterpret_cast<D*>(d.dst) + q0;
+      const uint32_t bytes = qn * np * (uint32_t)sizeof(S);
+#pragma unroll 2
+      for (uint32_t o = threadIdx.x * 16; o + 16 <= bytes; o += kTileThreads * 16) {
+        uint32_t w[4];
+        load_span<16>(src + o, w);
+        *reinterpret_cast<uint4*>(sm + o) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+      for (uint32_t e = (bytes & ~15u) / sizeof(S) + threadIdx.x; e < qn * np; e += kTileThreads)
+        reinterpret_cast<S*>(sm)[e] = reinterpret_cast<const S*>(src)[e];
+      __syncthreads();
+      if (t.vector_store) {
+        // With eight or more rows a warp covers eight of them by 64 bytes: neighbouring rows are neighbours in shared
+        // memory, where vectors of one row may be any number of banks apart (2^21 x 20 bf16: 16-way conflicts).
+        const uint32_t vr = (qn + E - 1) / E, pb = np >= 8 ? 8 : 1;
+        const uint32_t p_groups = (np + pb - 1) / pb, units = p_groups * pb * ((vr + 3) & ~3u);
+        for (uint32_t u = threadIdx.x; u < units; u += kTileThreads) {
+          uint32_t p, v;
+          if (pb == 8) {
+            const uint32_t r = u >> 5, g = r / p_groups;
+            p = (r - g * p_groups) * 8 + (u & 7), v = g * 4 + ((u >> 3) & 3);
+          } else {
+            const uint32_t vs = (vr + 3) & ~3u;
+            p = u / vs, v = u - p * vs;
+          }
+          if (p < np && v < vr) {
+            const S* s = el + (v * E) * np + p;
+            D* out = dst + (int64_t)p * t.p_dst + v * E;
+            if (v * E + E <= qn) {
+              alignas(16) D o[E];
+#pragma unroll
+              for (int k = 0; k < (int)E; ++k) o[k] = Convert<S, D, RAW>::one(s[k * np], op, arg);
+              *reinterpret_cast<uint4*>(out) = *reinterpret_cast<uint4*>(o);
+            } else {
+              for (uint32_t k = 0; v * E + k < qn; ++k) out[k] = Convert<S, D, RAW>::one(s[k * np], op, arg);
+            }
+          }
+        }
+      } else {
+        for (uint32_t p = 0; p < np; ++p)
+#pragma unroll 4
+          for (uint32_t q = threadIdx.x; q < qn; q += kTileThreads)
+            dst[(int64_t)p * t.p_dst + q] = Convert<S, D, RAW>::one(el[q * np + p], op, arg);
       }
       __syncthreads();
     }
@@ -734,15 +925,26 @@ static bool collapse(eux_xfer_desc& d) {
   return true;
 }
 
+static FastDiv fast_div(uint32_t d) {
+  int l = 0;
+  while (((uint64_t)1 << l) < d) ++l;
+  FastDiv f;
+  f.m = (uint32_t)(((uint64_t)1 << 32) * (((uint64_t)1 << l) - d) / d + 1);
+  f.s1 = l > 0 ? 1 : 0, f.s2 = l > 0 ? l - 1 : 0;
+  return f;
+}
+
 template <typename S, typename D, bool RAW>
-static void launch_gather(const XferArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
-  if (!t) xfer_gather_kernel<S, D, RAW><<<grid, kXferThreads, 0, st>>>(a);
+static void launch_gather(const GatherArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
+  if (!t && vector) xfer_gather_kernel<S, D, RAW, true><<<grid, kXferThreads, 0, st>>>(a);
+  else if (!t) xfer_gather_kernel<S, D, RAW, false><<<grid, kXferThreads, 0, st>>>(a);
+  else if (t->narrow) xfer_narrow_kernel<S, D, RAW><<<grid, kTileThreads, 0, st>>>(*t);
   else if (vector) xfer_tile_kernel<S, D, RAW, true><<<grid, kTileThreads, 0, st>>>(*t);
   else xfer_tile_kernel<S, D, RAW, false><<<grid, kTileThreads, 0, st>>>(*t);
 }
 template <typename S>
-static int launch_gather_from(const XferArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
-  switch (a.d.dst_dtype) {
+static int launch_gather_from(const GatherArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
+  switch (a.x.d.dst_dtype) {
     case EUX_DT_F32: launch_gather<S, float, false>(a, t, vector, grid, st); break;
     case EUX_DT_F16: launch_gather<S, __half, false>(a, t, vector, grid, st); break;
     case EUX_DT_BF16: launch_gather<S, __nv_bfloat16, false>(a, t, vector, grid, st); break;
@@ -784,13 +986,13 @@ static bool plan_tiles(const eux_xfer_desc& d, TileArgs& t, bool& vector) {
     batch *= (uint64_t)d.shape[k];
   }
   t.p_dst = dst_stride[p];
-  // 64 steps of P by 128 bytes of Q; where one of the two is shorter the tile is as much longer in the other
-  uint32_t qw_all = (t.nq + g - 1) / g, qw = 32, tp = 64;
+  // TP steps of P by 128 or 256 bytes of Q; where one of the two is shorter the tile is as much longer in the other
+  uint32_t qw_all = (t.nq + g - 1) / g, qw = tile_q(vector), tp = ssz == 1 ? tile_p<uint8_t>() : tile_p<uint16_t>();
   if (t.np < 64) {
     tp = t.np;
     qw = (uint32_t)(kTileWords / tp - 1) & ~3u;
     if (qw > qw_all) qw = qw_all;
-  } else if (qw_all < 32) {
+  } else if (qw_all < qw) {
     qw = qw_all;
     tp = ((uint32_t)kTileWords / (qw | 1u)) & ~15u;  // whole vectors of P
     if (tp > t.np) tp = t.np;
@@ -798,8 +1000,24 @@ static bool plan_tiles(const eux_xfer_desc& d, TileArgs& t, bool& vector) {
   t.pitch = qw | 1u;
   t.tp = tp, t.tq = qw * g < t.nq ? qw * g : t.nq;
   t.tiles_p = (t.np + tp - 1) / tp, t.tiles_q = (t.nq + t.tq - 1) / t.tq;
+  t.narrow = d.ndim == 2 && t.np < 64 && t.q_src == (int64_t)t.np && t.nq >= 1024;
+  if (t.narrow) {
+    t.tq = (uint32_t)(kNarrowBytes / (t.np * ssz)) & ~15u;  // whole vectors of Q
+    if (t.tq > 2048) t.tq = 2048;
+    t.tiles_q = (t.nq + t.tq - 1) / t.tq;
+  }
   t.tiles = batch * t.tiles_p * t.tiles_q;
   t.vector_store = store16;
+  return true;
+}
+
+// Whether every chunk of `chunk` elements is one aligned load of the source and one aligned store.
+static bool rows_aligned(const eux_xfer_desc& d, bool whole, int chunk, int ssz, int dsz) {
+  if (!whole || d.stride[d.ndim - 1] != 1 || d.shape[d.ndim - 1] % chunk) return false;
+  const uint64_t load = chunk * ssz >= 16 ? 16 : 8, store = chunk * dsz >= 16 ? 16 : 8;
+  if ((uintptr_t)d.src % load || (uintptr_t)d.dst % store) return false;
+  for (int k = 0; k + 1 < d.ndim; ++k)
+    if ((uint64_t)(d.stride[k] * ssz) % load) return false;
   return true;
 }
 
@@ -856,24 +1074,32 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     bool vector = false;
     const bool tiled = whole && !as_bytes && plan_tiles(a.d, t, vector);
     if (tiled) t.x = a;
-    // Eight tile CTAs (256 threads) and four gather CTAs (512) fill an SM's threads.
-    if (!ctas_given) max_ctas = (tiled ? 8 : 4) * sms;
-    const uint64_t per_cta = (uint64_t)kXferThreads * (raw ? 16 / (as_bytes ? 1 : dsz) : 8);
+    const int chunk = raw ? 16 / (as_bytes ? 1 : dsz) : 8;  // elements per chunk of the gather kernel
+    if (!tiled) vector = !as_bytes && rows_aligned(a.d, whole, chunk, ssz, dsz);
+    // Four gather CTAs fill an SM's threads. Tiles: a CTA each, whose loads then overlap other CTAs' stores (55 us against
+    // 60 on 8192 x 8192 bf16), or eight CTAs per SM where each one also has a flag's counter to go through.
+    if (!ctas_given) max_ctas = !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;
+    const uint64_t per_cta = (uint64_t)kXferThreads * chunk;
     grid = limit(tiled ? t.tiles : (a.d.n_elems + per_cta - 1) / per_cta);
     if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
     const TileArgs* tp = tiled ? &t : nullptr;
+    GatherArgs ga{a, {}, a.d.n_elems >> 32 == 0};
+    for (int k = 0; k < a.d.ndim; ++k) {
+      if (a.d.shape[k] >> 32) ga.small = 0;
+      else if (a.d.shape[k] > 0) ga.div[k] = fast_div((uint32_t)a.d.shape[k]);
+    }
     int rc = 0;
     if (raw) {
       const int esz = as_bytes ? 1 : ssz;
-      if (esz == 4) launch_gather<uint32_t, uint32_t, true>(a, tp, vector, grid, st);
-      else if (esz == 2) launch_gather<uint16_t, uint16_t, true>(a, tp, vector, grid, st);
-      else launch_gather<uint8_t, uint8_t, true>(a, tp, vector, grid, st);
+      if (esz == 4) launch_gather<uint32_t, uint32_t, true>(ga, tp, vector, grid, st);
+      else if (esz == 2) launch_gather<uint16_t, uint16_t, true>(ga, tp, vector, grid, st);
+      else launch_gather<uint8_t, uint8_t, true>(ga, tp, vector, grid, st);
     } else {
       switch (d->src_dtype) {
-        case EUX_DT_F32: rc = launch_gather_from<float>(a, tp, vector, grid, st); break;
-        case EUX_DT_F16: rc = launch_gather_from<__half>(a, tp, vector, grid, st); break;
-        case EUX_DT_BF16: rc = launch_gather_from<__nv_bfloat16>(a, tp, vector, grid, st); break;
-        case EUX_DT_F8E4M3: rc = launch_gather_from<__nv_fp8_e4m3>(a, tp, vector, grid, st); break;
+        case EUX_DT_F32: rc = launch_gather_from<float>(ga, tp, vector, grid, st); break;
+        case EUX_DT_F16: rc = launch_gather_from<__half>(ga, tp, vector, grid, st); break;
+        case EUX_DT_BF16: rc = launch_gather_from<__nv_bfloat16>(ga, tp, vector, grid, st); break;
+        case EUX_DT_F8E4M3: rc = launch_gather_from<__nv_fp8_e4m3>(ga, tp, vector, grid, st); break;
         default: rc = EUX_ERR_BAD_ARG;
       }
     }
@@ -1058,7 +1284,9 @@ int preload_one(K kernel) {
 }
 template <typename S, typename D, bool RAW>
 int preload_gather() {
-  int rc = preload_one(xfer_gather_kernel<S, D, RAW>);
+  int rc = preload_one(xfer_gather_kernel<S, D, RAW, true>);
+  if (!rc) rc = preload_one(xfer_gather_kernel<S, D, RAW, false>);
+  if (!rc) rc = preload_one(xfer_narrow_kernel<S, D, RAW>);
   if (!rc) rc = preload_one(xfer_tile_kernel<S, D, RAW, true>);
   if (!rc) rc = preload_one(xfer_tile_kernel<S, D, RAW, false>);
   return rc;
