@@ -20,6 +20,9 @@
 // arenas with peer loads and accumulates sum_k w_k * y_k in fp32 registers, so
 // the weighted combine is fused into the receive and no intermediate buffer
 // exists.
+#include <algorithm>
+#include <atomic>
+
 #include "eux_device.cuh"
 
 namespace eux {
@@ -34,82 +37,98 @@ __host__ __device__ __forceinline__ size_t moe_row_bytes(int hidden, int fp8) {
   return fp8 ? (((size_t)hidden + (size_t)(hidden / 128) * 4 + 127) / 128) * 128 : (size_t)hidden * 2;
 }
 
-// ---- routing: slot assignment, grouped by expert (single CTA) --------------
-// counters layout: [0,W) rows per dst rank | [W,W+E) rows per expert | [W+E] done-CTA word
-__global__ void __launch_bounds__(1024) moe_route_kernel(eux_moe_desc d) {
-  extern __shared__ int sm[];
-  int* cnt = sm;                    // [E]
-  int* off = sm + d.n_experts;      // [E]
-  int* cur = sm + 2 * d.n_experts;  // [E]
-  const int E = d.n_experts, W = d.world, EPR = E / W;
-  const int n = d.n_tokens * d.topk;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0, cur[e] = 0;
-  // Up to 32 routing entries per thread are fetched once, all loads in flight together, and
-  // serve both passes from registers (a single CTA is latency bound: 64 dependent global loads
-  // per thread otherwise). Larger batches fall back to re-reading.
-  constexpr int kCache = 32;
-  const bool cached = n <= kCache * (int)blockDim.x;
-  int ev[kCache];
-  if (cached) {
+// ---- dispatch: routing and the transfer in one cooperative launch -----------------------------------------
+// Every CTA owns a run of tokens. It counts their experts, adds its counts to the global ones (which returns where its
+// rows start inside each expert's group), waits for all CTAs at a grid barrier, and then knows every slot: the experts
+// before this one on the same rank, its CTA's start, and the rank inside the CTA. A single routing CTA in front of the
+// transfer took 5 us for 128 tokens and 13 for 4096 (top 8 of 256), plus a launch. All CTAs are resident (cooperative
+// launch), so the barrier ends; its wait is bounded all the same.
+// counters layout: [0,W) unused | [W,W+E) rows per expert | [W+E] done CTAs | [W+E+1] barrier; zero between launches
+__device__ __forceinline__ void moe_ld_v8(const void* p, uint32_t (&v)[8]) {
+  asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "l"(p));
+}
+__device__ __forceinline__ void moe_st_v8(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+struct MoeRouting {
+  int* local;  // [E] rows of this CTA per expert
+  int* base;   // [E] where they start inside the expert's group; after the barrier: inside the destination's region
+  int* total;  // [E] rows of all CTAs per expert
+};
+
+// Exclusive scan of v over the CTA; `sums`: one int per warp.
+__device__ __forceinline__ int cta_exclusive_scan(int v, int* sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
 #pragma unroll
-    for (int j = 0; j < kCache; ++j) {
-      const int i = threadIdx.x + j * blockDim.x;
-      ev[j] = i < n ? __ldg(d.topk_idx + i) : -1;
-    }
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
+  if (lane == 31) sums[warp] = x;
   __syncthreads();
-  if (cached) {
-#pragma unroll
-    for (int j = 0; j < kCache; ++j)
-      if (ev[j] >= 0 && ev[j] < E) atomicAdd(&cnt[ev[j]], 1);
-  } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      int e = d.topk_idx[i];
-      if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
-    }
-  }
+  int before = 0;
+  for (int w = 0; w < warp; ++w) before += sums[w];
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int base = (e / EPR) * EPR, s = 0;
-    for (int j = base; j < e; ++j) s += cnt[j];
-    off[e] = s;
-    d.counters[W + e] = cnt[e];
-  }
-  for (int r = threadIdx.x; r < W; r += blockDim.x) {
-    int s = 0;
-    for (int j = r * EPR; j < (r + 1) * EPR; ++j) s += cnt[j];
-    if (s > d.capacity) set_status(d.status, EUX_ST_OVERFLOW, 10);
-    d.counters[r] = s < d.capacity ? s : d.capacity;
-  }
-  __syncthreads();
-  if (cached) {
-#pragma unroll
-    for (int j = 0; j < kCache; ++j) {
-      const int i = threadIdx.x + j * blockDim.x;
-      if (i >= n) continue;
-      const int e = ev[j];
-      int slot = -1;
-      if (e >= 0 && e < E) {
-        slot = off[e] + atomicAdd(&cur[e], 1);
-        if (slot >= d.capacity) slot = -1;
-      }
-      d.slot_of[i] = slot;
-    }
-  } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      int e = d.topk_idx[i];
-      int slot = -1;
-      if (e >= 0 && e < E) {
-        slot = off[e] + atomicAdd(&cur[e], 1);
-        if (slot >= d.capacity) slot = -1;
-      }
-      d.slot_of[i] = slot;
-    }
-  }
+  return before + x - v;
 }
 
-__device__ __forceinline__ void moe_publish(const eux_moe_desc& d) {
-  // last CTA: send counts + arrival flags to every destination rank
+__device__ __forceinline__ bool moe_route(const eux_moe_desc& d, const MoeRouting& r, int t0, int t1) {
+  const int W = d.world, E = d.n_experts, EPR = E / W, K = d.topk;
+  int* const counts = d.counters + W;
+  uint32_t* const barrier = reinterpret_cast<uint32_t*>(d.counters + W + E + 1);
+  __shared__ int s_sums[kMoeThreads / 32];
+  __shared__ int s_ok;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) r.local[e] = 0;
+  __syncthreads();
+  for (int64_t i = (int64_t)t0 * K + threadIdx.x; i < (int64_t)t1 * K; i += blockDim.x) {
+    const int e = __ldg(d.topk_idx + i);
+    d.slot_of[i] = e >= 0 && e < E ? atomicAdd(&r.local[e], 1) : -1;  // the rank inside this CTA, for now
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) r.base[e] = r.local[e] ? atomicAdd(counts + e, r.local[e]) : 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(barrier, 1u);
+    s_ok = wait_u32_ge_gpu(barrier, gridDim.x, d.wait_timeout_ns);
+    if (!s_ok) set_status(d.status, EUX_ST_TIMEOUT, 10);
+  }
+  __syncthreads();
+  if (!s_ok) return false;
+  // every thread takes a run of consecutive experts: totals, and the exclusive sums over them
+  const int run = (E + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int e0 = (int)threadIdx.x * run, e1 = min(e0 + run, E);
+  int mine = 0;
+  for (int e = e0; e < e1; ++e) {
+    r.total[e] = __ldcg(counts + e);
+    mine += r.total[e];
+  }
+  int sum = cta_exclusive_scan(mine, s_sums);
+  for (int e = e0; e < e1; ++e) {
+    r.local[e] = sum;  // rows of all experts before e, whatever their rank
+    sum += r.total[e];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) r.base[e] += r.local[e] - r.local[(e / EPR) * EPR];
+  __syncthreads();
+  for (int64_t i = (int64_t)t0 * K + threadIdx.x; i < (int64_t)t1 * K; i += blockDim.x) {
+    int slot = d.slot_of[i];
+    if (slot >= 0) {
+      slot += r.base[__ldg(d.topk_idx + i)];
+      d.slot_of[i] = slot < d.capacity ? slot : -1;
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+// The last CTA sends counts and arrival flags to every destination rank and leaves the counters at zero.
+__device__ __forceinline__ void moe_publish(const eux_moe_desc& d, const MoeRouting& r) {
   __syncthreads();
   __shared__ int s_last;
   const int W = d.world, E = d.n_experts, EPR = E / W;
@@ -121,31 +140,72 @@ __device__ __forceinline__ void moe_publish(const eux_moe_desc& d) {
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (int i = threadIdx.x; i < W * EPR; i += blockDim.x) {
-    int dst = i / EPR, le = i - dst * EPR;
-    d.flag_peer[dst][3 * W + d.rank * EPR + le] = (uint64_t)d.counters[W + dst * EPR + le];
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    const int dst = e / EPR, le = e - dst * EPR;
+    d.flag_peer[dst][3 * W + d.rank * EPR + le] = (uint64_t)r.total[e];
+    d.counters[W + e] = 0;
   }
-  for (int dst = threadIdx.x; dst < W; dst += blockDim.x) d.flag_peer[dst][W + d.rank] = (uint64_t)d.counters[dst];
+  for (int dst = threadIdx.x; dst < W; dst += blockDim.x) {
+    const int last = dst * EPR + EPR - 1;
+    const int rows = r.local[last] - r.local[dst * EPR] + r.total[last];
+    if (rows > d.capacity) set_status(d.status, EUX_ST_OVERFLOW, 10);
+    d.flag_peer[dst][W + d.rank] = (uint64_t)(rows < d.capacity ? rows : d.capacity);
+  }
   __threadfence_system();
   __syncthreads();
   for (int dst = threadIdx.x; dst < W; dst += blockDim.x) st_release_sys(&d.flag_peer[dst][d.rank], d.seq);
-  if (threadIdx.x == 0) d.counters[W + E] = 0;
+  if (threadIdx.x < 2) d.counters[W + E + threadIdx.x] = 0;
+}
+
+// The routing entries of a token: lane k (< topk) owns slot k.
+struct MoeEntry {
+  int dst = -1, slot = -1, expert = -1;
+  float w = 0.f;
+  __device__ __forceinline__ MoeEntry(const eux_moe_desc& d, int t, int lane, int EPR) {
+    if (lane < d.topk) {
+      const int64_t i = (int64_t)t * d.topk + lane;
+      slot = d.slot_of[i];
+      if (slot >= 0) {
+        expert = __ldg(d.topk_idx + i);
+        dst = expert / EPR;
+        w = __ldg(d.topk_w + i);
+      }
+    }
+  }
+  __device__ __forceinline__ size_t row(const eux_moe_desc& d) const { return (size_t)d.rank * d.capacity + slot; }
+  __device__ __forceinline__ unsigned char* arena_row(const eux_moe_desc& d, size_t row_bytes) const {
+    return slot < 0 ? nullptr : reinterpret_cast<unsigned char*>(d.arena_peer[dst]) + row(d) * row_bytes;
+  }
+  __device__ __forceinline__ void store_header(const eux_moe_desc& d, int t, int lane, int EPR) const {
+    if (slot < 0) return;
+    uint4 h;
+    h.x = (uint32_t)t;
+    h.y = (uint32_t)lane | ((uint32_t)(expert - dst * EPR) << 16);
+    h.z = __float_as_uint(w);
+    h.w = (uint32_t)d.rank;
+    st_u4(reinterpret_cast<uint4*>(d.meta_peer[dst]) + row(d), h);
+  }
+};
+__device__ __forceinline__ unsigned char* shfl_ptr(unsigned char* p, int src) {
+  return (unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)p, src);
 }
 
 // ---- dispatch, bf16 rows ----------------------------------------------------
 // Work unit = (token, 128 consecutive 16-byte chunks): a warp loads 4 chunks per
 // lane once and stores them to each of the token's top-k destinations.
-__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_desc d) {
-  const int W = d.world, EPR = d.n_experts / W, K = d.topk;
+__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_desc d, int tokens_per_cta) {
+  extern __shared__ int moe_sm[];
+  const MoeRouting r{moe_sm, moe_sm + d.n_experts, moe_sm + 2 * d.n_experts};
+  const int t0 = min((int)blockIdx.x * tokens_per_cta, d.n_tokens), t1 = min(t0 + tokens_per_cta, d.n_tokens);
+  if (!moe_route(d, r, t0, t1)) return;
+  const int EPR = d.n_experts / d.world, K = d.topk;
   const int chunks = d.hidden / 8;  // uint4 per row
   const int upr = (chunks + 127) / 128;
   const size_t row_bytes = (size_t)d.hidden * 2;
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int64_t units = (int64_t)d.n_tokens * upr;
-  for (int64_t u = warp; u < units; u += nwarps) {
-    const int t = (int)(u / upr), part = (int)(u - (int64_t)t * upr);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int units = (t1 - t0) * upr;
+  for (int u = warp; u < units; u += nwarps) {
+    const int tl = u / upr, t = t0 + tl, part = u - tl * upr;
     const uint4* src = reinterpret_cast<const uint4*>(d.x) + (size_t)t * chunks;
     const int c0 = part * 128 + lane;
     uint4 v[4];
@@ -154,223 +214,99 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_
       int c = c0 + 32 * j;
       if (c < chunks) v[j] = ld_stream_u4(src + c);
     }
-    // lane k (< topk) owns the routing entry of slot k
-    int my_e = -1, my_slot = -1;
-    float my_w = 0.f;
-    if (lane < K) {
-      my_e = d.topk_idx[t * K + lane];
-      my_slot = d.slot_of[t * K + lane];
-      my_w = d.topk_w[t * K + lane];
-    }
+    const MoeEntry my(d, t, lane, EPR);
+    unsigned char* const my_out = my.arena_row(d, row_bytes);
     for (int k = 0; k < K; ++k) {
-      const int e = __shfl_sync(0xffffffffu, my_e, k);
-      const int slot = __shfl_sync(0xffffffffu, my_slot, k);
-      if (slot < 0) continue;
-      const int dst = e / EPR;
-      const size_t row = (size_t)d.rank * d.capacity + slot;
-      uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(d.arena_peer[dst]) + row * row_bytes);
+      uint4* out = reinterpret_cast<uint4*>(shfl_ptr(my_out, k));
+      if (!out) continue;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         int c = c0 + 32 * j;
         if (c < chunks) st_u4(out + c, v[j]);
       }
-      if (part == 0 && lane == k) {
-        uint4 h;
-        h.x = (uint32_t)t;
-        h.y = (uint32_t)k | ((uint32_t)(e - dst * EPR) << 16);
-        h.z = __float_as_uint(my_w);
-        h.w = (uint32_t)d.rank;
-        st_u4(reinterpret_cast<uint4*>(d.meta_peer[dst]) + row, h);
-      }
     }
+    if (part == 0) my.store_header(d, t, lane, EPR);
   }
-  moe_publish(d);
+  moe_publish(d, r);
 }
 
 // ---- dispatch, e4m3 rows with one fp32 scale per 128 elements ---------------
-// Work unit = (token, 512 elements): lane holds 16 elements; 8 lanes share a scale.
-__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_fp8_kernel(eux_moe_desc d) {
-  const int W = d.world, EPR = d.n_experts / W, K = d.topk;
-  const int upr = (d.hidden + 511) / 512;
-  const size_t row_bytes = moe_row_bytes(d.hidden, 1);
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int64_t units = (int64_t)d.n_tokens * upr;
-  for (int64_t u = warp; u < units; u += nwarps) {
-    const int t = (int)(u / upr), part = (int)(u - (int64_t)t * upr);
-    const int e0 = part * 512 + lane * 16;  // first element of this lane
-    const bool in = e0 < d.hidden;
-    float f[16];
-    if (in) {
-      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(d.x) + (size_t)t * d.hidden + e0);
-      uint4 a = ld_stream_u4(src), b = ld_stream_u4(src + 1);
-      const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
-      const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2 x = __bfloat1622float2(pa[j]), y = __bfloat1622float2(pb[j]);
-        f[2 * j] = x.x, f[2 * j + 1] = x.y, f[8 + 2 * j] = y.x, f[8 + 2 * j + 1] = y.y;
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) f[j] = 0.f;
-    }
-    float amax = 0.f;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-    const float scale = fmaxf(amax, 1e-10f) * (1.0f / 448.0f);
-    const float inv = 1.0f / scale;
-    uint4 q;
-    {
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j] * inv, f[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-        uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j + 2] * inv, f[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-        w[j] = lo | (hi << 16);
-      }
-      q = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-    int my_e = -1, my_slot = -1;
-    float my_w = 0.f;
-    if (lane < K) {
-      my_e = d.topk_idx[t * K + lane];
-      my_slot = d.slot_of[t * K + lane];
-      my_w = d.topk_w[t * K + lane];
-    }
-    for (int k = 0; k < K; ++k) {
-      const int e = __shfl_sync(0xffffffffu, my_e, k);
-      const int slot = __shfl_sync(0xffffffffu, my_slot, k);
-      if (slot < 0) continue;
-      const int dst = e / EPR;
-      const size_t row = (size_t)d.rank * d.capacity + slot;
-      unsigned char* out = reinterpret_cast<unsigned char*>(d.arena_peer[dst]) + row * row_bytes;
-      if (in) {
-        st_u4(out + e0, q);
-        if ((lane & 7) == 0) reinterpret_cast<float*>(out + d.hidden)[e0 >> 7] = scale;
-      }
-      if (part == 0 && lane == k) {
-        uint4 h;
-        h.x = (uint32_t)t;
-        h.y = (uint32_t)k | ((uint32_t)(e - dst * EPR) << 16);
-        h.z = __float_as_uint(my_w);
-        h.w = (uint32_t)d.rank;
-        st_u4(reinterpret_cast<uint4*>(d.meta_peer[dst]) + row, h);
-      }
-    }
-  }
-  moe_publish(d);
+// Work unit = (token, 1024 elements): a lane holds 32 elements, four lanes share a scale, and a warp's store into a row
+// is 1 KiB. The scales of a batch of tokens are collected in shared memory and leave as one coalesced store per row:
+// across NVLink a 4-byte store costs a packet of its own. (One warp per token row, which kept them in registers, left a
+// decode batch with a warp per token: 128 tokens of 7168 took 34 us, 20 now. 32-byte stores: with two of 16 bytes per
+// lane 4096 tokens took 89 us, 78 now.)
+constexpr int kMoeScaleFloats = 4096;  // per buffer; two buffers, so that one barrier per batch is enough
+__host__ __device__ __forceinline__ int moe_scale_batch(int hidden) {
+  const int b = kMoeScaleFloats / (hidden / 128);
+  return b < 1 ? 1 : (b > 16 ? 16 : b);
 }
+__host__ __device__ __forceinline__ int moe_scale_stride(int hidden) { return moe_scale_batch(hidden) * (hidden / 128); }
 
-// ---- dispatch, e4m3 rows, one warp per token row -------------------------------
-// Same bytes as moe_dispatch_fp8_kernel, but the 4-byte scales of a row are collected in
-// registers (lane L keeps groups L, 32+L, ...) and leave as one coalesced store per destination
-// at the end of the row: across NVLink a 4-byte store costs a packet of its own, and the
-// per-group stores of the kernel above made a fifth of all packets.
-__device__ __forceinline__ float pick4(const float (&r)[4], int i) {
-  return i == 0 ? r[0] : (i == 1 ? r[1] : (i == 2 ? r[2] : r[3]));
-}
-__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_fp8_rows_kernel(eux_moe_desc d) {
-  const int W = d.world, EPR = d.n_experts / W, K = d.topk;
-  const int upr = (d.hidden + 511) / 512;
+__global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_moe_desc d, int tokens_per_cta) {
+  extern __shared__ int moe_sm[];
+  const MoeRouting r{moe_sm, moe_sm + d.n_experts, moe_sm + 2 * d.n_experts};
+  float* const scales = reinterpret_cast<float*>(moe_sm + 3 * d.n_experts);
+  const int t0 = min((int)blockIdx.x * tokens_per_cta, d.n_tokens), t1 = min(t0 + tokens_per_cta, d.n_tokens);
+  if (!moe_route(d, r, t0, t1)) return;
+  const int EPR = d.n_experts / d.world, K = d.topk;
+  const int upr = (d.hidden + 1023) / 1024;
   const int ngroups = d.hidden / 128;
   const size_t row_bytes = moe_row_bytes(d.hidden, 1);
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int t = warp; t < d.n_tokens; t += nwarps) {
-    int my_e = -1, my_slot = -1;
-    float my_w = 0.f;
-    if (lane < K) {
-      my_e = d.topk_idx[t * K + lane];
-      my_slot = d.slot_of[t * K + lane];
-      my_w = d.topk_w[t * K + lane];
-    }
-    // this lane's destination row, for k = lane
-    unsigned char* my_out = nullptr;
-    if (my_slot >= 0) {
-      const int dst = my_e / EPR;
-      my_out = reinterpret_cast<unsigned char*>(d.arena_peer[dst]) + ((size_t)d.rank * d.capacity + my_slot) * row_bytes;
-    }
-    float sc[4] = {0.f, 0.f, 0.f, 0.f};
-    const __nv_bfloat16* xrow = reinterpret_cast<const __nv_bfloat16*>(d.x) + (size_t)t * d.hidden;
-    for (int part = 0; part < upr; ++part) {
-      const int e0 = part * 512 + lane * 16;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int batch = moe_scale_batch(d.hidden), stride = moe_scale_stride(d.hidden);
+  int buf = 0;
+  for (int tb = t0; tb < t1; tb += batch, buf ^= 1) {
+    const int nt = min(batch, t1 - tb);
+    float* const sc = scales + buf * stride;
+    for (int u = warp; u < nt * upr; u += nwarps) {
+      const int tl = u / upr, t = tb + tl, part = u - tl * upr;
+      const int e0 = part * 1024 + lane * 32;  // first element of this lane
       const bool in = e0 < d.hidden;
-      float f[16];
-      if (in) {
-        const uint4* src = reinterpret_cast<const uint4*>(xrow + e0);
-        uint4 a = ld_stream_u4(src), b = ld_stream_u4(src + 1);
-        const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
-        const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
+      uint4 raw[4];
+      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(d.x) + (size_t)t * d.hidden + e0);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 x = __bfloat1622float2(pa[j]), y = __bfloat1622float2(pb[j]);
-          f[2 * j] = x.x, f[2 * j + 1] = x.y, f[8 + 2 * j] = y.x, f[8 + 2 * j + 1] = y.y;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) f[j] = 0.f;
-      }
+      for (int j = 0; j < 4; ++j) raw[j] = in ? ld_stream_u4(src + j) : make_uint4(0, 0, 0, 0);
+      const MoeEntry my(d, t, lane, EPR);
+      unsigned char* const my_out = my.arena_row(d, row_bytes);
+      const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(raw);
       float amax = 0.f;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
+      for (int j = 0; j < 16; ++j) {
+        const float2 x = __bfloat1622float2(pairs[j]);
+        amax = fmaxf(amax, fmaxf(fabsf(x.x), fabsf(x.y)));
+      }
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
       const float scale = fmaxf(amax, 1e-10f) * (1.0f / 448.0f);
       const float inv = 1.0f / scale;
-      uint32_t w4[4];
+      uint32_t w[8];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j] * inv, f[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-        uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[4 * j + 2] * inv, f[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-        w4[j] = lo | (hi << 16);
+      for (int j = 0; j < 8; ++j) {
+        const float2 a = __bfloat1622float2(pairs[2 * j]), b = __bfloat1622float2(pairs[2 * j + 1]);
+        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a.x * inv, a.y * inv), __NV_SATFINITE, __NV_E4M3);
+        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(b.x * inv, b.y * inv), __NV_SATFINITE, __NV_E4M3);
+        w[j] = lo | (hi << 16);
       }
-      const uint4 q = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-      // the four scales of this part go to the lanes that keep them
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float sj = __shfl_sync(0xffffffffu, scale, 8 * j);
-        const int gi = part * 4 + j;
-        if (lane == (gi & 31)) {
-          const int r = gi >> 5;
-          if (r == 0) sc[0] = sj;
-          else if (r == 1) sc[1] = sj;
-          else if (r == 2) sc[2] = sj;
-          else sc[3] = sj;
-        }
-      }
+      if (in && (lane & 3) == 0) sc[tl * ngroups + (e0 >> 7)] = scale;
       for (int k = 0; k < K; ++k) {
-        unsigned char* out = (unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_out, k);
-        if (out && in) st_u4(out + e0, q);
+        unsigned char* out = shfl_ptr(my_out, k);
+        if (!out || !in) continue;
+        moe_st_v8(out + e0, w);
       }
+      if (part == 0) my.store_header(d, t, lane, EPR);
     }
-    for (int k = 0; k < K; ++k) {
-      unsigned char* out = (unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_out, k);
+    __syncthreads();
+    for (int u = warp; u < nt * K; u += nwarps) {
+      const int tl = u / K, k = u - tl * K;
+      const MoeEntry my(d, tb + tl, lane, EPR);
+      unsigned char* out = shfl_ptr(my.arena_row(d, row_bytes), k);
       if (!out) continue;
       float* so = reinterpret_cast<float*>(out + d.hidden);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int g = r * 32 + lane;
-        if (g < ngroups) so[g] = sc[r];
-      }
-    }
-    if (my_out) {  // lane k writes the header of the k-th destination row
-      const int dst = my_e / EPR;
-      uint4 h;
-      h.x = (uint32_t)t;
-      h.y = (uint32_t)lane | ((uint32_t)(my_e - dst * EPR) << 16);
-      h.z = __float_as_uint(my_w);
-      h.w = (uint32_t)d.rank;
-      st_u4(reinterpret_cast<uint4*>(d.meta_peer[dst]) + ((size_t)d.rank * d.capacity + my_slot), h);
+      for (int g = lane; g < ngroups; g += 32) so[g] = sc[tl * ngroups + g];
     }
   }
-  moe_publish(d);
+  moe_publish(d, r);
 }
 
 // ---- expert side: wait for every source, (identity expert), tell the sources -
@@ -485,11 +421,6 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_kernel(eux_moe_d
 // on one GPU, 403 -> 388 us when half the rows cross NVLink). A unit's eight rows are fetched as two
 // groups of four, and the next group is always requested before the current one is accumulated, so a
 // warp never sits out a whole memory round trip; the routing entries are read once per token.
-__device__ __forceinline__ void moe_ld_v8(const void* p, uint32_t (&v)[8]) {
-  asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "l"(p));
-}
 __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_stream_kernel(eux_moe_desc d) {
   if (!moe_wait_experts(d)) return;
   const int W = d.world, EPR = d.n_experts / W, K = d.topk;
@@ -654,6 +585,9 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_kernel(eux_moe_de
   }
 }
 
+__device__ __forceinline__ float pick4(const float (&r)[4], int i) {
+  return i == 0 ? r[0] : (i == 1 ? r[1] : (i == 2 ? r[2] : r[3]));
+}
 // ---- combine, fp8 rows, one warp per token (top-k <= 8, hidden <= 16384) -----------------
 // The scales of the k rows are fetched once per row (two coalesced loads per row instead of one
 // small load per 512 elements), already multiplied by the gate weight.
@@ -751,15 +685,48 @@ using namespace eux;
 
 extern "C" size_t eux_moe_row_bytes(int hidden, int fp8) { return moe_row_bytes(hidden, fp8); }
 
+// How many CTAs of a cooperative launch the device holds at once (asked once per device and amount of shared memory).
+template <auto KERNEL>
+static int moe_resident_ctas(int dev, size_t smem, int* out) {
+  static std::atomic<uint64_t> known[64];  // shared memory << 32 | CTAs, of the last question
+  const uint64_t k = known[dev].load(std::memory_order_acquire);
+  if (k && (k >> 32) == smem) {
+    *out = (int)(uint32_t)k;
+    return 0;
+  }
+  int per_sm = 0, sms = 0;
+  cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, kMoeThreads, smem);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return (int)e;
+  if (per_sm < 1) return EUX_ERR_UNSUPPORTED;
+  *out = per_sm * sms;
+  known[dev].store((uint64_t)smem << 32 | (uint32_t)*out, std::memory_order_release);
+  return 0;
+}
+template <auto KERNEL>
+static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream_t st) {
+  int dev = 0, resident = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return EUX_ERR_BAD_ARG;
+  if (int rc = moe_resident_ctas<KERNEL>(dev, smem, &resident)) return rc;
+  // two CTAs per SM where there are tokens for them
+  if (ctas <= 0) ctas = 296;
+  if (ctas > resident) ctas = resident;
+  int per = (d->n_tokens + ctas - 1) / ctas;
+  if (per < 1) per = 1;
+  int grid = (d->n_tokens + per - 1) / per;
+  if (grid < 1) grid = 1;
+  eux_moe_desc dd = *d;
+  void* args[] = {&dd, &per};
+  return (int)cudaLaunchCooperativeKernel((const void*)KERNEL, dim3(grid), dim3(kMoeThreads), args, smem, st);
+}
+
 extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* stream) {
   if (int rc = moe_check(d)) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (ctas <= 0) ctas = 296;
-  moe_route_kernel<<<1, 1024, 3 * d->n_experts * sizeof(int), st>>>(*d);
-  if (d->fp8 && d->hidden <= 16384) moe_dispatch_fp8_rows_kernel<<<ctas, kMoeThreads, 0, st>>>(*d);
-  else if (d->fp8) moe_dispatch_fp8_kernel<<<ctas, kMoeThreads, 0, st>>>(*d);
-  else moe_dispatch_bf16_kernel<<<ctas, kMoeThreads, 0, st>>>(*d);
-  return (int)cudaGetLastError();
+  const size_t routing = 3 * (size_t)d->n_experts * sizeof(int);
+  if (!d->fp8) return moe_dispatch<moe_dispatch_bf16_kernel>(d, ctas, routing, (cudaStream_t)stream);
+  return moe_dispatch<moe_dispatch_fp8_kernel>(d, ctas, routing + 2 * (size_t)moe_scale_stride(d->hidden) * sizeof(float), (cudaStream_t)stream);
 }
 
 extern "C" int eux_moe_expert_ready_launch(const eux_moe_desc* d, void* stream) {
@@ -886,7 +853,10 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
 
 extern "C" int eux_moe_combine_launch(const eux_moe_desc* d, int ctas, void* stream) {
   if (int rc = moe_check(d)) return rc;
-  if (ctas <= 0) ctas = 296;
+  if (ctas <= 0) {  // no CTA without a unit (of at least 512 elements of a token) for some warp: each polls the flags
+    const int64_t units = (int64_t)d->n_tokens * ((d->hidden + 511) / 512);
+    ctas = (int)std::min<int64_t>(296, std::max<int64_t>(1, (units + kMoeThreads / 32 - 1) / (kMoeThreads / 32)));
+  }
   if (d->fp8 && d->topk <= 8 && d->hidden <= 8192) moe_combine_fp8_stream_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
   else if (d->fp8 && d->topk <= 8 && d->hidden <= 16384) moe_combine_fp8_rows_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
   else if (d->fp8) moe_combine_fp8_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
@@ -899,10 +869,10 @@ extern "C" int eux_moe_combine_launch(const eux_moe_desc* d, int ctas, void* str
 // Loads every kernel of this file (see eux_xfer_preload for why a first launch must not be the one that loads).
 extern "C" int eux_moe_preload(void) {
   cudaFuncAttributes attr;
-  const void* kernels[] = {(const void*)moe_route_kernel,          (const void*)moe_dispatch_bf16_kernel,   (const void*)moe_dispatch_fp8_kernel,
-                           (const void*)moe_dispatch_fp8_rows_kernel, (const void*)moe_expert_ready_kernel, (const void*)moe_combine_bf16_kernel,
-                           (const void*)moe_combine_bf16_stream_kernel, (const void*)moe_combine_fp8_kernel, (const void*)moe_combine_fp8_rows_kernel,
-                           (const void*)moe_combine_fp8_stream_kernel};
+  const void* kernels[] = {(const void*)moe_dispatch_bf16_kernel,       (const void*)moe_dispatch_fp8_kernel,
+                           (const void*)moe_expert_ready_kernel,        (const void*)moe_combine_bf16_kernel,
+                           (const void*)moe_combine_bf16_stream_kernel, (const void*)moe_combine_fp8_kernel,
+                           (const void*)moe_combine_fp8_rows_kernel,    (const void*)moe_combine_fp8_stream_kernel};
   for (const void* k : kernels) {
     cudaError_t e = cudaFuncGetAttributes(&attr, k);
     if (e != cudaSuccess) return (int)e;

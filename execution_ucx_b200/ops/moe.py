@@ -96,7 +96,7 @@ class MoeAllToAll:
         d = self._desc()
         _native.check(_native.load().eux_moe_dispatch_launch(C.byref(d), ctas, C.c_void_p(_native.current_stream_ptr())),
                       "eux_moe_dispatch_launch")
-        _launches += 2
+        _launches += 1
 
     def expert_ready(self) -> None:
         global _launches

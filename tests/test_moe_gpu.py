@@ -115,3 +115,58 @@ def test_combine_pairs_each_row_with_its_own_weight_and_expert(cuda_device, worl
             y = (x * f.unsqueeze(1)).to(torch.bfloat16).float()      # what the expert stored for this (token, k)
             ref += ws[r][:, k].unsqueeze(1) * y
         torch.testing.assert_close(outs[r].float(), ref, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("t,hidden,topk,ne", [(1, 128, 1, 8), (3, 512, 32, 64), (128, 7168, 8, 256), (297, 1152, 6, 16),
+                                              (1000, 7040, 2, 4096), (40, 33024, 4, 8), (4096, 640, 8, 64)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dispatch_routes_in_one_launch(cuda_device, t, hidden, topk, ne, fp8):
+    """One token, a token per CTA, several tokens per CTA, more experts than threads, rows whose scales fill a buffer:
+    every (token, slot) has a row of its own in its expert's group, the row holds the token, and the scratch counters
+    come back zero (a second dispatch, from a captured graph, finds them so). bf16 rows are copies. fp8 rows are within
+    half a step of e4m3 (2^-4 of the value, 2^-10 of the block's largest) and carry a scale of largest / 448."""
+    from execution_ucx_b200.ops import moe
+    a2a = moe.MoeAllToAll.emulated(1, t, hidden, topk, ne, fp8=fp8)[0]
+    g = torch.Generator(device=cuda_device).manual_seed(t + hidden)
+    x = torch.randn(t, hidden, device=cuda_device, generator=g).to(torch.bfloat16)
+    idx = torch.randint(-1 if t > 1 else 0, ne, (t, topk), device=cuda_device, generator=g, dtype=torch.int32)
+    w = torch.rand(t, topk, device=cuda_device, generator=g)
+    for again in range(3):
+        if again == 2:
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                a2a.dispatch(x, idx, w)
+            graph.replay()
+        else:
+            a2a.dispatch(x, idx, w)
+        torch.cuda.synchronize()
+        a2a.check_status()
+        assert int(a2a.counters.abs().sum()) == 0
+        flat, slots = idx.view(-1).long(), a2a.slot_of.long()
+        valid = flat >= 0
+        assert bool((slots[~valid] == -1).all())
+        n = int(valid.sum())
+        assert int(a2a.recv_counts()[0]) == n
+        assert torch.equal(slots[valid].sort().values, torch.arange(n, device=cuda_device))
+        meta = a2a.recv_meta(0, n)[slots[valid]]
+        entry = valid.nonzero().view(-1)
+        assert torch.equal(meta[:, 0].long(), entry // topk)
+        assert torch.equal((meta[:, 1] & 0xffff).long(), entry % topk)
+        assert torch.equal((meta[:, 1] >> 16).long(), flat[valid])
+        assert torch.equal(meta[:, 2].contiguous().view(torch.float32), w.view(-1)[valid])
+        le = a2a.recv_meta(0, n)[:, 1] >> 16
+        assert bool((le[1:] >= le[:-1]).all())
+        rows = a2a.recv_rows(0, n)[slots[valid]]
+        want = x[entry // topk]
+        if not fp8:
+            assert torch.equal(rows.view(torch.bfloat16).view(n, hidden).view(torch.int16), want.view(torch.int16))
+            continue
+        q = rows[:, :hidden].contiguous().view(torch.float8_e4m3fn).double().view(n, hidden // 128, 128)
+        scale = rows[:, hidden:hidden + hidden // 32].contiguous().view(torch.float32).double()
+        blocks = want.double().view(n, hidden // 128, 128)
+        amax = blocks.abs().amax(-1)
+        assert bool(((scale * 448 - amax).abs() <= amax * 1e-6 + 1e-9).all())
+        err = (q * scale.unsqueeze(-1) - blocks).abs()
+        assert bool((err <= blocks.abs() * (2.0 ** -4 + 1e-6) + amax.unsqueeze(-1) * 2.0 ** -10).all())
+        a2a.recv_rows(0, n).zero_()
