@@ -540,6 +540,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const int total = m_blocks * n_blocks;
   const int k_all = p.K * p.elem_bytes / BKB;
   const int rank = SPLIT ? (int)cluster_cta_rank() : 0;
+  const int tile0 = SPLIT ? (int)blockIdx.x / p.split : 0;  // past the last tile: this cluster only helps to copy X
   const int k_begin = SPLIT ? k_all * rank / p.split : 0;  // this CTA's share of K
   const int k_iters = (SPLIT ? k_all * (rank + 1) / p.split : k_all) - k_begin;
   const int kelems = BKB / p.elem_bytes;  // elements of K per stage
@@ -557,7 +558,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       uint32_t ph = 0;
       for (int it = 0;; ++it) {
         int tile;
-        if (SPLIT) tile = it == 0 ? (int)blockIdx.x / p.split : total;  // one tile per cluster
+        if (SPLIT) tile = it == 0 ? tile0 : total;  // one tile per cluster
         else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
@@ -678,10 +679,10 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   tc_fence_before();
   __syncthreads();
-  if (SPLIT) {
+  if (SPLIT && tile0 < total) {
     tc_fence_after();
     int mb, nb;
-    tile_coords((int)blockIdx.x / p.split, m_blocks, n_blocks, p.head_blocks, mb, nb);
+    tile_coords(tile0, m_blocks, n_blocks, p.head_blocks, mb, nb);
     split_sum(p, tmem_base, smem_u32(smem), mb, nb, rank, 0, 1);
     tc_fence_before();
     __syncthreads();
@@ -834,6 +835,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   const int total = m_blocks * n_blocks;
   const int kscales = p.K / 128;
   const int rank = SPLIT ? (int)cluster_cta_rank() : 0;
+  const int tile0 = SPLIT ? (int)blockIdx.x / p.split : 0;  // past the last tile: this cluster only helps to copy X
   const int k_begin = SPLIT ? kscales * rank / p.split : 0;  // this CTA's share of K
   const int k_blocks = (SPLIT ? kscales * (rank + 1) / p.split : kscales) - k_begin;
   volatile int* abort = &s_abort;
@@ -848,7 +850,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       uint32_t ph = 0;
       for (int it = 0;; ++it) {
         int tile;
-        if (SPLIT) tile = it == 0 ? (int)blockIdx.x / p.split : total;  // one tile per cluster
+        if (SPLIT) tile = it == 0 ? tile0 : total;  // one tile per cluster
         else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
@@ -905,7 +907,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     // warps 2 and 3: X (and its scales) from the caller's memory into the staging buffer
     if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
   }
-  if (SPLIT && warp < 4) {  // the two barriers of split_sum_regs count every thread of the cluster
+  if (SPLIT && tile0 < total && warp < 4) {  // the two barriers of split_sum_regs count every thread of the cluster
     __syncwarp();
     cluster_sync_all();
     cluster_sync_all();
@@ -995,7 +997,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         bulk_commit();
       }
     }
-    if (SPLIT) split_sum_regs(p, acc, smem_u32(smem), (int)blockIdx.x / p.split, m_blocks, n_blocks, rank, half, row_local);
+    if (SPLIT && tile0 < total) split_sum_regs(p, acc, smem_u32(smem), tile0, m_blocks, n_blocks, rank, half, row_local);
     if (elected) {  // Y is complete before this CTA reports
       bulk_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");
@@ -1190,6 +1192,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   const int total = m_blocks * n_blocks;
   const int k_all = p.K * p.elem_bytes / BKB;
   const int share = SPLIT ? (int)(even >> 1) : 0;  // this pair's share of K
+  const int tile0 = SPLIT ? (int)blockIdx.x / (2 * p.split) : 0;  // past the last tile: this cluster only helps to copy X
   const int k_begin = SPLIT ? k_all * share / p.split : 0;
   const int k_iters = (SPLIT ? k_all * (share + 1) / p.split : k_all) - k_begin;
   const int kelems = BKB / p.elem_bytes;
@@ -1209,7 +1212,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       for (int it = 0;; ++it) {
         int tile;
         if (leader) {
-          if (SPLIT) tile = it == 0 ? (int)blockIdx.x / (2 * p.split) : total;  // one tile per cluster
+          if (SPLIT) tile = it == 0 ? tile0 : total;  // one tile per cluster
           else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
           const int slot = it & (TILE_RING - 1);
           s_tiles[slot] = tile;
@@ -1398,10 +1401,10 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 
   tc_fence_before();
   __syncthreads();
-  if (SPLIT) {
+  if (SPLIT && tile0 < total) {
     tc_fence_after();
     int mb, nb;
-    tile_coords((int)blockIdx.x / (2 * p.split), m_blocks, n_blocks, p.head_blocks, mb, nb);
+    tile_coords(tile0, m_blocks, n_blocks, p.head_blocks, mb, nb);
     split_sum(p, tmem_base, smem_u32(smem), 2 * mb + (int)rank, nb, share, (int)rank, 2);
     tc_fence_before();
   }
@@ -1791,8 +1794,9 @@ static int launch_clusters(int dev, int cluster, int grid, int threads, size_t s
 
 // Shares of K per tile (1, 2, 4 or 8) for `tiles` clusters of `ctas` CTAs per share: from 24 K steps on, as many as
 // leave eight steps to each while all clusters fit the device at once (asked of the driver, once per device and size).
+// `clusters`: how many of them fit.
 template <auto KERNEL>
-static int choose_split(int dev, int threads, size_t smem, int tiles, int ctas, int k_iters) {
+static int choose_split(int dev, int threads, size_t smem, int tiles, int ctas, int k_iters, int* clusters) {
   static std::atomic<int> resident[64][4];  // 1 + the number of clusters
   int split = 1;
   for (int i = 1; i < 4 && ctas << i <= 8; ++i) {
@@ -1808,7 +1812,7 @@ static int choose_split(int dev, int threads, size_t smem, int tiles, int ctas, 
       }
       resident[dev][i].store(n + 1, std::memory_order_release);
     }
-    if (tiles <= n) split = s;
+    if (tiles <= n) split = s, *clusters = n;
   }
   return split;
 }
@@ -1882,29 +1886,32 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   // (32 tiles) takes 49 us with four CTAs per tile and 72 with one, 128 x 512 x 8192 27 with eight and 59 with one;
   // 384 x 4096 x 1024, sixteen steps, loses 2 us. All clusters have to fit at once: a second wave costs more.
   if (!pull || copy_by_warps) {
+    int clusters = 0;
     if (mx) {
-      const int s = choose_split<remote_gemm_2cta_kernel<true, true>>(dev, GEMM_THREADS, PairCfg<true>::SMEM, tiles2, 2, k_iters);
+      const int s = choose_split<remote_gemm_2cta_kernel<true, true>>(dev, GEMM_THREADS, PairCfg<true>::SMEM, tiles2, 2, k_iters, &clusters);
       if (s > 1) {
+        if (!pull) clusters = tiles2;  // with X to copy, clusters without a tile help with that
         CUtensorMap mb2, msa, msb;
         if (int rc = make_map(&mb2, d->w_t, eb, (uint64_t)d->N, (uint64_t)d->K, BN / 2)) return rc;
         if (int rc = make_map_sf(&msa, p.x_scale_stage, (uint64_t)(d->M / 128) * (d->K / 128), 1)) return rc;
         if (int rc = make_map_sf(&msb, d->w_scale, (uint64_t)(d->N / 128) * (d->K / 128), 2)) return rc;
         p.split = s, p.copy_ctas = 0;
-        p.copy_warps = pull ? 2 * 2 * tiles2 * s : 0;
+        p.copy_warps = pull ? 2 * 2 * clusters * s : 0;
         p.panel_target = pull ? warp_target(p.copy_warps) : 0;
         if (pull && head_arg < 0) p.head_blocks = 2;
-        return launch_clusters<remote_gemm_2cta_kernel<true, true>>(dev, 2 * s, 2 * tiles2 * s, GEMM_THREADS, PairCfg<true>::SMEM, st, ma, mb2,
+        return launch_clusters<remote_gemm_2cta_kernel<true, true>>(dev, 2 * s, 2 * clusters * s, GEMM_THREADS, PairCfg<true>::SMEM, st, ma, mb2,
                                my, msa, msb, p);
       }
     } else {
-      const int s = d->fp8 ? choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters)
-                           : choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, tiles, 1, k_iters);
+      const int s = d->fp8 ? choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters, &clusters)
+                           : choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, tiles, 1, k_iters, &clusters);
       if (s > 1) {
+        if (!pull) clusters = tiles;
         p.split = s, p.copy_ctas = 0;
-        p.copy_warps = pull ? 2 * tiles * s : 0;
+        p.copy_warps = pull ? 2 * clusters * s : 0;
         p.panel_target = pull ? warp_target(p.copy_warps) : 0;
-        if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, tiles * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
-        return launch_clusters<remote_gemm_kernel<true>>(dev, s, tiles * s, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
+        if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, clusters * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
+        return launch_clusters<remote_gemm_kernel<true>>(dev, s, clusters * s, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
       }
     }
   }
