@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent.parent / "_lib" / "libeux_kernels.so"
@@ -71,6 +72,26 @@ class GemmDesc(C.Structure):
     ]
 
 
+# The same layouts for one pack call per launch: setting the fields of a ctypes structure one by one costs more host
+# time than the launch itself. The launch functions take the packed bytes where they take a pointer to the structure.
+XFER_HEAD = struct.Struct("<QQQiiifii")
+XFER_DIMS = struct.Struct("<8q8q")
+XFER_TAIL = struct.Struct("<8Q")
+MOE_DESC = struct.Struct("<8i12Q")
+GEMM_DESC = struct.Struct("<7Q4i6Q2i")
+assert XFER_HEAD.size + XFER_DIMS.size + XFER_TAIL.size == C.sizeof(XferDesc)
+assert MOE_DESC.size == C.sizeof(MoeDesc) and GEMM_DESC.size == C.sizeof(GemmDesc)
+
+
+def descriptor(packer: struct.Struct, cls, *values):
+    """The argument of a launch function: the packed values, or the structure where one of them is None or out of its
+    field's range, which ctypes takes as a null pointer and modulo the field's size."""
+    try:
+        return packer.pack(*values)
+    except (struct.error, OverflowError):
+        return C.byref(cls(*values))
+
+
 def lib_path() -> Path:
     return _LIB_PATH
 
@@ -87,8 +108,8 @@ def load():
         _build.build_kernels()
     lib = C.CDLL(str(_LIB_PATH), mode=C.RTLD_GLOBAL)
     P, I, U64 = C.c_void_p, C.c_int, C.c_uint64
-    lib.eux_xfer_launch.argtypes = [C.POINTER(XferDesc), P, I, P]
-    lib.eux_xfer_bulk_launch.argtypes = [C.POINTER(XferDesc), P, I, P]
+    lib.eux_xfer_launch.argtypes = [P, P, I, P]
+    lib.eux_xfer_bulk_launch.argtypes = [P, P, I, P]
     lib.eux_xfer_rpc_step_launch.argtypes = [C.POINTER(XferDesc), C.POINTER(XferDesc), C.POINTER(XferDesc), P, I, P]
     lib.eux_xfer_batch_launch.argtypes = [P, I, P]
     lib.eux_xfer_pull_batch_launch.argtypes = [C.POINTER(PullItem), I, P]
@@ -106,11 +127,11 @@ def load():
     lib.eux_error_string.restype = C.c_char_p
     lib.eux_moe_row_bytes.argtypes = [I, I]
     lib.eux_moe_row_bytes.restype = C.c_size_t
-    lib.eux_moe_dispatch_launch.argtypes = [C.POINTER(MoeDesc), I, P]
-    lib.eux_moe_expert_ready_launch.argtypes = [C.POINTER(MoeDesc), P]
-    lib.eux_moe_combine_launch.argtypes = [C.POINTER(MoeDesc), I, P]
+    lib.eux_moe_dispatch_launch.argtypes = [P, I, P]
+    lib.eux_moe_expert_ready_launch.argtypes = [P, P]
+    lib.eux_moe_combine_launch.argtypes = [P, I, P]
     if hasattr(lib, "eux_gemm_launch"):
-        lib.eux_gemm_launch.argtypes = [C.POINTER(GemmDesc), P]
+        lib.eux_gemm_launch.argtypes = [P, P]
         lib.eux_gemm_num_sms.argtypes = []
     if hasattr(lib, "eux_gemm_bf16_noalloc"):
         lib.eux_gemm_bf16_noalloc.argtypes = [P, P, P, I, I, I, P, U64, P]
@@ -159,4 +180,4 @@ def torch_dtype_code(dtype) -> int:
 
 def current_stream_ptr() -> int:
     import torch
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

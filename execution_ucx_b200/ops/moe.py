@@ -8,7 +8,6 @@ peer-mapped. ``dispatch`` routes and pushes rows to the expert ranks,
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import List, Optional
 
 import torch
@@ -73,19 +72,14 @@ class MoeAllToAll:
         return [cls(g, n_tokens, hidden, topk, n_experts, fp8, cap, (arenas[r], metas[r], flags[r]), rank=r)
                 for r in range(world)]
 
-    def _desc(self) -> _native.MoeDesc:
-        d = _native.MoeDesc()
-        d.rank, d.world, d.n_tokens, d.hidden = self.rank, self.world, self.n_tokens, self.hidden
-        d.topk, d.n_experts, d.fp8, d.capacity = self.topk, self.n_experts, int(self.fp8), self.capacity
-        d.x = self._x.data_ptr() if self._x is not None else None
-        d.topk_idx = self._idx.data_ptr() if self._idx is not None else None
-        d.topk_w = self._w.data_ptr() if self._w is not None else None
-        d.arena_peer = self.arena.ptr_table.data_ptr()
-        d.meta_peer = self.meta.ptr_table.data_ptr()
-        d.flag_peer = self.flags.ptr_table.data_ptr()
-        d.slot_of, d.counters, d.out = self.slot_of.data_ptr(), self.counters.data_ptr(), self.out.data_ptr()
-        d.seq, d.wait_timeout_ns, d.status = self.seq, 2_000_000_000, self.status.data_ptr()
-        return d
+    def _desc(self):
+        """An ``eux_moe_desc`` of the exchange under way."""
+        x, idx, w = self._x, self._idx, self._w
+        return _native.descriptor(
+            _native.MOE_DESC, _native.MoeDesc, self.rank, self.world, self.n_tokens, self.hidden, self.topk, self.n_experts, int(self.fp8), self.capacity,
+            x.data_ptr() if x is not None else 0, idx.data_ptr() if idx is not None else 0, w.data_ptr() if w is not None else 0,
+            self.arena.ptr_table.data_ptr(), self.meta.ptr_table.data_ptr(), self.flags.ptr_table.data_ptr(),
+            self.slot_of.data_ptr(), self.counters.data_ptr(), self.out.data_ptr(), self.seq, 2_000_000_000, self.status.data_ptr())
 
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, topk_w: torch.Tensor, ctas: int = 0) -> None:
         global _launches
@@ -93,23 +87,23 @@ class MoeAllToAll:
         assert topk_idx.dtype == torch.int32 and topk_w.dtype == torch.float32
         self._x, self._idx, self._w = x, topk_idx.contiguous(), topk_w.contiguous()
         self.seq += 1
-        d = self._desc()
-        _native.check(_native.load().eux_moe_dispatch_launch(C.byref(d), ctas, C.c_void_p(_native.current_stream_ptr())),
-                      "eux_moe_dispatch_launch")
+        rc = _native.load().eux_moe_dispatch_launch(self._desc(), ctas, _native.current_stream_ptr())
+        if rc:
+            _native.check(rc, "eux_moe_dispatch_launch")
         _launches += 1
 
     def expert_ready(self) -> None:
         global _launches
-        d = self._desc()
-        _native.check(_native.load().eux_moe_expert_ready_launch(C.byref(d), C.c_void_p(_native.current_stream_ptr())),
-                      "eux_moe_expert_ready_launch")
+        rc = _native.load().eux_moe_expert_ready_launch(self._desc(), _native.current_stream_ptr())
+        if rc:
+            _native.check(rc, "eux_moe_expert_ready_launch")
         _launches += 1
 
     def combine(self, ctas: int = 0) -> torch.Tensor:
         global _launches
-        d = self._desc()
-        _native.check(_native.load().eux_moe_combine_launch(C.byref(d), ctas, C.c_void_p(_native.current_stream_ptr())),
-                      "eux_moe_combine_launch")
+        rc = _native.load().eux_moe_combine_launch(self._desc(), ctas, _native.current_stream_ptr())
+        if rc:
+            _native.check(rc, "eux_moe_combine_launch")
         _launches += 1
         return self.out
 

@@ -7,7 +7,6 @@ the panels that have arrived) and writes Y into the caller's memory.
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import Optional
 
 import torch
@@ -19,6 +18,19 @@ _launches = 0
 
 def launch_count() -> int:
     return _launches
+
+
+def _launch(what: str, x: int, x_stage: int, w: int, y: int, xs: int, xs_stage: int, ws: int, m: int, n: int, k: int, fp8: int,
+            scratch, done_flag_ptr: int, done_value: int, timeout_ns: int, copy_ctas: int, flags: int) -> None:
+    """One ``eux_gemm_launch`` on the current stream; ``scratch`` holds panel_flags, sched and status."""
+    global _launches
+    desc = _native.descriptor(_native.GEMM_DESC, _native.GemmDesc, x, x_stage, w, y, xs, xs_stage, ws, m, n, k, fp8,
+                              scratch.panel_flags.data_ptr(), scratch.sched.data_ptr(), done_flag_ptr, done_value, timeout_ns,
+                              scratch.status.data_ptr(), copy_ctas, flags)
+    rc = _native.load().eux_gemm_launch(desc, _native.current_stream_ptr())
+    if rc:
+        _native.check(rc, what)
+    _launches += 1
 
 
 class RemoteGemm:
@@ -47,23 +59,13 @@ class RemoteGemm:
         A remote X is copied into the staging buffer by two spare warps of every CTA while the
         other warps compute (``copy_warps``, the default), or, when ``copy_ctas`` > 0 is given, by
         that many CTAs that copy first and compute afterwards."""
-        global _launches
         if m > self.max_m:
             raise ValueError("m exceeds the staging buffer")
-        d = _native.GemmDesc()
-        d.x_src = x_ptr
-        d.x_stage = x_ptr if x_is_local else self.x_stage.data_ptr()
-        d.w_t, d.y_dst = self.w_t.data_ptr(), y_ptr
-        d.M, d.N, d.K, d.fp8 = m, self.N, self.K, 0
-        d.panel_flags, d.sched = self.panel_flags.data_ptr(), self.sched.data_ptr()
-        d.done_flag, d.done_value = done_flag_ptr or None, done_value
-        d.wait_timeout_ns, d.status, d.copy_ctas = timeout_ns, self.status.data_ptr(), copy_ctas
         if copy_warps is None:
             copy_warps = copy_ctas == 0
-        d.flags = (1 if cta_pairs else 0) | (2 if copy_warps else 0) | (0 if head_blocks is None else ((head_blocks + 1) & 0xff) << 8)
-        _native.check(_native.load().eux_gemm_launch(C.byref(d), C.c_void_p(_native.current_stream_ptr())),
-                      "eux_gemm_launch")
-        _launches += 1
+        flags = (1 if cta_pairs else 0) | (2 if copy_warps else 0) | (0 if head_blocks is None else ((head_blocks + 1) & 0xff) << 8)
+        _launch("eux_gemm_launch", x_ptr, x_ptr if x_is_local else self.x_stage.data_ptr(), self.w_t.data_ptr(), y_ptr, 0, 0, 0,
+                m, self.N, self.K, 0, self, done_flag_ptr, done_value, timeout_ns, copy_ctas, flags)
 
     def check_status(self) -> None:
         s = int(self.status.item())
@@ -143,25 +145,14 @@ class RemoteGemmFp8:
     def __call__(self, xq_ptr: int, xs_ptr: int, m: int, y_ptr: int, *, x_is_local: bool, done_flag_ptr: int = 0,
                  done_value: int = 0, copy_ctas: int = 0, timeout_ns: int = 2_000_000_000,
                  copy_warps: Optional[bool] = None, head_blocks: Optional[int] = None) -> None:
-        global _launches
         if m > self.max_m:
             raise ValueError("m exceeds the staging buffer")
-        d = _native.GemmDesc()
         if copy_warps is None:
             copy_warps = copy_ctas == 0
-        d.flags = (2 if copy_warps else 0) | (0 if head_blocks is None else ((head_blocks + 1) & 0xff) << 8)
-        d.x_src = xq_ptr
-        d.x_stage = xq_ptr if x_is_local else self.x_stage.data_ptr()
-        d.x_scale = xs_ptr
-        d.x_scale_stage = xs_ptr if x_is_local else self.x_scale_stage.data_ptr()
-        d.w_t, d.w_scale, d.y_dst = self.w_q_t.data_ptr(), self.w_scale.data_ptr(), y_ptr
-        d.M, d.N, d.K, d.fp8 = m, self.N, self.K, 1
-        d.panel_flags, d.sched = self.panel_flags.data_ptr(), self.sched.data_ptr()
-        d.done_flag, d.done_value = done_flag_ptr or None, done_value
-        d.wait_timeout_ns, d.status, d.copy_ctas = timeout_ns, self.status.data_ptr(), copy_ctas
-        _native.check(_native.load().eux_gemm_launch(C.byref(d), C.c_void_p(_native.current_stream_ptr())),
-                      "eux_gemm_launch(fp8)")
-        _launches += 1
+        flags = (2 if copy_warps else 0) | (0 if head_blocks is None else ((head_blocks + 1) & 0xff) << 8)
+        _launch("eux_gemm_launch(fp8)", xq_ptr, xq_ptr if x_is_local else self.x_stage.data_ptr(), self.w_q_t.data_ptr(), y_ptr, xs_ptr,
+                xs_ptr if x_is_local else self.x_scale_stage.data_ptr(), self.w_scale.data_ptr(), m, self.N, self.K, 1, self,
+                done_flag_ptr, done_value, timeout_ns, copy_ctas, flags)
 
     def check_status(self) -> None:
         s = int(self.status.item())
@@ -221,25 +212,14 @@ class RemoteGemmMx:
     def __call__(self, xq_ptr: int, xs_ptr: int, m: int, y_ptr: int, *, x_is_local: bool, done_flag_ptr: int = 0,
                  done_value: int = 0, copy_ctas: int = 0, timeout_ns: int = 2_000_000_000,
                  copy_warps: Optional[bool] = None, head_blocks: Optional[int] = None) -> None:
-        global _launches
         if m > self.max_m or m % 256:
             raise ValueError("m exceeds the staging buffer or is not a multiple of 256")
-        d = _native.GemmDesc()
         if copy_warps is None:
             copy_warps = copy_ctas == 0
-        d.flags = (2 if copy_warps else 0) | (0 if head_blocks is None else ((head_blocks + 1) & 0xff) << 8)
-        d.x_src = xq_ptr
-        d.x_stage = xq_ptr if x_is_local else self.x_stage.data_ptr()
-        d.x_scale = xs_ptr
-        d.x_scale_stage = xs_ptr if x_is_local else self.x_scale_stage.data_ptr()
-        d.w_t, d.w_scale, d.y_dst = self.w_q_t.data_ptr(), self.w_chunks.data_ptr(), y_ptr
-        d.M, d.N, d.K, d.fp8 = m, self.N, self.K, 2
-        d.panel_flags, d.sched = self.panel_flags.data_ptr(), self.sched.data_ptr()
-        d.done_flag, d.done_value = done_flag_ptr or None, done_value
-        d.wait_timeout_ns, d.status, d.copy_ctas = timeout_ns, self.status.data_ptr(), copy_ctas
-        _native.check(_native.load().eux_gemm_launch(C.byref(d), C.c_void_p(_native.current_stream_ptr())),
-                      "eux_gemm_launch(mx)")
-        _launches += 1
+        flags = (2 if copy_warps else 0) | (0 if head_blocks is None else ((head_blocks + 1) & 0xff) << 8)
+        _launch("eux_gemm_launch(mx)", xq_ptr, xq_ptr if x_is_local else self.x_stage.data_ptr(), self.w_q_t.data_ptr(), y_ptr, xs_ptr,
+                xs_ptr if x_is_local else self.x_scale_stage.data_ptr(), self.w_chunks.data_ptr(), m, self.N, self.K, 2, self,
+                done_flag_ptr, done_value, timeout_ns, copy_ctas, flags)
 
     def check_status(self) -> None:
         s = int(self.status.item())

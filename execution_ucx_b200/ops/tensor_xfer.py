@@ -10,6 +10,7 @@ and ignores strides (rpc_core/utils/tensor_meta.hpp:91-104).
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Optional
 
 import torch
@@ -30,13 +31,16 @@ def _is_dense(t: torch.Tensor) -> bool:
 
 
 _scratch = {}
+_DENSE = bytes(_native.XFER_DIMS.size)
+_PAD = [(0,) * (_native.EUX_MAX_DIMS - n) for n in range(_native.EUX_MAX_DIMS + 1)]
 
 
-def _scratch_counter(device) -> torch.Tensor:
-    key = (device.index, torch.cuda.current_stream().cuda_stream)
-    if key not in _scratch:
-        _scratch[key] = torch.zeros(64, dtype=torch.int32, device=device)
-    return _scratch[key]
+def _scratch_counter(device_index: int, stream: int) -> torch.Tensor:
+    key = (device_index, stream)
+    counter = _scratch.get(key)
+    if counter is None:
+        counter = _scratch[key] = torch.zeros(64, dtype=torch.int32, device=torch.device("cuda", device_index))
+    return counter
 
 
 def make_desc(src: torch.Tensor, dst_ptr: int, dst_dtype: torch.dtype, op: int = OP_NONE, op_arg: float = 0.0,
@@ -85,13 +89,28 @@ def push(src: torch.Tensor, dst, *, dst_dtype: Optional[torch.dtype] = None, op:
     else:
         dst_ptr = int(dst)
         dst_dtype = dst_dtype or src.dtype
-    d = make_desc(src, dst_ptr, dst_dtype, op, op_arg, flag_ptr, flag_value, wait_flag_ptr, wait_value,
-                  wait_timeout_ns, status_ptr)
-    counter = _scratch_counter(src.device)
+    if _is_dense(src):
+        ndim, dims = 0, _DENSE
+    else:
+        ndim = src.dim()
+        if ndim > _native.EUX_MAX_DIMS:
+            raise ValueError("at most 8 dimensions")
+        pad = _PAD[ndim]
+        dims = _native.XFER_DIMS.pack(*src.shape, *pad, *src.stride(), *pad)
+    src_code, dst_code = _native.torch_dtype_code(src.dtype), _native.torch_dtype_code(dst_dtype)
+    try:
+        desc = _native.XFER_HEAD.pack(src.data_ptr(), dst_ptr, src.numel(), src_code, dst_code, op, op_arg, ndim, 0) + dims + \
+            _native.XFER_TAIL.pack(flag_ptr, flag_value, wait_flag_ptr, wait_value, wait_timeout_ns, status_ptr, 0, 0)
+    except (struct.error, OverflowError):  # None, or a number outside its field's range: as ctypes takes them
+        desc = C.byref(make_desc(src, dst_ptr, dst_dtype, op, op_arg, flag_ptr, flag_value, wait_flag_ptr, wait_value,
+                                 wait_timeout_ns, status_ptr))
+    stream = _native.current_stream_ptr()
+    counter = _scratch_counter(src.get_device(), stream)
     lib = _native.load()
     fn = lib.eux_xfer_bulk_launch if bulk else lib.eux_xfer_launch
-    _native.check(fn(C.byref(d), C.c_void_p(counter.data_ptr()), max_ctas,
-                     C.c_void_p(_native.current_stream_ptr())), "eux_xfer_bulk_launch" if bulk else "eux_xfer_launch")
+    rc = fn(desc, counter.data_ptr(), max_ctas, stream)
+    if rc:
+        _native.check(rc, "eux_xfer_bulk_launch" if bulk else "eux_xfer_launch")
     _launches += 1
 
 
@@ -138,9 +157,10 @@ class RpcEchoStep:
         self.resp.flag_value = seq
         self.resp.wait_value = seq
         self.done.wait_value = seq
-        counter = _scratch_counter(self._device)
-        _native.check(self._fn(*self._refs, C.c_void_p(counter.data_ptr() + 16), self._max_ctas,
-                               C.c_void_p(_native.current_stream_ptr())), "eux_xfer_rpc_step_launch")
+        stream = _native.current_stream_ptr()
+        counter = _scratch_counter(self._device.index, stream)
+        _native.check(self._fn(*self._refs, C.c_void_p(counter.data_ptr() + 16), self._max_ctas, C.c_void_p(stream)),
+                      "eux_xfer_rpc_step_launch")
         _launches += 1
 
 
