@@ -151,8 +151,7 @@ __device__ __forceinline__ void moe_publish(const eux_moe_desc& d, const MoeRout
     if (rows > d.capacity) set_status(d.status, EUX_ST_OVERFLOW, 10);
     d.flag_peer[dst][W + d.rank] = (uint64_t)(rows < d.capacity ? rows : d.capacity);
   }
-  __threadfence_system();
-  __syncthreads();
+  __syncthreads();  // the release below covers what the CTA's other threads wrote before this barrier
   for (int dst = threadIdx.x; dst < W; dst += blockDim.x) st_release_sys(&d.flag_peer[dst][d.rank], d.seq);
   if (threadIdx.x < 2) d.counters[W + E + threadIdx.x] = 0;
 }
@@ -324,7 +323,6 @@ __global__ void moe_expert_ready_kernel(eux_moe_desc d) {
   __syncthreads();
   // identity expert: the rows already are the expert output
   if ((int)threadIdx.x < W && s_ok) {
-    __threadfence_system();
     st_release_sys(&d.flag_peer[threadIdx.x][2 * W + d.rank], d.seq);
   }
 }

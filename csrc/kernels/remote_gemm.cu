@@ -380,7 +380,8 @@ __device__ __forceinline__ void copy_warp_role(const GemmParams& p, uint32_t war
 __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   __syncthreads();
   if (threadIdx.x != 0) return;
-  __threadfence_system();
+  if (p.done_flag) __threadfence_system();  // without a flag to publish the end of the launch is enough for Y
+  else __threadfence();
   const uint32_t old = atomicAdd(p.sched, 1u);
   if (old == gridDim.x - 1) {
     const bool all_ok = ok && p.sched[1] == 0;
@@ -392,7 +393,7 @@ __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
     __threadfence_system();
     // done_always: a caller that reads the status word learns of the end of the kernel either way (an RPC
     // handler must answer); otherwise the flag means "Y is complete" and stays silent after a failure
-    if ((all_ok || p.done_always) && p.done_flag) st_release_sys(p.done_flag, p.done_value);
+    if ((all_ok || p.done_always) && p.done_flag) st_relaxed_sys(p.done_flag, p.done_value);
   }
 }
 

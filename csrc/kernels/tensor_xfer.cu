@@ -84,11 +84,11 @@ __device__ __forceinline__ void cta_publish(const eux_xfer_desc& d, uint32_t* co
     if (old & 0x80000000u) ok = false;
     if (last) {
       *counter = 0;  // leave the scratch word clean for the next launch
-      __threadfence();
+      __threadfence_system();  // what the other CTAs wrote before they counted themselves comes before the flags
     }
   }
-  if (last && ok && d.flag) st_release_sys(d.flag, d.flag_value);
-  if (last && ok && d.flag2) st_release_sys(d.flag2, d.flag2_value);
+  if (last && ok && d.flag) st_relaxed_sys(d.flag, d.flag_value);
+  if (last && ok && d.flag2) st_relaxed_sys(d.flag2, d.flag2_value);
 }
 
 // Dense byte copy. A CTA works on one contiguous block at a time and the blocks are dealt
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(256) xfer_batch_kernel(const eux_xfer_desc* de
   __syncthreads();
   if (threadIdx.x == 0 && ok && d.flag) {
     __threadfence_system();
-    st_release_sys(d.flag, d.flag_value);
+    st_relaxed_sys(d.flag, d.flag_value);
   }
 }
 
@@ -1211,8 +1211,8 @@ __global__ void __launch_bounds__(kPullBatchThreads) xfer_pull_batch_kernel(cons
   __syncthreads();
   if (threadIdx.x == 0 && (d.flag || d.flag2)) {
     __threadfence_system();
-    if (d.flag) st_release_sys(d.flag, d.flag_value);
-    if (d.flag2) st_release_sys(d.flag2, d.flag2_value);
+    if (d.flag) st_relaxed_sys(d.flag, d.flag_value);
+    if (d.flag2) st_relaxed_sys(d.flag2, d.flag2_value);
   }
 }
 
