@@ -1391,7 +1391,7 @@ void Worker::fill_gather(eux_xfer_desc* d, const WireLayout& l) {
   if (l.src_dtype != l.dst_dtype) {  // converted on the way (the layout was checked: both are floating-point types of the kernel)
     d->src_dtype = l.src_dtype;
     d->dst_dtype = l.dst_dtype;
-    // a dense row-major source takes the vectorised kernel; anything else the element-wise one
+    // a dense row-major source takes the dense kernel; the launch finds the right one for any other layout
     bool dense = true;
     int64_t expect = 1;
     for (int i = l.ndim - 1; i >= 0 && dense; --i) {

@@ -708,8 +708,11 @@ static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return EUX_ERR_BAD_ARG;
   if (int rc = moe_resident_ctas<KERNEL>(dev, smem, &resident)) return rc;
-  // two CTAs per SM where there are tokens for them
-  if (ctas <= 0) ctas = 296;
+  // One CTA per SM, half of what fits: as fast as two (4096 x 7168, exchange: 209 us against 211), and a kernel of another
+  // stream that holds SMs while it waits for a peer does not keep this launch, and the peer, waiting.
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (ctas <= 0) ctas = sms;
   if (ctas > resident) ctas = resident;
   int per = (d->n_tokens + ctas - 1) / ctas;
   if (per < 1) per = 1;

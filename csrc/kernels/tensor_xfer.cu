@@ -1113,7 +1113,10 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     if (!ctas_given) max_ctas = !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;
     const uint64_t per_cta = (uint64_t)kXferThreads * chunk;
     grid = limit(tiled ? t.tiles : (a.d.n_elems + per_cta - 1) / per_cta);
-    if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
+    if (!scratch_counter) {  // up to 2048 elements, or when told to, one CTA does without
+      if (d->n_elems > (uint64_t)kXferThreads * 4 && max_ctas > 1) return EUX_ERR_BAD_ARG;
+      grid = 1;
+    }
     const TileArgs* tp = tiled ? &t : nullptr;
     GatherArgs ga{a, {}, a.d.n_elems >> 32 == 0};
     for (int k = 0; k < a.d.ndim; ++k) {
