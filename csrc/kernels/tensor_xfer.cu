@@ -335,10 +335,11 @@ __global__ void __launch_bounds__(kXferThreads) xfer_rpc_step_kernel(RpcStepArgs
 
 // ---- gathers ---------------------------------------------------------------------------------------
 // What the layout is, eux_xfer_launch finds out on the host (size-1 dimensions dropped, dimensions that are
-// contiguous with one another merged) and picks one of two kernels:
+// contiguous with one another merged) and picks one of three kernels:
 //   * xfer_gather_kernel: the elements of the innermost dimension are next to one another in the source (row
 //     slices, permuted outer dimensions, dense tensors at any offset), or no dimension has stride 1;
-//   * xfer_tile_kernel: some other dimension has stride 1 (transposes): tiles through shared memory.
+//   * xfer_tile_kernel: some other dimension has stride 1 (transposes): tiles through shared memory;
+//   * xfer_element_kernel: rows of a few elements, and tensors of a few thousand.
 
 __device__ __forceinline__ uint64_t div_u64(uint64_t a, uint64_t b) {
   if (((a | b) >> 32) == 0) return (uint32_t)a / (uint32_t)b;  // most tensors; a 64-bit division costs several times as much
@@ -489,6 +490,43 @@ __global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_
       uint64_t c;
       const int64_t row = gather_row(a, e, c);
       dst[e] = Convert<S, D, RAW>::one(src[row + (int64_t)c * inner], op, arg);
+    }
+  }
+  cta_publish(d, a.x.counter, ok);
+}
+
+// Small tensors (a step for every thread of the device, or less), and single bytes in rows of less than a chunk: one
+// element per thread at a time, four in flight, neighbouring threads on neighbouring elements. Bound by one trip to memory
+// and by the index arithmetic; the chunked kernel's unrolled row crossings are long, cold code to a launch that runs them
+// once (1000 matrices of 3 x 3 bytes, transposed: 12.5 us in chunks, 4.1 here; with a 64-bit division per dimension, as
+// every strided element once had, 7.0).
+template <typename S, typename D, bool RAW>
+__global__ void __launch_bounds__(kXferThreads) xfer_element_kernel(const __grid_constant__ GatherArgs a) {
+  const eux_xfer_desc& d = a.x.d;
+  const bool ok = cta_wait_arrival(d);
+  if (ok) {
+    constexpr int U = 4;
+    const S* src = reinterpret_cast<const S*>(d.src);
+    D* dst = reinterpret_cast<D*>(d.dst);
+    const uint64_t n = d.n_elems;
+    const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
+    const int64_t inner = d.stride[d.ndim - 1];
+    const int op = d.op;
+    const float arg = d.op_arg;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * nthreads) {
+      S v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (i0 + u * nthreads >= n) break;
+        uint64_t col;
+        const int64_t row = gather_row(a, i0 + u * nthreads, col);
+        v[u] = src[row + (int64_t)col * inner];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (i0 + u * nthreads >= n) break;
+        dst[i0 + u * nthreads] = Convert<S, D, RAW>::one(v[u], op, arg);
+      }
     }
   }
   cta_publish(d, a.x.counter, ok);
@@ -964,21 +1002,26 @@ static FastDiv fast_div(uint32_t d) {
   return f;
 }
 
+enum class Route { kElement, kGather, kGatherAligned, kTile, kTileVector, kNarrow };
+
 template <typename S, typename D, bool RAW>
-static void launch_gather(const GatherArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
-  if (!t && vector) xfer_gather_kernel<S, D, RAW, true><<<grid, kXferThreads, 0, st>>>(a);
-  else if (!t) xfer_gather_kernel<S, D, RAW, false><<<grid, kXferThreads, 0, st>>>(a);
-  else if (t->narrow) xfer_narrow_kernel<S, D, RAW><<<grid, kTileThreads, 0, st>>>(*t);
-  else if (vector) xfer_tile_kernel<S, D, RAW, true><<<grid, kTileThreads, 0, st>>>(*t);
-  else xfer_tile_kernel<S, D, RAW, false><<<grid, kTileThreads, 0, st>>>(*t);
+static void launch_gather(const GatherArgs& a, const TileArgs& t, Route route, int grid, cudaStream_t st) {
+  switch (route) {
+    case Route::kElement: xfer_element_kernel<S, D, RAW><<<grid, kXferThreads, 0, st>>>(a); break;
+    case Route::kGather: xfer_gather_kernel<S, D, RAW, false><<<grid, kXferThreads, 0, st>>>(a); break;
+    case Route::kGatherAligned: xfer_gather_kernel<S, D, RAW, true><<<grid, kXferThreads, 0, st>>>(a); break;
+    case Route::kTile: xfer_tile_kernel<S, D, RAW, false><<<grid, kTileThreads, 0, st>>>(t); break;
+    case Route::kTileVector: xfer_tile_kernel<S, D, RAW, true><<<grid, kTileThreads, 0, st>>>(t); break;
+    case Route::kNarrow: xfer_narrow_kernel<S, D, RAW><<<grid, kTileThreads, 0, st>>>(t); break;
+  }
 }
 template <typename S>
-static int launch_gather_from(const GatherArgs& a, const TileArgs* t, bool vector, int grid, cudaStream_t st) {
+static int launch_gather_from(const GatherArgs& a, const TileArgs& t, Route route, int grid, cudaStream_t st) {
   switch (a.x.d.dst_dtype) {
-    case EUX_DT_F32: launch_gather<S, float, false>(a, t, vector, grid, st); break;
-    case EUX_DT_F16: launch_gather<S, __half, false>(a, t, vector, grid, st); break;
-    case EUX_DT_BF16: launch_gather<S, __nv_bfloat16, false>(a, t, vector, grid, st); break;
-    case EUX_DT_F8E4M3: launch_gather<S, __nv_fp8_e4m3, false>(a, t, vector, grid, st); break;
+    case EUX_DT_F32: launch_gather<S, float, false>(a, t, route, grid, st); break;
+    case EUX_DT_F16: launch_gather<S, __half, false>(a, t, route, grid, st); break;
+    case EUX_DT_BF16: launch_gather<S, __nv_bfloat16, false>(a, t, route, grid, st); break;
+    case EUX_DT_F8E4M3: launch_gather<S, __nv_fp8_e4m3, false>(a, t, route, grid, st); break;
     default: return EUX_ERR_BAD_ARG;
   }
   return 0;
@@ -1038,7 +1081,9 @@ static bool plan_tiles(const eux_xfer_desc& d, TileArgs& t, bool& vector) {
   }
   t.tiles = batch * t.tiles_p * t.tiles_q;
   t.vector_store = store16;
-  return true;
+  // A tile costs a CTA two barriers and its index set-up however small it is. In tiles and in chunks, bf16: 2^20 matrices of
+  // 3 x 3 2821 and 45 us, 2^14 of 32 x 32 52 and 25, 2^12 of 64 x 64 21 and 25 (fp32: 60 and 45, 25 and 50).
+  return batch == 1 || (uint64_t)t.np * t.nq >= 1280;
 }
 
 // Whether every chunk of `chunk` elements is one aligned load of the source and one aligned store.
@@ -1104,20 +1149,27 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
       if (a.d.shape[k] < 1 && a.d.n_elems) return EUX_ERR_BAD_ARG;
     TileArgs t;
     bool vector = false;
-    const bool tiled = whole && !as_bytes && plan_tiles(a.d, t, vector);
-    if (tiled) t.x = a;
     const int chunk = raw ? 16 / (as_bytes ? 1 : dsz) : 8;  // elements per chunk of the gather kernel
-    if (!tiled) vector = !as_bytes && rows_aligned(a.d, whole, chunk, ssz, dsz);
+    const bool few = a.d.n_elems <= (uint64_t)sms * 2048;   // less than a step of four elements for every thread of the device
+    Route route = Route::kElement;
+    if (whole && !as_bytes && plan_tiles(a.d, t, vector) && (vector || !few)) {
+      route = t.narrow ? Route::kNarrow : vector ? Route::kTileVector : Route::kTile;
+      t.x = a;
+    } else if (!as_bytes && rows_aligned(a.d, whole, chunk, ssz, dsz)) {
+      route = Route::kGatherAligned;
+    } else if (as_bytes || !(few || (ssz * dsz == 1 && a.d.ndim > 2 && a.d.shape[a.d.ndim - 1] < chunk))) {
+      route = Route::kGather;
+    }
+    const bool tiled = route >= Route::kTile;
     // Four gather CTAs fill an SM's threads. Tiles: a CTA each, whose loads then overlap other CTAs' stores (55 us against
     // 60 on 8192 x 8192 bf16), or eight CTAs per SM where each one also has a flag's counter to go through.
     if (!ctas_given) max_ctas = !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;
-    const uint64_t per_cta = (uint64_t)kXferThreads * chunk;
+    const uint64_t per_cta = (uint64_t)kXferThreads * (route == Route::kElement ? 2 : chunk);
     grid = limit(tiled ? t.tiles : (a.d.n_elems + per_cta - 1) / per_cta);
     if (!scratch_counter) {  // up to 2048 elements, or when told to, one CTA does without
       if (d->n_elems > (uint64_t)kXferThreads * 4 && max_ctas > 1) return EUX_ERR_BAD_ARG;
       grid = 1;
     }
-    const TileArgs* tp = tiled ? &t : nullptr;
     GatherArgs ga{a, {}, a.d.n_elems >> 32 == 0};
     for (int k = 0; k < a.d.ndim; ++k) {
       if (a.d.shape[k] >> 32) ga.small = 0;
@@ -1126,15 +1178,15 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     int rc = 0;
     if (raw) {
       const int esz = as_bytes ? 1 : ssz;
-      if (esz == 4) launch_gather<uint32_t, uint32_t, true>(ga, tp, vector, grid, st);
-      else if (esz == 2) launch_gather<uint16_t, uint16_t, true>(ga, tp, vector, grid, st);
-      else launch_gather<uint8_t, uint8_t, true>(ga, tp, vector, grid, st);
+      if (esz == 4) launch_gather<uint32_t, uint32_t, true>(ga, t, route, grid, st);
+      else if (esz == 2) launch_gather<uint16_t, uint16_t, true>(ga, t, route, grid, st);
+      else launch_gather<uint8_t, uint8_t, true>(ga, t, route, grid, st);
     } else {
       switch (d->src_dtype) {
-        case EUX_DT_F32: rc = launch_gather_from<float>(ga, tp, vector, grid, st); break;
-        case EUX_DT_F16: rc = launch_gather_from<__half>(ga, tp, vector, grid, st); break;
-        case EUX_DT_BF16: rc = launch_gather_from<__nv_bfloat16>(ga, tp, vector, grid, st); break;
-        case EUX_DT_F8E4M3: rc = launch_gather_from<__nv_fp8_e4m3>(ga, tp, vector, grid, st); break;
+        case EUX_DT_F32: rc = launch_gather_from<float>(ga, t, route, grid, st); break;
+        case EUX_DT_F16: rc = launch_gather_from<__half>(ga, t, route, grid, st); break;
+        case EUX_DT_BF16: rc = launch_gather_from<__nv_bfloat16>(ga, t, route, grid, st); break;
+        case EUX_DT_F8E4M3: rc = launch_gather_from<__nv_fp8_e4m3>(ga, t, route, grid, st); break;
         default: rc = EUX_ERR_BAD_ARG;
       }
     }
@@ -1319,7 +1371,8 @@ int preload_one(K kernel) {
 }
 template <typename S, typename D, bool RAW>
 int preload_gather() {
-  int rc = preload_one(xfer_gather_kernel<S, D, RAW, true>);
+  int rc = preload_one(xfer_element_kernel<S, D, RAW>);
+  if (!rc) rc = preload_one(xfer_gather_kernel<S, D, RAW, true>);
   if (!rc) rc = preload_one(xfer_gather_kernel<S, D, RAW, false>);
   if (!rc) rc = preload_one(xfer_narrow_kernel<S, D, RAW>);
   if (!rc) rc = preload_one(xfer_tile_kernel<S, D, RAW, true>);

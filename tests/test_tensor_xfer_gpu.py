@@ -118,6 +118,40 @@ def test_gather_layouts(cuda_device, src_dtype, dst_dtype, op, shift):
         assert int(flag[0]) == i + 1, name
 
 
+def _push_us(view, dst, times=8):
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    best = []
+    for _ in range(times):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        tx.push(view, dst)
+        b.record()
+        torch.cuda.synchronize()
+        best.append(a.elapsed_time(b) * 1e3)
+    return min(best)
+
+
+@pytest.mark.parametrize("b,p,q", [(1 << 18, 3, 3), (1 << 17, 2, 8), (1 << 15, 16, 16), (20000, 7, 9), (1000, 56, 48), (999, 65, 33), (3000, 4, 128),
+                                   (40, 96, 4), (7, 5, 3)])
+@pytest.mark.parametrize("src_dtype,dst_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.uint8, torch.uint8),
+                                                 (torch.float32, torch.float8_e4m3fn), (torch.bfloat16, torch.float32)])
+def test_batches_of_small_transposes(cuda_device, b, p, q, src_dtype, dst_dtype):
+    """Every size below and above the tile kernel's smallest tile and the element kernel's largest tensor. Values are
+    equal to torch's, and no batch of small matrices costs many times a dense push of as many elements, as it does with
+    a CTA per matrix (2^18 matrices of 3 x 3: 700 us against 10). Five times, and a launch's 20 us, are allowed."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    g = torch.Generator(device=cuda_device).manual_seed(b + p + q)
+    x = torch.randint(0, 200, (b, p, q), device=cuda_device, generator=g).to(src_dtype)
+    view = x.mT
+    buf = torch.full((x.numel() + 32,), 9.0, device=cuda_device).to(dst_dtype)
+    dst = buf[16:16 + x.numel()]
+    tx.push(view, dst)
+    torch.cuda.synchronize()
+    assert torch.equal(dst.float(), view.contiguous().view(-1).to(dst_dtype).float())
+    assert bool((buf[:16].float() == 9).all()) and bool((buf[16 + x.numel():].float() == 9).all())
+    assert _push_us(view, dst) < 5 * _push_us(x, dst) + 20
+
+
 def test_batch(cuda_device):
     from execution_ucx_b200.ops import tensor_xfer as tx
     g = torch.Generator(device="cpu").manual_seed(3)
