@@ -1123,7 +1123,9 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     else xfer_bytes_kernel<false><<<grid, kXferThreads, 0, st>>>(a);
   } else if (a.d.ndim == 0 && d->src_dtype != EUX_DT_BYTES && (al & 15u) == 0) {
     // two CTAs per SM carry enough bytes when the source is fp32 (31 us against 33 with four), narrower ones take four
-    if (!ctas_given) max_ctas = (ssz == 4 ? 2 : 4) * sms;
+    // (narrow sources have 32 registers, fp32 ones up to 58). One that waits for its arrival keeps to half of an SM: kernels
+    // of other streams, the one that it waits for perhaps among them, find room.
+    if (!ctas_given) max_ctas = (d->wait_flag ? 1 : 2) * (ssz == 4 ? 1 : 2) * sms;
     grid = limit((d->n_elems / 8 + kXferThreads - 1) / kXferThreads);
     if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
     int rc = 0;
@@ -1163,7 +1165,9 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     const bool tiled = route >= Route::kTile;
     // Four gather CTAs fill an SM's threads. Tiles: a CTA each, whose loads then overlap other CTAs' stores (55 us against
     // 60 on 8192 x 8192 bf16), or eight CTAs per SM where each one also has a flag's counter to go through.
-    if (!ctas_given) max_ctas = !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;
+    // One that waits keeps to half of an SM (gathers have 64 registers and 512 threads), and all its CTAs wait at once, so
+    // that a limit passes once.
+    if (!ctas_given) max_ctas = d->wait_flag ? (tiled ? 2 : 1) * sms : !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;
     const uint64_t per_cta = (uint64_t)kXferThreads * (route == Route::kElement ? 2 : chunk);
     grid = limit(tiled ? t.tiles : (a.d.n_elems + per_cta - 1) / per_cta);
     if (!scratch_counter) {  // up to 2048 elements, or when told to, one CTA does without

@@ -152,6 +152,35 @@ def test_batches_of_small_transposes(cuda_device, b, p, q, src_dtype, dst_dtype)
     assert _push_us(view, dst) < 5 * _push_us(x, dst) + 20
 
 
+@pytest.mark.parametrize("layout", ["dense", "rows", "transposed"])
+def test_a_waiting_push_leaves_room(cuda_device, layout):
+    """A push of 2^26 elements waits for an arrival that never comes: it gives up after one limit, however many tiles it
+    has, and a small conversion on another stream runs meanwhile."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    x = torch.zeros(8192, 8192 + 8, dtype=torch.bfloat16, device=cuda_device)
+    view = {"dense": x.view(-1)[:1 << 26], "rows": x[:, 1:8193], "transposed": x[:, :8192].t()}[layout]
+    dst = torch.empty(view.numel(), dtype=torch.float32 if layout == "dense" else torch.bfloat16, device=cuda_device)
+    small, small_dst = torch.ones(4096, dtype=torch.bfloat16, device=cuda_device), torch.zeros(4096, device=cuda_device)
+    flag = torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    other = torch.cuda.Stream()
+    with torch.cuda.stream(other):
+        tx.push(small, small_dst)
+        small_dst.zero_()
+    tx.push(view, dst)
+    torch.cuda.synchronize()
+    begin, end, gave_up = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    begin.record()
+    tx.push(view, dst, wait_flag_ptr=flag.data_ptr(), wait_value=1, wait_timeout_ns=200_000_000, status_ptr=status.data_ptr())
+    gave_up.record()
+    with torch.cuda.stream(other):
+        tx.push(small, small_dst)
+        end.record()
+    torch.cuda.synchronize()
+    assert int(status) != 0 and 150 < begin.elapsed_time(gave_up) < 350
+    assert begin.elapsed_time(end) < 100 and torch.equal(small.float(), small_dst)
+
+
 def test_batch(cuda_device):
     from execution_ucx_b200.ops import tensor_xfer as tx
     g = torch.Generator(device="cpu").manual_seed(3)
