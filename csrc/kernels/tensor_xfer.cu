@@ -43,6 +43,11 @@ struct Elem<__nv_fp8_e4m3> {
   static __device__ __forceinline__ __nv_fp8_e4m3 from(float f) { return __nv_fp8_e4m3(f); }
 };
 
+template <>
+struct Elem<uint8_t> {
+  static __device__ __forceinline__ uint8_t from(float f) { return (uint8_t)f; }
+};
+
 template <int BYTES>
 struct PackT;
 template <>
@@ -1022,6 +1027,7 @@ static int launch_gather_from(const GatherArgs& a, const TileArgs& t, Route rout
     case EUX_DT_F16: launch_gather<S, __half, false>(a, t, route, grid, st); break;
     case EUX_DT_BF16: launch_gather<S, __nv_bfloat16, false>(a, t, route, grid, st); break;
     case EUX_DT_F8E4M3: launch_gather<S, __nv_fp8_e4m3, false>(a, t, route, grid, st); break;
+    case EUX_DT_BYTES: xfer_element_kernel<S, uint8_t, false><<<grid, kXferThreads, 0, st>>>(a); break;  // truncated
     default: return EUX_ERR_BAD_ARG;
   }
   return 0;
@@ -1113,6 +1119,8 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
   const int ssz = dtype_size(d->src_dtype), dsz = dtype_size(d->dst_dtype);
   const uintptr_t al = ((uintptr_t)d->src) | ((uintptr_t)d->dst);
   auto limit = [&](uint64_t want) { return (int)(want < 1 ? 1 : (want > (uint64_t)max_ctas ? max_ctas : want)); };
+  // Floating-point elements as bytes: an unaligned source or one described by a layout is taken, an aligned dense one is not.
+  const bool to_bytes = d->dst_dtype == EUX_DT_BYTES && !raw;
   int grid;
   if (a.d.ndim == 0 && raw && (al & 15u) == 0) {
     // 64 B per thread per step, one CTA per SM; small messages stay on one CTA (no counter traffic)
@@ -1121,7 +1129,7 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     if (grid > 1 && !scratch_counter) return EUX_ERR_BAD_ARG;
     if ((al & 31u) == 0) xfer_bytes_kernel<true><<<grid, kXferThreads, 0, st>>>(a);
     else xfer_bytes_kernel<false><<<grid, kXferThreads, 0, st>>>(a);
-  } else if (a.d.ndim == 0 && d->src_dtype != EUX_DT_BYTES && (al & 15u) == 0) {
+  } else if (a.d.ndim == 0 && d->src_dtype != EUX_DT_BYTES && (al & 15u) == 0 && !(to_bytes && d->ndim > 0)) {
     // two CTAs per SM carry enough bytes when the source is fp32 (31 us against 33 with four), narrower ones take four
     // (narrow sources have 32 registers, fp32 ones up to 58). One that waits for its arrival keeps to half of an SM: kernels
     // of other streams, the one that it waits for perhaps among them, find room.
@@ -1154,7 +1162,9 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     const int chunk = raw ? 16 / (as_bytes ? 1 : dsz) : 8;  // elements per chunk of the gather kernel
     const bool few = a.d.n_elems <= (uint64_t)sms * 2048;   // less than a step of four elements for every thread of the device
     Route route = Route::kElement;
-    if (whole && !as_bytes && plan_tiles(a.d, t, vector) && (vector || !few)) {
+    if (to_bytes) {
+      // one kernel
+    } else if (whole && !as_bytes && plan_tiles(a.d, t, vector) && (vector || !few)) {
       route = t.narrow ? Route::kNarrow : vector ? Route::kTileVector : Route::kTile;
       t.x = a;
     } else if (!as_bytes && rows_aligned(a.d, whole, chunk, ssz, dsz)) {
@@ -1390,6 +1400,7 @@ int preload_typed() {
   if (!rc) rc = preload_one(xfer_typed_kernel<S, __nv_bfloat16>);
   if (!rc) rc = preload_one(xfer_typed_kernel<S, __nv_fp8_e4m3>);
   if (!rc) rc = preload_one(xfer_rpc_step_kernel<S>);
+  if (!rc) rc = preload_one(xfer_element_kernel<S, uint8_t, false>);
   if (!rc) rc = preload_gather<S, float, false>();
   if (!rc) rc = preload_gather<S, __half, false>();
   if (!rc) rc = preload_gather<S, __nv_bfloat16, false>();

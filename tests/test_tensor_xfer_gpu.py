@@ -181,6 +181,39 @@ def test_a_waiting_push_leaves_room(cuda_device, layout):
     assert begin.elapsed_time(end) < 100 and torch.equal(small.float(), small_dst)
 
 
+def _launch(src_ptr, dst_ptr, n, src_dtype, dst_dtype, shape=(), stride=(), counter=0, max_ctas=0):
+    import ctypes as C
+    from execution_ucx_b200.ops import _native
+    d = _native.XferDesc()
+    d.src, d.dst, d.n_elems = src_ptr, dst_ptr, n
+    d.src_dtype, d.dst_dtype = _native.torch_dtype_code(src_dtype), _native.torch_dtype_code(dst_dtype)
+    d.ndim = len(shape)
+    for i in range(len(shape)):
+        d.shape[i], d.stride[i] = shape[i], stride[i]
+    rc = _native.load().eux_xfer_launch(C.byref(d), counter or None, max_ctas, _native.current_stream_ptr())
+    torch.cuda.synchronize()
+    return rc
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16, torch.float8_e4m3fn])
+def test_floating_point_to_bytes(cuda_device, dtype):
+    """Truncated, from a source that is unaligned or described by a layout (a dense one among them); an aligned dense
+    source without a layout has always been refused."""
+    g = torch.Generator(device=cuda_device).manual_seed(1)
+    x = (torch.rand(101, 203, device=cuda_device, generator=g) * 250).to(dtype)
+    counter = torch.zeros(4, dtype=torch.int32, device=cuda_device)
+    esz = x.element_size()
+    for view in (x.t(), x[:, 3:77], x[1:, 1:2], x, x.view(-1)[1:]):
+        n = view.numel()
+        dst = torch.full((n + 8,), 251, dtype=torch.uint8, device=cuda_device)
+        shape, stride = (view.shape, view.stride()) if view.dim() > 1 else ((), ())
+        assert _launch(view.data_ptr(), dst.data_ptr(), n, dtype, torch.uint8, shape, stride, counter.data_ptr()) == 0
+        assert torch.equal(dst[:n], view.contiguous().view(-1).float().to(torch.uint8)) and bool((dst[n:] == 251).all())
+    dst = torch.empty(x.numel(), dtype=torch.uint8, device=cuda_device)
+    assert _launch(x.data_ptr(), dst.data_ptr(), x.numel(), dtype, torch.uint8, counter=counter.data_ptr()) == 100001
+    assert esz * x.numel() > 0 and int(counter.abs().sum()) == 0
+
+
 def test_batch(cuda_device):
     from execution_ucx_b200.ops import tensor_xfer as tx
     g = torch.Generator(device="cpu").manual_seed(3)
