@@ -1121,6 +1121,7 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
   auto limit = [&](uint64_t want) { return (int)(want < 1 ? 1 : (want > (uint64_t)max_ctas ? max_ctas : want)); };
   // Floating-point elements as bytes: an unaligned source or one described by a layout is taken, an aligned dense one is not.
   const bool to_bytes = d->dst_dtype == EUX_DT_BYTES && !raw;
+  if (d->ndim > 0 && !scratch_counter && d->n_elems > (uint64_t)kXferThreads * 4 && max_ctas > 1) return EUX_ERR_BAD_ARG;
   int grid;
   if (a.d.ndim == 0 && raw && (al & 15u) == 0) {
     // 64 B per thread per step, one CTA per SM; small messages stay on one CTA (no counter traffic)
@@ -1154,7 +1155,7 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
       a.d.shape[0] = a.d.n_elems ? (int64_t)a.d.n_elems : 1;
       a.d.stride[0] = 1;
     }
-    if (!as_bytes && (((uintptr_t)d->src % ssz) || ((uintptr_t)d->dst % dsz))) return EUX_ERR_BAD_ARG;  // would fault
+    if (!as_bytes && d->n_elems && (((uintptr_t)d->src % ssz) || ((uintptr_t)d->dst % dsz))) return EUX_ERR_BAD_ARG;  // would fault
     for (int k = 0; k < a.d.ndim; ++k)
       if (a.d.shape[k] < 1 && a.d.n_elems) return EUX_ERR_BAD_ARG;
     TileArgs t;

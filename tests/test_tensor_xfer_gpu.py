@@ -214,6 +214,21 @@ def test_floating_point_to_bytes(cuda_device, dtype):
     assert esz * x.numel() > 0 and int(counter.abs().sum()) == 0
 
 
+def test_what_a_launch_refuses(cuda_device):
+    """Without a counter a layout may have 2048 elements, or more on one CTA, dense as it may be. Nothing to move is no
+    error, wherever it lies."""
+    f32 = torch.float32
+    x, y = torch.randn(64, 128, device=cuda_device), torch.zeros(64, 128, device=cuda_device)
+    for n, shape in ((2048, (16, 128)), (8192, (64, 128))):
+        for stride in ((128, 1), (1, shape[0])):
+            args = (x.data_ptr(), y.data_ptr(), n, f32, f32, shape, stride)
+            assert _launch(*args) == (0 if n == 2048 else 100001)
+            assert _launch(*args, max_ctas=1) == 0
+            assert torch.equal(y.view(-1)[:n], torch.as_strided(x, shape, stride).reshape(-1))
+    assert _launch(x.data_ptr() + 1, y.data_ptr(), 0, f32, f32, (0, 3), (1, 7)) == 0
+    assert _launch(x.data_ptr() + 1, y.data_ptr(), 0, f32, torch.bfloat16) == 0
+
+
 def test_batch(cuda_device):
     from execution_ucx_b200.ops import tensor_xfer as tx
     g = torch.Generator(device="cpu").manual_seed(3)
