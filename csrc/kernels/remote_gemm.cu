@@ -16,7 +16,8 @@
 //
 // Every wait is bounded: when one runs out the CTA raises an abort flag, stops
 // issuing work, lets its copies land, frees its TMEM and returns with
-// EUX_ST_TIMEOUT in the status word.
+// EUX_ST_TIMEOUT in the status word. (The cluster barriers have no limit: every
+// role comes to them once its own waits have ended.)
 #include <cuda.h>
 
 #include <atomic>
@@ -411,15 +412,23 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// One thread of a CTA that gave up: the other CTAs of the cluster of `n` learn of it.
+__device__ __forceinline__ void split_spread_abort(int* s_abort, uint32_t n) {
+  if (!*(volatile int*)s_abort) return;
+  for (uint32_t r = 0; r < n; ++r)
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32(s_abort), r)), "r"(1u) : "memory");
+}
 // The sum over a cluster whose CTAs have each computed a share of K of one 128 x 256 tile: CTA r owns 256 / split of
 // the columns, every CTA stores its partial sums (fp32) of the other owners' columns into their shared memory, and the
 // owner adds them up in the order of the ranks and writes its part of Y. All pipeline stages are idle by then: the
-// first cluster barrier comes after every CTA's last MMA. All eight warps take part; a thread handles one row.
+// first cluster barrier comes after every CTA's last MMA. All eight warps take part; a thread handles one row. A CTA
+// that gave up says so to all others between the two barriers, and none of them writes: as in the unsplit kernels, Y
+// stays as it was where a wait ran out.
 // Layout of a part: 16 bytes (four columns) of one row next to the same columns of the next row.
 // `rank` counts the shares of K; the CTA that has another share of the same rows is `stride` cluster ranks per share
 // further on from `first`. (mb, nb): the tile in blocks of 128 rows and 256 columns.
 __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_base, uint32_t smem0, int mb, int nb, int rank,
-                                          int first, int stride) {
+                                          int first, int stride, int* s_abort) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lg = warp & 3, side = warp >> 2;
   const int row = lg * 32 + lane;
@@ -429,6 +438,8 @@ __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_bas
   const uint32_t mine = smem0 + (uint32_t)row * 16u + (uint32_t)(side * half / 4) * (BM * 16u);
   __syncwarp();
   cluster_sync_all();
+  if (threadIdx.x == 0) split_spread_abort(s_abort, (uint32_t)(p.split * stride));
+  __syncwarp();
   for (int d = 1; d < p.split; ++d) {
     const int owner = (rank + d) % p.split;  // each CTA starts with another one
     const uint32_t slot = (uint32_t)(rank < owner ? rank : rank - 1);
@@ -446,6 +457,7 @@ __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_bas
   }
   __syncwarp();
   cluster_sync_all();
+  if (*(volatile int*)s_abort) return;
   unsigned char* out = p.y + ((size_t)(mb * BM + row) * p.N + (size_t)nb * BN + rank * width + side * half) * 2;
   for (int c = 0; c < half; c += 16) {
     uint32_t own[16];
@@ -611,6 +623,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           umma_commit(empty_bar(s));
           if (++s == STAGES) s = 0, ph ^= 1u;
         }
+        if (*abort) break;  // a tile that is not complete is not announced
         umma_commit(tfull_bar(buf));
       }
     }
@@ -684,7 +697,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     tc_fence_after();
     int mb, nb;
     tile_coords(tile0, m_blocks, n_blocks, p.head_blocks, mb, nb);
-    split_sum(p, tmem_base, smem_u32(smem), mb, nb, rank, 0, 1);
+    split_sum(p, tmem_base, smem_u32(smem), mb, nb, rank, 0, 1, &s_abort);
     tc_fence_before();
     __syncthreads();
   }
@@ -722,11 +735,13 @@ constexpr size_t GEMM8_SMEM = (size_t)STAGES8 * (A8_STAGE_BYTES + B8_STAGE_BYTES
 // split_sum for the block-scaled fp8 kernel, whose epilogue warps hold their sums in registers: thread (row, half) has
 // the 64 columns of its half of a 128 x 128 tile. Called by the epilogue warps; the others join the two barriers.
 __device__ __forceinline__ void split_sum_regs(const GemmParams& p, const float (&acc)[64], uint32_t smem0, int tile, int m_blocks,
-                                               int n_blocks, int rank, int half, int row) {
+                                               int n_blocks, int rank, int half, int row, int* s_abort) {
   const int width = 128 / p.split;  // columns per owner: 64, 32 or 16
   const uint32_t part_bytes = (uint32_t)width * BM * 4u;
   __syncwarp();
   cluster_sync_all();
+  if (half == 0 && row == 0) split_spread_abort(s_abort, (uint32_t)p.split);
+  __syncwarp();
 #pragma unroll
   for (int g = 0; g < 4; ++g) {  // 16 columns at a time: all of one owner's
     const int col = half * 64 + g * 16, owner = col / width;
@@ -742,6 +757,7 @@ __device__ __forceinline__ void split_sum_regs(const GemmParams& p, const float 
   }
   __syncwarp();
   cluster_sync_all();
+  if (*(volatile int*)s_abort) return;
   int mb, nb;
   tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
 #pragma unroll
@@ -920,7 +936,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const bool elected = lg == 0 && lane == 0;  // one per half: issues (and owns) that half's TMA stores
     const uint32_t sbuf = smem_u32(sEpi) + (uint32_t)half * EPI_SLAB_BYTES;
     uint32_t blk = 0;
-    float acc[64];
+    float acc[64] = {};
     for (int it = 0;; ++it) {
       const int tile = next_tile(it);
       if (epi_vote_any(1 + half, tile >= total)) break;  // the four warps of a half leave together
@@ -998,7 +1014,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         bulk_commit();
       }
     }
-    if (SPLIT && tile0 < total) split_sum_regs(p, acc, smem_u32(smem), tile0, m_blocks, n_blocks, rank, half, row_local);
+    if (SPLIT && tile0 < total) split_sum_regs(p, acc, smem_u32(smem), tile0, m_blocks, n_blocks, rank, half, row_local, &s_abort);
     if (elected) {  // Y is complete before this CTA reports
       bulk_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");
@@ -1294,6 +1310,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
           umma_commit_pair(map_to_cta(empty_bar(s), even | 1u));
           if (++s == STAGES2) s = 0, ph ^= 1u;
         }
+        if (*abort) break;  // a tile that is not complete is not announced
         umma_commit_pair(tfull_bar(buf));
         umma_commit_pair(map_to_cta(tfull_bar(buf), even | 1u));
       }
@@ -1406,7 +1423,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     tc_fence_after();
     int mb, nb;
     tile_coords(tile0, m_blocks, n_blocks, p.head_blocks, mb, nb);
-    split_sum(p, tmem_base, smem_u32(smem), 2 * mb + (int)rank, nb, share, (int)rank, 2);
+    split_sum(p, tmem_base, smem_u32(smem), 2 * mb + (int)rank, nb, share, (int)rank, 2, &s_abort);
     tc_fence_before();
   }
   cluster_sync_all();  // neither CTA leaves while the other may still touch its shared memory or TMEM

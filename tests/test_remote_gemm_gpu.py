@@ -181,3 +181,46 @@ def test_mxfp8_cta_pairs(cuda_device, m, n, k, pull):
         full = x @ w
         assert float((y.float() - full).abs().max()) < 0.1 * float(full.abs().max())
         assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+
+
+@pytest.mark.parametrize("fmt,m,n,k", [("bf16", 128, 256, 8192), ("bf16", 640, 768, 2048), ("bf16", 1024, 1024, 1024), ("bf16", 4096, 4096, 512),
+                                       ("fp8_block", 128, 128, 8192), ("fp8_block", 256, 640, 3200), ("fp8_block", 256, 256, 1024),
+                                       ("fp8_block", 1920, 2688, 2048), ("mxfp8", 256, 256, 8192), ("mxfp8", 512, 768, 3200),
+                                       ("mxfp8", 1024, 1024, 1024)])
+def test_a_wait_that_runs_out(cuda_device, fmt, m, n, k):
+    """Rows of X that never arrive (the counter from which the copying warps draw their work says that all of it is taken):
+    the call gives up after its limit, says so in the status word, leaves Y and the done flag alone and its scratch at
+    zero, whether one CTA, a pair or a cluster shares a tile, and the next call is right."""
+    from execution_ucx_b200.ops import remote_gemm as rg
+    torch.manual_seed(m + n + k)
+    x = torch.randn(m, k, device=cuda_device)
+    w = torch.randn(k, n, device=cuda_device) * 0.02
+    if fmt == "bf16":
+        g, args = rg.RemoteGemm(w.to(torch.bfloat16), m), [x.to(torch.bfloat16)]
+    elif fmt == "fp8_block":
+        g, args = rg.RemoteGemmFp8(w, m), list(rg.quantize_rows_1x128(x))
+    else:
+        xq, sf = rg.quantize_mx(x)
+        g, args = rg.RemoteGemmMx(w, m), [xq, rg.mx_scale_chunks(sf, False)]
+    y = torch.full((m, n), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    done = torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    ptrs = [a.data_ptr() for a in args]
+    for part in (0, 1):  # nothing arrives; the first panel alone does not
+        g.sched[3] = 0x7fffffff if part == 0 else (128 * k * x.element_size() // (2 if fmt == "bf16" else 4) >> 13) + (0 if fmt == "bf16" else (4 * k + 8191) >> 13)
+        g(*ptrs, m, y.data_ptr(), x_is_local=False, done_flag_ptr=done.data_ptr(), done_value=1, timeout_ns=20_000_000)
+        torch.cuda.synchronize()
+        assert int(g.status) != 0 and int(done) == 0
+        if part == 0 or m == 128:
+            assert bool((y == 7).all())
+        else:  # the rows of the missing panel; with CTA pairs the panel beside it too
+            assert bool((y[:128] == 7).all())
+        assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+        g.status.zero_()
+    g(*ptrs, m, y.data_ptr(), x_is_local=False, done_flag_ptr=done.data_ptr(), done_value=1)
+    torch.cuda.synchronize()
+    g.check_status()
+    assert int(done) == 1
+    want = torch.empty_like(y)
+    g(*ptrs, m, want.data_ptr(), x_is_local=True)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
