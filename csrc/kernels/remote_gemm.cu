@@ -114,15 +114,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Tiles in groups of GROUP_M row blocks (row block fastest inside a group) so that one wave of CTAs
@@ -412,83 +403,94 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The sum over a cluster whose CTAs have each computed a share of K of one tile of 128 rows: CTA r owns rows
+// [r * 128 / split, (r + 1) * 128 / split), every CTA stores its partial sums (fp32) of an owner's rows into the owner's
+// shared memory, and the owner adds the parts up in the order of the ranks and writes its rows of Y, full 128-byte
+// lines of each (Y may be the caller's memory across NVLink). All pipeline stages are idle by then: the first cluster
+// barrier comes after every CTA's last MMA. A CTA that gave up says so to all others between the two barriers, and none
+// of them writes: as in the unsplit kernels, Y stays as it was where a wait ran out.
+// `rank` counts the shares of K; the CTA that has another share of the same rows is `stride` cluster ranks per share
+// further on from `first`.
+// Layout of a part: 16 bytes (four columns) of one row next to the same columns of the next row, so that a warp's store
+// is one run of 512 bytes (rows further apart: 3 us more per tile); neighbours within eight rows are exchanged by the
+// number of the column group, so that the owner's reads along a row meet eight different banks.
+template <int COLS>
+struct SplitParts {
+  uint32_t base;  // of this CTA's parts: [share][group of four columns][row of the owner]
+  int split, rank, first, stride;
+  __device__ __forceinline__ int rows() const { return BM / split; }
+  static __device__ __forceinline__ uint32_t at(int rows, int group, int row) { return (uint32_t)(group * rows + (row ^ (group & 7))) * 16u; }
+  // this CTA's share in the shared memory of the CTA that owns `row`, as a shared::cluster address
+  __device__ __forceinline__ uint32_t out(int row) const {
+    return map_to_cta(base + (uint32_t)(rank * rows()) * COLS * 4u, (uint32_t)(first + row / rows() * stride));
+  }
+  // N columns of `row` from group `group` on (a multiple of eight)
+  template <int N>
+  __device__ __forceinline__ void store(uint32_t dst, int group, int row, const float* v) const {
+#pragma unroll
+    for (int q = 0; q < N / 4; ++q)
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + at(rows(), group + q, row % rows())), "f"(v[4 * q]),
+                   "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                   : "memory");
+  }
+};
 // One thread of a CTA that gave up: the other CTAs of the cluster of `n` learn of it.
 __device__ __forceinline__ void split_spread_abort(int* s_abort, uint32_t n) {
   if (!*(volatile int*)s_abort) return;
   for (uint32_t r = 0; r < n; ++r)
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32(s_abort), r)), "r"(1u) : "memory");
 }
-// The sum over a cluster whose CTAs have each computed a share of K of one 128 x 256 tile: CTA r owns 256 / split of
-// the columns, every CTA stores its partial sums (fp32) of the other owners' columns into their shared memory, and the
-// owner adds them up in the order of the ranks and writes its part of Y. All pipeline stages are idle by then: the
-// first cluster barrier comes after every CTA's last MMA. All eight warps take part; a thread handles one row. A CTA
-// that gave up says so to all others between the two barriers, and none of them writes: as in the unsplit kernels, Y
-// stays as it was where a wait ran out.
-// Layout of a part: 16 bytes (four columns) of one row next to the same columns of the next row.
-// `rank` counts the shares of K; the CTA that has another share of the same rows is `stride` cluster ranks per share
-// further on from `first`. (mb, nb): the tile in blocks of 128 rows and 256 columns.
+// The owner's rows of Y, by eight warps (`warp` from 0): a warp per row, 256 bytes of it in one store.
+template <int COLS>
+__device__ __forceinline__ void split_write(const GemmParams& p, const SplitParts<COLS>& s, unsigned char* y_tile, int warp, int lane) {
+  const int rows = s.rows();
+  for (int r = warp; r < rows; r += 8) {
+    unsigned char* out = y_tile + (size_t)(s.rank * rows + r) * p.N * 2;
+#pragma unroll
+    for (int c = 0; c < COLS; c += 128) {
+      const int col = c + lane * 4;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int k = 0; k < s.split; ++k) {
+        float v[4];
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                     : "r"(s.base + (uint32_t)(k * rows) * COLS * 4u + SplitParts<COLS>::at(rows, col / 4, r))
+                     : "memory");
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] += v[j];
+      }
+      uint2 o;
+      __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
+      q[0] = __floats2bfloat162_rn(acc[0], acc[1]);
+      q[1] = __floats2bfloat162_rn(acc[2], acc[3]);
+      *reinterpret_cast<uint2*>(out + (size_t)col * 2) = o;
+    }
+  }
+}
+// The whole of it for a 128 x 256 tile in TMEM. All eight warps take part. (mb, nb): the tile in blocks of 128 rows and
+// 256 columns.
 __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_base, uint32_t smem0, int mb, int nb, int rank,
                                           int first, int stride, int* s_abort) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lg = warp & 3, side = warp >> 2;
-  const int row = lg * 32 + lane;
-  const int width = BN / p.split, half = width / 2;  // this thread: columns [side * half, +half) of an owner's
-  const uint32_t part_bytes = (uint32_t)width * BM * 4u;
-  const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * half);
-  const uint32_t mine = smem0 + (uint32_t)row * 16u + (uint32_t)(side * half / 4) * (BM * 16u);
+  const SplitParts<BN> parts{smem0, p.split, rank, first, stride};
+  const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * (BN / 2));
+  const uint32_t dst = parts.out(lg * 32 + lane);
   __syncwarp();
   cluster_sync_all();
   if (threadIdx.x == 0) split_spread_abort(s_abort, (uint32_t)(p.split * stride));
   __syncwarp();
-  for (int d = 1; d < p.split; ++d) {
-    const int owner = (rank + d) % p.split;  // each CTA starts with another one
-    const uint32_t slot = (uint32_t)(rank < owner ? rank : rank - 1);
-    const uint32_t dst = map_to_cta(mine + slot * part_bytes, (uint32_t)(first + owner * stride));
-    for (int c = 0; c < half; c += 16) {
-      uint32_t r[16];
-      tmem_ld16(tbase + (uint32_t)(owner * width + c), r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(c / 4 + q) * (BM * 16u)), "r"(r[4 * q]),
-                     "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
-                     : "memory");
-    }
+#pragma unroll 1
+  for (int c = 0; c < BN / 2; c += 32) {
+    uint32_t r[32];
+    tmem_ld32(tbase + (uint32_t)c, r);
+    tmem_ld_wait();
+    parts.store<32>(dst, (side * (BN / 2) + c) / 4, lg * 32 + lane, reinterpret_cast<const float*>(r));
   }
   __syncwarp();
   cluster_sync_all();
   if (*(volatile int*)s_abort) return;
-  unsigned char* out = p.y + ((size_t)(mb * BM + row) * p.N + (size_t)nb * BN + rank * width + side * half) * 2;
-  for (int c = 0; c < half; c += 16) {
-    uint32_t own[16];
-    tmem_ld16(tbase + (uint32_t)(rank * width + c), own);
-    tmem_ld_wait();
-    float acc[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-    for (int r = 0; r < p.split; ++r) {
-      const uint32_t src = mine + (uint32_t)(r < rank ? r : r - 1) * part_bytes + (uint32_t)(c / 4) * (BM * 16u);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t v[4] = {own[4 * q], own[4 * q + 1], own[4 * q + 2], own[4 * q + 3]};
-        if (r != rank)
-          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-                       : "r"(src + (uint32_t)q * (BM * 16u))
-                       : "memory");
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[4 * q + j] += __uint_as_float(v[j]);
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint4 o;
-      __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) q[j] = __floats2bfloat162_rn(acc[8 * h + 2 * j], acc[8 * h + 2 * j + 1]);
-      st_u4(out + c * 2 + h * 16, o);
-    }
-  }
+  split_write(p, parts, p.y + ((size_t)mb * BM * p.N + (size_t)nb * BN) * 2, warp, lane);
 }
 
 template <bool SPLIT>
@@ -736,62 +738,19 @@ constexpr size_t GEMM8_SMEM = (size_t)STAGES8 * (A8_STAGE_BYTES + B8_STAGE_BYTES
 // the 64 columns of its half of a 128 x 128 tile. Called by the epilogue warps; the others join the two barriers.
 __device__ __forceinline__ void split_sum_regs(const GemmParams& p, const float (&acc)[64], uint32_t smem0, int tile, int m_blocks,
                                                int n_blocks, int rank, int half, int row, int* s_abort) {
-  const int width = 128 / p.split;  // columns per owner: 64, 32 or 16
-  const uint32_t part_bytes = (uint32_t)width * BM * 4u;
+  const SplitParts<BN8> parts{smem0, p.split, rank, 0, 1};
+  const uint32_t dst = parts.out(row);
   __syncwarp();
   cluster_sync_all();
   if (half == 0 && row == 0) split_spread_abort(s_abort, (uint32_t)p.split);
   __syncwarp();
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {  // 16 columns at a time: all of one owner's
-    const int col = half * 64 + g * 16, owner = col / width;
-    if (owner == rank) continue;
-    const uint32_t dst = map_to_cta(smem0 + (uint32_t)(rank < owner ? rank : rank - 1) * part_bytes + (uint32_t)row * 16u +
-                                        (uint32_t)((col - owner * width) / 4) * (BM * 16u),
-                                    (uint32_t)owner);
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)q * (BM * 16u)), "f"(acc[g * 16 + 4 * q]),
-                   "f"(acc[g * 16 + 4 * q + 1]), "f"(acc[g * 16 + 4 * q + 2]), "f"(acc[g * 16 + 4 * q + 3])
-                   : "memory");
-  }
+  parts.store<64>(dst, half * 16, row, acc);
   __syncwarp();
   cluster_sync_all();
   if (*(volatile int*)s_abort) return;
   int mb, nb;
   tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    const int col = half * 64 + g * 16;
-    if (col / width != rank) continue;
-    float sum[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) sum[j] = 0.f;
-    for (int r = 0; r < p.split; ++r) {
-      const uint32_t src = smem0 + (uint32_t)(r < rank ? r : r - 1) * part_bytes + (uint32_t)row * 16u +
-                           (uint32_t)((col - rank * width) / 4) * (BM * 16u);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float v[4] = {acc[g * 16 + 4 * q], acc[g * 16 + 4 * q + 1], acc[g * 16 + 4 * q + 2], acc[g * 16 + 4 * q + 3]};
-        if (r != rank)
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                       : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                       : "r"(src + (uint32_t)q * (BM * 16u))
-                       : "memory");
-#pragma unroll
-        for (int j = 0; j < 4; ++j) sum[4 * q + j] += v[j];
-      }
-    }
-    unsigned char* out = p.y + ((size_t)(mb * BM + row) * p.N + (size_t)nb * BN8 + col) * 2;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      uint4 o;
-      __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) q[j] = __floats2bfloat162_rn(sum[8 * h + 2 * j], sum[8 * h + 2 * j + 1]);
-      st_u4(out + h * 16, o);
-    }
-  }
+  split_write(p, parts, p.y + ((size_t)mb * BM * p.N + (size_t)nb * BN8) * 2, half * 4 + (row >> 5), row & 31);
 }
 
 template <bool SPLIT>
