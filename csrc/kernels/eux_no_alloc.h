@@ -20,9 +20,10 @@
  *     M*K elements, which is not "modest", so that mode stays with eux_gemm_launch.
  *   - The static array (EUX_NOALLOC_GEMM_SCRATCH_BYTES) exists once per GPU that loads
  *     the library, for the life of the process.
- *   - The first call on a device looks up the array's device address
- *     (cudaGetSymbolAddress) and raises the kernel's shared-memory limit; make that
- *     first call before any stream capture begins.
+ *   - The first call on a device, of any shape, looks up the array's device address
+ *     (cudaGetSymbolAddress) and sets up every kernel that a later call of another shape
+ *     may take (loads it, raises its shared-memory limit, asks how many clusters fit);
+ *     make that first call before any stream capture begins.
  *   - Every call uses the same array and finds there what the previous call left, so the
  *     entry point clears it on `stream` before the kernel. Two calls whose kernels can
  *     overlap on the GPU (different streams, no dependency) race on it: keep calls on

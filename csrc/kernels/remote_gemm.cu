@@ -1949,6 +1949,20 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
 
 static __device__ __align__(256) uint32_t g_noalloc_gemm_scratch[EUX_NOALLOC_GEMM_SCRATCH_BYTES / 4];
 
+// Everything that a first launch of one of the bf16 kernels would set up: which of them a call takes depends on its shape.
+static int prepare_bf16(int dev) {
+  const void* kernels[] = {(const void*)remote_gemm_kernel<false>, (const void*)remote_gemm_kernel<true>,
+                           (const void*)remote_gemm_2cta_kernel<false, false>};
+  cudaFuncAttributes attr;
+  for (const void* k : kernels)
+    if (cudaError_t e = cudaFuncGetAttributes(&attr, k); e != cudaSuccess) return (int)e;
+  cudaError_t e = allow_smem<remote_gemm_kernel<false>>(dev, GEMM_SMEM);
+  if (e == cudaSuccess) e = allow_smem<remote_gemm_2cta_kernel<false, false>>(dev, PairCfg<false>::SMEM);
+  int clusters = 0;  // one tile and a long K: every size of cluster is asked about
+  choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, 1, 1, 64, &clusters);
+  return (int)e;
+}
+
 extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, int M, int N, int K, uint32_t* status,
                                      uint64_t wait_timeout_ns, void* stream) {
   if (!x || !w_t || !y || M <= 0 || N <= 0 || K <= 0) return EUX_ERR_BAD_ARG;
@@ -1956,7 +1970,7 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
   // The shapes the kernels take, checked here so that a call that is going to be refused has put
   // nothing on the stream: the clear below touches the array that every call shares.
   if (M % 128 || N % 256 || K % 64) return EUX_ERR_BAD_ARG;
-  // Set-up, once per device, with that device current: the device address of the static array.
+  // Set-up, once per device, with that device current: the device address of the static array, and the kernels.
   // Host threads may race to be first; they would all store the same address, atomically.
   static std::atomic<uint32_t*> scratch_addr[64];
   int dev = 0;
@@ -1968,6 +1982,7 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
     uint32_t* ptr = nullptr;
     e = cudaGetSymbolAddress((void**)&ptr, g_noalloc_gemm_scratch);
     if (e != cudaSuccess) return (int)e;
+    if (int rc = prepare_bf16(dev)) return rc;
     scratch_addr[dev].store(ptr, std::memory_order_release);
     scratch = ptr;
   }
@@ -1988,7 +2003,7 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
   d.wait_timeout_ns = wait_timeout_ns;
   d.status = status;
   d.copy_ctas = 0;
-  d.flags = EUX_GEMM_FLAG_CTA_PAIRS;  // taken when M is a multiple of 256
+  d.flags = EUX_GEMM_FLAG_CTA_PAIRS;  // where there are enough tiles; eux_gemm_launch has the rule
   return eux_gemm_launch(&d, stream);
 }
 

@@ -56,3 +56,37 @@ def test_noalloc_gemm_matches_regular_entry_point(cuda_device, m):
     rc = fn(C.c_void_p(x.data_ptr()), C.c_void_p(w_t.data_ptr()), C.c_void_p(got.data_ptr()), m + 64, n, k,
             C.c_void_p(status.data_ptr()), 0, stream)
     assert rc == 100001
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 256, 8192), (128, 768, 1536), (384, 512, 4096), (640, 768, 2048)])
+def test_noalloc_gemm_split_over_clusters(cuda_device, m, n, k):
+    """Few tiles and a long K: clusters share a tile. A call of another shape has done the set-up; this one is captured.
+    fp32 sums in another order (1e-5 of a row's largest result) and one rounding to bf16 (2^-8 of the value)."""
+    from execution_ucx_b200.ops import _native
+    fn = _native.load().eux_gemm_bf16_noalloc
+    torch.manual_seed(m + n + k)
+    x = torch.randn(m, k, device=cuda_device).to(torch.bfloat16)
+    w_t = (torch.randn(n, k, device=cuda_device) * 0.02).to(torch.bfloat16)
+    y = torch.zeros(m, n, dtype=torch.bfloat16, device=cuda_device)
+    status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+
+    def call(m, n, k):
+        return fn(x.data_ptr(), w_t.data_ptr(), y.data_ptr(), m, n, k, status.data_ptr(), 2_000_000_000, torch.cuda.current_stream().cuda_stream)
+
+    assert call(128, 256, 64) == 0
+    torch.cuda.synchronize()
+    ref = x.double() @ w_t.double().t()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert call(m, n, k) == 0
+    for _ in range(3):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0
+        assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
+    free_before, _ = torch.cuda.mem_get_info()
+    assert call(m, n, k) == 0
+    torch.cuda.synchronize()
+    free_after, _ = torch.cuda.mem_get_info()
+    assert free_after == free_before
