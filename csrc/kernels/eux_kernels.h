@@ -171,7 +171,7 @@ typedef struct eux_moe_desc {
   uint64_t* const* meta_peer; /* device array [world]: row headers, 16 B each */
   uint64_t* const* flag_peer; /* device array [world]: [world] arrival flags + [world] counts */
   int32_t* slot_of;           /* [n_tokens, topk] scratch+output: slot inside (src,dst) region */
-  int32_t* counters;          /* scratch [world + n_experts + 8] zero on entry, zero on exit (clear it after a time-out) */
+  int32_t* counters;          /* scratch [world + n_experts + 8] zero on entry, zero on exit */
   void* out;                  /* combine output [n_tokens, hidden] bf16 */
   uint64_t seq;               /* flag value of this dispatch/combine exchange (monotonic) */
   uint64_t wait_timeout_ns;

@@ -21,7 +21,6 @@
 // the weighted combine is fused into the receive and no intermediate buffer
 // exists.
 #include <algorithm>
-#include <atomic>
 
 #include "eux_device.cuh"
 
@@ -37,13 +36,17 @@ __host__ __device__ __forceinline__ size_t moe_row_bytes(int hidden, int fp8) {
   return fp8 ? (((size_t)hidden + (size_t)(hidden / 128) * 4 + 127) / 128) * 128 : (size_t)hidden * 2;
 }
 
-// ---- dispatch: routing and the transfer in one cooperative launch -----------------------------------------
-// Every CTA owns a run of tokens. It counts their experts, adds its counts to the global ones (which returns where its
-// rows start inside each expert's group), waits for all CTAs at a grid barrier, and then knows every slot: the experts
-// before this one on the same rank, its CTA's start, and the rank inside the CTA. A single routing CTA in front of the
-// transfer took 5 us for 128 tokens and 13 for 4096 (top 8 of 256), plus a launch. All CTAs are resident (cooperative
-// launch), so the barrier ends; its wait is bounded all the same.
-// counters layout: [0,W) unused | [W,W+E) rows per expert | [W+E] done CTAs | [W+E+1] barrier; zero between launches
+// ---- dispatch: routing, then the transfer -------------------------------------------------------------------
+// Every CTA owns a run of tokens and has to know where its rows go: the rows of the experts before each one on the same
+// rank, and the rows of the same expert from tokens of the CTAs before it.
+//   * Few entries (kRouteSelf): every CTA reads all of them (out of L2) and counts for itself. No CTA waits for another
+//     one, so nothing depends on how many of them run at a time.
+//   * More: moe_count_kernel in front of the dispatch adds the counts up and gives every entry its place inside its
+//     expert's group; the end of that launch is the barrier.
+// (A grid barrier inside one cooperative launch needed all CTAs resident at once, which a kernel of another stream can
+// prevent for as long as it waits for this dispatch, and a barrier that ran out left its counters behind. Exchange of 128
+// tokens of 7168, fp8: 24.8 us with the barrier, 24.1 now; 4096 tokens, bf16: 207.8 and 210.8, 219 with one routing CTA.)
+// counters layout: [0,W) unused | [W,W+E) rows per expert | [W+E] done CTAs; zero between launches
 __device__ __forceinline__ void moe_ld_v8(const void* p, uint32_t (&v)[8]) {
   asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -55,10 +58,14 @@ __device__ __forceinline__ void moe_st_v8(void* p, const uint32_t (&v)[8]) {
                : "memory");
 }
 struct MoeRouting {
-  int* local;  // [E] rows of this CTA per expert
-  int* base;   // [E] where they start inside the expert's group; after the barrier: inside the destination's region
+  int* local;  // [E] rows of this CTA per expert; then rows of all experts before e, whatever their rank
+  int* base;   // [E] where this CTA's rows start inside the destination's region
   int* total;  // [E] rows of all CTAs per expert
 };
+// The tokens [t0, t1) of CTA `b` of `grid`: all shares within one token of one another.
+__device__ __forceinline__ int moe_first_token(const eux_moe_desc& d, int b, int grid) {
+  return (int)((int64_t)d.n_tokens * b / grid);
+}
 
 // Exclusive scan of v over the CTA; `sums`: one int per warp.
 __device__ __forceinline__ int cta_exclusive_scan(int v, int* sums) {
@@ -77,54 +84,94 @@ __device__ __forceinline__ int cta_exclusive_scan(int v, int* sums) {
   return before + x - v;
 }
 
-__device__ __forceinline__ bool moe_route(const eux_moe_desc& d, const MoeRouting& r, int t0, int t1) {
-  const int W = d.world, E = d.n_experts, EPR = E / W, K = d.topk;
-  int* const counts = d.counters + W;
-  uint32_t* const barrier = reinterpret_cast<uint32_t*>(d.counters + W + E + 1);
-  __shared__ int s_sums[kMoeThreads / 32];
-  __shared__ int s_ok;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) r.local[e] = 0;
+constexpr int kRouteSelf = 4096;
+
+// The place of every entry inside its expert's group: a CTA takes a run of entries, ranks them, and adds its counts to the
+// global ones, which returns where its rows start. (The additions go out in the order of the experts, a warp's 32 in one
+// line; where each expert's first entry made it, 4096 x 7168 took 4 us more.)
+__global__ void __launch_bounds__(kMoeThreads) moe_count_kernel(eux_moe_desc d) {
+  extern __shared__ int moe_sm[];
+  int* const local = moe_sm;
+  int* const base = moe_sm + d.n_experts;
+  const int E = d.n_experts;
+  const int64_t n = (int64_t)d.n_tokens * d.topk;
+  const int64_t i0 = n * blockIdx.x / gridDim.x, i1 = n * (blockIdx.x + 1) / gridDim.x;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) local[e] = 0;
   __syncthreads();
-  for (int64_t i = (int64_t)t0 * K + threadIdx.x; i < (int64_t)t1 * K; i += blockDim.x) {
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const int e = __ldg(d.topk_idx + i);
-    d.slot_of[i] = e >= 0 && e < E ? atomicAdd(&r.local[e], 1) : -1;  // the rank inside this CTA, for now
+    d.slot_of[i] = e >= 0 && e < E ? atomicAdd(&local[e], 1) : -1;  // the rank inside this CTA, for now
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) r.base[e] = r.local[e] ? atomicAdd(counts + e, r.local[e]) : 0;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) base[e] = local[e] ? atomicAdd(d.counters + d.world + e, local[e]) : 0;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(barrier, 1u);
-    s_ok = wait_u32_ge_gpu(barrier, gridDim.x, d.wait_timeout_ns);
-    if (!s_ok) set_status(d.status, EUX_ST_TIMEOUT, 10);
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    const int rank = d.slot_of[i];
+    if (rank >= 0) d.slot_of[i] = rank + base[__ldg(d.topk_idx + i)];
+  }
+}
+
+// The slots of tokens [t0, t1). `counted`: moe_count_kernel has run. What a thread knows of its entries stays in its
+// registers until the slots are known: a trip to memory more costs as much as all of the arithmetic.
+__device__ __forceinline__ void moe_route(const eux_moe_desc& d, const MoeRouting& r, int t0, int t1, bool counted) {
+  constexpr int PER = kRouteSelf / kMoeThreads;
+  const int W = d.world, E = d.n_experts, EPR = E / W, K = d.topk;
+  const int64_t lo = (int64_t)t0 * K, hi = (int64_t)t1 * K;
+  const int n = counted ? 0 : d.n_tokens * K;  // entries that this CTA counts: at most kRouteSelf
+  __shared__ int s_sums[kMoeThreads / 32];
+  int expert[PER], rank[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int i = (int)threadIdx.x + j * kMoeThreads;
+    expert[j] = i < n ? __ldg(d.topk_idx + i) : -1;
+  }
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    r.local[e] = 0, r.base[e] = 0;
+    r.total[e] = counted ? __ldcg(d.counters + W + e) : 0;
   }
   __syncthreads();
-  if (!s_ok) return false;
-  // every thread takes a run of consecutive experts: totals, and the exclusive sums over them
+  if (!counted) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = (int)threadIdx.x + j * kMoeThreads, e = expert[j];
+      if (e < 0 || e >= E) expert[j] = -1;
+      else if (i >= lo && i < hi) rank[j] = atomicAdd(&r.local[e], 1);
+      else atomicAdd(i < lo ? &r.base[e] : &r.total[e], 1);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) r.total[e] += r.base[e] + r.local[e];
+    __syncthreads();
+  }
+  // every thread takes a run of consecutive experts
   const int run = (E + (int)blockDim.x - 1) / (int)blockDim.x;
   const int e0 = (int)threadIdx.x * run, e1 = min(e0 + run, E);
   int mine = 0;
-  for (int e = e0; e < e1; ++e) {
-    r.total[e] = __ldcg(counts + e);
-    mine += r.total[e];
-  }
+  for (int e = e0; e < e1; ++e) mine += r.total[e];
   int sum = cta_exclusive_scan(mine, s_sums);
   for (int e = e0; e < e1; ++e) {
-    r.local[e] = sum;  // rows of all experts before e, whatever their rank
+    r.local[e] = sum;
     sum += r.total[e];
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) r.base[e] += r.local[e] - r.local[(e / EPR) * EPR];
   __syncthreads();
-  for (int64_t i = (int64_t)t0 * K + threadIdx.x; i < (int64_t)t1 * K; i += blockDim.x) {
-    int slot = d.slot_of[i];
-    if (slot >= 0) {
-      slot += r.base[__ldg(d.topk_idx + i)];
-      d.slot_of[i] = slot < d.capacity ? slot : -1;
+  auto place = [&](int64_t i, int e, int in_group) {
+    const int slot = e >= 0 ? r.base[e] + in_group : -1;
+    d.slot_of[i] = slot < d.capacity ? slot : -1;
+  };
+  if (counted) {
+    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+      const int in_group = d.slot_of[i];
+      place(i, in_group >= 0 ? __ldg(d.topk_idx + i) : -1, in_group);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = (int)threadIdx.x + j * kMoeThreads;
+      if (i >= lo && i < hi) place(i, expert[j], rank[j]);
     }
   }
   __syncthreads();
-  return true;
 }
 
 // The last CTA sends counts and arrival flags to every destination rank and leaves the counters at zero.
@@ -153,7 +200,7 @@ __device__ __forceinline__ void moe_publish(const eux_moe_desc& d, const MoeRout
   }
   __syncthreads();  // the release below covers what the CTA's other threads wrote before this barrier
   for (int dst = threadIdx.x; dst < W; dst += blockDim.x) st_release_sys(&d.flag_peer[dst][d.rank], d.seq);
-  if (threadIdx.x < 2) d.counters[W + E + threadIdx.x] = 0;
+  if (threadIdx.x == 0) d.counters[W + E] = 0;
 }
 
 // The routing entries of a token: lane k (< topk) owns slot k.
@@ -192,11 +239,11 @@ __device__ __forceinline__ unsigned char* shfl_ptr(unsigned char* p, int src) {
 // ---- dispatch, bf16 rows ----------------------------------------------------
 // Work unit = (token, 128 consecutive 16-byte chunks): a warp loads 4 chunks per
 // lane once and stores them to each of the token's top-k destinations.
-__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_desc d, int tokens_per_cta) {
+__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_desc d, int counted) {
   extern __shared__ int moe_sm[];
   const MoeRouting r{moe_sm, moe_sm + d.n_experts, moe_sm + 2 * d.n_experts};
-  const int t0 = min((int)blockIdx.x * tokens_per_cta, d.n_tokens), t1 = min(t0 + tokens_per_cta, d.n_tokens);
-  if (!moe_route(d, r, t0, t1)) return;
+  const int t0 = moe_first_token(d, blockIdx.x, gridDim.x), t1 = moe_first_token(d, blockIdx.x + 1, gridDim.x);
+  moe_route(d, r, t0, t1, counted != 0);
   const int EPR = d.n_experts / d.world, K = d.topk;
   const int chunks = d.hidden / 8;  // uint4 per row
   const int upr = (chunks + 127) / 128;
@@ -242,12 +289,12 @@ __host__ __device__ __forceinline__ int moe_scale_batch(int hidden) {
 }
 __host__ __device__ __forceinline__ int moe_scale_stride(int hidden) { return moe_scale_batch(hidden) * (hidden / 128); }
 
-__global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_moe_desc d, int tokens_per_cta) {
+__global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_moe_desc d, int counted) {
   extern __shared__ int moe_sm[];
   const MoeRouting r{moe_sm, moe_sm + d.n_experts, moe_sm + 2 * d.n_experts};
   float* const scales = reinterpret_cast<float*>(moe_sm + 3 * d.n_experts);
-  const int t0 = min((int)blockIdx.x * tokens_per_cta, d.n_tokens), t1 = min(t0 + tokens_per_cta, d.n_tokens);
-  if (!moe_route(d, r, t0, t1)) return;
+  const int t0 = moe_first_token(d, blockIdx.x, gridDim.x), t1 = moe_first_token(d, blockIdx.x + 1, gridDim.x);
+  moe_route(d, r, t0, t1, counted != 0);
   const int EPR = d.n_experts / d.world, K = d.topk;
   const int upr = (d.hidden + 1023) / 1024;
   const int ngroups = d.hidden / 128;
@@ -683,44 +730,26 @@ using namespace eux;
 
 extern "C" size_t eux_moe_row_bytes(int hidden, int fp8) { return moe_row_bytes(hidden, fp8); }
 
-// How many CTAs of a cooperative launch the device holds at once (asked once per device and amount of shared memory).
-template <auto KERNEL>
-static int moe_resident_ctas(int dev, size_t smem, int* out) {
-  static std::atomic<uint64_t> known[64];  // shared memory << 32 | CTAs, of the last question
-  const uint64_t k = known[dev].load(std::memory_order_acquire);
-  if (k && (k >> 32) == smem) {
-    *out = (int)(uint32_t)k;
-    return 0;
-  }
-  int per_sm = 0, sms = 0;
-  cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, kMoeThreads, smem);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return (int)e;
-  if (per_sm < 1) return EUX_ERR_UNSUPPORTED;
-  *out = per_sm * sms;
-  known[dev].store((uint64_t)smem << 32 | (uint32_t)*out, std::memory_order_release);
-  return 0;
-}
 template <auto KERNEL>
 static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream_t st) {
-  int dev = 0, resident = 0;
+  int dev = 0, sms = 148;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return EUX_ERR_BAD_ARG;
-  if (int rc = moe_resident_ctas<KERNEL>(dev, smem, &resident)) return rc;
-  // One CTA per SM, half of what fits: as fast as two (4096 x 7168, exchange: 209 us against 211), and a kernel of another
-  // stream that holds SMs while it waits for a peer does not keep this launch, and the peer, waiting.
-  int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (ctas <= 0) ctas = sms;
-  if (ctas > resident) ctas = resident;
-  int per = (d->n_tokens + ctas - 1) / ctas;
-  if (per < 1) per = 1;
-  int grid = (d->n_tokens + per - 1) / per;
-  if (grid < 1) grid = 1;
-  eux_moe_desc dd = *d;
-  void* args[] = {&dd, &per};
-  return (int)cudaLaunchCooperativeKernel((const void*)KERNEL, dim3(grid), dim3(kMoeThreads), args, smem, st);
+  // A CTA per token, up to one per SM: a second one counts all entries again (256 tokens, fp8: 28.2 us for the exchange
+  // with one, 30.2 with two). fp8 rows of more than eight tokens per CTA have two, one of which works while the other
+  // waits at its barriers (32768 x 1024: 235 us against 280).
+  if (ctas <= 0) ctas = d->fp8 && d->n_tokens > 8 * sms ? 2 * sms : sms;
+  const int grid = std::max(1, std::min(ctas, d->n_tokens));
+  if (smem > 40 * 1024)  // with the kernel's static arrays near the 48 KiB that need no leave
+    if (cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); e != cudaSuccess) return (int)e;
+  const int64_t entries = (int64_t)d->n_tokens * d->topk;
+  const int counted = entries > kRouteSelf;
+  if (counted) {
+    const int64_t want = (entries + kMoeThreads - 1) / kMoeThreads;
+    moe_count_kernel<<<(int)std::min<int64_t>(want, sms), kMoeThreads, 2 * (size_t)d->n_experts * sizeof(int), st>>>(*d);
+  }
+  KERNEL<<<grid, kMoeThreads, smem, st>>>(*d, counted);
+  return (int)cudaGetLastError();
 }
 
 extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* stream) {
@@ -870,7 +899,8 @@ extern "C" int eux_moe_combine_launch(const eux_moe_desc* d, int ctas, void* str
 // Loads every kernel of this file (see eux_xfer_preload for why a first launch must not be the one that loads).
 extern "C" int eux_moe_preload(void) {
   cudaFuncAttributes attr;
-  const void* kernels[] = {(const void*)moe_dispatch_bf16_kernel,       (const void*)moe_dispatch_fp8_kernel,
+  const void* kernels[] = {(const void*)moe_count_kernel,
+                           (const void*)moe_dispatch_bf16_kernel,       (const void*)moe_dispatch_fp8_kernel,
                            (const void*)moe_expert_ready_kernel,        (const void*)moe_combine_bf16_kernel,
                            (const void*)moe_combine_bf16_stream_kernel, (const void*)moe_combine_fp8_kernel,
                            (const void*)moe_combine_fp8_rows_kernel,    (const void*)moe_combine_fp8_stream_kernel};

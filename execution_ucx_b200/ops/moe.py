@@ -16,6 +16,7 @@ from . import _native
 from ..parallel.peer import PeerGroup, SymmetricBuffer
 
 _launches = 0
+_ROUTE_SELF = 4096  # routing entries up to which the dispatch is one launch (kRouteSelf of moe_dispatch.cu)
 
 
 def launch_count() -> int:
@@ -90,7 +91,7 @@ class MoeAllToAll:
         rc = _native.load().eux_moe_dispatch_launch(self._desc(), ctas, _native.current_stream_ptr())
         if rc:
             _native.check(rc, "eux_moe_dispatch_launch")
-        _launches += 1
+        _launches += 1 if self.n_tokens * self.topk <= _ROUTE_SELF else 2
 
     def expert_ready(self) -> None:
         global _launches

@@ -170,3 +170,76 @@ def test_dispatch_routes_in_one_launch(cuda_device, t, hidden, topk, ne, fp8):
         err = (q * scale.unsqueeze(-1) - blocks).abs()
         assert bool((err <= blocks.abs() * (2.0 ** -4 + 1e-6) + amax.unsqueeze(-1) * 2.0 ** -10).all())
         a2a.recv_rows(0, n).zero_()
+
+
+def _check_routed(a2a, x, idx, w):
+    """Every valid (token, slot) has a row of its own that holds the token, grouped by expert; scratch is left at zero."""
+    a2a.check_status()
+    assert int(a2a.counters.abs().sum()) == 0
+    k, flat, slots = idx.shape[1], idx.view(-1).long(), a2a.slot_of.long()
+    n = flat.numel()
+    assert int(a2a.recv_counts()[0]) == n
+    assert torch.equal(slots.sort().values, torch.arange(n, device=x.device))
+    meta, entry = a2a.recv_meta(0, n)[slots], torch.arange(n, device=x.device)
+    assert torch.equal(meta[:, 0].long(), entry // k) and torch.equal((meta[:, 1] & 0xffff).long(), entry % k)
+    assert torch.equal((meta[:, 1] >> 16).long(), flat)
+    le = a2a.recv_meta(0, n)[:, 1] >> 16
+    assert bool((le[1:] >= le[:-1]).all())
+    if not a2a.fp8:
+        assert torch.equal(a2a.recv_rows(0, n)[slots].view(torch.int16), x[entry // k].view(torch.int16))
+
+
+@pytest.mark.parametrize("t,topk", [(512, 8), (513, 8), (4096, 1), (4097, 1), (149, 8), (296, 8), (300, 32)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dispatch_waits_for_nothing(cuda_device, t, topk, fp8):
+    """Around the number of entries that every CTA counts for itself, with one token more than there are SMs, and with
+    the shortest limit there is: a dispatch has no wait that could run out, now or in the calls behind it."""
+    import ctypes as C
+    from execution_ucx_b200.ops import _native, moe
+    a2a = moe.MoeAllToAll.emulated(1, t, 256, topk, 64, fp8=fp8)[0]
+    g = torch.Generator(device=cuda_device).manual_seed(t)
+    x = torch.randn(t, 256, device=cuda_device, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, 64, (t, topk), device=cuda_device, generator=g, dtype=torch.int32)
+    w = torch.rand(t, topk, device=cuda_device, generator=g)
+    for limit in (1, 1, 2_000_000_000):
+        a2a.dispatch(x, idx, w)
+        d = a2a._desc()
+        d = _native.MoeDesc.from_buffer_copy(d)
+        d.wait_timeout_ns = limit
+        a2a.arena.local.zero_()
+        rc = _native.load().eux_moe_dispatch_launch(C.byref(d), 0, _native.current_stream_ptr())
+        assert rc == 0
+        torch.cuda.synchronize()
+        _check_routed(a2a, x, idx, w)
+
+
+@pytest.mark.parametrize("t", [128, 1024])
+def test_dispatch_runs_on_the_sms_that_are_free(cuda_device, t):
+    """A transfer that waits for an arrival (which never comes; it gives up after half a second) holds the registers
+    of all SMs but two. The dispatch on another stream needs no more than what is left."""
+    from execution_ucx_b200.ops import moe, tensor_xfer as tx
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    a2a = moe.MoeAllToAll.emulated(1, t, 512, 8, 64)[0]
+    g = torch.Generator(device=cuda_device).manual_seed(t)
+    x = torch.randn(t, 512, device=cuda_device, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, 64, (t, 8), device=cuda_device, generator=g, dtype=torch.int32)
+    w = torch.rand(t, 8, device=cuda_device, generator=g)
+    a2a.dispatch(x, idx, w)
+    src = torch.zeros(1 << 23, device=cuda_device)
+    dst = torch.empty(1 << 23, dtype=torch.bfloat16, device=cuda_device)
+    tx.push(src, dst)
+    flag = torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    status = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    torch.cuda.synchronize()
+    other = torch.cuda.Stream()
+    begin, end, gave_up = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    begin.record()
+    tx.push(src, dst, wait_flag_ptr=flag.data_ptr(), wait_value=1, wait_timeout_ns=500_000_000, status_ptr=status.data_ptr(), max_ctas=2 * sms - 2)
+    gave_up.record()
+    with torch.cuda.stream(other):
+        a2a.dispatch(x, idx, w)
+        end.record()
+    torch.cuda.synchronize()
+    assert int(status) != 0 and begin.elapsed_time(gave_up) > 400
+    assert begin.elapsed_time(end) < 250
+    _check_routed(a2a, x, idx, w)
