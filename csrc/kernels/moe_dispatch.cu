@@ -338,7 +338,12 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
       for (int k = 0; k < K; ++k) {
         unsigned char* out = shfl_ptr(my_out, k);
         if (!out || !in) continue;
-        moe_st_v8(out + e0, w);
+        if (((uintptr_t)out & 31u) == 0) {
+          moe_st_v8(out + e0, w);
+        } else {  // an arena has to start on 16 bytes only
+          st_u4(out + e0, make_uint4(w[0], w[1], w[2], w[3]));
+          st_u4(out + e0 + 16, make_uint4(w[4], w[5], w[6], w[7]));
+        }
       }
       if (part == 0) my.store_header(d, t, lane, EPR);
     }

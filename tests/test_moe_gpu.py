@@ -243,3 +243,29 @@ def test_dispatch_runs_on_the_sms_that_are_free(cuda_device, t):
     assert int(status) != 0 and begin.elapsed_time(gave_up) > 400
     assert begin.elapsed_time(end) < 250
     _check_routed(a2a, x, idx, w)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dispatch_into_an_arena_on_16_bytes(cuda_device, fp8):
+    """The same rows, wherever an arena starts that is aligned to 16 bytes."""
+    import ctypes as C
+    from execution_ucx_b200.ops import _native, moe
+    t, hidden, topk, ne = 40, 1152, 4, 16
+    a2a = moe.MoeAllToAll.emulated(1, t, hidden, topk, ne, fp8=fp8, capacity=t * topk + 1)[0]
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    x = torch.randn(t, hidden, device=cuda_device, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, ne, (t, topk), device=cuda_device, generator=g, dtype=torch.int32)
+    w = torch.rand(t, topk, device=cuda_device, generator=g)
+    a2a.dispatch(x, idx, w)
+    torch.cuda.synchronize()
+    used = hidden + hidden // 32 if fp8 else 2 * hidden
+    n = t * topk
+    want = a2a.recv_rows(0, n)[a2a.slot_of.long(), :used].clone()
+    a2a.arena.local.zero_()
+    table = torch.tensor([a2a.arena.local.data_ptr() + 16], dtype=torch.int64, device=cuda_device)
+    d = _native.MoeDesc.from_buffer_copy(a2a._desc())
+    d.arena_peer = table.data_ptr()
+    assert _native.load().eux_moe_dispatch_launch(C.byref(d), 0, _native.current_stream_ptr()) == 0
+    torch.cuda.synchronize()
+    rows = a2a.arena.local[16:16 + n * a2a.row_bytes].view(n, a2a.row_bytes)
+    assert torch.equal(rows[a2a.slot_of.long(), :used], want)
