@@ -79,8 +79,8 @@ typedef struct eux_xfer_desc {
   uint64_t wait_value;
   uint64_t wait_timeout_ns;
   uint32_t* status; /* local device (or mapped host) word; may be NULL */
-  uint64_t* flag2;  /* a second word published together with `flag` (the sender's own completion word when
-                       `flag` belongs to the receiver); may be NULL */
+  uint64_t* flag2;  /* a second word published together with `flag` (the sender's own completion word when `flag`
+                       belongs to the receiver): both behind the data, in no order between them; may be NULL */
   uint64_t flag2_value;
 } eux_xfer_desc;
 
@@ -114,7 +114,8 @@ typedef struct eux_pull_item {
   uint64_t nbytes;
   uint64_t* flag; /* mapped pinned host memory or device memory; may be NULL */
   uint64_t flag_value;
-  uint64_t* flag2; /* a second word published with the first (sender-side completion of a push); may be NULL */
+  uint64_t* flag2; /* a second word published together with the first, in no order (sender-side completion of a push);
+                      may be NULL */
   uint64_t flag2_value;
 } eux_pull_item;
 EUX_API int eux_xfer_pull_batch_launch(const eux_pull_item* items, int n, void* stream);

@@ -1859,9 +1859,10 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   const int tiles = (d->M / BM) * (d->N / bn), tiles2 = m_pairs * n_pairs;
   const int waves = (tiles + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
   // Few tiles: the K of a tile is shared out over a cluster of CTAs (or CTA pairs), which add their sums up through
-  // distributed shared memory. A K step costs a CTA about half a microsecond, the sum about three: 128 x 8192 x 8192
-  // (32 tiles) takes 49 us with four CTAs per tile and 72 with one, 128 x 512 x 8192 27 with eight and 59 with one;
-  // 384 x 4096 x 1024, sixteen steps, loses 2 us. All clusters have to fit at once: a second wave costs more.
+  // distributed shared memory. A K step costs a CTA about half a microsecond, the sum about three. Calls in a loop:
+  // 128 x 8192 x 8192 (32 tiles) 35 us with four CTAs per tile and 59 with one, 128 x 512 x 8192 18 with eight and 46 with
+  // one; 384 x 4096 x 1024, sixteen steps, 16.5 with two and 14.3 with one. All clusters have to fit at once: a second
+  // wave costs more.
   if (!pull || copy_by_warps) {
     int clusters = 0;
     if (mx) {
@@ -1892,16 +1893,16 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
       }
     }
   }
-  // bf16 on CTA pairs (bit 0 of the descriptor's flags): a K step of a 256 x 256 tile takes 0.41 us, one of a single
-  // CTA's 128 x 256 tile 0.47, so pairs are taken unless half a tile of padding (M an odd number of 128-row blocks)
-  // costs them a wave or K is short (640 x 8192 x 8192: 98 us against 113, 640 x 4096 x 1024: 25 against 23). CTAs
-  // that copy X before they compute keep to whole tiles.
+  // bf16 on CTA pairs (bit 0 of the descriptor's flags): a K step of a 256 x 256 tile takes 0.35 us, one of a single
+  // CTA's 128 x 256 tile 0.40, so pairs are taken unless half a tile of padding (M an odd number of 128-row blocks)
+  // costs them a wave or K is short (calls in a loop: 640 x 8192 x 8192 90 us against 102, 640 x 4096 x 1024 16.3 against
+  // 14.6). CTAs that copy X before they compute keep to whole tiles.
   const bool pairs_bf16 = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) && !d->fp8 &&
                           (d->M % (2 * BM) == 0 || ((!pull || copy_by_warps) && waves2 <= waves && k_iters >= 24));
-  // Block-scaled fp8 on CTA pairs: a K-block takes 0.76 us of a pair's 256 x 256 tile and 0.53 us of a CTA's 128 x 128
-  // tile (1920 x 4608 x 7168: 89 us against 113; 512 x 4096 x 7168, one wave of either: 54 against 42), so the pairs are
-  // taken when they need at most 7 / 10 of the waves and K is not short. Pulled scales are read through L1, which is sound while no line
-  // holds rows of two panels: their staging buffer starts on a line.
+  // Block-scaled fp8 on CTA pairs: a K-block takes 0.7 to 0.8 us of a pair's 256 x 256 tile and 0.5 to 0.6 us of a CTA's
+  // 128 x 128 tile (calls in a loop: 1920 x 4608 x 7168 78 us against 104; 512 x 4096 x 7168, one wave of either, 44
+  // against 35), so the pairs are taken when they need at most 7 / 10 of the waves and K is not short. Pulled scales are
+  // read through L1, which is sound while no line holds rows of two panels: their staging buffer starts on a line.
   const bool pairs_fp8 = d->fp8 && !mx && (!pull || (copy_by_warps && ((uintptr_t)d->x_scale_stage & 127u) == 0)) &&
                          waves2 * 10 <= waves * 7 && k_iters >= 16;
   if (mx || pairs_bf16 || pairs_fp8) {

@@ -266,7 +266,7 @@ __device__ __forceinline__ void store8(T* p, bool wide, T (&v)[8]) {
 
 // Dense typed path: 8 elements per step, two steps in flight, cast + handler fused. Bound by DRAM: what it takes is bytes
 // in flight and whole sectors per access (2^26 elements, one step with 16-byte accesses and two CTAs per SM -> now:
-// bf16 to e4m3 53 -> 40 us, e4m3 to bf16 50 -> 41, bf16 to fp32 75 -> 71, fp32 to e4m3 of 4096 x 7168 35 -> 31).
+// bf16 to e4m3 51 -> 33 us, e4m3 to bf16 52 -> 40, bf16 to fp32 level at 76, fp32 to e4m3 of 4096 x 7168 30 -> 26).
 template <typename S, typename D>
 __device__ __forceinline__ void typed_body(const eux_xfer_desc& d) {
   const S* src = reinterpret_cast<const S*>(d.src);
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kXferThreads) xfer_rpc_step_kernel(RpcStepArgs
 //   * xfer_gather_kernel: the elements of the innermost dimension are next to one another in the source (row
 //     slices, permuted outer dimensions, dense tensors at any offset), or no dimension has stride 1;
 //   * xfer_tile_kernel: some other dimension has stride 1 (transposes): tiles through shared memory;
-//   * xfer_element_kernel: rows of a few elements, and tensors of a few thousand.
+//   * xfer_element_kernel: tensors of up to 2048 elements per SM, and single bytes in short rows.
 
 __device__ __forceinline__ uint64_t div_u64(uint64_t a, uint64_t b) {
   if (((a | b) >> 32) == 0) return (uint32_t)a / (uint32_t)b;  // most tensors; a 64-bit division costs several times as much
@@ -549,8 +549,8 @@ __global__ void __launch_bounds__(kXferThreads) xfer_element_kernel(const __grid
 constexpr int kTileThreads = 256;
 template <typename S>
 constexpr int tile_p() { return sizeof(S) == 1 ? 128 : 64; }  // every thread has a 16-byte load
-// Words of Q: 256 bytes of a destination row where loads are 16 bytes wide (8192 x 8192 bf16: 68 us with 128 bytes, 55
-// with 256), 128 otherwise (8191 x 8193 bytes: 68 us with 128, 94 with 256).
+// Words of Q: 256 bytes of a destination row where loads are 16 bytes wide (8192 x 8192 bf16: 56 us with 128 bytes, 47
+// with 256), 128 otherwise (8191 x 8193 bytes: 64 us; with 256 it took 1.4 times as long).
 constexpr int tile_q(bool vector) { return vector ? 64 : 32; }
 constexpr int kNarrowBytes = 24576;
 constexpr int kTileWords = 64 * 33;  // of a tile of any other shape
@@ -1131,7 +1131,7 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     if ((al & 31u) == 0) xfer_bytes_kernel<true><<<grid, kXferThreads, 0, st>>>(a);
     else xfer_bytes_kernel<false><<<grid, kXferThreads, 0, st>>>(a);
   } else if (a.d.ndim == 0 && d->src_dtype != EUX_DT_BYTES && (al & 15u) == 0 && !(to_bytes && d->ndim > 0)) {
-    // two CTAs per SM carry enough bytes when the source is fp32 (31 us against 33 with four), narrower ones take four
+    // two CTAs per SM carry enough bytes when the source is fp32 (4096 x 7168 to e4m3: 25 us, 29 with four), narrower ones take four
     // (narrow sources have 32 registers, fp32 ones up to 58). One that waits for its arrival keeps to half of an SM: kernels
     // of other streams, the one that it waits for perhaps among them, find room.
     if (!ctas_given) max_ctas = (d->wait_flag ? 1 : 2) * (ssz == 4 ? 1 : 2) * sms;
@@ -1174,8 +1174,8 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
       route = Route::kGather;
     }
     const bool tiled = route >= Route::kTile;
-    // Four gather CTAs fill an SM's threads. Tiles: a CTA each, whose loads then overlap other CTAs' stores (55 us against
-    // 60 on 8192 x 8192 bf16), or eight CTAs per SM where each one also has a flag's counter to go through.
+    // Four gather CTAs fill an SM's threads. Tiles: a CTA each, whose loads then overlap other CTAs' stores (47 us against
+    // 51 on 8192 x 8192 bf16), or eight CTAs per SM where each one also has a flag's counter to go through.
     // One that waits keeps to half of an SM (gathers have 64 registers and 512 threads), and all its CTAs wait at once, so
     // that a limit passes once.
     if (!ctas_given) max_ctas = d->wait_flag ? (tiled ? 2 : 1) * sms : !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;

@@ -54,7 +54,9 @@ class RemoteGemm:
         ``cta_pairs`` selects the kernel that computes 256 x 256 tiles on pairs of CTAs
         (tcgen05 cta_group::2); shapes that half a tile of padding would cost a wave, and
         ``cta_pairs=False``, run the kernel with one CTA per 128 x 256 tile. With few tiles a cluster
-        of CTAs shares the K of each (its sums are added up in a fixed order). ``head_blocks``
+        of CTAs shares the K of each. Its sums are added up in an order that is fixed for a shape, so a
+        call repeats itself bit by bit, but the low bits of a row can differ between calls with other
+        numbers of rows, whose tiles are shared by more CTAs or fewer. ``head_blocks``
         overrides the height (in row blocks) of the first group of tiles when X is remote.
         A remote X is copied into the staging buffer by two spare warps of every CTA while the
         other warps compute (``copy_warps``, the default), or, when ``copy_ctas`` > 0 is given, by
