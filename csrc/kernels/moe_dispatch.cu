@@ -283,9 +283,10 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_
 // decode batch with a warp per token: 128 tokens of 7168 took 34 us, 20 now. 32-byte stores: with two of 16 bytes per
 // lane 4096 tokens took 89 us, 78 now.)
 constexpr int kMoeScaleFloats = 4096;  // per buffer; two buffers, so that one barrier per batch is enough
+// Tokens per batch; none for rows whose scales do not fit a buffer: those leave one by one.
 __host__ __device__ __forceinline__ int moe_scale_batch(int hidden) {
   const int b = kMoeScaleFloats / (hidden / 128);
-  return b < 1 ? 1 : (b > 16 ? 16 : b);
+  return b > 16 ? 16 : b;
 }
 __host__ __device__ __forceinline__ int moe_scale_stride(int hidden) { return moe_scale_batch(hidden) * (hidden / 128); }
 
@@ -300,7 +301,9 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
   const int ngroups = d.hidden / 128;
   const size_t row_bytes = moe_row_bytes(d.hidden, 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const int batch = moe_scale_batch(d.hidden), stride = moe_scale_stride(d.hidden);
+  const int stride = moe_scale_stride(d.hidden);
+  const bool collect = stride > 0;
+  const int batch = collect ? moe_scale_batch(d.hidden) : 1;
   int buf = 0;
   for (int tb = t0; tb < t1; tb += batch, buf ^= 1) {
     const int nt = min(batch, t1 - tb);
@@ -334,7 +337,8 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
         const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(b.x * inv, b.y * inv), __NV_SATFINITE, __NV_E4M3);
         w[j] = lo | (hi << 16);
       }
-      if (in && (lane & 3) == 0) sc[tl * ngroups + (e0 >> 7)] = scale;
+      const bool keeps = in && (lane & 3) == 0;
+      if (keeps && collect) sc[tl * ngroups + (e0 >> 7)] = scale;
       for (int k = 0; k < K; ++k) {
         unsigned char* out = shfl_ptr(my_out, k);
         if (!out || !in) continue;
@@ -344,9 +348,11 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
           st_u4(out + e0, make_uint4(w[0], w[1], w[2], w[3]));
           st_u4(out + e0 + 16, make_uint4(w[4], w[5], w[6], w[7]));
         }
+        if (keeps && !collect) reinterpret_cast<float*>(out + d.hidden)[e0 >> 7] = scale;
       }
       if (part == 0) my.store_header(d, t, lane, EPR);
     }
+    if (!collect) continue;
     __syncthreads();
     for (int u = warp; u < nt * K; u += nwarps) {
       const int tl = u / K, k = u - tl * K;

@@ -269,3 +269,23 @@ def test_dispatch_into_an_arena_on_16_bytes(cuda_device, fp8):
     torch.cuda.synchronize()
     rows = a2a.arena.local[16:16 + n * a2a.row_bytes].view(n, a2a.row_bytes)
     assert torch.equal(rows[a2a.slot_of.long(), :used], want)
+
+
+@pytest.mark.parametrize("hidden", [524288, 524416, 1 << 22])
+def test_dispatch_of_rows_with_many_scales(cuda_device, hidden):
+    """The longest row whose scales are collected in shared memory, the next one, and one whose scales would not fit it.
+    The whole exchange against its statement in fp32: one rounding to bf16 (2^-8 of the value)."""
+    from execution_ucx_b200.ops import moe
+    t, topk, ne = 3, 2, 4
+    a2a = moe.MoeAllToAll.emulated(1, t, hidden, topk, ne, fp8=True)[0]
+    g = torch.Generator(device=cuda_device).manual_seed(hidden)
+    x = torch.randn(t, hidden, device=cuda_device, generator=g).to(torch.bfloat16)
+    idx = torch.randint(0, ne, (t, topk), device=cuda_device, generator=g, dtype=torch.int32)
+    w = torch.rand(t, topk, device=cuda_device, generator=g)
+    a2a.dispatch(x, idx, w)
+    a2a.expert_ready()
+    out = a2a.combine()
+    torch.cuda.synchronize()
+    a2a.check_status()
+    ref = moe.reference_dispatch_combine(x, idx, w, True)
+    assert bool(((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
