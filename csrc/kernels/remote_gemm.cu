@@ -440,30 +440,44 @@ __device__ __forceinline__ void split_spread_abort(int* s_abort, uint32_t n) {
   for (uint32_t r = 0; r < n; ++r)
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to_cta(smem_u32(s_abort), r)), "r"(1u) : "memory");
 }
-// The owner's rows of Y, by eight warps (`warp` from 0): a warp per row, 256 bytes of it in one store.
+// The owner's rows of Y, by eight warps (`warp` from 0): a warp per row, 256 bytes of it in one store. Two parts of the row
+// at a time, all their loads in flight together; they are added in the order of the ranks.
 template <int COLS>
 __device__ __forceinline__ void split_write(const GemmParams& p, const SplitParts<COLS>& s, unsigned char* y_tile, int warp, int lane) {
+  constexpr int C = COLS / 128;
   const int rows = s.rows();
   for (int r = warp; r < rows; r += 8) {
-    unsigned char* out = y_tile + (size_t)(s.rank * rows + r) * p.N * 2;
+    float acc[C][4];
 #pragma unroll
-    for (int c = 0; c < COLS; c += 128) {
-      const int col = c + lane * 4;
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int k = 0; k < s.split; ++k) {
-        float v[4];
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                     : "r"(s.base + (uint32_t)(k * rows) * COLS * 4u + SplitParts<COLS>::at(rows, col / 4, r))
-                     : "memory");
+    for (int c = 0; c < C; ++c)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] += v[j];
-      }
+      for (int j = 0; j < 4; ++j) acc[c][j] = 0.f;
+#pragma unroll 1
+    for (int k = 0; k < s.split; k += 2) {  // 2, 4 or 8 parts
+      float v[2][C][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[u][c][0]), "=f"(v[u][c][1]), "=f"(v[u][c][2]), "=f"(v[u][c][3])
+                       : "r"(s.base + (uint32_t)((k + u) * rows) * COLS * 4u + SplitParts<COLS>::at(rows, c * 32 + lane, r))
+                       : "memory");
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[c][j] += v[u][c][j];
+    }
+    unsigned char* out = y_tile + (size_t)(s.rank * rows + r) * p.N * 2 + lane * 8;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
       uint2 o;
       __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
-      q[0] = __floats2bfloat162_rn(acc[0], acc[1]);
-      q[1] = __floats2bfloat162_rn(acc[2], acc[3]);
-      *reinterpret_cast<uint2*>(out + (size_t)col * 2) = o;
+      q[0] = __floats2bfloat162_rn(acc[c][0], acc[c][1]);
+      q[1] = __floats2bfloat162_rn(acc[c][2], acc[c][3]);
+      *reinterpret_cast<uint2*>(out + c * 256) = o;
     }
   }
 }
@@ -480,7 +494,7 @@ __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_bas
   cluster_sync_all();
   if (threadIdx.x == 0) split_spread_abort(s_abort, (uint32_t)(p.split * stride));
   __syncwarp();
-#pragma unroll 1
+#pragma unroll 2
   for (int c = 0; c < BN / 2; c += 32) {
     uint32_t r[32];
     tmem_ld32(tbase + (uint32_t)c, r);
