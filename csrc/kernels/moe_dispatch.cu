@@ -45,7 +45,7 @@ __host__ __device__ __forceinline__ size_t moe_row_bytes(int hidden, int fp8) {
 //     expert's group; the end of that launch is the barrier.
 // (A grid barrier inside one cooperative launch needed all CTAs resident at once, which a kernel of another stream can
 // prevent for as long as it waits for this dispatch, and a barrier that ran out left its counters behind. Exchange of 128
-// tokens of 7168, fp8: 24.8 us with the barrier, 24.1 now; 4096 tokens, bf16: 207.8 and 210.8, 219 with one routing CTA.)
+// tokens of 7168, fp8: 24.8 us with the barrier, 24.1 now; 4096 tokens, bf16: 207.5 and 208.5, 219 with one routing CTA.)
 // counters layout: [0,W) unused | [W,W+E) rows per expert | [W+E] done CTAs; zero between launches
 __device__ __forceinline__ void moe_ld_v8(const void* p, uint32_t (&v)[8]) {
   asm volatile("ld.global.cg.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -96,16 +96,21 @@ __global__ void __launch_bounds__(kMoeThreads) moe_count_kernel(eux_moe_desc d) 
   const int E = d.n_experts;
   const int64_t n = (int64_t)d.n_tokens * d.topk;
   const int64_t i0 = n * blockIdx.x / gridDim.x, i1 = n * (blockIdx.x + 1) / gridDim.x;
+  const int64_t first = i0 + threadIdx.x;  // all of a thread's entries up to 512 per SM: stays in registers
+  int e0 = first < i1 ? __ldg(d.topk_idx + first) : -1, rank0 = -1;
+  if (e0 >= E) e0 = -1;
   for (int e = threadIdx.x; e < E; e += blockDim.x) local[e] = 0;
   __syncthreads();
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+  if (e0 >= 0) rank0 = atomicAdd(&local[e0], 1);
+  for (int64_t i = first + blockDim.x; i < i1; i += blockDim.x) {
     const int e = __ldg(d.topk_idx + i);
     d.slot_of[i] = e >= 0 && e < E ? atomicAdd(&local[e], 1) : -1;  // the rank inside this CTA, for now
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) base[e] = local[e] ? atomicAdd(d.counters + d.world + e, local[e]) : 0;
   __syncthreads();
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+  if (first < i1) d.slot_of[first] = e0 >= 0 ? base[e0] + rank0 : -1;
+  for (int64_t i = first + blockDim.x; i < i1; i += blockDim.x) {
     const int rank = d.slot_of[i];
     if (rank >= 0) d.slot_of[i] = rank + base[__ldg(d.topk_idx + i)];
   }
@@ -125,6 +130,8 @@ __device__ __forceinline__ void moe_route(const eux_moe_desc& d, const MoeRoutin
     const int i = (int)threadIdx.x + j * kMoeThreads;
     expert[j] = i < n ? __ldg(d.topk_idx + i) : -1;
   }
+  const int64_t first = lo + threadIdx.x;
+  if (counted && first < hi) expert[0] = __ldg(d.topk_idx + first), rank[0] = d.slot_of[first];
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     r.local[e] = 0, r.base[e] = 0;
     r.total[e] = counted ? __ldcg(d.counters + W + e) : 0;
@@ -160,7 +167,8 @@ __device__ __forceinline__ void moe_route(const eux_moe_desc& d, const MoeRoutin
     d.slot_of[i] = slot < d.capacity ? slot : -1;
   };
   if (counted) {
-    for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+    if (first < hi) place(first, rank[0] >= 0 ? expert[0] : -1, rank[0]);
+    for (int64_t i = first + blockDim.x; i < hi; i += blockDim.x) {
       const int in_group = d.slot_of[i];
       place(i, in_group >= 0 ? __ldg(d.topk_idx + i) : -1, in_group);
     }
