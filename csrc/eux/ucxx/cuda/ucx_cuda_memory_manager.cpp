@@ -370,7 +370,9 @@ const UcxCudaMemoryResourceManager::Registration* UcxCudaMemoryResourceManager::
     }
   }
   std::lock_guard lk(mu_);
-  auto [it, ok] = regs_.emplace(reinterpret_cast<uintptr_t>(base), reg);
+  // An earlier allocation may be remembered at this very base: one that ended before `ptr`, so that the search above did
+  // not find it. It is gone, the driver has just named the one that is there now.
+  auto [it, added] = regs_.insert_or_assign(reinterpret_cast<uintptr_t>(base), reg);
   return &it->second;
 }
 

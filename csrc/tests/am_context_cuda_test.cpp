@@ -1,6 +1,7 @@
 // ucx_am_context with device memory on a real GPU: the CUDA forms of the context tests (the reference runs each
 // of its context tests with host and with CUDA buffers, ucx_am_context_test.cpp:1377-1945). Two contexts in one
 // process on GPU 0. Run by tests/test_native_gpu.py; needs a GPU, so it is not among the CPU test binaries.
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 
 #include <cstdlib>
@@ -293,6 +294,56 @@ EUX_TEST(a_device_transfer_in_flight_is_not_torn_by_a_stop_request) {
   auto again = pattern(4096, 3);
   UcxBuffer small = device_copy(p.cli.mr, again);
   CHECK(round(p, small, 2) == again);
+}
+
+template <typename Fn>
+static Fn driver(const char* name) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  CHECK(cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess);
+  return reinterpret_cast<Fn>(p);
+}
+
+// A tensor library's cache gives a segment back and gets a longer one at the same address: a tensor behind the end of
+// the old one is described by the new one.
+EUX_TEST(a_longer_allocation_at_a_remembered_base_is_exported) {
+  CHECK_EQ(cudaFree(nullptr), cudaSuccess);
+  auto granularity = driver<decltype(&cuMemGetAllocationGranularity)>("cuMemGetAllocationGranularity");
+  auto reserve = driver<decltype(&cuMemAddressReserve)>("cuMemAddressReserve");
+  auto give_back = driver<decltype(&cuMemAddressFree)>("cuMemAddressFree");
+  auto create = driver<decltype(&cuMemCreate)>("cuMemCreate");
+  auto release = driver<decltype(&cuMemRelease)>("cuMemRelease");
+  auto map = driver<decltype(&cuMemMap)>("cuMemMap");
+  auto unmap = driver<decltype(&cuMemUnmap)>("cuMemUnmap");
+  auto access = driver<decltype(&cuMemSetAccess)>("cuMemSetAccess");
+  CUmemAllocationProp prop{};
+  prop.type = CU_MEM_ALLOCATION_TYPE_PINNED;
+  prop.location.type = CU_MEM_LOCATION_TYPE_DEVICE;
+  prop.location.id = 0;
+  prop.requestedHandleTypes = CU_MEM_HANDLE_TYPE_POSIX_FILE_DESCRIPTOR;
+  size_t unit = 0;
+  CHECK_EQ(granularity(&unit, &prop, CU_MEM_ALLOC_GRANULARITY_MINIMUM), CUDA_SUCCESS);
+  CUdeviceptr base = 0;
+  CHECK_EQ(reserve(&base, 4 * unit, 0, 0, 0), CUDA_SUCCESS);
+  UcxCudaMemoryResourceManager mr(Node::options());
+  for (size_t units : {1, 4, 2}) {
+    CUmemGenericAllocationHandle h;
+    CHECK_EQ(create(&h, units * unit, &prop, 0), CUDA_SUCCESS);
+    CHECK_EQ(map(base, units * unit, 0, h, 0), CUDA_SUCCESS);
+    CUmemAccessDesc rw{};
+    rw.location = prop.location;
+    rw.flags = CU_MEM_ACCESS_FLAGS_PROT_READWRITE;
+    CHECK_EQ(access(base, units * unit, &rw, 1), CUDA_SUCCESS);
+    PeerRegionDesc d;
+    const size_t at = (units - 1) * unit + 512;  // behind the end of the allocation before
+    CHECK(mr.export_region(reinterpret_cast<void*>(base + at), 1024, &d));
+    CHECK_EQ(d.base, base);
+    CHECK_EQ(d.offset, at);
+    CHECK(!mr.export_region(reinterpret_cast<void*>(base + at), units * unit - at + 1, &d));
+    CHECK_EQ(unmap(base, units * unit), CUDA_SUCCESS);
+    CHECK_EQ(release(h), CUDA_SUCCESS);
+  }
+  CHECK_EQ(give_back(base, 4 * unit), CUDA_SUCCESS);
 }
 
 EUX_TEST_MAIN()
