@@ -63,10 +63,69 @@ struct GemmParams {
   const float* w_scale;       // [N/128, K/128], local
 };
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+// The loading role and the MMA role run as whole warps, and one elected lane issues: every TMA and tcgen05 instruction below
+// carries the election as a predicate (`issue`) instead of standing in a branch for lane 0, and the waits in front of them
+// end for all lanes at once. A K step of the tensor pipe takes 512 cycles. In a branch, a step's instructions alone took the
+// MMA thread 360 (bf16) to 530 (MX, with its scale copies) and the loading thread about 250 and 110 more for each load.
+// Calls of 4096^3 MXFP8 62 us before, 53 now; block-scaled fp8 on single CTAs, 512 x 4096 x 7168, 32.2 and 25.5; bf16, whose
+// K step is bound by the tensor pipe alone, level.
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e;
+}
+// One try by a whole warp, the same answer in every lane. CLUSTER: what the arriving CTA of the cluster wrote before its
+// arrive is visible afterwards.
+template <bool CLUSTER>
+__device__ __forceinline__ bool mbar_try_warp(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  if (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  return ok != 0;
+}
+// mbar_wait by a whole warp, which stays together: all lanes leave with the same answer
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort, uint64_t timeout_ns) {
+  uint64_t t0 = 0;
+  for (uint32_t it = 0; it < 0x7fffffffu; ++it) {
+    if (mbar_try_warp<CLUSTER>(bar, parity)) return true;
+    if ((it & 255u) == 255u) {
+      if (__any_sync(0xffffffffu, *abort != 0)) return false;
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, now - t0 > (timeout_ns ? timeout_ns : 2000000000ull))) break;
+    }
+  }
+  *abort = 1;
+  return false;
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t issue, uint32_t bar, uint32_t bytes) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-      "l"(map), "r"(bar), "r"(x), "r"(y)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t issue, uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
+      "l"(map), "r"(bar), "r"(x), "r"(y), "r"(issue)
       : "memory");
 }
 
@@ -81,23 +140,26 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 }
 
 template <bool FP8>
-__device__ __forceinline__ void umma(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma(uint32_t issue, uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   if (FP8) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
         : "memory");
   } else {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
         : "memory");
   }
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t issue, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(issue)
+      : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -389,6 +451,17 @@ __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   }
 }
 
+// The loading warp's wait for a panel of X that is on its way into the staging buffer. On time-out all roles are told.
+__device__ __forceinline__ bool panel_wait_warp(const GemmParams& p, int panel, int lane, volatile int* abort) {
+  bool arrived = true;
+  if (lane == 0) arrived = wait_u32_ge_gpu(p.panel_flags + panel, p.panel_target, p.timeout_ns);
+  arrived = __all_sync(0xffffffffu, arrived);
+  if (!arrived) *abort = 1;
+  __syncwarp();  // what lane 0 acquired is there for the lane that issues
+  asm volatile("fence.proxy.async;" ::: "memory");
+  return arrived;
+}
+
 __device__ __forceinline__ uint32_t cluster_cta_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -579,36 +652,42 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (!mbar_wait(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
     return *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
   };
+  auto next_tile_warp = [&](int it) -> int {
+    int tile = total;
+    if (mbar_wait_warp(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns))
+      tile = *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
+    return __shfl_sync(0xffffffffu, tile, 0);
+  };
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      for (int it = 0;; ++it) {
-        int tile;
-        if (SPLIT) tile = it == 0 ? tile0 : total;  // one tile per cluster
-        else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+    const uint32_t issue = elect_lane();
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0;; ++it) {
+      int tile = it == 0 ? tile0 : total;  // SPLIT: one tile per cluster
+      if (lane == 0) {
+        if (!SPLIT) tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
-        if (tile >= total) break;
-        int mb, nb;
-        tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-        if (p.panel_target > 0) {
-          if (!wait_u32_ge_gpu(p.panel_flags + mb, p.panel_target, p.timeout_ns)) {
-            *abort = 1;
-            break;
-          }
-          asm volatile("fence.proxy.async;" ::: "memory");
-        }
-        for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-          mbar_expect_tx(full_bar(s), A_STAGE_BYTES + B_STAGE_BYTES);
-          tma_load_2d(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_bar(s), (k_begin + k) * kelems, mb * BM);
-          tma_load_2d(smem_u32(sB + (size_t)s * B_STAGE_BYTES), &map_b, full_bar(s), (k_begin + k) * kelems, nb * BN);
-          if (++s == STAGES) s = 0, ph ^= 1u;
-        }
       }
+      tile = __shfl_sync(0xffffffffu, tile, 0);
+      if (tile >= total) break;
+      int mb, nb;
+      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+      if (p.panel_target > 0 && !panel_wait_warp(p, mb, lane, abort)) break;
+      int k = 0;
+      for (; k < k_iters; ++k) {
+        if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+        mbar_expect_tx(issue, full_bar(s), A_STAGE_BYTES + B_STAGE_BYTES);
+        tma_load_2d(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_bar(s), (k_begin + k) * kelems, mb * BM);
+        tma_load_2d(issue, b0 + (uint32_t)s * B_STAGE_BYTES, &map_b, full_bar(s), (k_begin + k) * kelems, nb * BN);
+        if (++s == STAGES) s = 0, ph ^= 1u;
+      }
+      if (k < k_iters) break;
+    }
+    if (lane == 0) {
       if (*abort) {  // let copies that are still in flight land before the CTA retires
         const uint64_t t0 = globaltimer_ns();
         while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -616,32 +695,30 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc<false, BN>();
-      int s = 0;
-      uint32_t ph = 0;
-      for (int it = 0;; ++it) {
-        if (next_tile(it) >= total) break;
-        const int buf = it & 1;
-        const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-        if (!mbar_wait(tempty_bar(buf), tph ^ 1u, abort, p.timeout_ns)) break;
+    constexpr uint32_t idesc = make_idesc<false, BN>();
+    const uint32_t issue = elect_lane();
+    const uint64_t adesc0 = umma_desc_sw128(smem_u32(sA)), bdesc0 = umma_desc_sw128(smem_u32(sB));
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0;; ++it) {
+      if (next_tile_warp(it) >= total) break;
+      const int buf = it & 1;
+      const uint32_t tph = (uint32_t)(it >> 1) & 1u;
+      if (!mbar_wait_warp(tempty_bar(buf), tph ^ 1u, abort, p.timeout_ns)) break;
+      tc_fence_after();
+      const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
+      int k = 0;
+      for (; k < k_iters; ++k) {
+        if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
         tc_fence_after();
-        const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
-        for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait(full_bar(s), ph, abort, p.timeout_ns)) break;
-          tc_fence_after();
-          const uint32_t a0 = smem_u32(sA + (size_t)s * A_STAGE_BYTES);
-          const uint32_t b0 = smem_u32(sB + (size_t)s * B_STAGE_BYTES);
+        const uint64_t ad = adesc0 + (uint32_t)s * (A_STAGE_BYTES >> 4), bd = bdesc0 + (uint32_t)s * (B_STAGE_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BKB / 32; ++kk) {
-            umma<false>(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)((k | kk) != 0));
-          }
-          umma_commit(empty_bar(s));
-          if (++s == STAGES) s = 0, ph ^= 1u;
-        }
-        if (*abort) break;  // a tile that is not complete is not announced
-        umma_commit(tfull_bar(buf));
+        for (int kk = 0; kk < BKB / 32; ++kk) umma<false>(issue, tacc, ad + kk * 2, bd + kk * 2, idesc, (uint32_t)((k | kk) != 0));
+        umma_commit(issue, empty_bar(s));
+        if (++s == STAGES) s = 0, ph ^= 1u;
       }
+      if (k < k_iters) break;  // a tile that is not complete is not announced
+      umma_commit(issue, tfull_bar(buf));
     }
   } else if (warp < 4) {
     // warps 2 and 3: X (and its scales) from the caller's memory into the staging buffer
@@ -833,65 +910,71 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     if (!mbar_wait(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
     return *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
   };
+  auto next_tile_warp = [&](int it) -> int {
+    int tile = total;
+    if (mbar_wait_warp(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns))
+      tile = *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
+    return __shfl_sync(0xffffffffu, tile, 0);
+  };
 
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      for (int it = 0;; ++it) {
-        int tile;
-        if (SPLIT) tile = it == 0 ? tile0 : total;  // one tile per cluster
-        else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+    const uint32_t issue = elect_lane();
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0;; ++it) {
+      int tile = it == 0 ? tile0 : total;  // SPLIT: one tile per cluster
+      if (lane == 0) {
+        if (!SPLIT) tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
-        if (tile >= total) break;
-        int mb, nb;
-        tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-        if (p.panel_target > 0) {
-          if (!wait_u32_ge_gpu(p.panel_flags + mb, p.panel_target, p.timeout_ns)) {
-            *abort = 1;
-            break;
-          }
-          asm volatile("fence.proxy.async;" ::: "memory");
-        }
-        for (int k = 0; k < k_blocks; ++k) {
-          if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-          mbar_expect_tx(full_bar(s), A8_STAGE_BYTES + B8_STAGE_BYTES);
-          tma_load_2d(smem_u32(sA + (size_t)s * A8_STAGE_BYTES), &map_a, full_bar(s), (k_begin + k) * 128, mb * BM);
-          tma_load_2d(smem_u32(sB + (size_t)s * B8_STAGE_BYTES), &map_b, full_bar(s), (k_begin + k) * 128, nb * BN8);
-          if (++s == STAGES8) s = 0, ph ^= 1u;
-        }
       }
+      tile = __shfl_sync(0xffffffffu, tile, 0);
+      if (tile >= total) break;
+      int mb, nb;
+      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+      if (p.panel_target > 0 && !panel_wait_warp(p, mb, lane, abort)) break;
+      int k = 0;
+      for (; k < k_blocks; ++k) {
+        if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+        mbar_expect_tx(issue, full_bar(s), A8_STAGE_BYTES + B8_STAGE_BYTES);
+        tma_load_2d(issue, a0 + (uint32_t)s * A8_STAGE_BYTES, &map_a, full_bar(s), (k_begin + k) * 128, mb * BM);
+        tma_load_2d(issue, b0 + (uint32_t)s * B8_STAGE_BYTES, &map_b, full_bar(s), (k_begin + k) * 128, nb * BN8);
+        if (++s == STAGES8) s = 0, ph ^= 1u;
+      }
+      if (k < k_blocks) break;
+    }
+    if (lane == 0) {
       if (*abort) {
         const uint64_t t0 = globaltimer_ns();
         while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc<true, BN8>();
-      int s = 0;
-      uint32_t ph = 0;
-      uint32_t blk = 0;  // running K-block count: selects the TMEM buffer and its phase
-      for (int it = 0;; ++it) {
-        if (next_tile(it) >= total || *abort) break;
-        for (int k = 0; k < k_blocks && !*abort; ++k, ++blk) {
-          const int buf = blk & (TBUF8 - 1);
-          const uint32_t tph = (blk / TBUF8) & 1u;
-          if (!mbar_wait(tempty_bar(buf), tph ^ 1u, abort, p.timeout_ns)) break;
-          if (!mbar_wait(full_bar(s), ph, abort, p.timeout_ns)) break;
-          tc_fence_after();
-          const uint32_t tacc = tmem_base + (uint32_t)buf * BN8;
-          const uint32_t a0 = smem_u32(sA + (size_t)s * A8_STAGE_BYTES);
-          const uint32_t b0 = smem_u32(sB + (size_t)s * B8_STAGE_BYTES);
+    constexpr uint32_t idesc = make_idesc<true, BN8>();
+    const uint32_t issue = elect_lane();
+    const uint64_t adesc0 = umma_desc_sw128(smem_u32(sA)), bdesc0 = umma_desc_sw128(smem_u32(sB));
+    int s = 0;
+    uint32_t ph = 0;
+    uint32_t blk = 0;  // running K-block count: selects the TMEM buffer and its phase
+    for (int it = 0;; ++it) {
+      if (next_tile_warp(it) >= total) break;
+      int k = 0;
+      for (; k < k_blocks; ++k, ++blk) {
+        const int buf = blk & (TBUF8 - 1);
+        const uint32_t tph = (blk / TBUF8) & 1u;
+        if (!mbar_wait_warp(tempty_bar(buf), tph ^ 1u, abort, p.timeout_ns)) break;
+        if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
+        tc_fence_after();
+        const uint32_t tacc = tmem_base + (uint32_t)buf * BN8;
+        const uint64_t ad = adesc0 + (uint32_t)s * (A8_STAGE_BYTES >> 4), bd = bdesc0 + (uint32_t)s * (B8_STAGE_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BKB / 32; ++kk)
-            umma<true>(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)(kk != 0));
-          umma_commit(empty_bar(s));
-          umma_commit(tfull_bar(buf));
-          if (++s == STAGES8) s = 0, ph ^= 1u;
-        }
+        for (int kk = 0; kk < BKB / 32; ++kk) umma<true>(issue, tacc, ad + kk * 2, bd + kk * 2, idesc, (uint32_t)(kk != 0));
+        umma_commit(issue, tfull_bar(buf));
+        umma_commit(issue, empty_bar(s));
+        if (++s == STAGES8) s = 0, ph ^= 1u;
       }
+      if (k < k_blocks) break;
     }
   } else if (warp < 4) {
     // warps 2 and 3: X (and its scales) from the caller's memory into the staging buffer
@@ -1079,39 +1162,51 @@ __device__ __forceinline__ void mbar_arrive_remote_tmem(uint32_t cluster_addr) {
 }
 // per-CTA tile load of a CTA pair: the bytes land in this CTA, the completion is counted on `bar`, a
 // shared::cluster address (the even CTA's barrier)
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster, int x, int y) {
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t issue, uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster, int x, int y) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-      "l"(map), "r"(bar_cluster), "r"(x), "r"(y)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
+      "l"(map), "r"(bar_cluster), "r"(x), "r"(y), "r"(issue)
       : "memory");
 }
-__device__ __forceinline__ void umma_pair(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_pair(uint32_t issue, uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
-// arrives on one barrier (shared::cluster address) when the pair's MMAs issued so far are done
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster) : "memory");
+// arrives on the barrier at this offset in every CTA of `mask` (bits are cluster ranks) when the pair's MMAs issued so far
+// are done: one commit for both CTAs
+__device__ __forceinline__ void umma_commit_pair(uint32_t issue, uint32_t bar, uint32_t mask) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t.reg .b16 m;\n\tsetp.ne.b32 q, %2, 0;\n\tcvt.u16.u32 m, %1;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(bar),
+      "r"(mask), "r"(issue)
+      : "memory");
 }
 
 // 128 rows x 4 scale bytes (512 bytes of shared memory, rows of 16 bytes, 8-row groups 128 bytes apart) into
 // four TMEM columns of every lane quarter, in both CTAs of the pair
-__device__ __forceinline__ void sf_to_tmem_pair(uint32_t tmem_col, uint32_t smem_addr) {
+__device__ __forceinline__ uint64_t sf_desc(uint32_t smem_addr) {
   uint64_t d = 0;
   d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
   d |= (uint64_t)(128u >> 4) << 32;  // stride byte offset
   d |= (uint64_t)1 << 46;            // descriptor version; no swizzle
-  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(d) : "memory");
+  return d;
 }
-__device__ __forceinline__ void umma_mx_pair(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t tmem_sfa,
-                                             uint32_t tmem_sfb, uint32_t accumulate) {
+__device__ __forceinline__ void sf_to_tmem_pair(uint32_t issue, uint32_t tmem_col, uint64_t desc) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(tmem_c),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n\t}" ::"r"(tmem_col), "l"(desc), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void umma_mx_pair(uint32_t issue, uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(tmem_c),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb), "r"(issue)
       : "memory");
 }
 
@@ -1193,99 +1288,106 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     if (!mbar_wait_cluster(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
     return *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
   };
+  auto next_tile_warp = [&](int it) -> int {
+    int tile = total;
+    if (mbar_wait_warp<true>(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns))
+      tile = *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
+    return __shfl_sync(0xffffffffu, tile, 0);
+  };
 
   if (warp == 0) {
     // ---------------- loads: both CTAs, completion counted in the even CTA ----------------
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      for (int it = 0;; ++it) {
-        int tile;
-        if (leader) {
-          if (SPLIT) tile = it == 0 ? tile0 : total;  // one tile per cluster
-          else tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+    const uint32_t issue = elect_lane();
+    const uint32_t issue_leader = leader ? issue : 0u;
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB), f0 = smem_u32(sSF);
+    const uint32_t full0 = map_to_cta(full_bar(0), even);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int it = 0;; ++it) {
+      int tile = it == 0 ? tile0 : total;  // SPLIT: one tile per cluster
+      if (leader) {
+        if (lane == 0) {
+          if (!SPLIT) tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
           const int slot = it & (TILE_RING - 1);
           s_tiles[slot] = tile;
           mbar_arrive(tile_bar(slot));
           st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), even | 1u), (uint32_t)tile);
           mbar_arrive_remote(map_to_cta(tile_bar(slot), even | 1u));
-        } else {
-          tile = next_tile(it);
         }
-        if (tile >= total) break;
-        int mb, nb;
-        tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-        if (p.panel_target > 0 && (2 * mb + (int)rank) * BM < p.M) {  // this CTA's 128 rows of the 256-row block
-          if (!wait_u32_ge_gpu(p.panel_flags + 2 * mb + (int)rank, p.panel_target, p.timeout_ns)) {
-            *abort = 1;
-            break;
-          }
-          asm volatile("fence.proxy.async;" ::: "memory");
-        }
-        for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-          const uint32_t full_leader = map_to_cta(full_bar(s), even);
-          if (leader) mbar_expect_tx(full_bar(s), 2 * PairCfg<MX>::STAGE_BYTES);
-          tma_load_2d_pair(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_leader, (k_begin + k) * kelems, mb * 2 * BM + (int)rank * BM);
-          tma_load_2d_pair(smem_u32(sB + (size_t)s * B2_STAGE_BYTES), &map_b, full_leader, (k_begin + k) * kelems, nb * BN + (int)rank * (BN / 2));
-          if (MX) {  // this CTA's X scales of the step, and the whole tile's Wt scales (each CTA needs all 256 in its TMEM)
-            const uint32_t sf = smem_u32(sSF + (size_t)s * SF_STAGE_BYTES);
-            tma_load_2d_pair(sf, &map_sfa, full_leader, 0, (mb * 2 + (int)rank) * k_all + k_begin + k);
-            tma_load_2d_pair(sf + 512, &map_sfb, full_leader, 0, (k_begin + k) * (p.N / 128) + nb * 2);
-          }
-          if (++s == STAGES2) s = 0, ph ^= 1u;
-        }
+        tile = __shfl_sync(0xffffffffu, tile, 0);
+      } else {
+        tile = next_tile_warp(it);
       }
-      if (*abort) {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+      if (tile >= total) break;
+      int mb, nb;
+      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+      const int panel = 2 * mb + (int)rank;  // this CTA's 128 rows of the 256-row block
+      if (p.panel_target > 0 && panel * BM < p.M && !panel_wait_warp(p, panel, lane, abort)) break;
+      int k = 0;
+      for (; k < k_iters; ++k) {
+        if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+        const uint32_t full_leader = full0 + 8u * (uint32_t)s;
+        mbar_expect_tx(issue_leader, full_bar(s), 2 * PairCfg<MX>::STAGE_BYTES);
+        tma_load_2d_pair(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_leader, (k_begin + k) * kelems, panel * BM);
+        tma_load_2d_pair(issue, b0 + (uint32_t)s * B2_STAGE_BYTES, &map_b, full_leader, (k_begin + k) * kelems, nb * BN + (int)rank * (BN / 2));
+        if (MX) {  // this CTA's X scales of the step, and the whole tile's Wt scales (each CTA needs all 256 in its TMEM)
+          const uint32_t sf = f0 + (uint32_t)s * SF_STAGE_BYTES;
+          tma_load_2d_pair(issue, sf, &map_sfa, full_leader, 0, panel * k_all + k_begin + k);
+          tma_load_2d_pair(issue, sf + 512, &map_sfb, full_leader, 0, (k_begin + k) * (p.N / 128) + nb * 2);
+        }
+        if (++s == STAGES2) s = 0, ph ^= 1u;
       }
+      if (k < k_iters) break;
     }
+    if (*abort && lane == 0) {  // let copies that are still in flight land before the CTA retires
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
+    __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA: the even CTA issues for the pair ----------------
-    if (leader && lane == 0) {
+    if (leader) {
       // bf16: D fp32 (bit 4), A and B bf16 (bits 7, 10). MX: A and B e4m3 (zero), scales UE8M0 (bit 23); the
       // 32-element block of the K-step goes into bits 29..30 (X scales) and 4..5 (Wt scales) per instruction.
       constexpr uint32_t idesc = (MX ? (1u << 23) : ((1u << 4) | (1u << 7) | (1u << 10))) | ((uint32_t)(BN >> 3) << 17) |
                                  ((uint32_t)((2 * BM) >> 4) << 24);
+      const uint32_t issue = elect_lane();
+      const uint32_t both = 3u << even;
+      const uint64_t adesc0 = umma_desc_sw128(smem_u32(sA)), bdesc0 = umma_desc_sw128(smem_u32(sB));
+      const uint64_t sdesc0 = sf_desc(smem_u32(sSF));
+      const uint32_t tsf = tmem_base + SF_TMEM_COL;
       int s = 0;
       uint32_t ph = 0;
       for (int it = 0;; ++it) {
-        if (next_tile(it) >= total || *abort) break;
+        if (next_tile_warp(it) >= total) break;
         const int buf = it % NBUF;
         const uint32_t tph = (uint32_t)(it / NBUF) & 1u;
-        if (!mbar_wait(tempty_bar(buf), tph ^ 1u, abort, p.timeout_ns)) break;
+        if (!mbar_wait_warp(tempty_bar(buf), tph ^ 1u, abort, p.timeout_ns)) break;
         tc_fence_after();
         const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
-        for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait(full_bar(s), ph, abort, p.timeout_ns)) break;
+        int k = 0;
+        for (; k < k_iters; ++k) {
+          if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
           tc_fence_after();
-          const uint32_t a0 = smem_u32(sA + (size_t)s * A_STAGE_BYTES);
-          const uint32_t b0 = smem_u32(sB + (size_t)s * B2_STAGE_BYTES);
+          const uint64_t ad = adesc0 + (uint32_t)s * (A_STAGE_BYTES >> 4), bd = bdesc0 + (uint32_t)s * (B2_STAGE_BYTES >> 4);
           if (MX) {
             // the step's scale factors into TMEM, in both CTAs; the tensor pipe runs them before the MMAs below
-            const uint32_t sf = smem_u32(sSF + (size_t)s * SF_STAGE_BYTES);
-            const uint32_t tsf = tmem_base + SF_TMEM_COL;
-            sf_to_tmem_pair(tsf, sf);
-            sf_to_tmem_pair(tsf + 4, sf + 512);
-            sf_to_tmem_pair(tsf + 8, sf + 1024);
+            const uint64_t sd = sdesc0 + (uint32_t)s * (SF_STAGE_BYTES >> 4);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) sf_to_tmem_pair(issue, tsf + 4 * i, sd + i * (512 >> 4));
 #pragma unroll
             for (int kk = 0; kk < BKB / 32; ++kk)
-              umma_mx_pair(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32),
-                           idesc | ((uint32_t)kk << 29) | ((uint32_t)kk << 4), tsf, tsf + 4, (uint32_t)((k | kk) != 0));
+              umma_mx_pair(issue, tacc, ad + kk * 2, bd + kk * 2, idesc | ((uint32_t)kk << 29) | ((uint32_t)kk << 4), tsf, tsf + 4,
+                           (uint32_t)((k | kk) != 0));
           } else {
 #pragma unroll
-            for (int kk = 0; kk < BKB / 32; ++kk)
-              umma_pair(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)((k | kk) != 0));
+            for (int kk = 0; kk < BKB / 32; ++kk) umma_pair(issue, tacc, ad + kk * 2, bd + kk * 2, idesc, (uint32_t)((k | kk) != 0));
           }
-          // the stage is free in both CTAs once these MMAs have read it
-          umma_commit_pair(empty_bar(s));
-          umma_commit_pair(map_to_cta(empty_bar(s), even | 1u));
+          umma_commit_pair(issue, empty_bar(s), both);  // the stage is free in both CTAs once these MMAs have read it
           if (++s == STAGES2) s = 0, ph ^= 1u;
         }
-        if (*abort) break;  // a tile that is not complete is not announced
-        umma_commit_pair(tfull_bar(buf));
-        umma_commit_pair(map_to_cta(tfull_bar(buf), even | 1u));
+        if (k < k_iters) break;  // a tile that is not complete is not announced
+        umma_commit_pair(issue, tfull_bar(buf), both);
       }
     }
   } else if (warp < 4) {
@@ -1436,11 +1538,11 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-__device__ __forceinline__ void umma_fp8_pair(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_fp8_pair(uint32_t issue, uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_c),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
 
@@ -1501,76 +1603,84 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     if (!mbar_wait_cluster(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
     return *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
   };
+  auto next_tile_warp = [&](int it) -> int {
+    int tile = total;
+    if (mbar_wait_warp<true>(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns))
+      tile = *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
+    return __shfl_sync(0xffffffffu, tile, 0);
+  };
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS8P_OTHERS));
     if (warp == 0) {
       // ---------------- loads: both CTAs, completion counted in the even CTA ----------------
-      if (lane == 0) {
-        int s = 0;
-        uint32_t ph = 0;
-        for (int it = 0;; ++it) {
-          int tile;
-          if (leader) {
+      const uint32_t issue = elect_lane();
+      const uint32_t issue_leader = leader ? issue : 0u;
+      const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+      const uint32_t full0 = map_to_cta(full_bar(0), 0);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int it = 0;; ++it) {
+        int tile = 0;
+        if (leader) {
+          if (lane == 0) {
             tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
             const int slot = it & (TILE_RING - 1);
             s_tiles[slot] = tile;
             mbar_arrive(tile_bar(slot));
             st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), 1), (uint32_t)tile);
             mbar_arrive_remote(map_to_cta(tile_bar(slot), 1));
-          } else {
-            tile = next_tile(it);
           }
-          if (tile >= total) break;
-          int mb, nb;
-          tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-          const int panel = 2 * mb + (int)rank;  // this CTA's 128 rows (past M for the odd CTA of a last half block)
-          if (p.panel_target > 0 && panel * BM < p.M) {
-            if (!wait_u32_ge_gpu(p.panel_flags + panel, p.panel_target, p.timeout_ns)) {
-              *abort = 1;
-              break;
-            }
-            asm volatile("fence.proxy.async;" ::: "memory");
-          }
-          for (int k = 0; k < k_blocks; ++k) {
-            if (!mbar_wait(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-            const uint32_t full_leader = map_to_cta(full_bar(s), 0);
-            if (leader) mbar_expect_tx(full_bar(s), 2 * STAGE8P_BYTES);
-            tma_load_2d_pair(smem_u32(sA + (size_t)s * A_STAGE_BYTES), &map_a, full_leader, k * 128, panel * BM);
-            tma_load_2d_pair(smem_u32(sB + (size_t)s * B2_STAGE_BYTES), &map_b, full_leader, k * 128, nb * BN + (int)rank * (BN / 2));
-            if (++s == STAGES8P) s = 0, ph ^= 1u;
-          }
+          tile = __shfl_sync(0xffffffffu, tile, 0);
+        } else {
+          tile = next_tile_warp(it);
         }
-        if (*abort) {
-          const uint64_t t0 = globaltimer_ns();
-          while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+        if (tile >= total) break;
+        int mb, nb;
+        tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+        const int panel = 2 * mb + (int)rank;  // this CTA's 128 rows (past M for the odd CTA of a last half block)
+        if (p.panel_target > 0 && panel * BM < p.M && !panel_wait_warp(p, panel, lane, abort)) break;
+        int k = 0;
+        for (; k < k_blocks; ++k) {
+          if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+          const uint32_t full_leader = full0 + 8u * (uint32_t)s;
+          mbar_expect_tx(issue_leader, full_bar(s), 2 * STAGE8P_BYTES);
+          tma_load_2d_pair(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_leader, k * 128, panel * BM);
+          tma_load_2d_pair(issue, b0 + (uint32_t)s * B2_STAGE_BYTES, &map_b, full_leader, k * 128, nb * BN + (int)rank * (BN / 2));
+          if (++s == STAGES8P) s = 0, ph ^= 1u;
         }
+        if (k < k_blocks) break;
       }
+      if (*abort && lane == 0) {
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+      }
+      __syncwarp();
     } else if (warp == 1) {
       // ---------------- MMA: the even CTA issues for the pair, one partial product per K-block ----------------
-      if (leader && lane == 0) {
+      if (leader) {
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+        const uint32_t issue = elect_lane();
+        const uint64_t adesc0 = umma_desc_sw128(smem_u32(sA)), bdesc0 = umma_desc_sw128(smem_u32(sB));
         int s = 0;
         uint32_t ph = 0, blk = 0;
         for (int it = 0;; ++it) {
-          if (next_tile(it) >= total || *abort) break;
-          for (int k = 0; k < k_blocks && !*abort; ++k, ++blk) {
+          if (next_tile_warp(it) >= total) break;
+          int k = 0;
+          for (; k < k_blocks; ++k, ++blk) {
             const int buf = blk & 1u;
-            if (!mbar_wait(tempty_bar(buf), ((blk >> 1) & 1u) ^ 1u, abort, p.timeout_ns)) break;
-            if (!mbar_wait(full_bar(s), ph, abort, p.timeout_ns)) break;
+            if (!mbar_wait_warp(tempty_bar(buf), ((blk >> 1) & 1u) ^ 1u, abort, p.timeout_ns)) break;
+            if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
             tc_fence_after();
             const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
-            const uint32_t a0 = smem_u32(sA + (size_t)s * A_STAGE_BYTES);
-            const uint32_t b0 = smem_u32(sB + (size_t)s * B2_STAGE_BYTES);
+            const uint64_t ad = adesc0 + (uint32_t)s * (A_STAGE_BYTES >> 4), bd = bdesc0 + (uint32_t)s * (B2_STAGE_BYTES >> 4);
 #pragma unroll
-            for (int kk = 0; kk < BKB / 32; ++kk)
-              umma_fp8_pair(tacc, umma_desc_sw128(a0 + kk * 32), umma_desc_sw128(b0 + kk * 32), idesc, (uint32_t)(kk != 0));
-            umma_commit_pair(tfull_bar(buf));
-            umma_commit_pair(map_to_cta(tfull_bar(buf), 1));
-            umma_commit_pair(empty_bar(s));
-            umma_commit_pair(map_to_cta(empty_bar(s), 1));
+            for (int kk = 0; kk < BKB / 32; ++kk) umma_fp8_pair(issue, tacc, ad + kk * 2, bd + kk * 2, idesc, (uint32_t)(kk != 0));
+            umma_commit_pair(issue, tfull_bar(buf), 3u);
+            umma_commit_pair(issue, empty_bar(s), 3u);
             if (++s == STAGES8P) s = 0, ph ^= 1u;
           }
+          if (k < k_blocks) break;
         }
       }
     } else {
