@@ -1515,29 +1515,36 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 }
 
 // ---------------------------------------------------------------------------
-// Block-scaled fp8 on CTA pairs: the promotion scheme of remote_gemm_fp8_kernel on 256 x 256 tiles. What bounds the
-// 128 x 128 kernel is the operand feed from L2 (about 13 TB/s over all SMs, 46 bytes per SM and cycle): its K-block
-// brings 32 KiB into an SM for 256 cycles of MMA. Here the same 32 KiB serve twice the MMAs. A CTA's 128 x 256 partial
-// product fills half of its TMEM, so two are in flight; each of the eight epilogue warps folds 32 rows by 128 columns
-// into 128 registers (the register file is split unevenly: setmaxnreg). Rows and columns past M and N (both are
-// multiples of 128, a tile is 256) are zero-filled loads, and nothing is stored for them.
+// Block-scaled fp8 on CTA pairs: the promotion scheme of remote_gemm_fp8_kernel on 256 x 256 tiles, half the operand bytes
+// per flop. What bounds it is the fold: a K-block is 512 cycles of MMA and takes about 1000. So:
+//   * Sixteen warps fold, 32 rows by 64 columns each. The arithmetic of the fold is 280 cycles per K-block; the rest of a
+//     warp's chain (waiting, TMEM loads, the arrive) is latency, which four warps per scheduler hide better than two.
+//   * The loading warp multiplies and stages the scales, eight K-blocks at a time, so that a fold reads one word. Staged by
+//     the folding warps they cost each of them 200 cycles per K-block. It holds a batch in registers while it issues loads.
+// 1920 x 4608 x 7168: 74.9 us with eight folding warps that staged their scales, 64.6 now (calls in a loop). Tried: the two
+// halves of the columns as products of their own, four in flight (66.5 to 74: the MMA warp waits and commits more often).
+// Twenty warps of 96 registers fill the register file; a twenty-first would leave each 80.
+// Rows and columns past M and N (both are multiples of 128, a tile is 256) are zero-filled loads, and nothing is stored
+// for them.
 // ---------------------------------------------------------------------------
 constexpr int STAGES8P = 5;
-constexpr int GEMM8P_THREADS = 384;  // warp 0 TMA, warp 1 MMA (even CTA), warps 2 and 3 copy X, warps 4..11 epilogue
+constexpr int FOLD_WARPS = 16;
+constexpr int GEMM8P_THREADS = (4 + FOLD_WARPS) * 32;  // warp 0 TMA and scales, warp 1 MMA (even CTA), 2 and 3 copy X, 4..19 fold
 constexpr int STAGE8P_BYTES = A_STAGE_BYTES + B2_STAGE_BYTES;
-constexpr int SCALE8P_K = 8;                                // K-blocks of scales per batch
-constexpr int SCALE8P_FLOATS = 33 * (SCALE8P_K + 1);        // 32 rows of X scales and one of Wt scales, odd pitch
-constexpr size_t GEMM8P_SMEM =
-    (size_t)STAGES8P * STAGE8P_BYTES + 2 * EPI_SLAB_BYTES + 8 * 2 * SCALE8P_FLOATS * sizeof(float) + 1024 + 256;
-// 168 registers per thread at launch; 128 x 96 + 256 x 200 = 63488 of the 384 x 168 = 64512 that the block has
-constexpr int REGS8P_OTHERS = 96, REGS8P_EPILOGUE = 200;
+constexpr int SCALE8P_K = 8;               // K-blocks of scales per batch
+constexpr int SCALE8P_PITCH = BM + 4;      // words from one K-block to the next: the staging stores meet 32 different banks
+constexpr int SCALE8P_FLOATS = 2 * SCALE8P_K * SCALE8P_PITCH;  // a batch, for both halves of the columns
+constexpr int EPI8P_BYTES = 16 * 128;      // a folding warp's own slab: 16 rows of 64 columns
+constexpr size_t GEMM8P_SMEM = (size_t)STAGES8P * STAGE8P_BYTES + FOLD_WARPS * EPI8P_BYTES + 2 * SCALE8P_FLOATS * sizeof(float) + 1024 + 256;
 
-__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-
 __device__ __forceinline__ void umma_fp8_pair(uint32_t issue, uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
@@ -1553,10 +1560,11 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = smem;
   unsigned char* sB = smem + (size_t)STAGES8P * A_STAGE_BYTES;
-  unsigned char* sEpi = smem + (size_t)STAGES8P * STAGE8P_BYTES;  // one slab per half
-  float* sScale = reinterpret_cast<float*>(sEpi + 2 * EPI_SLAB_BYTES);  // two batches for each epilogue warp
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sScale + 8 * 2 * SCALE8P_FLOATS);
-  // bars: [0,S) full (used in the even CTA), [S,2S) empty, then 2 tmem_full, 2 tmem_empty (even CTA), TILE_RING tile slots
+  unsigned char* sEpi = smem + (size_t)STAGES8P * STAGE8P_BYTES;
+  float* sScale = reinterpret_cast<float*>(sEpi + FOLD_WARPS * EPI8P_BYTES);  // two batches
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sScale + 2 * SCALE8P_FLOATS);
+  // bars: [0,S) full (used in the even CTA), [S,2S) empty, then 2 tmem_full, 2 tmem_empty (even CTA), 2 scale_full,
+  // 2 scale_empty, TILE_RING tile slots
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
   __shared__ int s_tiles[TILE_RING];
@@ -1568,7 +1576,9 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   auto empty_bar = [&](int s) { return bar0 + 8u * (STAGES8P + s); };
   auto tfull_bar = [&](int b) { return bar0 + 8u * (2 * STAGES8P + b); };
   auto tempty_bar = [&](int b) { return bar0 + 8u * (2 * STAGES8P + 2 + b); };
-  auto tile_bar = [&](int i) { return bar0 + 8u * (2 * STAGES8P + 4 + i); };
+  auto sfull_bar = [&](int b) { return bar0 + 8u * (2 * STAGES8P + 4 + b); };
+  auto sempty_bar = [&](int b) { return bar0 + 8u * (2 * STAGES8P + 6 + b); };
+  auto tile_bar = [&](int i) { return bar0 + 8u * (2 * STAGES8P + 8 + i); };
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int i = 0; i < TILE_RING; ++i) mbar_init(tile_bar(i), 1);
@@ -1578,7 +1588,9 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 16);  // eight epilogue warps in each CTA of the pair
+      mbar_init(tempty_bar(b), 2 * FOLD_WARPS);  // of both CTAs
+      mbar_init(sfull_bar(b), 1);
+      mbar_init(sempty_bar(b), FOLD_WARPS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1599,10 +1611,6 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   const int total = m_blocks * n_blocks;
   const int k_blocks = p.K / 128;
   volatile int* abort = &s_abort;
-  auto next_tile = [&](int it) -> int {
-    if (!mbar_wait_cluster(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns)) return total;
-    return *(volatile int*)&s_tiles[it & (TILE_RING - 1)];
-  };
   auto next_tile_warp = [&](int it) -> int {
     int tile = total;
     if (mbar_wait_warp<true>(tile_bar(it & (TILE_RING - 1)), (uint32_t)(it / TILE_RING) & 1u, abort, p.timeout_ns))
@@ -1610,157 +1618,149 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     return __shfl_sync(0xffffffffu, tile, 0);
   };
 
-  if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS8P_OTHERS));
-    if (warp == 0) {
-      // ---------------- loads: both CTAs, completion counted in the even CTA ----------------
-      const uint32_t issue = elect_lane();
-      const uint32_t issue_leader = leader ? issue : 0u;
-      const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
-      const uint32_t full0 = map_to_cta(full_bar(0), 0);
-      int s = 0;
-      uint32_t ph = 0;
-      for (int it = 0;; ++it) {
-        int tile = 0;
-        if (leader) {
-          if (lane == 0) {
-            tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
-            const int slot = it & (TILE_RING - 1);
-            s_tiles[slot] = tile;
-            mbar_arrive(tile_bar(slot));
-            st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), 1), (uint32_t)tile);
-            mbar_arrive_remote(map_to_cta(tile_bar(slot), 1));
-          }
-          tile = __shfl_sync(0xffffffffu, tile, 0);
-        } else {
-          tile = next_tile_warp(it);
+  if (warp == 0) {
+    // ---------------- loads: both CTAs, completion counted in the even CTA; and the scales ----------------
+    const uint32_t issue = elect_lane();
+    const uint32_t issue_leader = leader ? issue : 0u;
+    const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+    const uint32_t full0 = map_to_cta(full_bar(0), 0);
+    int s = 0;
+    uint32_t ph = 0, batch = 0;
+    const int k8 = lane & 7, r4 = lane >> 3;
+    for (int it = 0;; ++it) {
+      int tile = 0;
+      if (leader) {
+        if (lane == 0) {
+          tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+          const int slot = it & (TILE_RING - 1);
+          s_tiles[slot] = tile;
+          mbar_arrive(tile_bar(slot));
+          st_shared_remote_u32(map_to_cta(smem_u32(&s_tiles[slot]), 1), (uint32_t)tile);
+          mbar_arrive_remote(map_to_cta(tile_bar(slot), 1));
         }
-        if (tile >= total) break;
-        int mb, nb;
-        tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-        const int panel = 2 * mb + (int)rank;  // this CTA's 128 rows (past M for the odd CTA of a last half block)
-        if (p.panel_target > 0 && panel * BM < p.M && !panel_wait_warp(p, panel, lane, abort)) break;
+        tile = __shfl_sync(0xffffffffu, tile, 0);
+      } else {
+        tile = next_tile_warp(it);
+      }
+      if (tile >= total) break;
+      int mb, nb;
+      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+      const int panel = 2 * mb + (int)rank;  // this CTA's 128 rows (past M for the odd CTA of a last half block)
+      const bool rows_inside = panel * BM < p.M;
+      if (p.panel_target > 0 && rows_inside && !panel_wait_warp(p, panel, lane, abort)) break;  // X and its scales
+      // A batch of scales: eight lanes read eight K-blocks of a row, one sector, from L2 (where pulled scales arrive).
+      const float* sx = p.x_scale_stage + (size_t)(panel * BM + r4) * k_blocks + k8;
+      const float* sw = p.w_scale + (size_t)(nb * 2) * k_blocks + k8;
+      const bool right = nb * 2 + 1 < p.N / 128;
+      float v[BM / 4], w0, w1;
+      auto fetch = [&](int k) {
+        const bool in = rows_inside && k + k8 < k_blocks;
+#pragma unroll
+        for (int i = 0; i < BM / 4; ++i) v[i] = in ? __ldcg(sx + (size_t)(i * 4) * k_blocks + k) : 0.f;
+        w0 = in ? __ldg(sw + k) : 0.f;
+        w1 = in && right ? __ldg(sw + k_blocks + k) : 0.f;
+      };
+      fetch(0);
+      int k = 0;
+      for (; k < k_blocks; ++k) {
+        if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+        const uint32_t full_leader = full0 + 8u * (uint32_t)s;
+        mbar_expect_tx(issue_leader, full_bar(s), 2 * STAGE8P_BYTES);
+        tma_load_2d_pair(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_leader, k * 128, panel * BM);
+        tma_load_2d_pair(issue, b0 + (uint32_t)s * B2_STAGE_BYTES, &map_b, full_leader, k * 128, nb * BN + (int)rank * (BN / 2));
+        if (++s == STAGES8P) s = 0, ph ^= 1u;
+        // Four steps into a batch its scales leave: the loads have come back by then, and no product of the batch is done.
+        // (The two batches before it are at most seven steps of loads and products behind, so this wait is short.)
+        if (k % SCALE8P_K == 3 || (k == k_blocks - 1 && k % SCALE8P_K < 3)) {
+          if (!mbar_wait_warp(sempty_bar((int)(batch & 1u)), ((batch >> 1) & 1u) ^ 1u, abort, p.timeout_ns)) break;
+          float* out = sScale + (batch & 1u) * SCALE8P_FLOATS + k8 * SCALE8P_PITCH + r4;
+#pragma unroll
+          for (int i = 0; i < BM / 4; ++i) {
+            out[i * 4] = v[i] * w0;
+            out[SCALE8P_K * SCALE8P_PITCH + i * 4] = v[i] * w1;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sfull_bar((int)(batch & 1u)));
+          ++batch;
+          if (k / SCALE8P_K * SCALE8P_K + SCALE8P_K < k_blocks) fetch(k / SCALE8P_K * SCALE8P_K + SCALE8P_K);
+        }
+      }
+      if (k < k_blocks) break;
+    }
+    if (*abort && lane == 0) {  // loads in flight still write shared memory: give them time to land
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------- MMA: the even CTA issues for the pair, one partial product per K-block ----------------
+    if (leader) {
+      constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+      const uint32_t issue = elect_lane();
+      const uint64_t adesc0 = umma_desc_sw128(smem_u32(sA)), bdesc0 = umma_desc_sw128(smem_u32(sB));
+      int s = 0;
+      uint32_t ph = 0, blk = 0;
+      for (int it = 0;; ++it) {
+        if (next_tile_warp(it) >= total) break;
         int k = 0;
-        for (; k < k_blocks; ++k) {
-          if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-          const uint32_t full_leader = full0 + 8u * (uint32_t)s;
-          mbar_expect_tx(issue_leader, full_bar(s), 2 * STAGE8P_BYTES);
-          tma_load_2d_pair(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_leader, k * 128, panel * BM);
-          tma_load_2d_pair(issue, b0 + (uint32_t)s * B2_STAGE_BYTES, &map_b, full_leader, k * 128, nb * BN + (int)rank * (BN / 2));
+        for (; k < k_blocks; ++k, ++blk) {
+          const int buf = blk & 1u;
+          if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
+          if (!mbar_wait_warp(tempty_bar(buf), ((blk >> 1) & 1u) ^ 1u, abort, p.timeout_ns)) break;
+          tc_fence_after();
+          const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
+          const uint64_t ad = adesc0 + (uint32_t)s * (A_STAGE_BYTES >> 4), bd = bdesc0 + (uint32_t)s * (B2_STAGE_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < BKB / 32; ++kk) umma_fp8_pair(issue, tacc, ad + kk * 2, bd + kk * 2, idesc, (uint32_t)(kk != 0));
+          umma_commit_pair(issue, tfull_bar(buf), 3u);
+          umma_commit_pair(issue, empty_bar(s), 3u);
           if (++s == STAGES8P) s = 0, ph ^= 1u;
         }
         if (k < k_blocks) break;
       }
-      if (*abort && lane == 0) {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-      }
-      __syncwarp();
-    } else if (warp == 1) {
-      // ---------------- MMA: the even CTA issues for the pair, one partial product per K-block ----------------
-      if (leader) {
-        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
-        const uint32_t issue = elect_lane();
-        const uint64_t adesc0 = umma_desc_sw128(smem_u32(sA)), bdesc0 = umma_desc_sw128(smem_u32(sB));
-        int s = 0;
-        uint32_t ph = 0, blk = 0;
-        for (int it = 0;; ++it) {
-          if (next_tile_warp(it) >= total) break;
-          int k = 0;
-          for (; k < k_blocks; ++k, ++blk) {
-            const int buf = blk & 1u;
-            if (!mbar_wait_warp(tempty_bar(buf), ((blk >> 1) & 1u) ^ 1u, abort, p.timeout_ns)) break;
-            if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
-            tc_fence_after();
-            const uint32_t tacc = tmem_base + (uint32_t)buf * BN;
-            const uint64_t ad = adesc0 + (uint32_t)s * (A_STAGE_BYTES >> 4), bd = bdesc0 + (uint32_t)s * (B2_STAGE_BYTES >> 4);
-#pragma unroll
-            for (int kk = 0; kk < BKB / 32; ++kk) umma_fp8_pair(issue, tacc, ad + kk * 2, bd + kk * 2, idesc, (uint32_t)(kk != 0));
-            umma_commit_pair(issue, tfull_bar(buf), 3u);
-            umma_commit_pair(issue, empty_bar(s), 3u);
-            if (++s == STAGES8P) s = 0, ph ^= 1u;
-          }
-          if (k < k_blocks) break;
-        }
-      }
-    } else {
-      // ---------------- warps 2 and 3: X and its scales from the caller's memory into the staging buffer ----------------
-      if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
     }
-    __syncwarp();
+  } else if (warp < 4) {
+    // ---------------- warps 2 and 3: X and its scales from the caller's memory into the staging buffer ----------------
+    if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS8P_EPILOGUE));
-    const int lg = (warp - 4) & 3;     // TMEM lane group
-    const int half = (warp - 4) >> 2;  // which 128 columns of the tile: one block of W's scales
-    const int row_local = lg * 32 + lane;
-    const bool elected = lg == 0 && lane == 0;
-    const uint32_t sbuf = smem_u32(sEpi) + (uint32_t)half * EPI_SLAB_BYTES;
+    // ---------------- fold: a warp has 32 rows (the TMEM lanes it may read) by 64 columns ----------------
+    const int lg = warp & 3;
+    const int quarter = (warp - 4) >> 2;  // which 64 columns of the tile
+    const int half = quarter >> 1;        // 128 columns: one block of W's scales
+    const uint32_t sbuf = smem_u32(sEpi) + (uint32_t)(warp - 4) * EPI8P_BYTES;
     const uint32_t tempty0 = map_to_cta(tempty_bar(0), 0);
-    float* my_scales = sScale + (size_t)(warp - 4) * 2 * SCALE8P_FLOATS;
-    uint32_t blk = 0;
+    const uint32_t tcol = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(quarter * 64);
+    const uint32_t sc0 = smem_u32(sScale) + (uint32_t)(half * SCALE8P_K * SCALE8P_PITCH + lg * 32 + lane) * 4u;
+    uint32_t blk = 0, batch = 0;
     for (int it = 0;; ++it) {
-      const int tile = next_tile(it);
-      if (epi_vote_any(1 + half, tile >= total)) break;
-      int mb, nb;
-      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
-      const int panel = 2 * mb + (int)rank;
-      const int nblk = nb * 2 + half;
-      const bool inside = panel * BM < p.M && nblk * 128 < p.N;  // the same for all threads of a half
-      const float* sx = p.x_scale_stage + (size_t)(panel * BM + lg * 32) * k_blocks;  // of this warp's first row
-      const float* sw = p.w_scale + (size_t)nblk * k_blocks;
-      float acc[128];
+      const int tile = next_tile_warp(it);
+      if (tile >= total) break;
+      float acc[64];
 #pragma unroll
-      for (int j = 0; j < 128; ++j) acc[j] = 0.f;
-      bool ok = true;
-      if (p.panel_target > 0 && inside) {  // the scales of pulled rows are there once their panel is reported
-        int arrived = 1;
-        if (lane == 0) arrived = wait_u32_ge_gpu(p.panel_flags + panel, p.panel_target, p.timeout_ns) ? 1 : 0;
-        arrived = __shfl_sync(0xffffffffu, arrived, 0);
-        if (!arrived) {
-          *abort = 1;
-          ok = false;
-        }
-      }
-      // Eight K-blocks of this warp's scales at a time: asynchronous copies into the warp's own buffer, one batch
-      // ahead. (Fetched into registers K-block by K-block, the loads in flight held up the arrive below, which waits
-      // for them: 171 us instead of 85 on 1920 x 4608 x 7168.)
-      auto stage_scales = [&](int batch) {
-        float* buf = my_scales + (batch & 1) * SCALE8P_FLOATS;
-        if (ok && inside) {
-#pragma unroll
-          for (int i = 0; i < SCALE8P_K; ++i) {
-            const int row = i * 4 + (lane >> 3), k = batch * SCALE8P_K + (lane & 7);
-            if (k < k_blocks) cp_async_4(smem_u32(buf + row * (SCALE8P_K + 1) + (lane & 7)), sx + (size_t)row * k_blocks + k);
-          }
-          const int k = batch * SCALE8P_K + lane;
-          if (lane < SCALE8P_K && k < k_blocks) cp_async_4(smem_u32(buf + 32 * (SCALE8P_K + 1) + lane), sw + k);
-        }
-        cp_async_commit();
-      };
-      __syncwarp();
-      stage_scales(0);
-      for (int k = 0; ok && k < k_blocks; ++k, ++blk) {
+      for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+      int k = 0;
+      for (; k < k_blocks; ++k, ++blk) {
         const int j8 = k % SCALE8P_K;
         if (j8 == 0) {
-          __syncwarp();  // every lane has read the buffer that the next batch goes into
-          stage_scales(k / SCALE8P_K + 1);
-          cp_async_wait_1();
-          __syncwarp();
+          if (k > 0) {  // this warp has read the batch before
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sempty_bar((int)(batch & 1u)));
+            ++batch;
+          }
+          if (!mbar_wait_warp(sfull_bar((int)(batch & 1u)), (batch >> 1) & 1u, abort, p.timeout_ns)) break;
         }
+        float scale;
+        asm volatile("ld.shared.f32 %0, [%1];"
+                     : "=f"(scale)
+                     : "r"(sc0 + (uint32_t)((batch & 1u) * SCALE8P_FLOATS + j8 * SCALE8P_PITCH) * 4u)
+                     : "memory");
         const int buf = blk & 1u;
-        const uint32_t tph = (blk >> 1) & 1u;
-        if (!mbar_wait(tfull_bar(buf), tph, abort, p.timeout_ns)) {
-          ok = false;
-          break;
-        }
+        if (!mbar_wait_warp(tfull_bar(buf), (blk >> 1) & 1u, abort, p.timeout_ns)) break;
         tc_fence_after();
-        const float* sc = my_scales + ((k / SCALE8P_K) & 1) * SCALE8P_FLOATS;
-        const float scale = inside ? sc[lane * (SCALE8P_K + 1) + j8] * sc[32 * (SCALE8P_K + 1) + j8] : 0.f;
-        const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)buf * BN + (uint32_t)half * 128;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tbase + c * 32, r);
+          uint32_t r[16];
+          tmem_ld16(tcol + (uint32_t)(buf * BN + c * 16), r);
           tmem_ld_wait();
           if (c == 3) {
             tc_fence_before();
@@ -1768,34 +1768,42 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
             if (lane == 0) mbar_arrive_remote_tmem(tempty0 + 8u * buf);  // in registers: the buffer may be overwritten
           }
 #pragma unroll
-          for (int j = 0; j < 32; j += 2)
-            ffma2(acc[c * 32 + j], acc[c * 32 + j + 1], __uint_as_float(r[j]), __uint_as_float(r[j + 1]), scale);
+          for (int j = 0; j < 16; j += 2)
+            ffma2(acc[c * 16 + j], acc[c * 16 + j + 1], __uint_as_float(r[j]), __uint_as_float(r[j + 1]), scale);
         }
       }
-      if (epi_vote_any(1 + half, !ok)) break;
-      if (!inside) continue;
+      if (k < k_blocks) break;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sempty_bar((int)(batch & 1u)));
+      ++batch;
+      int mb, nb;
+      tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+      const int row0 = (2 * mb + (int)rank) * BM + lg * 32, col0 = nb * BN + quarter * 64;
+      if (row0 >= p.M || col0 >= p.N) continue;
+      // 16 rows at a time through the warp's slab, so that Y is written in full lines
 #pragma unroll
-      for (int sl = 0; sl < 2; ++sl) {
-        if (elected) bulk_wait_read_0();  // the store before this one has read the slab
-        epi_bar_sync(1 + half);
+      for (int h = 0; h < 2; ++h) {
+        if (lane == 0) bulk_wait_read_0();  // the store before this one has read the slab
+        __syncwarp();
+        if ((lane >> 4) == h) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint4 o;
-          __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
+          for (int c = 0; c < 8; ++c) {
+            uint4 o;
+            __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            q[j] = __floats2bfloat162_rn(acc[sl * 64 + c * 8 + 2 * j], acc[sl * 64 + c * 8 + 2 * j + 1]);
-          st_shared_u4(sbuf + (uint32_t)row_local * 128u + (uint32_t)((c ^ (row_local & 7)) * 16), o);
+            for (int j = 0; j < 4; ++j) q[j] = __floats2bfloat162_rn(acc[c * 8 + 2 * j], acc[c * 8 + 2 * j + 1]);
+            st_shared_u4(sbuf + (uint32_t)(lane & 15) * 128u + (uint32_t)((c ^ (lane & 7)) * 16), o);
+          }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        epi_bar_sync(1 + half);
-        if (elected) {
-          tma_store_2d(&map_y, sbuf, nblk * 128 + sl * 64, panel * BM);
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&map_y, sbuf, col0, row0 + h * 16);
           bulk_commit();
         }
       }
     }
-    if (elected) {
+    if (lane == 0) {
       bulk_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");
     }
@@ -2023,15 +2031,17 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   // 14.6). CTAs that copy X before they compute keep to whole tiles.
   const bool pairs_bf16 = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) && !d->fp8 &&
                           (d->M % (2 * BM) == 0 || ((!pull || copy_by_warps) && waves2 <= waves && k_iters >= 24));
-  // Block-scaled fp8 on CTA pairs: a K-block takes 0.7 to 0.8 us of a pair's 256 x 256 tile and 0.5 to 0.6 us of a CTA's
-  // 128 x 128 tile (calls in a loop: 1920 x 4608 x 7168 78 us against 104; 512 x 4096 x 7168, one wave of either, 44
-  // against 35), so the pairs are taken when they need at most 7 / 10 of the waves and K is not short. Pulled scales are
-  // read through L1, which is sound while no line holds rows of two panels: their staging buffer starts on a line.
-  const bool pairs_fp8 = d->fp8 && !mx && (!pull || (copy_by_warps && ((uintptr_t)d->x_scale_stage & 127u) == 0)) &&
-                         waves2 * 10 <= waves * 7 && k_iters >= 16;
+  // Block-scaled fp8 on CTA pairs: a K-block takes 0.54 us of a pair's 256 x 256 tile and 0.35 us of a CTA's 128 x 128
+  // tile, so the pairs are taken when they need at most 5 / 8 of the waves and K is not short (calls in a loop, pairs and
+  // single CTAs: 1920 x 4608 x 7168, two waves of four, 65 and 84 us; 2560 x 4096 x 4096, three of five, 58 and 62;
+  // 1536 x 4096 x 2048, two of three, 27 and 24; 4096 x 4096 x 512 23 and 23).
+  const bool pairs_fp8 = d->fp8 && !mx && (!pull || copy_by_warps) && waves2 * 8 <= waves * 5 && k_iters >= 16;
   if (mx || pairs_bf16 || pairs_fp8) {
     CUtensorMap mb2;  // this CTA's half of a Wt tile: 128 rows
     if (int rc = make_map(&mb2, d->w_t, eb, (uint64_t)d->N, (uint64_t)d->K, BN / 2)) return rc;
+    // the folding warps of block-scaled fp8 store 16 rows at a time
+    if (pairs_fp8)
+      if (int rc = make_map(&my, d->y_dst, 2, (uint64_t)d->M, (uint64_t)d->N, 16)) return rc;
     int copy_pairs = pull ? (copy_ctas + 1) / 2 : 0;
     if (copy_pairs > sms / 2 - 1) copy_pairs = sms / 2 - 1;
     p.copy_ctas = 2 * copy_pairs;

@@ -224,3 +224,32 @@ def test_a_wait_that_runs_out(cuda_device, fmt, m, n, k):
     g(*ptrs, m, want.data_ptr(), x_is_local=True)
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("m,n,k", [(1408, 2944, 2176), (1408, 2944, 2304), (1920, 4480, 2560), (3968, 2688, 2944), (2048, 4096, 2048)])
+@pytest.mark.parametrize("pull", [False, "warps"])
+def test_block_scaled_fp8_pairs_fold(cuda_device, m, n, k, pull):
+    """At most 5 / 8 of the waves: CTA pairs, whose scales come in batches of eight K-blocks. One to three tiles per pair,
+    half tiles at the end of M and of N, last batches of one, two, four, seven and eight K-blocks."""
+    test_block_scaled_fp8_pairs(cuda_device, m, n, k, pull)
+
+
+def test_block_scaled_fp8_pairs_give_up(cuda_device):
+    test_a_wait_that_runs_out(cuda_device, "fp8_block", 1920, 4480, 2048)
+
+
+def test_block_scaled_fp8_pairs_scales_off_a_line(cuda_device):
+    """Pulled scales whose staging buffer starts on 16 bytes and no more: the same result as with scales in place."""
+    from execution_ucx_b200.ops import remote_gemm as rg
+    m, n, k = 1408, 2944, 2304
+    torch.manual_seed(5)
+    g = rg.RemoteGemmFp8(torch.randn(k, n, device=cuda_device) * 0.02, m)
+    g.x_scale_stage = torch.empty(g.x_scale_stage.numel() + 4, device=cuda_device)[4:].view(g.x_scale_stage.shape)
+    assert g.x_scale_stage.data_ptr() % 128 == 16
+    xq, xs = rg.quantize_rows_1x128(torch.randn(m, k, device=cuda_device))
+    y, want = (torch.empty(m, n, dtype=torch.bfloat16, device=cuda_device) for _ in range(2))
+    g(xq.data_ptr(), xs.data_ptr(), m, y.data_ptr(), x_is_local=False)
+    g(xq.data_ptr(), xs.data_ptr(), m, want.data_ptr(), x_is_local=True)
+    torch.cuda.synchronize()
+    g.check_status()
+    assert torch.equal(y, want)
