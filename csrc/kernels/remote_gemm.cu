@@ -395,23 +395,29 @@ __device__ __forceinline__ void copy_warp_role(const GemmParams& p, uint32_t war
   };
   auto count = [&](int panel) {
     __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      red_release_gpu_add(p.panel_flags + panel, 1u);
-    }
+    if (lane == 0) red_release_gpu_add(p.panel_flags + panel, 1u);  // covers the warp's stores from before the barrier
   };
   int pending = -1;  // panel of the unit whose stores have been issued but not counted
   uint32_t u = draw();
   while (u < total) {
     const uint32_t panel = u / per_panel, w = u % per_panel;
     if (w < scale_units) {
-      // a slice of this panel's scales: few and small, copied and counted at once
+      // a slice of this panel's scales, counted at once
       const size_t begin = (size_t)panel * scale_panel_bytes + ((size_t)w << 13);
-      const size_t end = min((size_t)panel * scale_panel_bytes + scale_panel_bytes, begin + 8192);
-      const unsigned char* ss = reinterpret_cast<const unsigned char*>(p.x_scale_src);
-      unsigned char* sd = reinterpret_cast<unsigned char*>(p.x_scale_stage);
-      for (size_t i = begin + (size_t)lane * 16; i < end; i += 512)
-        *reinterpret_cast<uint4*>(sd + i) = __ldcg(reinterpret_cast<const uint4*>(ss + i));
+      const int n = (int)min(scale_panel_bytes - ((size_t)w << 13), (size_t)8192) - lane * 16;  // bytes from this lane's first on
+      const unsigned char* ss = reinterpret_cast<const unsigned char*>(p.x_scale_src) + begin + lane * 16;
+      unsigned char* sd = reinterpret_cast<unsigned char*>(p.x_scale_stage) + begin + lane * 16;
+      // half a unit's loads on their way before the first is stored: one by one, a unit took ten microseconds, and no panel
+      // was complete before its scales (first tiles of 4096^3 MXFP8 from 14 us on, now from 8)
+#pragma unroll 1
+      for (int b = 0; b < n; b += 4096) {
+        uint4 q[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) q[j] = b + j * 512 < n ? __ldcg(reinterpret_cast<const uint4*>(ss + b + j * 512)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+          if (b + j * 512 < n) *reinterpret_cast<uint4*>(sd + b + j * 512) = q[j];
+      }
       const uint32_t next = draw();
       count((int)panel);
       u = next;
