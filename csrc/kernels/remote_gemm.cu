@@ -439,6 +439,13 @@ __device__ __forceinline__ void copy_warp_role(const GemmParams& p, uint32_t war
   if (lane == 0) __threadfence();  // the counts are in before this CTA is counted as done: the last one clears them
 }
 
+// Programmatic dependent launch: a GEMM may be launched while the kernel before it in the stream still runs, sets up its
+// barriers and TMEM on SMs that have become free, and waits here until that kernel is complete and visible, before it
+// touches anything in memory. (Nothing to wait for in a plain launch.) 2 to 2.5 us per call otherwise, between the end of one
+// kernel and the first load of the next: 128 x 8192 x 8192 bf16 32.8 us without and 30.4 with, fp8 20.5 and 18.6.
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   __syncthreads();
   if (threadIdx.x != 0) return;
@@ -604,7 +611,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
+  allow_next_launch();
   if ((int)blockIdx.x < p.copy_ctas) {
+    wait_for_launch_before();
     // first the transfer of X, then this CTA computes tiles like the others
     const bool ok = copy_role_n(p, GEMM_THREADS, smem_raw);
     if (!ok) {
@@ -656,6 +665,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  wait_for_launch_before();
 
   const int m_blocks = p.M / BM, n_blocks = p.N / BN;
   const int total = m_blocks * n_blocks;
@@ -868,7 +878,9 @@ __global__ void __launch_bounds__(GEMM8_THREADS, 1)
 remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
+  allow_next_launch();
   if ((int)blockIdx.x < p.copy_ctas) {
+    wait_for_launch_before();
     // first the transfer of X and its scales, then this CTA computes tiles like the others
     const bool ok = copy_role_n(p, GEMM8_THREADS, smem_raw);
     if (!ok) {
@@ -917,6 +929,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  wait_for_launch_before();
   const int m_blocks = p.M / BM, n_blocks = p.N / BN8;
   const int total = m_blocks * n_blocks;
   const int kscales = p.K / 128;
@@ -1238,7 +1251,9 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   constexpr int NBUF = PairCfg<MX>::NBUF;
   extern __shared__ unsigned char smem_raw[];
   bool copy_ok = true;
+  allow_next_launch();
   if ((int)blockIdx.x < p.copy_ctas) {
+    wait_for_launch_before();
     // whole pairs copy X first (copy_ctas is even). A CTA whose copy failed still walks through the
     // rest with its abort flag set: its partner waits for it at the cluster barriers.
     copy_ok = copy_role_n(p, GEMM_THREADS, smem_raw);
@@ -1291,6 +1306,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   cluster_sync_all();  // the partner's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  wait_for_launch_before();
 
   const int m_blocks = (p.M + 2 * BM - 1) / (2 * BM), n_blocks = p.N / BN;
   const int total = m_blocks * n_blocks;
@@ -1576,6 +1592,7 @@ __global__ void __launch_bounds__(GEMM8P_THREADS, 1)
 remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                             const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
+  allow_next_launch();
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = smem;
   unsigned char* sB = smem + (size_t)STAGES8P * A_STAGE_BYTES;
@@ -1625,6 +1642,7 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   cluster_sync_all();  // the partner's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  wait_for_launch_before();
 
   const int m_blocks = (p.M + 2 * BM - 1) / (2 * BM), n_blocks = (p.N + BN - 1) / BN;
   const int total = m_blocks * n_blocks;
@@ -1900,16 +1918,18 @@ static cudaError_t allow_smem(int dev, size_t smem) {
 
 struct ClusterLaunch {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   ClusterLaunch(int cluster, int grid, int threads, size_t smem, cudaStream_t st) {
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = cluster > 1 ? 1 : 0;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
   }
 };
 

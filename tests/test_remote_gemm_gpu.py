@@ -253,3 +253,38 @@ def test_block_scaled_fp8_pairs_scales_off_a_line(cuda_device):
     torch.cuda.synchronize()
     g.check_status()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("m,k", [(128, 2048), (640, 1024), (1024, 1024), (2304, 2048)])
+@pytest.mark.parametrize("pull", [False, True, "ctas"])
+def test_calls_behind_one_another(cuda_device, m, k, pull):
+    """A call may be launched while the kernel before it runs. A chain of calls in which every X is the Y of the call before
+    (by turns as it is and after an elementwise kernel), on one scratch: the same bits as with a synchronisation after each,
+    from plain calls and from a captured graph."""
+    from execution_ucx_b200.ops.remote_gemm import RemoteGemm
+    torch.manual_seed(m + k)
+    x = torch.randn(m, k, device=cuda_device).to(torch.bfloat16)
+    g = RemoteGemm((torch.randn(k, k, device=cuda_device) * k ** -0.5).to(torch.bfloat16), m)
+    bufs = [torch.empty_like(x) for _ in range(9)]
+
+    def chain(sync):
+        bufs[0].copy_(x)
+        for i in range(8):
+            g(bufs[i].data_ptr(), m, bufs[i + 1].data_ptr(), x_is_local=not pull, copy_ctas=16 if pull == "ctas" else 0)
+            if i & 1:
+                bufs[i + 1].mul_(0.5)
+            if sync:
+                torch.cuda.synchronize()
+
+    chain(True)
+    want = [b.clone() for b in bufs]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(False)
+    for run in (lambda: chain(False), graph.replay):
+        for b in bufs:
+            b.zero_()
+        run()
+        torch.cuda.synchronize()
+        g.check_status()
+        assert all(torch.equal(b, w) for b, w in zip(bufs, want))
