@@ -57,13 +57,6 @@ __device__ __forceinline__ void moe_st_v8(void* p, const uint32_t (&v)[8]) {
                "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
-// Programmatic dependent launch, which takes the 2 to 2.5 us between two kernels of a stream out of the exchange: what
-// follows may be launched while this kernel runs ... (The dispatch behind its count launch and the expert flag behind the
-// dispatch: 1024 bf16 tokens of 7168 69 -> 64 us, 4096 209 -> 205. Not the combine: while the expert flag waits for peers,
-// its CTAs would hold every SM against the kernels of other streams, perhaps the very ones that the peers wait for.)
-__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// ... and waits here until everything before it is complete and visible. (Nothing to wait for in a plain launch.)
-__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 struct MoeRouting {
   int* local;  // [E] rows of this CTA per expert; then rows of all experts before e, whatever their rank
   int* base;   // [E] where this CTA's rows start inside the destination's region
@@ -99,7 +92,6 @@ constexpr int kRouteSelf = 4096;
 // line; where each expert's first entry made it, 4096 x 7168 took 4 us more.)
 __global__ void __launch_bounds__(kMoeThreads) moe_count_kernel(eux_moe_desc d) {
   extern __shared__ int moe_sm[];
-  allow_next_launch();
   int* const local = moe_sm;
   int* const base = moe_sm + d.n_experts;
   const int E = d.n_experts;
@@ -266,12 +258,10 @@ __device__ __forceinline__ unsigned char* shfl_ptr(unsigned char* p, int src) {
 // lane once and stores them to each of the token's top-k destinations.
 __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_bf16_kernel(eux_moe_desc d, int counted) {
   extern __shared__ int moe_sm[];
-  allow_next_launch();
   const MoeRouting r{moe_sm, moe_sm + d.n_experts, moe_sm + 2 * d.n_experts};
   const int t0 = moe_first_token(d, blockIdx.x, gridDim.x), t1 = moe_first_token(d, blockIdx.x + 1, gridDim.x);
   __shared__ uint64_t* flags[kMaxWorld];
   if ((int)threadIdx.x < d.world) flags[threadIdx.x] = d.flag_peer[threadIdx.x];
-  wait_for_launch_before();
   moe_route(d, r, t0, t1, counted != 0);
   moe_send_counts(d, r, flags);
   const int EPR = d.n_experts / d.world, K = d.topk;
@@ -322,13 +312,11 @@ __host__ __device__ __forceinline__ int moe_scale_stride(int hidden) { return mo
 
 __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_moe_desc d, int counted) {
   extern __shared__ int moe_sm[];
-  allow_next_launch();
   const MoeRouting r{moe_sm, moe_sm + d.n_experts, moe_sm + 2 * d.n_experts};
   float* const scales = reinterpret_cast<float*>(moe_sm + 3 * d.n_experts);
   const int t0 = moe_first_token(d, blockIdx.x, gridDim.x), t1 = moe_first_token(d, blockIdx.x + 1, gridDim.x);
   __shared__ uint64_t* flags[kMaxWorld];
   if ((int)threadIdx.x < d.world) flags[threadIdx.x] = d.flag_peer[threadIdx.x];
-  wait_for_launch_before();
   moe_route(d, r, t0, t1, counted != 0);
   moe_send_counts(d, r, flags);
   const int EPR = d.n_experts / d.world, K = d.topk;
@@ -403,7 +391,6 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
 
 // ---- expert side: wait for every source, (identity expert), tell the sources -
 __global__ void moe_expert_ready_kernel(eux_moe_desc d) {
-  wait_for_launch_before();
   const int W = d.world;
   __shared__ int s_ok;
   if (threadIdx.x == 0) s_ok = 1;
@@ -777,19 +764,6 @@ using namespace eux;
 
 extern "C" size_t eux_moe_row_bytes(int hidden, int fp8) { return moe_row_bytes(hidden, fp8); }
 
-// A launch that may begin while the kernel before it in the stream is still running: the kernel has to wait for that itself.
-template <typename... Args>
-static int launch_early(void (*kernel)(Args...), int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem, cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr, cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 template <auto KERNEL>
 static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream_t st) {
   int dev = 0, sms = 148;
@@ -807,7 +781,6 @@ static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream
   if (counted) {
     const int64_t want = (entries + kMoeThreads - 1) / kMoeThreads;
     moe_count_kernel<<<(int)std::min<int64_t>(want, sms), kMoeThreads, 2 * (size_t)d->n_experts * sizeof(int), st>>>(*d);
-    return launch_early(KERNEL, grid, kMoeThreads, smem, st, *d, counted);
   }
   KERNEL<<<grid, kMoeThreads, smem, st>>>(*d, counted);
   return (int)cudaGetLastError();
@@ -822,7 +795,8 @@ extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* st
 
 extern "C" int eux_moe_expert_ready_launch(const eux_moe_desc* d, void* stream) {
   if (int rc = moe_check(d)) return rc;
-  return launch_early(moe_expert_ready_kernel, 1, 32, 0, (cudaStream_t)stream, *d);
+  moe_expert_ready_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(*d);
+  return (int)cudaGetLastError();
 }
 
 // ---- combine, fp8 rows, top-k <= 8, hidden <= 8192: the streaming scheme of the bf16 kernel. A unit is 1024
