@@ -49,6 +49,26 @@ __device__ __forceinline__ void red_release_gpu_add(uint32_t* p, uint32_t v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Programmatic dependent launch, which takes the 2 to 2.5 us between the end of one kernel of a stream and the first load of
+// the next away: what follows may be launched while this kernel runs (a kernel that waits for another GPU or stream does not
+// call this: what it lets in would hold SMs for as long) ...
+__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// ... and a kernel launched so waits here until everything before it in the stream is complete and visible, before it touches
+// memory. (Nothing to wait for in a plain launch.)
+__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The launch of a kernel that calls wait_for_launch_before.
+template <typename... Args>
+static inline int launch_early(void (*kernel)(Args...), int grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid), cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Spin until *flag >= value. Gives up after timeout_ns (0 = 2 s default) or
 // 2^31 polls, whichever comes first; returns false on give-up.
 __device__ __forceinline__ bool wait_flag_ge(const uint64_t* flag, uint64_t value, uint64_t timeout_ns) {

@@ -439,13 +439,6 @@ __device__ __forceinline__ void copy_warp_role(const GemmParams& p, uint32_t war
   if (lane == 0) __threadfence();  // the counts are in before this CTA is counted as done: the last one clears them
 }
 
-// Programmatic dependent launch: a GEMM may be launched while the kernel before it in the stream still runs, sets up its
-// barriers and TMEM on SMs that have become free, and waits here until that kernel is complete and visible, before it
-// touches anything in memory. (Nothing to wait for in a plain launch.) 2 to 2.5 us per call otherwise, between the end of one
-// kernel and the first load of the next: 128 x 8192 x 8192 bf16 32.8 us without and 30.4 with, fp8 20.5 and 18.6.
-__device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   __syncthreads();
   if (threadIdx.x != 0) return;
@@ -1924,6 +1917,8 @@ struct ClusterLaunch {
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
+    // A GEMM may be launched while the kernel before it in the stream still runs: a CTA sets up its barriers and TMEM on an
+    // SM that has become free and waits there (128 x 8192 x 8192 bf16 32.8 us per call without and 30.4 with, fp8 20.5 and 18.6).
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;

@@ -357,3 +357,43 @@ def test_rpc_echo_step_single_launch(cuda_device, n, op, arg):
                      flags.data_ptr(), flags.data_ptr() + 8, 7, status_ptr=status.data_ptr(), wait_timeout_ns=20_000_000)
     torch.cuda.synchronize()
     assert int(status[0]) & 0xff == 1 and int(flags[0]) == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(64, 96), (1000, 1040), (3000, 2056)])
+def test_pushes_behind_one_another(cuda_device, rows, cols):
+    """A push may be launched while the one before it runs. A chain over every route (typed, tiles, bytes, gathers, single
+    elements, thin matrices), each reading what the one before it wrote, with an elementwise kernel of another library in
+    between: what torch computes for the chain, from plain calls and from a captured graph."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    x = torch.randn(rows, cols, device=cuda_device)
+    a = torch.empty(rows, cols, dtype=torch.bfloat16, device=cuda_device)
+    b = torch.empty(cols, rows, dtype=torch.bfloat16, device=cuda_device)
+    c = torch.empty_like(b)
+    d = torch.empty(cols, rows - 8, dtype=torch.float32, device=cuda_device)
+    e = torch.empty(cols * (rows - 8) - 1, dtype=torch.float32, device=cuda_device)
+    f = torch.empty((cols * (rows - 8) - 2) // 3, 3, dtype=torch.float32, device=cuda_device)
+    g = torch.empty(3, f.shape[0], dtype=torch.float32, device=cuda_device)
+
+    def chain():
+        tx.push(x, a, op=tx.OP_MUL, op_arg=0.5)
+        tx.push(a.t(), b)
+        tx.push(b, c)
+        c.add_(1.0)
+        tx.push(c[:, 8:], d)
+        tx.push(d.view(-1)[1:], e)
+        tx.push(e[:f.numel()].view(-1, 3), f)
+        tx.push(f.t(), g, op=tx.OP_ADD, op_arg=2.0)
+
+    want = ((x * 0.5).to(torch.bfloat16).t().contiguous() + 1.0)[:, 8:].float().reshape(-1)[1:]
+    want = want[:f.numel()].view(-1, 3).t() + 2.0
+    graph = torch.cuda.CUDAGraph()
+    chain()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        chain()
+    for run in (chain, chain, graph.replay, graph.replay):
+        for buf in (a, b, c, d, e, f, g):
+            buf.zero_()
+        run()
+        torch.cuda.synchronize()
+        assert torch.equal(g, want)
