@@ -22,6 +22,7 @@
 // exists.
 #include <algorithm>
 
+#include "eux_bulk.cuh"
 #include "eux_device.cuh"
 
 namespace eux {
@@ -386,6 +387,167 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
       for (int g = lane; g < ngroups; g += 32) so[g] = sc[tl * ngroups + g];
     }
   }
+  moe_publish(d, flags);
+}
+
+// ---- dispatch, e4m3 rows, two tokens per CTA and more: row images in shared memory, moved by bulk copies -------------------
+// Twelve warps quantise units of (token, 1024 elements) into images of whole rows (values, scales, padding) in a ring of
+// slots; four warps send the finished images to their top-k rows, a bulk copy each. The kernel above has what its registers
+// hold in flight and a barrier in front of the scales: 43 % of the DRAM's rate at 4096 tokens of 7168. Dispatches in a
+// loop, above and here: 4096 x 7168 75.1 and 65.0 us, 4096 x 2048 32.6 and 25.9, 1024 x 7168 25.7 and 23.0, 300 x 7168 16.0
+// and 15.9, 128 x 7168 13.3 and 14.1 (with one sending warp 65.4, 34.0, 22.8, 15.8: its look-ups are a trip to L2 per token).
+// Token tl of the CTA: slot tl % slots, barriers tl % 32, sending warp tl % 4. The number of slots is a multiple of four
+// too, so everything about a token belongs to one of four classes, each of which one warp sends in order. A quantising warp
+// has a unit of token tl - 12 as well (same class), for which it saw token tl - 12 - slots sent: no wait can meet a barrier
+// that is a whole ring behind or ahead.
+constexpr int kMoeBars = 32;
+constexpr int kMoeSenders = 4;
+constexpr int kMoeMinSlots = 8;
+__host__ __device__ __forceinline__ int moe_image_slots(int hidden) {  // 16, 12 or 8; 0: the rows are too wide
+  const int n = (int)(112 * 1024 / moe_row_bytes(hidden, 1)) / 4 * 4;
+  return n > 16 ? 16 : n < kMoeMinSlots ? 0 : n;
+}
+// 16 bf16 values (32 bytes) as e4m3 with the given 1 / scale
+__device__ __forceinline__ uint4 moe_quantize16(const uint32_t (&raw)[8], float inv) {
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[2 * j]));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[2 * j + 1]));
+    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a.x * inv, a.y * inv), __NV_SATFINITE, __NV_E4M3);
+    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(b.x * inv, b.y * inv), __NV_SATFINITE, __NV_E4M3);
+    w[j] = lo | (hi << 16);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__global__ void __launch_bounds__(kMoeThreads) moe_dispatch_fp8_bulk_kernel(eux_moe_desc d, int counted, int slots) {
+  extern __shared__ __align__(128) unsigned char moe_image_sm[];
+  __shared__ uint64_t bars[2 * kMoeBars];
+  __shared__ uint64_t* flags[kMaxWorld];
+  __shared__ unsigned char* arenas[kMaxWorld];
+  __shared__ uint4* metas[kMaxWorld];
+  __shared__ int s_abort;
+  const size_t row_bytes = moe_row_bytes(d.hidden, 1);
+  unsigned char* const ring = reinterpret_cast<unsigned char*>(((uintptr_t)moe_image_sm + 127) & ~(uintptr_t)127);
+  int* const tables = reinterpret_cast<int*>(ring + (size_t)slots * row_bytes);
+  const MoeRouting r{tables, tables + d.n_experts, tables + 2 * d.n_experts};
+  const int t0 = moe_first_token(d, blockIdx.x, gridDim.x), t1 = moe_first_token(d, blockIdx.x + 1, gridDim.x);
+  const int EPR = d.n_experts / d.world;
+  const int upr = (d.hidden + 1023) / 1024;
+  const int ngroups = d.hidden / 128;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWorkers = kMoeThreads / 32 - kMoeSenders;
+  static_assert(kWorkers % kMoeSenders == 0 && kMoeBars % kMoeSenders == 0, "classes of tokens");
+  const uint32_t ring0 = smem_u32(ring), bar0 = smem_u32(bars);
+  auto full_bar = [&](int tl) { return bar0 + 8u * (tl % kMoeBars); };
+  auto empty_bar = [&](int tl) { return bar0 + 8u * (kMoeBars + tl % kMoeBars); };
+  auto phase = [](int tl) { return (uint32_t)(tl / kMoeBars) & 1u; };
+  volatile int* abort = &s_abort;
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int i = 0; i < kMoeBars; ++i) {
+      mbar_init(full_bar(i), (uint32_t)upr);
+      mbar_init(empty_bar(i), 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if ((int)threadIdx.x < d.world) {
+    flags[threadIdx.x] = d.flag_peer[threadIdx.x];
+    arenas[threadIdx.x] = reinterpret_cast<unsigned char*>(d.arena_peer[threadIdx.x]);
+    metas[threadIdx.x] = reinterpret_cast<uint4*>(d.meta_peer[threadIdx.x]);
+  }
+  for (int s = warp; s < slots; s += kMoeThreads / 32)  // the padding behind the scales
+    for (int b = d.hidden + ngroups * 4 + lane * 4; b < (int)row_bytes; b += 128) *reinterpret_cast<uint32_t*>(ring + s * row_bytes + b) = 0;
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  moe_route(d, r, t0, t1, counted != 0);
+  moe_send_counts(d, r, flags);
+  const int units = (t1 - t0) * upr;
+  if (warp < kWorkers) {
+    // a lane has 16 elements of either half of the unit: 32-byte loads, conflict-free stores
+    uint32_t v[2][8];
+    auto load = [&](int u) {
+      const int tl = u / upr, e0 = (u - tl * upr) * 1024 + lane * 16;
+      const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(d.x) + (size_t)(t0 + tl) * d.hidden + e0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (e0 + h * 512 < d.hidden) {
+          const uint4 a = ld_stream_u4(src + h * 512), b = ld_stream_u4(src + h * 512 + 8);
+          v[h][0] = a.x, v[h][1] = a.y, v[h][2] = a.z, v[h][3] = a.w, v[h][4] = b.x, v[h][5] = b.y, v[h][6] = b.z, v[h][7] = b.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[h][j] = 0;
+        }
+    };
+    if (warp < units) load(warp);
+    for (int u = warp; u < units; u += kWorkers) {
+      const int tl = u / upr, part = u - tl * upr, s = tl % slots;
+      uint4 q[2];
+      float scale[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float amax = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[h][j]));
+          amax = fmaxf(amax, fmaxf(fabsf(x.x), fabsf(x.y)));
+        }
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+        scale[h] = fmaxf(amax, 1e-10f) * (1.0f / 448.0f);
+        q[h] = moe_quantize16(v[h], 1.0f / scale[h]);
+      }
+      if (u + kWorkers < units) load(u + kWorkers);
+      if (tl >= slots && __any_sync(0xffffffffu, !mbar_wait(empty_bar(tl - slots), phase(tl - slots), abort, 0))) break;
+      unsigned char* const image = ring + (size_t)s * row_bytes;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e0 = part * 1024 + h * 512 + lane * 16;
+        if (e0 < d.hidden) {
+          *reinterpret_cast<uint4*>(image + e0) = q[h];
+          if ((lane & 7) == 0) reinterpret_cast<float*>(image + d.hidden)[e0 >> 7] = scale[h];
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full_bar(tl));
+    }
+  } else {
+    // lane k owns row k; the routing entries of the next token are on their way while this one's image is waited for
+    int slot = -1, expert = 0;
+    float w = 0.f;
+    auto fetch = [&](int t) {
+      slot = -1;
+      if (lane < d.topk) {
+        const int64_t i = (int64_t)t * d.topk + lane;
+        slot = d.slot_of[i], expert = __ldg(d.topk_idx + i), w = __ldg(d.topk_w + i);
+      }
+    };
+    const int first = warp - kWorkers;
+    if (t0 + first < t1) fetch(t0 + first);
+    for (int tl = first; tl < t1 - t0; tl += kMoeSenders) {
+      const int t = t0 + tl, s = tl % slots;
+      unsigned char* out = nullptr;
+      if (slot >= 0) {
+        const int dst = expert / EPR;
+        const size_t row = (size_t)d.rank * d.capacity + slot;
+        out = arenas[dst] + row * row_bytes;
+        st_u4(metas[dst] + row, make_uint4((uint32_t)t, (uint32_t)lane | ((uint32_t)(expert - dst * EPR) << 16), __float_as_uint(w), (uint32_t)d.rank));
+      }
+      if (tl + kMoeSenders < t1 - t0) fetch(t + kMoeSenders);
+      if (__any_sync(0xffffffffu, !mbar_wait(full_bar(tl), phase(tl), abort, 0))) break;
+      if (out) bulk_s2g(out, ring0 + (uint32_t)(s * row_bytes), (uint32_t)row_bytes);
+      bulk_commit();
+      bulk_wait_read_1();  // the copies of the image before this one have read their slot
+      __syncwarp();
+      if (lane == 0 && tl >= kMoeSenders) mbar_arrive(empty_bar(tl - kMoeSenders));
+    }
+    bulk_wait_all();
+    asm volatile("fence.proxy.async;" ::: "memory");
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_abort) set_status(d.status, EUX_ST_TIMEOUT, 13);
   moe_publish(d, flags);
 }
 
@@ -764,15 +926,16 @@ using namespace eux;
 
 extern "C" size_t eux_moe_row_bytes(int hidden, int fp8) { return moe_row_bytes(hidden, fp8); }
 
-template <auto KERNEL>
-static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream_t st) {
+static int moe_sms() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // A CTA per token, up to one per SM: a second one counts all entries again (256 tokens, fp8: 28.2 us for the exchange
-  // with one, 30.2 with two). fp8 rows of more than eight tokens per CTA have two, one of which works while the other
-  // waits at its barriers (32768 x 1024: 235 us against 280).
-  if (ctas <= 0) ctas = d->fp8 && d->n_tokens > 8 * sms ? 2 * sms : sms;
+  return sms;
+}
+
+// The count launch, where there are too many entries for every CTA to count them all, and the dispatch.
+template <auto KERNEL, typename... More>
+static int moe_dispatch(const eux_moe_desc* d, int ctas, int sms, size_t smem, cudaStream_t st, More... more) {
   const int grid = std::max(1, std::min(ctas, d->n_tokens));
   if (smem > 40 * 1024)  // with the kernel's static arrays near the 48 KiB that need no leave
     if (cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); e != cudaSuccess) return (int)e;
@@ -782,15 +945,25 @@ static int moe_dispatch(const eux_moe_desc* d, int ctas, size_t smem, cudaStream
     const int64_t want = (entries + kMoeThreads - 1) / kMoeThreads;
     moe_count_kernel<<<(int)std::min<int64_t>(want, sms), kMoeThreads, 2 * (size_t)d->n_experts * sizeof(int), st>>>(*d);
   }
-  KERNEL<<<grid, kMoeThreads, smem, st>>>(*d, counted);
+  KERNEL<<<grid, kMoeThreads, smem, st>>>(*d, counted, more...);
   return (int)cudaGetLastError();
 }
 
 extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* stream) {
   if (int rc = moe_check(d)) return rc;
   const size_t routing = 3 * (size_t)d->n_experts * sizeof(int);
-  if (!d->fp8) return moe_dispatch<moe_dispatch_bf16_kernel>(d, ctas, routing, (cudaStream_t)stream);
-  return moe_dispatch<moe_dispatch_fp8_kernel>(d, ctas, routing + 2 * (size_t)moe_scale_stride(d->hidden) * sizeof(float), (cudaStream_t)stream);
+  const cudaStream_t st = (cudaStream_t)stream;
+  const int sms = moe_sms();
+  // A CTA per token, up to one per SM: a second one counts all entries again (256 tokens, fp8: 28.2 us for the exchange
+  // with one, 30.2 with two).
+  const int one = ctas > 0 ? ctas : sms;
+  if (!d->fp8) return moe_dispatch<moe_dispatch_bf16_kernel>(d, one, sms, routing, st);
+  if (const int slots = moe_image_slots(d->hidden); slots > 0 && d->n_tokens >= 2 * (int64_t)one)
+    return moe_dispatch<moe_dispatch_fp8_bulk_kernel>(d, one, sms, routing + 128 + (size_t)slots * moe_row_bytes(d->hidden, 1), st, slots);
+  // Rows too wide for images and more than eight tokens per CTA: two per SM, one of which works while the other waits at its
+  // barriers.
+  if (ctas <= 0) ctas = d->n_tokens > 8 * sms ? 2 * sms : sms;
+  return moe_dispatch<moe_dispatch_fp8_kernel>(d, ctas, sms, routing + 2 * (size_t)moe_scale_stride(d->hidden) * sizeof(float), st);
 }
 
 extern "C" int eux_moe_expert_ready_launch(const eux_moe_desc* d, void* stream) {
@@ -935,6 +1108,7 @@ extern "C" int eux_moe_preload(void) {
   cudaFuncAttributes attr;
   const void* kernels[] = {(const void*)moe_count_kernel,
                            (const void*)moe_dispatch_bf16_kernel,       (const void*)moe_dispatch_fp8_kernel,
+                           (const void*)moe_dispatch_fp8_bulk_kernel,
                            (const void*)moe_expert_ready_kernel,        (const void*)moe_combine_bf16_kernel,
                            (const void*)moe_combine_bf16_stream_kernel, (const void*)moe_combine_fp8_kernel,
                            (const void*)moe_combine_fp8_rows_kernel,    (const void*)moe_combine_fp8_stream_kernel};

@@ -289,3 +289,17 @@ def test_dispatch_of_rows_with_many_scales(cuda_device, hidden):
     a2a.check_status()
     ref = moe.reference_dispatch_combine(x, idx, w, True)
     assert bool(((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
+
+
+@pytest.mark.parametrize("t,hidden,topk,ne", [(295, 128, 1, 8), (296, 1152, 8, 16), (1300, 512, 3, 64), (6000, 256, 2, 8), (5000, 5120, 1, 16),
+                                              (4000, 7168, 1, 8), (2500, 8192, 2, 4096), (1700, 12928, 4, 8), (700, 14464, 2, 8), (333, 2048, 32, 64)])
+def test_fp8_dispatch_of_row_images(cuda_device, t, hidden, topk, ne):
+    """Around two tokens per CTA, from where rows leave as bulk copies of whole images: rings of 16, 12 and 8 slots that go
+    round several times, units per token from one to fourteen (with partial ones), rows too wide for images, the last unit a
+    partial one, entries without an expert."""
+    test_dispatch_routes_in_one_launch(cuda_device, t, hidden, topk, ne, True)
+
+
+@pytest.mark.parametrize("world", [2, 8])
+def test_fp8_dispatch_of_row_images_to_ranks(cuda_device, world):
+    test_dispatch_combine(cuda_device, True, world, 400, 3200, 4, 16)
