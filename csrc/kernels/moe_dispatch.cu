@@ -659,10 +659,13 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_kernel(eux_moe_d
 
 // ---- combine, bf16, top-k <= 8: a warp streams through a contiguous run of (token, 1 KiB) units. Every load
 // is 32 bytes per lane, 1 KiB of one row per warp instruction (measured against 16-byte loads: 132 -> 113 us
-// on one GPU, 403 -> 388 us when half the rows cross NVLink). A unit's eight rows are fetched as two
-// groups of four, and the next group is always requested before the current one is accumulated, so a
-// warp never sits out a whole memory round trip; the routing entries are read once per token.
-__global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_stream_kernel(eux_moe_desc d) {
+// on one GPU, 403 -> 388 us when half the rows cross NVLink). A unit's rows are fetched as G groups of R (eight as two
+// groups of four, four and fewer as one, two and fewer as one of two), and the next group is always requested before the
+// current one is accumulated, so a warp never sits out a whole memory round trip; the routing entries are read once per
+// token. (With eight rows for every top-k, 4096 tokens of 4096 took 25.8 us at top-1, 27.6 at 2, 39.5 at 4; 12.7, 15.0 and 36.3
+// so. Groups of two rows for more than two, at 64 registers and two CTAs per SM: 44.7 at top-4, 103 against 93 at 8 x 7168.)
+template <int R, int G>
+__global__ void __launch_bounds__(kMoeThreads, R < 4 ? 2 : 1) moe_combine_bf16_stream_kernel(eux_moe_desc d) {
   if (!moe_wait_experts(d)) return;
   const int W = d.world, EPR = d.n_experts / W, K = d.topk;
   const int chunks = d.hidden / 16;  // 32-byte pieces per row
@@ -696,18 +699,18 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_stream_kernel(eu
       }
     }
   };
-  auto issue = [&](int c, int k0, uint32_t (&v)[4][8]) {
+  auto issue = [&](int c, int k0, uint32_t (&v)[R][8]) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < R; ++k) {
       const unsigned char* row = (const unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, k0 + k);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[k][j] = 0u;
       if (row && c < chunks) moe_ld_v8(row + (size_t)c * 32, v[k]);
     }
   };
-  auto accumulate = [&](const uint32_t (&v)[4][8], float w_lane, int k0, float (&acc)[16]) {
+  auto accumulate = [&](const uint32_t (&v)[R][8], float w_lane, int k0, float (&acc)[16]) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < R; ++k) {
       const float w = __shfl_sync(0xffffffffu, w_lane, k0 + k);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -718,23 +721,27 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_stream_kernel(eu
     }
   };
   if (u0 >= u1) return;
-  uint32_t a[4][8], b[4][8];
+  uint32_t a[R][8], b[R][8];
   int t, c;
-  locate(u0, t, c);
+  int64_t u = u0;
+  locate(u, t, c);
   issue(c, 0, a);
-  for (int64_t u = u0; u < u1; ++u) {
+  // one unit, whose first group is in x: what comes next is requested into the buffer that is not being accumulated
+  auto unit = [&](uint32_t (&x)[R][8], uint32_t (&y)[R][8]) {
     const float w_lane = my_w;
     const int tu = t, cu = c;
-    issue(cu, 4, b);
+    if (G == 2) issue(cu, R, y);
     float acc[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-    accumulate(a, w_lane, 0, acc);
+    if (G == 2) accumulate(x, w_lane, 0, acc);
     if (u + 1 < u1) {
       locate(u + 1, t, c);
-      issue(c, 0, a);
+      if (G == 2) issue(c, 0, x);
+      else issue(c, 0, y);
     }
-    accumulate(b, w_lane, 4, acc);
+    if (G == 2) accumulate(y, w_lane, R, acc);
+    else accumulate(x, w_lane, 0, acc);
     if (cu < chunks) {
       uint4 o0, o1;
       __nv_bfloat162* q0 = reinterpret_cast<__nv_bfloat162*>(&o0);
@@ -748,7 +755,14 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_stream_kernel(eu
       st_stream_u4(out, o0);
       st_stream_u4(out + 1, o1);
     }
-  }
+    return ++u < u1;
+  };
+  if (G == 2)
+    while (unit(a, b)) {
+    }
+  else
+    while (unit(a, b) && unit(b, a)) {
+    }
 }
 
 // ---- combine, fp8 rows: lane owns 16 elements; dequantise while accumulating --
@@ -973,9 +987,11 @@ extern "C" int eux_moe_expert_ready_launch(const eux_moe_desc* d, void* stream) 
 }
 
 // ---- combine, fp8 rows, top-k <= 8, hidden <= 8192: the streaming scheme of the bf16 kernel. A unit is 1024
-// elements of a token (32 bytes per lane, 1 KiB of a row per warp instruction); its eight rows are fetched as
-// four groups of two, the next group always requested before the current one is dequantised and
+// elements of a token (32 bytes per lane, 1 KiB of a row per warp instruction); its rows are fetched as G
+// groups of two (2 G >= top-k), the next group always requested before the current one is dequantised and
 // accumulated. Lane L keeps gate weight x scale of groups L and 32 + L of every row, loaded once per token.
+// (4096 tokens of 4096, with eight rows for every top-k and so: 25.2 and 18.5 us at top-1, 30.9 and 26.6 at 4, 40.0 and 38.7 at 6.)
+template <int G>
 __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux_moe_desc d) {
   if (!moe_wait_experts(d)) return;
   const int W = d.world, EPR = d.n_experts / W, K = d.topk;
@@ -992,8 +1008,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
   if (u0 >= u1) return;
   int cur_t = -1;
   const unsigned char* my_row = nullptr;
-  float scw[8][2];
-  // steps: 4 per unit; step s of unit u fetches rows 2s and 2s + 1
+  float scw[2 * G][2];
   auto locate = [&](int64_t u, int& t, int& e0) {
     t = (int)(u / upr);
     e0 = (int)(u - (int64_t)t * upr) * 1024 + lane * 32;
@@ -1011,7 +1026,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
       }
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < 2 * G; ++k) {
       const unsigned char* row = (const unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, k);
       const float wk = __shfl_sync(0xffffffffu, my_w, k);
 #pragma unroll
@@ -1031,49 +1046,52 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
     }
   };
   int t, e0;
-  locate(u0, t, e0);
+  int64_t u = u0;
+  locate(u, t, e0);
   new_token(t);
   uint32_t a[2][8], b[2][8];
   issue(e0, 0, a);
-  for (int64_t u = u0; u < u1; ++u) {
+  // one unit, whose first group is in x; the first group of the next one ends up in x where G is even, in y where it is odd
+  auto unit = [&](uint32_t (&x)[2][8], uint32_t (&y)[2][8]) {
     const int tu = t, eu = e0;
     const int gi = eu >> 7;  // scale group of this lane's 32 elements
     float acc[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) acc[j] = 0.f;
     // the weights of this unit's token, fetched before the routing entries may move on to the next one
-    float wk[8];
+    float wk[2 * G];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) wk[k] = __shfl_sync(0xffffffffu, (gi >> 5) ? scw[k][1] : scw[k][0], gi & 31);
-    auto accumulate = [&](const uint32_t (&v)[2][8], int k0) {
+    for (int k = 0; k < 2 * G; ++k) wk[k] = __shfl_sync(0xffffffffu, (gi >> 5) ? scw[k][1] : scw[k][0], gi & 31);
+    auto accumulate = [&](const uint32_t (&v)[2][8], float w0, float w1) {
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const float w = k0 == 0 ? wk[k] : k0 == 2 ? wk[2 + k] : k0 == 4 ? wk[4 + k] : wk[6 + k];
+        const float w = k == 0 ? w0 : w1;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           __half2_raw lo = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(v[k][j] & 0xffffu), __NV_E4M3);
           __half2_raw hi = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(v[k][j] >> 16), __NV_E4M3);
-          const float2 x = __half22float2(*reinterpret_cast<__half2*>(&lo));
-          const float2 y = __half22float2(*reinterpret_cast<__half2*>(&hi));
-          acc[4 * j] = fmaf(w, x.x, acc[4 * j]);
-          acc[4 * j + 1] = fmaf(w, x.y, acc[4 * j + 1]);
-          acc[4 * j + 2] = fmaf(w, y.x, acc[4 * j + 2]);
-          acc[4 * j + 3] = fmaf(w, y.y, acc[4 * j + 3]);
+          const float2 p = __half22float2(*reinterpret_cast<__half2*>(&lo));
+          const float2 q = __half22float2(*reinterpret_cast<__half2*>(&hi));
+          acc[4 * j] = fmaf(w, p.x, acc[4 * j]);
+          acc[4 * j + 1] = fmaf(w, p.y, acc[4 * j + 1]);
+          acc[4 * j + 2] = fmaf(w, q.x, acc[4 * j + 2]);
+          acc[4 * j + 3] = fmaf(w, q.y, acc[4 * j + 3]);
         }
       }
     };
-    issue(eu, 2, b);
-    accumulate(a, 0);
-    issue(eu, 4, a);
-    accumulate(b, 2);
-    issue(eu, 6, b);
-    accumulate(a, 4);
-    if (u + 1 < u1) {
-      locate(u + 1, t, e0);
-      if (t != cur_t) new_token(t);
-      issue(e0, 0, a);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      uint32_t (&now)[2][8] = g & 1 ? y : x;
+      uint32_t (&then)[2][8] = g & 1 ? x : y;
+      if (g + 1 < G) {
+        issue(eu, 2 * (g + 1), then);
+      } else if (u + 1 < u1) {
+        locate(u + 1, t, e0);
+        if (t != cur_t) new_token(t);
+        issue(e0, 0, then);
+      }
+      accumulate(now, wk[2 * g], wk[2 * g + 1]);
     }
-    accumulate(b, 6);
     if (eu < d.hidden) {
       uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(d.out) + (size_t)tu * d.hidden + eu);
 #pragma unroll
@@ -1085,7 +1103,14 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
         st_stream_u4(out + q, o);
       }
     }
-  }
+    return ++u < u1;
+  };
+  if (G % 2 == 0)
+    while (unit(a, b)) {
+    }
+  else
+    while (unit(a, b) && unit(b, a)) {
+    }
 }
 
 extern "C" int eux_moe_combine_launch(const eux_moe_desc* d, int ctas, void* stream) {
@@ -1094,11 +1119,18 @@ extern "C" int eux_moe_combine_launch(const eux_moe_desc* d, int ctas, void* str
     const int64_t units = (int64_t)d->n_tokens * ((d->hidden + 511) / 512);
     ctas = (int)std::min<int64_t>(296, std::max<int64_t>(1, (units + kMoeThreads / 32 - 1) / (kMoeThreads / 32)));
   }
-  if (d->fp8 && d->topk <= 8 && d->hidden <= 8192) moe_combine_fp8_stream_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
-  else if (d->fp8 && d->topk <= 8 && d->hidden <= 16384) moe_combine_fp8_rows_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
-  else if (d->fp8) moe_combine_fp8_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
-  else if (d->topk <= 8) moe_combine_bf16_stream_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
-  else moe_combine_bf16_kernel<<<ctas, kMoeThreads, 0, (cudaStream_t)stream>>>(*d);
+  const cudaStream_t st = (cudaStream_t)stream;
+  if (d->fp8 && d->topk <= 8 && d->hidden <= 8192) {
+    if (d->topk <= 2) moe_combine_fp8_stream_kernel<1><<<ctas, kMoeThreads, 0, st>>>(*d);
+    else if (d->topk <= 4) moe_combine_fp8_stream_kernel<2><<<ctas, kMoeThreads, 0, st>>>(*d);
+    else if (d->topk <= 6) moe_combine_fp8_stream_kernel<3><<<ctas, kMoeThreads, 0, st>>>(*d);
+    else moe_combine_fp8_stream_kernel<4><<<ctas, kMoeThreads, 0, st>>>(*d);
+  } else if (d->fp8 && d->topk <= 8 && d->hidden <= 16384) moe_combine_fp8_rows_kernel<<<ctas, kMoeThreads, 0, st>>>(*d);
+  else if (d->fp8) moe_combine_fp8_kernel<<<ctas, kMoeThreads, 0, st>>>(*d);
+  else if (d->topk <= 2) moe_combine_bf16_stream_kernel<2, 1><<<ctas, kMoeThreads, 0, st>>>(*d);
+  else if (d->topk <= 4) moe_combine_bf16_stream_kernel<4, 1><<<ctas, kMoeThreads, 0, st>>>(*d);
+  else if (d->topk <= 8) moe_combine_bf16_stream_kernel<4, 2><<<ctas, kMoeThreads, 0, st>>>(*d);
+  else moe_combine_bf16_kernel<<<ctas, kMoeThreads, 0, st>>>(*d);
   return (int)cudaGetLastError();
 }
 
@@ -1110,8 +1142,11 @@ extern "C" int eux_moe_preload(void) {
                            (const void*)moe_dispatch_bf16_kernel,       (const void*)moe_dispatch_fp8_kernel,
                            (const void*)moe_dispatch_fp8_bulk_kernel,
                            (const void*)moe_expert_ready_kernel,        (const void*)moe_combine_bf16_kernel,
-                           (const void*)moe_combine_bf16_stream_kernel, (const void*)moe_combine_fp8_kernel,
-                           (const void*)moe_combine_fp8_rows_kernel,    (const void*)moe_combine_fp8_stream_kernel};
+                           (const void*)moe_combine_bf16_stream_kernel<2, 1>, (const void*)moe_combine_bf16_stream_kernel<4, 1>,
+                           (const void*)moe_combine_bf16_stream_kernel<4, 2>, (const void*)moe_combine_fp8_kernel,
+                           (const void*)moe_combine_fp8_rows_kernel,    (const void*)moe_combine_fp8_stream_kernel<1>,
+                           (const void*)moe_combine_fp8_stream_kernel<2>, (const void*)moe_combine_fp8_stream_kernel<3>,
+                           (const void*)moe_combine_fp8_stream_kernel<4>};
   for (const void* k : kernels) {
     cudaError_t e = cudaFuncGetAttributes(&attr, k);
     if (e != cudaSuccess) return (int)e;

@@ -303,3 +303,28 @@ def test_fp8_dispatch_of_row_images(cuda_device, t, hidden, topk, ne):
 @pytest.mark.parametrize("world", [2, 8])
 def test_fp8_dispatch_of_row_images_to_ranks(cuda_device, world):
     test_dispatch_combine(cuda_device, True, world, 400, 3200, 4, 16)
+
+
+@pytest.mark.parametrize("topk", [1, 2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("t,hidden", [(1, 128), (333, 1152), (3001, 2176)])
+def test_combine_fetches_as_many_rows_as_there_are(cuda_device, topk, fp8, t, hidden):
+    """Every number of row groups a combine is compiled for, full and partial, with one unit per warp and several (an odd
+    and an even number of them), and entries without an expert: sums in fp32 and one rounding to bf16, 2^-8 of the value and
+    1e-5 of the token's largest; fp8 rows are dequantised exactly as the reference does."""
+    from execution_ucx_b200.ops import moe
+    (rk,) = moe.MoeAllToAll.emulated(1, t, hidden, topk, 16, fp8=fp8)
+    g = torch.Generator(device=cuda_device).manual_seed(topk + t)
+    x = torch.randn(t, hidden, device=cuda_device, generator=g).to(torch.bfloat16)
+    idx = torch.randint(-1 if t > 1 else 0, 16, (t, topk), device=cuda_device, generator=g, dtype=torch.int32)
+    w = torch.rand(t, topk, device=cuda_device, generator=g)
+    for _ in range(2):
+        rk.dispatch(x, idx, w)
+        rk.expert_ready()
+        rk.out.fill_(float("nan"))
+        out = rk.combine()
+        torch.cuda.synchronize()
+        rk.check_status()
+        ref = moe.reference_dispatch_combine(x, idx, w, fp8)
+        bound = ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True) + 1e-30
+        assert bool(((out.float() - ref).abs() <= bound).all())
