@@ -199,19 +199,21 @@ __device__ __forceinline__ void moe_send_counts(const eux_moe_desc& d, const Moe
     flags[dst][W + d.rank] = (uint64_t)(rows < d.capacity ? rows : d.capacity);
   }
 }
-// The last CTA sends the arrival flags and leaves the counters at zero. Two system-scope fences, a microsecond each, are on
-// the way of a flag: every CTA's between its rows and its count, and the last one's between the counts and the flag. (With
-// counts and flags both sent here, behind a release each, an exchange of 16 tokens of 4096 took 20.4 us, 18.8 now.)
+// The last CTA sends the arrival flags and leaves the counters at zero. A CTA's fence between its rows and its count is for
+// this GPU, where the last CTA sees the counts; that one's fence for everyone stands between them and the flags and covers the
+// rows of all CTAs. (System-scope fences queue up at 31 ns each: with one per CTA a dispatch of 128 fp8 tokens of 7168 took
+// 12.4 us, 9.0 so, graph replays. With counts and flags both sent here, behind a release each, an exchange of 16 tokens of
+// 4096 took 20.4 us, 18.8 without.)
 __device__ __forceinline__ void moe_publish(const eux_moe_desc& d, uint64_t* const* flags) {
   __syncthreads();
   __shared__ int s_last;
   const int W = d.world, E = d.n_experts;
   if (threadIdx.x == 0) {
-    __threadfence_system();
+    fence_gpu();
     const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(d.counters + W + E), 1u);
     s_last = (old == gridDim.x - 1);
     if (s_last) {
-      __threadfence_system();
+      fence_sys();
       for (int dst = 0; dst < W; ++dst) st_relaxed_sys(flags[dst] + d.rank, d.seq);
     }
   }

@@ -443,12 +443,12 @@ __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   __syncthreads();
   if (threadIdx.x != 0) return;
   // Without a flag to publish the end of the launch is enough for Y: no fence here and none in the last CTA (a call of
-  // 640 x 4096 x 1024 took 13.1 us with them and 11.3 without). A CTA that gave up has said so before it is counted.
-  if (p.done_flag) __threadfence_system();
-  else if (!ok) __threadfence();
+  // 640 x 4096 x 1024 took 13.1 us with them and 11.3 without). With one, the last CTA's fence for everyone covers what the
+  // others wrote before they counted themselves. A CTA that gave up has said so before it is counted.
+  if (p.done_flag || !ok) fence_gpu();
   const uint32_t old = atomicAdd(p.sched, 1u);
   if (old == gridDim.x - 1) {
-    if (p.done_flag) __threadfence();
+    if (p.done_flag) fence_gpu();
     const bool all_ok = ok && __ldcg(p.sched + 1) == 0;
     for (int i = 0; i < p.M / BM; ++i) p.panel_flags[i] = 0;
     p.sched[0] = 0;
@@ -456,7 +456,7 @@ __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
     p.sched[2] = 0;  // the tile counter
     p.sched[3] = 0;  // the copy warps' unit counter
     if (!p.done_flag) return;
-    __threadfence_system();
+    fence_sys();
     // done_always: a caller that reads the status word learns of the end of the kernel either way (an RPC
     // handler must answer); otherwise the flag means "Y is complete" and stays silent after a failure
     if (all_ok || p.done_always) st_relaxed_sys(p.done_flag, p.done_value);

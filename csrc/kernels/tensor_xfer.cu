@@ -81,23 +81,27 @@ __device__ __forceinline__ bool cta_wait_arrival(const eux_xfer_desc& d) {
 // All stores of this CTA are done; the last CTA of the grid publishes the flag, and only if no CTA
 // of the grid gave up: every CTA runs its own bounded wait, so near the deadline one can time out (and
 // skip its share of the copy) while the last one to arrive succeeded. The scratch word counts arrivals
-// in its low 31 bits; a CTA that failed sets the top bit before it counts itself.
+// in its low 31 bits; a CTA that failed sets the top bit before it counts itself. A CTA's fence before it counts itself is for
+// this GPU, where the last CTA sees the counts; that one's fence for everyone then covers what all of them wrote, into a
+// peer's memory too. (System-scope fences queue up at 31 ns each: with one per CTA, flagged transfers in a loop took, 16 MiB of
+// bytes 10.2 us, of fp32 to bf16 12.5, of bf16 at an odd offset 21.3, 4099 x 4096 fp32 transposed to bf16 29.4; now 7.2, 5.5,
+// 8.4 and 20.9.)
 __device__ __forceinline__ void cta_publish(const eux_xfer_desc& d, uint32_t* counter, bool ok) {
   if (!d.flag && !d.flag2) return;  // nobody is told: the end of the launch is enough
   __syncthreads();
   if (threadIdx.x != 0) return;
-  __threadfence_system();
   bool last = true;
   if (gridDim.x > 1) {
+    fence_gpu();
     if (!ok) atomicOr(counter, 0x80000000u);
     const uint32_t old = atomicAdd(counter, 1u);
     last = ((old & 0x7fffffffu) == gridDim.x - 1);
     if (old & 0x80000000u) ok = false;
     if (last) {
       *counter = 0;  // leave the scratch word clean for the next launch
-      __threadfence_system();  // what the other CTAs wrote before they counted themselves comes before the flags
     }
   }
+  if (last) fence_sys();  // what all CTAs wrote, the others before they counted themselves, comes before the flags
   if (last && ok && d.flag) st_relaxed_sys(d.flag, d.flag_value);
   if (last && ok && d.flag2) st_relaxed_sys(d.flag2, d.flag2_value);
 }
@@ -1196,10 +1200,13 @@ extern "C" int eux_xfer_launch(const eux_xfer_desc* d, uint32_t* scratch_counter
     }
     const bool tiled = route >= Route::kTile;
     // Four gather CTAs fill an SM's threads. Tiles: a CTA each, whose loads then overlap other CTAs' stores (47 us against
-    // 51 on 8192 x 8192 bf16), or eight CTAs per SM where each one also has a flag's counter to go through.
+    // 51 on 8192 x 8192 bf16).
+    // With a flag: five tile CTAs per SM, which are resident at once, and two gather CTAs, fewer CTAs that have to be counted
+    // (4099 x 4096 fp32 to bf16 transposed 20.9 us, 22.5 with eight; 16 MiB of bf16 at an odd offset 8.4, 9.6 with four).
     // One that waits keeps to half of an SM (gathers have 64 registers and 512 threads), and all its CTAs wait at once, so
     // that a limit passes once.
-    if (!ctas_given) max_ctas = d->wait_flag ? (tiled ? 2 : 1) * sms : !tiled ? 4 * sms : (d->flag || d->flag2) ? 8 * sms : 0x7fffffff;
+    const bool flagged = d->flag || d->flag2;
+    if (!ctas_given) max_ctas = d->wait_flag ? (tiled ? 2 : 1) * sms : !tiled ? (flagged ? 2 : 4) * sms : flagged ? 5 * sms : 0x7fffffff;
     const uint64_t per_cta = (uint64_t)kXferThreads * (route == Route::kElement ? 2 : chunk);
     grid = limit(tiled ? t.tiles : (a.d.n_elems + per_cta - 1) / per_cta);
     if (!scratch_counter) {  // up to 2048 elements, or when told to, one CTA does without
