@@ -1117,9 +1117,13 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
 
 extern "C" int eux_moe_combine_launch(const eux_moe_desc* d, int ctas, void* stream) {
   if (int rc = moe_check(d)) return rc;
-  if (ctas <= 0) {  // no CTA without a unit (of at least 512 elements of a token) for some warp: each polls the flags
+  if (ctas <= 0) {
+    // As many as are resident: a CTA streams through its share and would start anew in a second wave (calls of 4096 x 7168,
+    // top-8, an exchange of bf16 205.3 us with two waves and 202.2 with one, fp8 133.9 and 131.4; 1024 x 7168 62.5 and 59.3).
+    // And no CTA without a unit (of at least 512 elements of a token) for some warp: each polls the flags.
     const int64_t units = (int64_t)d->n_tokens * ((d->hidden + 511) / 512);
-    ctas = (int)std::min<int64_t>(296, std::max<int64_t>(1, (units + kMoeThreads / 32 - 1) / (kMoeThreads / 32)));
+    const int64_t resident = (int64_t)moe_sms() * (!d->fp8 && d->topk <= 2 ? 2 : 1);
+    ctas = (int)std::min<int64_t>(resident, std::max<int64_t>(1, (units + kMoeThreads / 32 - 1) / (kMoeThreads / 32)));
   }
   const cudaStream_t st = (cudaStream_t)stream;
   if (d->fp8 && d->topk <= 8 && d->hidden <= 8192) {
