@@ -572,23 +572,72 @@ __global__ void moe_expert_ready_kernel(eux_moe_desc d) {
   if ((int)threadIdx.x < W && s_ok) st_release_sys(peer + 2 * W + d.rank, d.seq);
 }
 
-__device__ __forceinline__ bool moe_wait_experts(const eux_moe_desc& d) {
+// The experts' arenas are fetched while the flags are polled.
+struct MoeArenas {
+  const unsigned char* of[kMaxWorld];
+};
+__device__ __forceinline__ bool moe_wait_experts(const eux_moe_desc& d, MoeArenas& arenas) {
   __shared__ int s_ok;
   if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
   if ((int)threadIdx.x < d.world) {
+    const void* const arena = d.arena_peer[threadIdx.x];
     if (!wait_flag_ge(&d.flag_peer[d.rank][2 * d.world + threadIdx.x], d.seq, d.wait_timeout_ns)) {
       set_status(d.status, EUX_ST_TIMEOUT, 12);
       s_ok = 0;
     }
+    arenas.of[threadIdx.x] = reinterpret_cast<const unsigned char*>(arena);
   }
   __syncthreads();
   return s_ok != 0;
 }
 
+// The rows of a token and their weights, lane k (< top-k) row k, for a warp that goes from token to token: the routing entries
+// of the next token are on their way while this one's rows are read, a trip to L2 that a warp waited for at every token
+// (combines in a loop: 4096 x 7168, top-8, bf16 90.0 and 85.5 us, 1024 x 7168 27.6 and 25.4). Not AHEAD: where the registers
+// are short (two CTAs per SM; 4096 x 4096, top-2: 15.2 us, 16.8 ahead).
+template <bool AHEAD>
+struct MoeRows {
+  const eux_moe_desc& d;
+  const MoeArenas& arenas;
+  const size_t row_bytes;
+  const int lane, EPR;
+  const unsigned char* row = nullptr;
+  float w = 0.f;
+  int next_expert = 0, next_slot = -1;
+  float next_w = 0.f;
+  __device__ __forceinline__ MoeRows(const eux_moe_desc& d_, const MoeArenas& arenas_, size_t row_bytes_, int lane_)
+      : d(d_), arenas(arenas_), row_bytes(row_bytes_), lane(lane_), EPR(d_.n_experts / d_.world) {}
+  __device__ __forceinline__ void fetch(int t) {
+    next_slot = -1;
+    if (lane < d.topk && t < d.n_tokens) {
+      const int64_t i = (int64_t)t * d.topk + lane;
+      next_expert = d.topk_idx[i], next_slot = d.slot_of[i], next_w = d.topk_w[i];
+    }
+  }
+  // token t, which comes behind the one before (or is the first and has been fetched), is the current one now
+  __device__ __forceinline__ void enter(int t) {
+    row = nullptr, w = 0.f;
+    if (AHEAD) {
+      if (next_slot >= 0) row = arenas.of[next_expert / EPR] + ((size_t)d.rank * d.capacity + next_slot) * row_bytes, w = next_w;
+      fetch(t + 1);
+    } else if (lane < d.topk) {
+      const int e = d.topk_idx[t * d.topk + lane], slot = d.slot_of[t * d.topk + lane];
+      if (slot >= 0) {
+        row = reinterpret_cast<const unsigned char*>(d.arena_peer[e / EPR]) + ((size_t)d.rank * d.capacity + slot) * row_bytes;
+        w = d.topk_w[t * d.topk + lane];
+      }
+    }
+  }
+  __device__ __forceinline__ const unsigned char* of(int k) const {
+    return (const unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)row, k);
+  }
+};
+
 // ---- combine, bf16: unit = (token, 64 chunks); 16 peer loads in flight per lane
 __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_kernel(eux_moe_desc d) {
-  if (!moe_wait_experts(d)) return;
+  __shared__ MoeArenas arenas;
+  if (!moe_wait_experts(d, arenas)) return;
   const int W = d.world, EPR = d.n_experts / W, K = d.topk;
   const int chunks = d.hidden / 8;
   const int upr = (chunks + 63) / 64;
@@ -607,7 +656,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_kernel(eux_moe_d
       int slot = d.slot_of[t * K + lane];
       if (slot >= 0) {
         int dst = e / EPR;
-        my_row = reinterpret_cast<const unsigned char*>(d.arena_peer[dst]) + ((size_t)d.rank * d.capacity + slot) * row_bytes;
+        my_row = arenas.of[dst] + ((size_t)d.rank * d.capacity + slot) * row_bytes;
         my_w = d.topk_w[t * K + lane];
       }
     }
@@ -668,8 +717,8 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_bf16_kernel(eux_moe_d
 // so. Groups of two rows for more than two, at 64 registers and two CTAs per SM: 44.7 at top-4, 103 against 93 at 8 x 7168.)
 template <int R, int G>
 __global__ void __launch_bounds__(kMoeThreads, R < 4 ? 2 : 1) moe_combine_bf16_stream_kernel(eux_moe_desc d) {
-  if (!moe_wait_experts(d)) return;
-  const int W = d.world, EPR = d.n_experts / W, K = d.topk;
+  __shared__ MoeArenas arenas;
+  if (!moe_wait_experts(d, arenas)) return;
   const int chunks = d.hidden / 16;  // 32-byte pieces per row
   const int upr = (chunks + 31) / 32;
   const size_t row_bytes = (size_t)d.hidden * 2;
@@ -680,31 +729,21 @@ __global__ void __launch_bounds__(kMoeThreads, R < 4 ? 2 : 1) moe_combine_bf16_s
   const int64_t per = (units + nwarps - 1) / nwarps;
   const int64_t u0 = (int64_t)warp * per;
   const int64_t u1 = u0 + per < units ? u0 + per : units;
-  int cur_t = -1;
-  const unsigned char* my_row = nullptr;
-  float my_w = 0.f;
+  if (u0 >= u1) return;
+  int cur_t = (int)(u0 / upr);
+  MoeRows<(R == 4)> rows(d, arenas, row_bytes, lane);
+  if (R == 4) rows.fetch(cur_t);
+  rows.enter(cur_t);
   auto locate = [&](int64_t u, int& t, int& c) {
     t = (int)(u / upr);
     const int part = (int)(u - (int64_t)t * upr);
     c = part * 32 + lane;
-    if (t != cur_t) {
-      cur_t = t;
-      my_row = nullptr;
-      my_w = 0.f;
-      if (lane < K) {
-        const int e = d.topk_idx[t * K + lane];
-        const int slot = d.slot_of[t * K + lane];
-        if (slot >= 0) {
-          my_row = reinterpret_cast<const unsigned char*>(d.arena_peer[e / EPR]) + ((size_t)d.rank * d.capacity + slot) * row_bytes;
-          my_w = d.topk_w[t * K + lane];
-        }
-      }
-    }
+    if (t != cur_t) rows.enter(cur_t = t);
   };
   auto issue = [&](int c, int k0, uint32_t (&v)[R][8]) {
 #pragma unroll
     for (int k = 0; k < R; ++k) {
-      const unsigned char* row = (const unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, k0 + k);
+      const unsigned char* row = rows.of(k0 + k);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[k][j] = 0u;
       if (row && c < chunks) moe_ld_v8(row + (size_t)c * 32, v[k]);
@@ -722,7 +761,6 @@ __global__ void __launch_bounds__(kMoeThreads, R < 4 ? 2 : 1) moe_combine_bf16_s
       }
     }
   };
-  if (u0 >= u1) return;
   uint32_t a[R][8], b[R][8];
   int t, c;
   int64_t u = u0;
@@ -730,7 +768,7 @@ __global__ void __launch_bounds__(kMoeThreads, R < 4 ? 2 : 1) moe_combine_bf16_s
   issue(c, 0, a);
   // one unit, whose first group is in x: what comes next is requested into the buffer that is not being accumulated
   auto unit = [&](uint32_t (&x)[R][8], uint32_t (&y)[R][8]) {
-    const float w_lane = my_w;
+    const float w_lane = rows.w;
     const int tu = t, cu = c;
     if (G == 2) issue(cu, R, y);
     float acc[16];
@@ -769,7 +807,8 @@ __global__ void __launch_bounds__(kMoeThreads, R < 4 ? 2 : 1) moe_combine_bf16_s
 
 // ---- combine, fp8 rows: lane owns 16 elements; dequantise while accumulating --
 __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_kernel(eux_moe_desc d) {
-  if (!moe_wait_experts(d)) return;
+  __shared__ MoeArenas arenas;
+  if (!moe_wait_experts(d, arenas)) return;
   const int W = d.world, EPR = d.n_experts / W, K = d.topk;
   const int upr = (d.hidden + 511) / 512;
   const size_t row_bytes = moe_row_bytes(d.hidden, 1);
@@ -788,7 +827,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_kernel(eux_moe_de
       int slot = d.slot_of[t * K + lane];
       if (slot >= 0) {
         int dst = e / EPR;
-        my_row = reinterpret_cast<const unsigned char*>(d.arena_peer[dst]) + ((size_t)d.rank * d.capacity + slot) * row_bytes;
+        my_row = arenas.of[dst] + ((size_t)d.rank * d.capacity + slot) * row_bytes;
         my_w = d.topk_w[t * K + lane];
       }
     }
@@ -849,7 +888,8 @@ __device__ __forceinline__ float pick4(const float (&r)[4], int i) {
 // The scales of the k rows are fetched once per row (two coalesced loads per row instead of one
 // small load per 512 elements), already multiplied by the gate weight.
 __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_rows_kernel(eux_moe_desc d) {
-  if (!moe_wait_experts(d)) return;
+  __shared__ MoeArenas arenas;
+  if (!moe_wait_experts(d, arenas)) return;
   const int W = d.world, EPR = d.n_experts / W, K = d.topk;
   const int upr = (d.hidden + 511) / 512;
   const int ngroups = d.hidden / 128;
@@ -865,7 +905,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_rows_kernel(eux_m
       int slot = d.slot_of[t * K + lane];
       if (slot >= 0) {
         int dst = e / EPR;
-        my_row = reinterpret_cast<const unsigned char*>(d.arena_peer[dst]) + ((size_t)d.rank * d.capacity + slot) * row_bytes;
+        my_row = arenas.of[dst] + ((size_t)d.rank * d.capacity + slot) * row_bytes;
         my_w = d.topk_w[t * K + lane];
       }
     }
@@ -991,12 +1031,12 @@ extern "C" int eux_moe_expert_ready_launch(const eux_moe_desc* d, void* stream) 
 // ---- combine, fp8 rows, top-k <= 8, hidden <= 8192: the streaming scheme of the bf16 kernel. A unit is 1024
 // elements of a token (32 bytes per lane, 1 KiB of a row per warp instruction); its rows are fetched as G
 // groups of two (2 G >= top-k), the next group always requested before the current one is dequantised and
-// accumulated. Lane L keeps gate weight x scale of groups L and 32 + L of every row, loaded once per token.
+// accumulated. Lane L keeps the scales of groups L and 32 + L of every row, loaded once per token.
 // (4096 tokens of 4096, with eight rows for every top-k and so: 25.2 and 18.5 us at top-1, 30.9 and 26.6 at 4, 40.0 and 38.7 at 6.)
 template <int G>
 __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux_moe_desc d) {
-  if (!moe_wait_experts(d)) return;
-  const int W = d.world, EPR = d.n_experts / W, K = d.topk;
+  __shared__ MoeArenas arenas;
+  if (!moe_wait_experts(d, arenas)) return;
   const int upr = (d.hidden + 1023) / 1024;
   const int ngroups = d.hidden / 128;
   const size_t row_bytes = moe_row_bytes(d.hidden, 1);
@@ -1008,40 +1048,31 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
   const int64_t u0 = (int64_t)warp * per;
   const int64_t u1 = u0 + per < units ? u0 + per : units;
   if (u0 >= u1) return;
-  int cur_t = -1;
-  const unsigned char* my_row = nullptr;
+  int cur_t = (int)(u0 / upr);
+  MoeRows<true> rows(d, arenas, row_bytes, lane);
+  rows.fetch(cur_t);
+  rows.enter(cur_t);
   float scw[2 * G][2];
   auto locate = [&](int64_t u, int& t, int& e0) {
     t = (int)(u / upr);
     e0 = (int)(u - (int64_t)t * upr) * 1024 + lane * 32;
   };
-  auto new_token = [&](int t) {
-    cur_t = t;
-    my_row = nullptr;
-    float my_w = 0.f;
-    if (lane < K) {
-      const int e = d.topk_idx[t * K + lane];
-      const int slot = d.slot_of[t * K + lane];
-      if (slot >= 0) {
-        my_row = reinterpret_cast<const unsigned char*>(d.arena_peer[e / EPR]) + ((size_t)d.rank * d.capacity + slot) * row_bytes;
-        my_w = d.topk_w[t * K + lane];
-      }
-    }
+  // the scales of the current token's rows, requested behind its first values and multiplied when they are used
+  auto scales = [&]() {
 #pragma unroll
     for (int k = 0; k < 2 * G; ++k) {
-      const unsigned char* row = (const unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, k);
-      const float wk = __shfl_sync(0xffffffffu, my_w, k);
+      const unsigned char* row = rows.of(k);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int g = r * 32 + lane;
-        scw[k][r] = (row && g < ngroups) ? wk * __ldcg(reinterpret_cast<const float*>(row + d.hidden) + g) : 0.f;
+        scw[k][r] = (row && g < ngroups) ? __ldcg(reinterpret_cast<const float*>(row + d.hidden) + g) : 0.f;
       }
     }
   };
   auto issue = [&](int e0, int k0, uint32_t (&v)[2][8]) {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      const unsigned char* row = (const unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)my_row, k0 + k);
+      const unsigned char* row = rows.of(k0 + k);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[k][j] = 0u;
       if (row && e0 < d.hidden) moe_ld_v8(row + e0, v[k]);
@@ -1050,9 +1081,9 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
   int t, e0;
   int64_t u = u0;
   locate(u, t, e0);
-  new_token(t);
   uint32_t a[2][8], b[2][8];
   issue(e0, 0, a);
+  scales();
   // one unit, whose first group is in x; the first group of the next one ends up in x where G is even, in y where it is odd
   auto unit = [&](uint32_t (&x)[2][8], uint32_t (&y)[2][8]) {
     const int tu = t, eu = e0;
@@ -1063,7 +1094,8 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
     // the weights of this unit's token, fetched before the routing entries may move on to the next one
     float wk[2 * G];
 #pragma unroll
-    for (int k = 0; k < 2 * G; ++k) wk[k] = __shfl_sync(0xffffffffu, (gi >> 5) ? scw[k][1] : scw[k][0], gi & 31);
+    for (int k = 0; k < 2 * G; ++k)
+      wk[k] = __shfl_sync(0xffffffffu, rows.w, k) * __shfl_sync(0xffffffffu, (gi >> 5) ? scw[k][1] : scw[k][0], gi & 31);
     auto accumulate = [&](const uint32_t (&v)[2][8], float w0, float w1) {
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
@@ -1089,8 +1121,10 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_stream_kernel(eux
         issue(eu, 2 * (g + 1), then);
       } else if (u + 1 < u1) {
         locate(u + 1, t, e0);
-        if (t != cur_t) new_token(t);
+        const bool entered = t != cur_t;
+        if (entered) rows.enter(cur_t = t);
         issue(e0, 0, then);
+        if (entered) scales();
       }
       accumulate(now, wk[2 * g], wk[2 * g + 1]);
     }
