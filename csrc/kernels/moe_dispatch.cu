@@ -1013,7 +1013,13 @@ extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* st
   // A CTA per token, up to one per SM: a second one counts all entries again (256 tokens, fp8: 28.2 us for the exchange
   // with one, 30.2 with two).
   const int one = ctas > 0 ? ctas : sms;
-  if (!d->fp8) return moe_dispatch<moe_dispatch_bf16_kernel>(d, one, sms, routing, st);
+  if (!d->fp8) {
+    // Rows for more than twice the L2: six CTAs per SM, the last ones of which begin as SMs become free, so that no SM's share
+    // ends late (top-8 of 7168, the exchange with one and with six per SM: 2048 tokens, 235 MB, 104.5 and 104.3 us; 2560
+    // 128.7 and 126.6; 4096 197.8 and 192.0; 8192 376.1 and 360.6).
+    const bool large = (int64_t)d->n_tokens * d->topk * d->hidden * 2 >= (int64_t(256) << 20) && d->n_tokens >= 12 * sms;
+    return moe_dispatch<moe_dispatch_bf16_kernel>(d, ctas > 0 ? ctas : large ? 6 * sms : sms, sms, routing, st);
+  }
   if (const int slots = moe_image_slots(d->hidden); slots > 0 && d->n_tokens >= 2 * (int64_t)one)
     return moe_dispatch<moe_dispatch_fp8_bulk_kernel>(d, one, sms, routing + 128 + (size_t)slots * moe_row_bytes(d->hidden, 1), st, slots);
   // Rows too wide for images and more than eight tokens per CTA: two per SM, one of which works while the other waits at its

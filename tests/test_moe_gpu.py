@@ -328,3 +328,9 @@ def test_combine_fetches_as_many_rows_as_there_are(cuda_device, topk, fp8, t, hi
         ref = moe.reference_dispatch_combine(x, idx, w, fp8)
         bound = ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True) + 1e-30
         assert bool(((out.float() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("t,hidden,topk", [(1775, 9472, 8), (1776, 9472, 8), (2561, 6656, 8)])
+def test_bf16_dispatch_of_more_than_the_l2_holds(cuda_device, t, hidden, topk):
+    """On both sides of the number of tokens and bytes from which a dispatch has several CTAs per SM."""
+    test_dispatch_routes_in_one_launch(cuda_device, t, hidden, topk, 64, False)
