@@ -503,9 +503,9 @@ __device__ __forceinline__ void cluster_sync_all() {
 // further on from `first`.
 // Layout of a part: 16 bytes (four columns) of one row next to the same columns of the next row, so that a warp's store
 // is one run of 512 bytes (rows further apart: 3 us more per tile); neighbours within eight rows are exchanged by the
-// number of the column group, so that the owner's reads along a row meet eight different banks. The exchange takes 3.7 of
-// the 28 us of 128 x 8192 x 8192: 16 bytes per cycle and SM is what the network between SMs carries (stores, asynchronous
-// stores and bulk copies alike); the K loop before it runs at 6.3 TB/s of W.
+// number of the column group, so that the owner's reads along a row meet eight different banks. The network between SMs
+// carries 16 bytes per cycle and SM (stores, asynchronous stores and bulk copies alike), which is what the exchange takes:
+// 3.7 us for four shares of 128 x 256.
 template <int COLS>
 struct SplitParts {
   uint32_t base;  // of this CTA's parts: [share][group of four columns][row of the owner]
@@ -599,7 +599,6 @@ __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_bas
   split_write(p, parts, p.y + ((size_t)mb * BM * p.N + (size_t)nb * BN) * 2, warp, lane);
 }
 
-template <bool SPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_y, GemmParams p) {
@@ -662,11 +661,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   const int m_blocks = p.M / BM, n_blocks = p.N / BN;
   const int total = m_blocks * n_blocks;
-  const int k_all = p.K * p.elem_bytes / BKB;
-  const int rank = SPLIT ? (int)cluster_cta_rank() : 0;
-  const int tile0 = SPLIT ? (int)blockIdx.x / p.split : 0;  // past the last tile: this cluster only helps to copy X
-  const int k_begin = SPLIT ? k_all * rank / p.split : 0;  // this CTA's share of K
-  const int k_iters = (SPLIT ? k_all * (rank + 1) / p.split : k_all) - k_begin;
+  const int k_iters = p.K * p.elem_bytes / BKB;
   const int kelems = BKB / p.elem_bytes;  // elements of K per stage
   volatile int* abort = &s_abort;
   // the next tile as the consumer roles see it: bounded wait on the ring slot, then its content
@@ -688,9 +683,9 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     int s = 0;
     uint32_t ph = 0;
     for (int it = 0;; ++it) {
-      int tile = it == 0 ? tile0 : total;  // SPLIT: one tile per cluster
+      int tile = total;
       if (lane == 0) {
-        if (!SPLIT) tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+        tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
       }
@@ -703,8 +698,8 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (; k < k_iters; ++k) {
         if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
         mbar_expect_tx(issue, full_bar(s), A_STAGE_BYTES + B_STAGE_BYTES);
-        tma_load_2d(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_bar(s), (k_begin + k) * kelems, mb * BM);
-        tma_load_2d(issue, b0 + (uint32_t)s * B_STAGE_BYTES, &map_b, full_bar(s), (k_begin + k) * kelems, nb * BN);
+        tma_load_2d(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_bar(s), k * kelems, mb * BM);
+        tma_load_2d(issue, b0 + (uint32_t)s * B_STAGE_BYTES, &map_b, full_bar(s), k * kelems, nb * BN);
         if (++s == STAGES) s = 0, ph ^= 1u;
       }
       if (k < k_iters) break;
@@ -763,7 +758,6 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint32_t tph = (uint32_t)(it >> 1) & 1u;
       const bool got = mbar_wait(tfull_bar(buf), tph, abort, p.timeout_ns);
       if (epi_vote_any(1, !got)) break;  // all four warps or none: the slab barriers below need everyone
-      if (SPLIT) break;  // summed over the cluster below
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)buf * BN;
 #pragma unroll 1
@@ -800,7 +794,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
       }
     }
-    if (!SPLIT && elected) {  // Y is complete before this CTA reports
+    if (elected) {  // Y is complete before this CTA reports
       bulk_wait_all();
       asm volatile("fence.proxy.async;" ::: "memory");
     }
@@ -808,14 +802,6 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   tc_fence_before();
   __syncthreads();
-  if (SPLIT && tile0 < total) {
-    tc_fence_after();
-    int mb, nb;
-    tile_coords(tile0, m_blocks, n_blocks, p.head_blocks, mb, nb);
-    split_sum(p, tmem_base, smem_u32(smem), mb, nb, rank, 0, 1, &s_abort);
-    tc_fence_before();
-    __syncthreads();
-  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
@@ -1543,6 +1529,201 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 }
 
 // ---------------------------------------------------------------------------
+// bf16 with few tiles: a CTA pair computes a tile of 128 rows of X by 256 of Wt the other way round, Wt as the tensor core's
+// A operand (M = 256, 128 rows of it per CTA) and X as B (N = 128, 64 rows per CTA), so that
+//   * an accumulator is 128 x 128 per CTA, half of what one CTA that has the tile for itself holds, for the same operand
+//     bytes per CTA (192 rows a K step): half as many shares of K keep as many CTAs busy, and the sum over them, which the
+//     network between SMs carries at 16 bytes per cycle and SM, is a third of the bytes (two shares of 64 KiB instead of
+//     four of 128) or nothing (one share instead of two);
+//   * a K step brings 24 KiB into a CTA: eight stages.
+// K is shared out over p.split pairs of a cluster (1, 2 or 4), which add their sums up in the order of the shares.
+// One tile per cluster; clusters past the last tile only help to copy X.
+// 128 x 8192 x 8192 takes 27.5 us a call (30.1 with four single CTAs to a tile), 20.5 of them W at the rate of HBM.
+// ---------------------------------------------------------------------------
+constexpr int FEW_STAGES = 8;
+constexpr int FEW_X_BYTES = (BM / 2) * BKB;
+constexpr int FEW_STAGE_BYTES = A_STAGE_BYTES + FEW_X_BYTES;
+constexpr size_t FEW_SMEM = (size_t)FEW_STAGES * FEW_STAGE_BYTES + 1024 + 256;
+constexpr int FEW_TMEM_COLS = BM;
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+remote_gemm_few_tiles_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, GemmParams p) {
+  extern __shared__ unsigned char smem_raw[];
+  allow_next_launch();
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sW = smem;
+  unsigned char* sX = smem + (size_t)FEW_STAGES * A_STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)FEW_STAGES * FEW_STAGE_BYTES);
+  // bars: [0,S) full (used in the even CTA), [S,2S) empty, 2S the accumulator is complete
+  __shared__ uint32_t s_tmem_base;
+  __shared__ int s_abort;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_cta_rank() & 1u;   // within the pair
+  const uint32_t even = cluster_cta_rank() & ~1u;  // cluster rank of the pair's even CTA
+  const uint32_t bar0 = smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (FEW_STAGES + s); };
+  const uint32_t done_bar = bar0 + 8u * (2 * FEW_STAGES);
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int s = 0; s < FEW_STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(done_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                 "r"((uint32_t)FEW_TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the partner's barriers exist before anything arrives on them
+  tc_fence_after();
+  const uint32_t tmem_base = s_tmem_base;
+  wait_for_launch_before();
+
+  const int m_blocks = p.M / BM, n_blocks = p.N / BN, total = m_blocks * n_blocks;
+  const int share = (int)(even >> 1);
+  const int tile = (int)blockIdx.x / (2 * p.split);
+  const int k_all = p.K * p.elem_bytes / BKB;
+  const int k_begin = k_all * share / p.split, k_iters = k_all * (share + 1) / p.split - k_begin;
+  const int kelems = BKB / p.elem_bytes;
+  volatile int* abort = &s_abort;
+  int mb = 0, nb = 0;
+  if (tile < total) tile_coords(tile, m_blocks, n_blocks, p.head_blocks, mb, nb);
+
+  if (warp == 2 || warp == 3) {
+    // ---------------- X from the caller's memory into the staging buffer ----------------
+    if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
+  } else if (tile < total) {
+    if (warp == 0) {
+      // ---------------- loads: both CTAs, completion counted in the even CTA ----------------
+      const uint32_t issue = elect_lane();
+      const uint32_t issue_leader = rank == 0 ? issue : 0u;
+      const uint32_t w0 = smem_u32(sW), x0 = smem_u32(sX);
+      const uint32_t full0 = map_to_cta(full_bar(0), even);
+      if (p.panel_target <= 0 || panel_wait_warp(p, mb, lane, abort)) {
+        int s = 0;
+        uint32_t ph = 0;
+        for (int k = 0; k < k_iters; ++k) {
+          if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+          const uint32_t full_leader = full0 + 8u * (uint32_t)s;
+          mbar_expect_tx(issue_leader, full_bar(s), 2 * FEW_STAGE_BYTES);
+          tma_load_2d_pair(issue, w0 + (uint32_t)s * A_STAGE_BYTES, &map_w, full_leader, (k_begin + k) * kelems, nb * BN + (int)rank * BM);
+          tma_load_2d_pair(issue, x0 + (uint32_t)s * FEW_X_BYTES, &map_x, full_leader, (k_begin + k) * kelems, mb * BM + (int)rank * (BM / 2));
+          if (++s == FEW_STAGES) s = 0, ph ^= 1u;
+        }
+      }
+      if (*abort && lane == 0) {  // let copies that are still in flight land before shared memory is used for the sum
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // ---------------- MMA: the even CTA issues for the pair ----------------
+      if (rank == 0) {
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+        const uint32_t issue = elect_lane();
+        const uint32_t both = 3u << even;
+        const uint64_t wdesc0 = umma_desc_sw128(smem_u32(sW)), xdesc0 = umma_desc_sw128(smem_u32(sX));
+        int s = 0, k = 0;
+        uint32_t ph = 0;
+        for (; k < k_iters; ++k) {
+          if (!mbar_wait_warp(full_bar(s), ph, abort, p.timeout_ns)) break;
+          tc_fence_after();
+          const uint64_t wd = wdesc0 + (uint32_t)s * (A_STAGE_BYTES >> 4), xd = xdesc0 + (uint32_t)s * (FEW_X_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < BKB / 32; ++kk) umma_pair(issue, tmem_base, wd + kk * 2, xd + kk * 2, idesc, (uint32_t)((k | kk) != 0));
+          umma_commit_pair(issue, empty_bar(s), both);
+          if (++s == FEW_STAGES) s = 0, ph ^= 1u;
+        }
+        if (k == k_iters) umma_commit_pair(issue, done_bar, both);  // a tile that is not complete is not announced
+      }
+    } else {
+      mbar_wait(done_bar, 0, abort, p.timeout_ns);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+
+  if (tile < total) {
+    // Share q owns rows [q * 128 / split, ...) of X: every CTA stores its part of them (fp32, its 128 columns of Y) into the
+    // owner's shared memory, 16 bytes (four rows) of one column next to the next column's. The two columns that a lane of
+    // the owner reads are neighbours: columns 8..15 of 16 are stored in pairs the other way round, so that the 16-byte
+    // reads of eight lanes meet 32 different banks.
+    tc_fence_after();
+    const int lg = warp & 3, side = warp >> 2;
+    const int rows = BM / p.split;
+    const uint32_t base = smem_u32(smem);
+    __syncwarp();
+    cluster_sync_relaxed();  // every CTA's last MMA is behind it: the stages are free
+    if (threadIdx.x == 0) split_spread_abort(&s_abort, (uint32_t)(2 * p.split));
+    __syncwarp();
+    const uint32_t column = (uint32_t)(lg * 32 + lane) ^ (uint32_t)(lane >> 3 & 1);
+    const uint32_t tcol = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(side * (BM / 2));
+#pragma unroll
+    for (int c = 0; c < BM / 2; c += 32) {
+      uint32_t r[32];
+      tmem_ld32(tcol + (uint32_t)c, r);
+      tmem_ld_wait();
+      const int row = side * (BM / 2) + c;  // 32 rows of X: of one owner
+      const uint32_t out = map_to_cta(base + (uint32_t)(share * rows + row % rows) * (BM * 4u) + column * 16u, 2u * (uint32_t)(row / rows) + rank);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out + (uint32_t)q * (BM * 16u)), "r"(r[4 * q]),
+                     "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
+                     : "memory");
+    }
+    tc_fence_before();
+    __syncwarp();
+    cluster_sync_all();
+    if (!*abort) {
+      // a warp writes 128 bytes of four rows at a time
+      for (int u = warp; u < rows / 2; u += GEMM_THREADS / 32) {
+        const int group = u >> 1, col = (u & 1) * 64 + 2 * lane;
+        const uint32_t slot = (uint32_t)col ^ (uint32_t)(col >> 3 & 1);
+        float acc[2][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] = 0.f;
+        for (int q = 0; q < p.split; ++q) {
+          const uint32_t in = base + (uint32_t)(q * rows + group * 4) * (BM * 4u);
+          float v[2][4];
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[i][0]), "=f"(v[i][1]), "=f"(v[i][2]), "=f"(v[i][3])
+                         : "r"(in + (slot ^ (uint32_t)i) * 16u)
+                         : "memory");
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i >> 2][i & 3] += v[i >> 2][i & 3];
+        }
+        unsigned char* out = p.y + (((size_t)mb * BM + share * rows + group * 4) * p.N + (size_t)nb * BN + rank * BM + col) * 2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<__nv_bfloat162*>(out + (size_t)j * p.N * 2) = __floats2bfloat162_rn(acc[0][j], acc[1][j]);
+      }
+    }
+    __syncthreads();
+  }
+  cluster_sync_all();  // neither CTA leaves while the other may still touch its shared memory or TMEM
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)FEW_TMEM_COLS) : "memory");
+  }
+  const bool ok = s_abort == 0;
+  if (!ok && threadIdx.x == 0) {
+    set_status(p.status, EUX_ST_TIMEOUT, 20);
+    atomicExch(p.sched + 1, 1u);
+  }
+  finish_cta(p, ok);
+}
+
+// ---------------------------------------------------------------------------
 // Block-scaled fp8 on CTA pairs: the promotion scheme of remote_gemm_fp8_kernel on 256 x 256 tiles, half the operand bytes
 // per flop. What bounds it is the fold: a K-block is 512 cycles of MMA and takes about 1000. So:
 //   * Sixteen warps fold, 32 rows by 64 columns each. The arithmetic of the fold is 280 cycles per K-block; the rest of a
@@ -1935,16 +2116,16 @@ static int launch_clusters(int dev, int cluster, int grid, int threads, size_t s
   return (int)cudaLaunchKernelEx(&l.cfg, KERNEL, args...);
 }
 
-// Shares of K per tile (1, 2, 4 or 8) for `tiles` clusters of `ctas` CTAs per share: from 24 K steps on, as many as
-// leave eight steps to each while all clusters fit the device at once (asked of the driver, once per device and size).
+// Shares of K per tile (1, 2, 4 or 8) for `tiles` clusters of `ctas` CTAs per share: from `from` K steps on, as many as
+// leave `least` steps to each while all clusters fit the device at once (asked of the driver, once per device and size).
 // `clusters`: how many of them fit.
 template <auto KERNEL>
-static int choose_split(int dev, int threads, size_t smem, int tiles, int ctas, int k_iters, int* clusters) {
+static int choose_split(int dev, int threads, size_t smem, int tiles, int ctas, int k_iters, int from, int least, int* clusters) {
   static std::atomic<int> resident[64][4];  // 1 + the number of clusters
   int split = 1;
   for (int i = 1; i < 4 && ctas << i <= 8; ++i) {
     const int s = 1 << i;
-    if (k_iters < 24 || k_iters < 8 * s) break;
+    if (k_iters < from || k_iters < least * s) break;
     int n = resident[dev][i].load(std::memory_order_acquire) - 1;
     if (n < 0) {
       n = 0;
@@ -2025,14 +2206,17 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   const int tiles = (d->M / BM) * (d->N / bn), tiles2 = m_pairs * n_pairs;
   const int waves = (tiles + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
   // Few tiles: the K of a tile is shared out over a cluster of CTAs (or CTA pairs), which add their sums up through
-  // distributed shared memory. A K step costs a CTA about half a microsecond, the sum about three. Calls in a loop:
-  // 128 x 8192 x 8192 (32 tiles) 35 us with four CTAs per tile and 59 with one, 128 x 512 x 8192 18 with eight and 46 with
-  // one; 384 x 4096 x 1024, sixteen steps, 16.5 with two and 14.3 with one. All clusters have to fit at once: a second
-  // wave costs more.
+  // distributed shared memory. All clusters have to fit at once: a second wave costs more.
+  // bf16: wherever there is a pair of SMs for each 128 x 256 tile, and several pairs per tile from eight K steps on, four or
+  // more for each. Against single CTAs that shared K from 24 steps on, eight or more for each (calls in a loop):
+  // 128 x 8192 x 8192 30.1 -> 27.8 us, 128 x 512 x 8192 12.8 -> 11.2, 256 x 8192 x 8192 40.5 -> 37.5, 128 x 8192 x 1024
+  // 10.1 -> 8.1 (8.7 without sharing K), 128 x 512 x 512 7.3 -> 6.5, 1152 x 2048 x 1024 (72 tiles) 10.3 -> 9.1.
+  // 256 x 256 tiles whose K is shared: 256 x 8192 x 2048 13.7 against 11.7 us, 256 x 8192 x 8192 35.2 against 35.5.
+  // fp8 and MXFP8, whose partial sums are twice as large for a CTA's operand bytes: from 24 steps on, eight for each.
   if (!pull || copy_by_warps) {
     int clusters = 0;
     if (mx) {
-      const int s = choose_split<remote_gemm_2cta_kernel<true, true>>(dev, GEMM_THREADS, PairCfg<true>::SMEM, tiles2, 2, k_iters, &clusters);
+      const int s = choose_split<remote_gemm_2cta_kernel<true, true>>(dev, GEMM_THREADS, PairCfg<true>::SMEM, tiles2, 2, k_iters, 24, 8, &clusters);
       if (s > 1) {
         if (!pull) clusters = tiles2;  // with X to copy, clusters without a tile help with that
         CUtensorMap mb2, msa, msb;
@@ -2046,16 +2230,27 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
         return launch_clusters<remote_gemm_2cta_kernel<true, true>>(dev, 2 * s, 2 * clusters * s, GEMM_THREADS, PairCfg<true>::SMEM, st, ma, mb2,
                                my, msa, msb, p);
       }
+    } else if (!d->fp8) {
+      clusters = sms / 2;
+      const int s = choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, tiles, 2, k_iters, 8, 4, &clusters);
+      if (tiles <= clusters) {
+        if (!pull) clusters = tiles;
+        CUtensorMap mx2, mb2;  // a CTA's half of either operand
+        if (int rc = make_map(&mx2, d->x_stage, eb, (uint64_t)d->M, (uint64_t)d->K, BM / 2)) return rc;
+        if (int rc = make_map(&mb2, d->w_t, eb, (uint64_t)d->N, (uint64_t)d->K, BN / 2)) return rc;
+        p.split = s, p.copy_ctas = 0;
+        p.copy_warps = pull ? 2 * 2 * clusters * s : 0;
+        p.panel_target = pull ? warp_target(p.copy_warps) : 0;
+        return launch_clusters<remote_gemm_few_tiles_kernel>(dev, 2 * s, 2 * clusters * s, GEMM_THREADS, FEW_SMEM, st, mx2, mb2, p);
+      }
     } else {
-      const int s = d->fp8 ? choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters, &clusters)
-                           : choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, tiles, 1, k_iters, &clusters);
+      const int s = choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters, 24, 8, &clusters);
       if (s > 1) {
         if (!pull) clusters = tiles;
         p.split = s, p.copy_ctas = 0;
         p.copy_warps = pull ? 2 * clusters * s : 0;
         p.panel_target = pull ? warp_target(p.copy_warps) : 0;
-        if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, clusters * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
-        return launch_clusters<remote_gemm_kernel<true>>(dev, s, clusters * s, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
+        return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, clusters * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
       }
     }
   }
@@ -2105,7 +2300,7 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
     p.panel_target = warp_target(p.copy_warps);
   }
   if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<false>>(dev, 1, grid, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
-  return launch_clusters<remote_gemm_kernel<false>>(dev, 1, grid, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
+  return launch_clusters<remote_gemm_kernel>(dev, 1, grid, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -2120,15 +2315,16 @@ static __device__ __align__(256) uint32_t g_noalloc_gemm_scratch[EUX_NOALLOC_GEM
 
 // Everything that a first launch of one of the bf16 kernels would set up: which of them a call takes depends on its shape.
 static int prepare_bf16(int dev) {
-  const void* kernels[] = {(const void*)remote_gemm_kernel<false>, (const void*)remote_gemm_kernel<true>,
+  const void* kernels[] = {(const void*)remote_gemm_kernel, (const void*)remote_gemm_few_tiles_kernel,
                            (const void*)remote_gemm_2cta_kernel<false, false>};
   cudaFuncAttributes attr;
   for (const void* k : kernels)
     if (cudaError_t e = cudaFuncGetAttributes(&attr, k); e != cudaSuccess) return (int)e;
-  cudaError_t e = allow_smem<remote_gemm_kernel<false>>(dev, GEMM_SMEM);
+  cudaError_t e = allow_smem<remote_gemm_kernel>(dev, GEMM_SMEM);
   if (e == cudaSuccess) e = allow_smem<remote_gemm_2cta_kernel<false, false>>(dev, PairCfg<false>::SMEM);
   int clusters = 0;  // one tile and a long K: every size of cluster is asked about
-  choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, 1, 1, 64, &clusters);
+  if (e == cudaSuccess) e = allow_smem<remote_gemm_few_tiles_kernel>(dev, FEW_SMEM);
+  choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, 1, 2, 64, 8, 4, &clusters);
   return (int)e;
 }
 
@@ -2181,7 +2377,7 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
 // that loads): a service that launches on behalf of a peer calls this when it is set up.
 extern "C" int eux_gemm_preload(void) {
   cudaFuncAttributes attr;
-  const void* kernels[] = {(const void*)remote_gemm_kernel<false>,           (const void*)remote_gemm_kernel<true>,
+  const void* kernels[] = {(const void*)remote_gemm_kernel,                  (const void*)remote_gemm_few_tiles_kernel,
                            (const void*)remote_gemm_fp8_kernel<false>,       (const void*)remote_gemm_fp8_kernel<true>,
                            (const void*)remote_gemm_2cta_kernel<false, false>, (const void*)remote_gemm_2cta_kernel<true, false>,
                            (const void*)remote_gemm_2cta_kernel<true, true>, (const void*)remote_gemm_fp8_2cta_kernel};

@@ -288,3 +288,18 @@ def test_calls_behind_one_another(cuda_device, m, k, pull):
         torch.cuda.synchronize()
         g.check_status()
         assert all(torch.equal(b, w) for b, w in zip(bufs, want))
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 256, 64), (128, 512, 512), (384, 256, 8 * 64 + 64), (128, 9472, 1024 - 64), (1280, 1792, 15 * 64),
+                                   (128, 4096, 16 * 64)])
+@pytest.mark.parametrize("pull", [False, True])
+def test_few_tiles_of_any_k(cuda_device, m, n, k, pull):
+    """A pair of SMs for each tile: one K step and more than there are stages, one, two and four shares of K of unequal
+    length, one tile, and as many as there are pairs. The tolerance of test_few_tiles."""
+    test_few_tiles(cuda_device, "bf16", m, n, k, pull)
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 256, 512), (256, 1792, 4096), (384, 4352, 2048)])
+def test_few_tiles_give_up(cuda_device, m, n, k):
+    """X never arrives: four shares of K, four with clusters that only copy, and one."""
+    test_a_wait_that_runs_out(cuda_device, "bf16", m, n, k)
