@@ -1607,15 +1607,24 @@ remote_gemm_few_tiles_kernel(const __grid_constant__ CUtensorMap map_x, const __
       const uint32_t issue_leader = rank == 0 ? issue : 0u;
       const uint32_t w0 = smem_u32(sW), x0 = smem_u32(sX);
       const uint32_t full0 = map_to_cta(full_bar(0), even);
+      auto load_w = [&](int k, int s) {
+        mbar_expect_tx(issue_leader, full_bar(s), 2 * FEW_STAGE_BYTES);
+        tma_load_2d_pair(issue, w0 + (uint32_t)s * A_STAGE_BYTES, &map_w, full0 + 8u * (uint32_t)s, (k_begin + k) * kelems,
+                         nb * BN + (int)rank * BM);
+      };
+      // W does not wait for X: the stages' halves of it are on their way while the copying warps bring the panel
+      const int ahead = k_iters < FEW_STAGES ? k_iters : FEW_STAGES;
+      for (int k = 0; k < ahead; ++k) load_w(k, k);
       if (p.panel_target <= 0 || panel_wait_warp(p, mb, lane, abort)) {
         int s = 0;
         uint32_t ph = 0;
         for (int k = 0; k < k_iters; ++k) {
-          if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
-          const uint32_t full_leader = full0 + 8u * (uint32_t)s;
-          mbar_expect_tx(issue_leader, full_bar(s), 2 * FEW_STAGE_BYTES);
-          tma_load_2d_pair(issue, w0 + (uint32_t)s * A_STAGE_BYTES, &map_w, full_leader, (k_begin + k) * kelems, nb * BN + (int)rank * BM);
-          tma_load_2d_pair(issue, x0 + (uint32_t)s * FEW_X_BYTES, &map_x, full_leader, (k_begin + k) * kelems, mb * BM + (int)rank * (BM / 2));
+          if (k >= ahead) {
+            if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
+            load_w(k, s);
+          }
+          tma_load_2d_pair(issue, x0 + (uint32_t)s * FEW_X_BYTES, &map_x, full0 + 8u * (uint32_t)s, (k_begin + k) * kelems,
+                           mb * BM + (int)rank * (BM / 2));
           if (++s == FEW_STAGES) s = 0, ph ^= 1u;
         }
       }
