@@ -349,7 +349,6 @@ __device__ bool copy_role_n(const GemmParams& p, const int nthreads, unsigned ch
       if (p.status) set_status(p.status, EUX_ST_TIMEOUT, 9);
       atomicExch(p.sched + 1, 1u);
     }
-    __threadfence();  // the counts are in before this CTA is counted as done: the last one clears them
   }
   __syncthreads();
   return cp_abort == 0;
@@ -436,21 +435,25 @@ __device__ __forceinline__ void copy_warp_role(const GemmParams& p, uint32_t war
     u = next;
   }
   if (pending >= 0) count(pending);
-  if (lane == 0) __threadfence();  // the counts are in before this CTA is counted as done: the last one clears them
 }
 
 __device__ __forceinline__ void finish_cta(const GemmParams& p, bool ok) {
   __syncthreads();
   if (threadIdx.x != 0) return;
-  // Without a flag to publish the end of the launch is enough for Y: no fence here and none in the last CTA (a call of
-  // 640 x 4096 x 1024 took 13.1 us with them and 11.3 without). With one, the last CTA's fence for everyone covers what the
-  // others wrote before they counted themselves. A CTA that gave up has said so before it is counted.
-  if (p.done_flag || !ok) fence_gpu();
+  // The last CTA clears the scratch. What any CTA did to it (panels counted and polled, units of X drawn, a failure noted)
+  // comes before that by this thread's fence, which covers the CTA's other threads through the barrier above, and by the
+  // last CTA's. With X in place and no failure there is only the tile counter: its draws and the clearing are writes of one
+  // word, and a CTA is counted after its last draw, the leader of a pair for both through the cluster's barriers.
+  // Without a flag to publish the end of the launch is enough for Y, so such a call has no fence per CTA (640 x 4096 x 1024
+  // took 13.1 us with one and 11.3 without). With a flag, the last CTA's fence for everyone covers what the others wrote
+  // before they counted themselves.
+  if (p.done_flag || p.panel_target > 0 || !ok) fence_gpu();
   const uint32_t old = atomicAdd(p.sched, 1u);
   if (old == gridDim.x - 1) {
-    if (p.done_flag) fence_gpu();
+    fence_gpu();
     const bool all_ok = ok && __ldcg(p.sched + 1) == 0;
-    for (int i = 0; i < p.M / BM; ++i) p.panel_flags[i] = 0;
+    if (p.panel_target > 0)  // otherwise nobody has touched them
+      for (int i = 0; i < p.M / BM; ++i) p.panel_flags[i] = 0;
     p.sched[0] = 0;
     p.sched[1] = 0;
     p.sched[2] = 0;  // the tile counter

@@ -303,3 +303,39 @@ def test_few_tiles_of_any_k(cuda_device, m, n, k, pull):
 def test_few_tiles_give_up(cuda_device, m, n, k):
     """X never arrives: four shares of K, four with clusters that only copy, and one."""
     test_a_wait_that_runs_out(cuda_device, "bf16", m, n, k)
+
+
+def _operands(fmt, m, n, k, calls, dev):
+    """The op with its weight, the arguments of `calls` calls, and their products in 64 bits."""
+    from execution_ucx_b200.ops import remote_gemm as rg
+    torch.manual_seed(m + n + k)
+    w = torch.randn(k, n, device=dev) * 0.02
+    xs = [torch.randn(m, k, device=dev) for _ in range(calls)]
+    if fmt == "bf16":
+        g, args = rg.RemoteGemm(w.to(torch.bfloat16), m), [[x.to(torch.bfloat16)] for x in xs]
+        return g, args, [x.double() @ w.to(torch.bfloat16).double() for (x,) in args]
+    if fmt == "fp8_block":
+        g, args = rg.RemoteGemmFp8(w, m), [list(rg.quantize_rows_1x128(x)) for x in xs]
+        return g, args, [rg.dequantized_reference(q.double(), s.double(), g.w_q_t.double(), g.w_scale.double()).double() for q, s in args]
+    g, quantized = rg.RemoteGemmMx(w, m), [rg.quantize_mx(x) for x in xs]
+    return (g, [[q, rg.mx_scale_chunks(s, False)] for q, s in quantized],
+            [rg.mx_dequantized_reference(q.double(), s.double(), g.w_q_t.double(), g.w_sf.double()).double() for q, s in quantized])
+
+
+@pytest.mark.parametrize("fmt,m,n,k", [("bf16", 640, 4096, 1024), ("bf16", 2304, 2304, 1024), ("bf16", 256, 1792, 4096),
+                                       ("fp8_block", 640, 2048, 1024), ("fp8_block", 256, 640, 3200), ("fp8_block", 1920, 4480, 2560),
+                                       ("mxfp8", 1024, 1024, 1024), ("mxfp8", 512, 768, 3200)])
+def test_scratch_of_calls_without_a_flag(cuda_device, fmt, m, n, k):
+    """Calls with X streamed in and in place by turns, each with an X of its own, behind one another on one scratch and
+    without a completion flag, on every kernel: a panel counted too early, or a count that outlives the clearing, would bring
+    rows of the call before. fp32 sums (1e-5 of a row's largest result) and one rounding to bf16 (2^-8 of the value)."""
+    g, args, refs = _operands(fmt, m, n, k, 4, cuda_device)
+    ys = [torch.zeros(m, n, dtype=torch.bfloat16, device=cuda_device) for _ in range(12)]
+    for i, y in enumerate(ys):
+        g(*[a.data_ptr() for a in args[i % 4]], m, y.data_ptr(), x_is_local=i % 3 == 2)
+    torch.cuda.synchronize()
+    g.check_status()
+    assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+    for i, y in enumerate(ys):
+        ref = refs[i % 4]
+        assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
