@@ -488,8 +488,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
   return out;
 }
-// The same without ordering memory, for the point at which every CTA has seen the end of its MMAs: nothing written before
-// it is read behind it, and the release in a full barrier waits for whatever the CTA has in flight
+// The same without ordering memory, for the point at which every CTA has seen the end of its MMAs: no CTA reads behind it
+// what another one wrote before it, and the release in a full barrier waits for whatever the CTA has in flight. What a
+// CTA's own warps have to tell one another there (that one of them gave up) goes over a barrier of the CTA in front of it.
 __device__ __forceinline__ void cluster_sync_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
@@ -837,11 +838,13 @@ constexpr int TBUF8 = 4;  // partial products in flight: four 128-column TMEM bu
 constexpr size_t GEMM8_SMEM = (size_t)STAGES8 * (A8_STAGE_BYTES + B8_STAGE_BYTES) + 2 * 16384 /* output slabs */ + 1024 + 256;
 
 // split_sum for the block-scaled fp8 kernel, whose epilogue warps hold their sums in registers: thread (row, half) has
-// the 64 columns of its half of a 128 x 128 tile. Called by the epilogue warps; the others join the two barriers.
+// the 64 columns of its half of a 128 x 128 tile. Called by the epilogue warps; the others join the three barriers.
+__device__ __forceinline__ void split_cta_sync() { asm volatile("barrier.sync 3, %0;" ::"n"(GEMM8_THREADS) : "memory"); }
 __device__ __forceinline__ void split_sum_regs(const GemmParams& p, const float (&acc)[64], uint32_t smem0, int tile, int m_blocks,
                                                int n_blocks, int rank, int half, int row, int* s_abort) {
   const SplitParts<BN8> parts{smem0, p.split, rank, 0, 1};
   const uint32_t dst = parts.out(row);
+  split_cta_sync();
   __syncwarp();
   cluster_sync_relaxed();
   if (half == 0 && row == 0) split_spread_abort(s_abort, (uint32_t)p.split);
@@ -994,7 +997,8 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     // warps 2 and 3: X (and its scales) from the caller's memory into the staging buffer
     if (p.copy_warps > 0) copy_warp_role(p, (uint32_t)blockIdx.x * 2u + (uint32_t)(warp - 2), lane);
   }
-  if (SPLIT && tile0 < total && warp < 4) {  // the two barriers of split_sum_regs count every thread of the cluster
+  if (SPLIT && tile0 < total && warp < 4) {  // the barriers of split_sum_regs count every thread of the CTA and of the cluster
+    split_cta_sync();
     __syncwarp();
     cluster_sync_relaxed();
     cluster_sync_all();

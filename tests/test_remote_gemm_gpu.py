@@ -339,3 +339,10 @@ def test_scratch_of_calls_without_a_flag(cuda_device, fmt, m, n, k):
     for i, y in enumerate(ys):
         ref = refs[i % 4]
         assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 7936, 3328), (256, 1280, 4096), (384, 512, 8192)])
+def test_block_scaled_fp8_shares_give_up(cuda_device, m, n, k):
+    """K shared by two, four and eight CTAs, one of whose warps finds that X never arrives: what it says has reached the
+    thread that tells the other CTAs, and none of them writes."""
+    test_a_wait_that_runs_out(cuda_device, "fp8_block", m, n, k)
