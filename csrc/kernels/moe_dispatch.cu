@@ -203,16 +203,19 @@ __device__ __forceinline__ void moe_send_counts(const eux_moe_desc& d, const Moe
 // this GPU, where the last CTA sees the counts; that one's fence for everyone stands between them and the flags and covers the
 // rows of all CTAs. (System-scope fences queue up at 31 ns each: with one per CTA a dispatch of 128 fp8 tokens of 7168 took
 // 12.4 us, 9.0 so, graph replays. With counts and flags both sent here, behind a release each, an exchange of 16 tokens of
-// 4096 took 20.4 us, 18.8 without.)
-__device__ __forceinline__ void moe_publish(const eux_moe_desc& d, uint64_t* const* flags) {
+// 4096 took 20.4 us, 18.8 without.) Nobody is told of an exchange of which a CTA gave up, as a transfer or a GEMM tells
+// nobody: the receivers' own waits run out. Such a CTA sets the top bit of the count before it adds itself.
+__device__ __forceinline__ void moe_publish(const eux_moe_desc& d, uint64_t* const* flags, bool ok = true) {
   __syncthreads();
   __shared__ int s_last;
   const int W = d.world, E = d.n_experts;
   if (threadIdx.x == 0) {
+    uint32_t* const done = reinterpret_cast<uint32_t*>(d.counters + W + E);
     fence_gpu();
-    const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(d.counters + W + E), 1u);
-    s_last = (old == gridDim.x - 1);
-    if (s_last) {
+    if (!ok) atomicOr(done, 0x80000000u);
+    const uint32_t old = atomicAdd(done, 1u);
+    s_last = ((old & 0x7fffffffu) == gridDim.x - 1);
+    if (s_last && !(old & 0x80000000u)) {
       fence_sys();
       for (int dst = 0; dst < W; ++dst) st_relaxed_sys(flags[dst] + d.rank, d.seq);
     }
@@ -409,6 +412,18 @@ __host__ __device__ __forceinline__ int moe_image_slots(int hidden) {  // 16, 12
   const int n = (int)(112 * 1024 / moe_row_bytes(hidden, 1)) / 4 * 4;
   return n > 16 ? 16 : n < kMoeMinSlots ? 0 : n;
 }
+// mbar_wait for waits that last microseconds: the clock is read after every failing try (one takes 4 us).
+__device__ __forceinline__ bool moe_wait(uint32_t bar, uint32_t parity, volatile int* abort, uint64_t timeout_ns) {
+  if (mbar_try(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+  for (uint32_t it = 0; it < 0x7fffffffu; ++it) {
+    if (mbar_try(bar, parity)) return true;
+    if (*abort) return false;
+    if (globaltimer_ns() - t0 > (timeout_ns ? timeout_ns : 2000000000ull)) break;
+  }
+  *abort = 1;
+  return false;
+}
 // 16 bf16 values (32 bytes) as e4m3 with the given 1 / scale
 __device__ __forceinline__ uint4 moe_quantize16(const uint32_t (&raw)[8], float inv) {
   uint32_t w[4];
@@ -501,7 +516,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_fp8_bulk_kernel(eux_
         q[h] = moe_quantize16(v[h], 1.0f / scale[h]);
       }
       if (u + kWorkers < units) load(u + kWorkers);
-      if (tl >= slots && __any_sync(0xffffffffu, !mbar_wait(empty_bar(tl - slots), phase(tl - slots), abort, 0))) break;
+      if (tl >= slots && __any_sync(0xffffffffu, !moe_wait(empty_bar(tl - slots), phase(tl - slots), abort, d.wait_timeout_ns))) break;
       unsigned char* const image = ring + (size_t)s * row_bytes;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -538,7 +553,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_fp8_bulk_kernel(eux_
         st_u4(metas[dst] + row, make_uint4((uint32_t)t, (uint32_t)lane | ((uint32_t)(expert - dst * EPR) << 16), __float_as_uint(w), (uint32_t)d.rank));
       }
       if (tl + kMoeSenders < t1 - t0) fetch(t + kMoeSenders);
-      if (__any_sync(0xffffffffu, !mbar_wait(full_bar(tl), phase(tl), abort, 0))) break;
+      if (__any_sync(0xffffffffu, !moe_wait(full_bar(tl), phase(tl), abort, d.wait_timeout_ns))) break;
       if (out) bulk_s2g(out, ring0 + (uint32_t)(s * row_bytes), (uint32_t)row_bytes);
       bulk_commit();
       bulk_wait_read_1();  // the copies of the image before this one have read their slot
@@ -549,8 +564,9 @@ __global__ void __launch_bounds__(kMoeThreads) moe_dispatch_fp8_bulk_kernel(eux_
     asm volatile("fence.proxy.async;" ::: "memory");
   }
   __syncthreads();
-  if (threadIdx.x == 0 && s_abort) set_status(d.status, EUX_ST_TIMEOUT, 13);
-  moe_publish(d, flags);
+  const bool ok = s_abort == 0;
+  if (threadIdx.x == 0 && !ok) set_status(d.status, EUX_ST_TIMEOUT, 13);
+  moe_publish(d, flags, ok);
 }
 
 // ---- expert side: wait for every source, (identity expert), tell the sources -

@@ -334,3 +334,43 @@ def test_combine_fetches_as_many_rows_as_there_are(cuda_device, topk, fp8, t, hi
 def test_bf16_dispatch_of_more_than_the_l2_holds(cuda_device, t, hidden, topk):
     """On both sides of the number of tokens and bytes from which a dispatch has several CTAs per SM."""
     test_dispatch_routes_in_one_launch(cuda_device, t, hidden, topk, 64, False)
+
+
+@pytest.mark.parametrize("t,hidden,topk,world", [(1200, 13056, 2, 1), (600, 7168, 8, 2)])
+def test_a_dispatch_that_gives_up_tells_nobody(cuda_device, t, hidden, topk, world):
+    """fp8 row images whose tokens come from pinned host memory, tens of microseconds each, and a limit of one: the dispatch
+    gives up, says so in its status word and sends no arrival flag, its counters are back at zero, and the next one on the
+    same buffers is right. One launch and two (more than 4096 routing entries)."""
+    import struct
+    from execution_ucx_b200.ops import _native, moe
+    ranks = moe.MoeAllToAll.emulated(world, t, hidden, topk, 8, fp8=True)
+    rk = ranks[0]
+    x = torch.randn(t, hidden, device=cuda_device).to(torch.bfloat16)
+    idx, w = _routing(t, topk, 8, cuda_device, t)
+    whole = rk._desc
+
+    def short():
+        desc = bytearray(whole())
+        struct.pack_into("<Q", desc, _native.MoeDesc.wait_timeout_ns.offset, 1000)
+        return bytes(desc)
+
+    rk._desc = short
+    rk.dispatch(x.cpu().pin_memory(), idx, w)
+    torch.cuda.synchronize()
+    assert int(rk.status) & 0xff == 1 and int(rk.status) >> 8 == 13
+    for dst in ranks:
+        assert int(dst.flags.view(torch.int64, world)[0]) == 0
+    assert int(rk.counters.abs().sum()) == 0
+    rk.status.zero_()
+    rk._desc = whole
+    for r in ranks:
+        r.seq = 1
+        r.dispatch(x, idx, w)
+    for r in ranks:
+        r.expert_ready()
+    outs = [r.combine().clone() for r in ranks]
+    torch.cuda.synchronize()
+    ref = moe.reference_dispatch_combine(x, idx, w, True)
+    for r, out in zip(ranks, outs):
+        r.check_status()
+        assert bool(((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
