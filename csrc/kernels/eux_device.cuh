@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "eux_kernels.h"
 
 namespace eux {
@@ -71,6 +73,18 @@ static inline int launch_early(void (*kernel)(Args...), int grid, int threads, s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr, cfg.numAttrs = 1;
   return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// The kernel's shared memory limit, raised before its first launch on a device to the most that any launch takes (threads
+// that race do it twice). Set to each launch's own size, a smaller launch of another thread could lower it in between.
+template <auto KERNEL>
+static cudaError_t allow_smem(int dev, size_t most) {
+  static std::atomic<bool> done[64];
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  if (e == cudaSuccess) done[dev].store(true, std::memory_order_release);
+  return e;
 }
 
 // Spin until *flag >= value. Gives up after timeout_ns (0 = 2 s default) or

@@ -29,6 +29,7 @@ namespace eux {
 
 constexpr int kMoeThreads = 512;
 constexpr int kMaxWorld = 16;
+constexpr int kMaxExperts = 4096;
 
 __host__ __device__ __forceinline__ size_t moe_row_bytes(int hidden, int fp8) {
   // fp8 rows: values, then one fp32 scale per 128 values, padded to whole 128-byte lines so that
@@ -408,8 +409,9 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
 constexpr int kMoeBars = 32;
 constexpr int kMoeSenders = 4;
 constexpr int kMoeMinSlots = 8;
+constexpr size_t kMoeImageBytes = 112 * 1024;
 __host__ __device__ __forceinline__ int moe_image_slots(int hidden) {  // 16, 12 or 8; 0: the rows are too wide
-  const int n = (int)(112 * 1024 / moe_row_bytes(hidden, 1)) / 4 * 4;
+  const int n = (int)(kMoeImageBytes / moe_row_bytes(hidden, 1)) / 4 * 4;
   return n > 16 ? 16 : n < kMoeMinSlots ? 0 : n;
 }
 // mbar_wait for waits that last microseconds: the clock is read after every failing try (one takes 4 us).
@@ -988,7 +990,7 @@ __global__ void __launch_bounds__(kMoeThreads) moe_combine_fp8_rows_kernel(eux_m
 static int moe_check(const eux_moe_desc* d) {
   if (!d || d->world < 1 || d->world > kMaxWorld || d->rank < 0 || d->rank >= d->world) return EUX_ERR_BAD_ARG;
   if (d->n_experts % d->world || d->hidden % 128 || d->hidden <= 0 || d->topk < 1 || d->topk > 32) return EUX_ERR_BAD_ARG;
-  if (d->n_experts > 4096 || d->capacity < 1 || d->n_tokens < 0) return EUX_ERR_BAD_ARG;
+  if (d->n_experts > kMaxExperts || d->capacity < 1 || d->n_tokens < 0) return EUX_ERR_BAD_ARG;
   return 0;
 }
 
@@ -998,19 +1000,21 @@ using namespace eux;
 
 extern "C" size_t eux_moe_row_bytes(int hidden, int fp8) { return moe_row_bytes(hidden, fp8); }
 
-static int moe_sms() {
+static int moe_sms(int* dev_out = nullptr) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (dev_out) *dev_out = dev;
   return sms;
 }
 
-// The count launch, where there are too many entries for every CTA to count them all, and the dispatch.
+// The count launch, where there are too many entries for every CTA to count them all, and the dispatch, with the routing
+// tables and `extra` bytes of shared memory, at most `most_extra` in any launch of this kernel.
 template <auto KERNEL, typename... More>
-static int moe_dispatch(const eux_moe_desc* d, int ctas, int sms, size_t smem, cudaStream_t st, More... more) {
+static int moe_dispatch(const eux_moe_desc* d, int ctas, int dev, int sms, size_t extra, size_t most_extra, cudaStream_t st, More... more) {
   const int grid = std::max(1, std::min(ctas, d->n_tokens));
-  if (smem > 40 * 1024)  // with the kernel's static arrays near the 48 KiB that need no leave
-    if (cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); e != cudaSuccess) return (int)e;
+  const size_t smem = 3 * (size_t)d->n_experts * sizeof(int) + extra;
+  if (cudaError_t e = allow_smem<KERNEL>(dev, 3 * (size_t)kMaxExperts * sizeof(int) + most_extra); e != cudaSuccess) return (int)e;
   const int64_t entries = (int64_t)d->n_tokens * d->topk;
   const int counted = entries > kRouteSelf;
   if (counted) {
@@ -1023,9 +1027,9 @@ static int moe_dispatch(const eux_moe_desc* d, int ctas, int sms, size_t smem, c
 
 extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* stream) {
   if (int rc = moe_check(d)) return rc;
-  const size_t routing = 3 * (size_t)d->n_experts * sizeof(int);
   const cudaStream_t st = (cudaStream_t)stream;
-  const int sms = moe_sms();
+  int dev = 0;
+  const int sms = moe_sms(&dev);
   // A CTA per token, up to one per SM: a second one counts all entries again (256 tokens, fp8: 28.2 us for the exchange
   // with one, 30.2 with two).
   const int one = ctas > 0 ? ctas : sms;
@@ -1034,14 +1038,15 @@ extern "C" int eux_moe_dispatch_launch(const eux_moe_desc* d, int ctas, void* st
     // ends late (top-8 of 7168, the exchange with one and with six per SM: 2048 tokens, 235 MB, 104.5 and 104.3 us; 2560
     // 128.7 and 126.6; 4096 197.8 and 192.0; 8192 376.1 and 360.6).
     const bool large = (int64_t)d->n_tokens * d->topk * d->hidden * 2 >= (int64_t(256) << 20) && d->n_tokens >= 12 * sms;
-    return moe_dispatch<moe_dispatch_bf16_kernel>(d, ctas > 0 ? ctas : large ? 6 * sms : sms, sms, routing, st);
+    return moe_dispatch<moe_dispatch_bf16_kernel>(d, ctas > 0 ? ctas : large ? 6 * sms : sms, dev, sms, 0, 0, st);
   }
   if (const int slots = moe_image_slots(d->hidden); slots > 0 && d->n_tokens >= 2 * (int64_t)one)
-    return moe_dispatch<moe_dispatch_fp8_bulk_kernel>(d, one, sms, routing + 128 + (size_t)slots * moe_row_bytes(d->hidden, 1), st, slots);
+    return moe_dispatch<moe_dispatch_fp8_bulk_kernel>(d, one, dev, sms, 128 + (size_t)slots * moe_row_bytes(d->hidden, 1), 128 + kMoeImageBytes, st, slots);
   // Rows too wide for images and more than eight tokens per CTA: two per SM, one of which works while the other waits at its
   // barriers.
   if (ctas <= 0) ctas = d->n_tokens > 8 * sms ? 2 * sms : sms;
-  return moe_dispatch<moe_dispatch_fp8_kernel>(d, ctas, sms, routing + 2 * (size_t)moe_scale_stride(d->hidden) * sizeof(float), st);
+  return moe_dispatch<moe_dispatch_fp8_kernel>(d, ctas, dev, sms, 2 * (size_t)moe_scale_stride(d->hidden) * sizeof(float),
+                                               2 * (size_t)kMoeScaleFloats * sizeof(float), st);
 }
 
 extern "C" int eux_moe_expert_ready_launch(const eux_moe_desc* d, void* stream) {

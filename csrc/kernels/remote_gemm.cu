@@ -2096,16 +2096,6 @@ static int make_map_sf(CUtensorMap* m, const void* base, uint64_t chunks, uint32
   return r == CUDA_SUCCESS ? 0 : EUX_ERR_BAD_ARG;
 }
 
-// The kernel's shared memory limit, raised before its first launch on a device (threads that race do it twice).
-template <auto KERNEL>
-static cudaError_t allow_smem(int dev, size_t smem) {
-  static std::atomic<bool> done[64];
-  if (done[dev].load(std::memory_order_acquire)) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) done[dev].store(true, std::memory_order_release);
-  return e;
-}
-
 struct ClusterLaunch {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];

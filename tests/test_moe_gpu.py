@@ -374,3 +374,40 @@ def test_a_dispatch_that_gives_up_tells_nobody(cuda_device, t, hidden, topk, wor
     for r, out in zip(ranks, outs):
         r.check_status()
         assert bool(((out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
+
+
+def test_dispatches_of_several_threads(cuda_device):
+    """Threads that launch dispatches as fast as they can, each on its own stream and buffers, with more shared memory or
+    less: none is refused because another thread's launch takes less, and every row is where it belongs."""
+    import threading
+    from execution_ucx_b200.ops import _native, moe
+    t, launch = 4, _native.load().eux_moe_dispatch_launch
+    start, refused, work = threading.Barrier(4), [], []
+    for hidden, ne in [(12928, 4096), (7168, 8), (12928, 4096), (11008, 8)]:
+        (rk,) = moe.MoeAllToAll.emulated(1, t, hidden, 2, ne, fp8=True)
+        work.append((rk, torch.randn(t, hidden, device=cuda_device).to(torch.bfloat16), *_routing(t, 2, ne, cuda_device, hidden)))
+
+    def loop(rk, x, idx, w):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            rk.dispatch(x, idx, w, ctas=1)
+            desc = rk._desc()
+            for _ in range(60):
+                start.wait()
+                refused.extend(rc for rc in [launch(desc, 1, stream.cuda_stream) for _ in range(100)] if rc)
+                stream.synchronize()
+            rk.expert_ready()
+            rk.combine()
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=loop, args=a) for a in work]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert not refused, (len(refused), refused[0])
+    for rk, x, idx, w in work:
+        rk.check_status()
+        ref = moe.reference_dispatch_combine(x, idx, w, True)
+        assert bool(((rk.out.float() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
