@@ -56,8 +56,11 @@ __device__ __forceinline__ void red_release_gpu_add(uint32_t* p, uint32_t v) {
 }
 
 // Programmatic dependent launch, which takes the 2 to 2.5 us between the end of one kernel of a stream and the first load of
-// the next away: what follows may be launched while this kernel runs (a kernel that waits for another GPU or stream does not
-// call this: what it lets in would hold SMs for as long) ...
+// the next away: what follows may be launched once every CTA has called this (a kernel that waits for another GPU or stream
+// does not: what it lets in would hold SMs for as long). What is let in sits on the SMs until this kernel ends, where kernels
+// of other streams find no room, so a CTA calls it when it has no more work to begin: the launch is through before the last
+// tile is (called at the start, 8192^3 let a transfer of its stream hold up those of others for 0.7 ms, and calls in a loop
+// were no faster: 128 x 8192 x 8192 bf16 30.2 and 30.3 us, 640 x 4096 x 1024 11.7 and 11.6) ...
 __device__ __forceinline__ void allow_next_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // ... and a kernel launched so waits here until everything before it in the stream is complete and visible, before it touches
 // memory. (Nothing to wait for in a plain launch.)

@@ -607,7 +607,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
-  allow_next_launch();
   if ((int)blockIdx.x < p.copy_ctas) {
     wait_for_launch_before();
     // first the transfer of X, then this CTA computes tiles like the others
@@ -708,6 +707,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
       if (k < k_iters) break;
     }
+    allow_next_launch();
     if (lane == 0) {
       if (*abort) {  // let copies that are still in flight land before the CTA retires
         const uint64_t t0 = globaltimer_ns();
@@ -863,7 +863,6 @@ __global__ void __launch_bounds__(GEMM8_THREADS, 1)
 remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                        const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
-  allow_next_launch();
   if ((int)blockIdx.x < p.copy_ctas) {
     wait_for_launch_before();
     // first the transfer of X and its scales, then this CTA computes tiles like the others
@@ -961,6 +960,7 @@ remote_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
       if (k < k_blocks) break;
     }
+    allow_next_launch();
     if (lane == 0) {
       if (*abort) {
         const uint64_t t0 = globaltimer_ns();
@@ -1237,7 +1237,6 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
   constexpr int NBUF = PairCfg<MX>::NBUF;
   extern __shared__ unsigned char smem_raw[];
   bool copy_ok = true;
-  allow_next_launch();
   if ((int)blockIdx.x < p.copy_ctas) {
     wait_for_launch_before();
     // whole pairs copy X first (copy_ctas is even). A CTA whose copy failed still walks through the
@@ -1360,6 +1359,7 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
       }
       if (k < k_iters) break;
     }
+    allow_next_launch();
     if (*abort && lane == 0) {  // let copies that are still in flight land before the CTA retires
       const uint64_t t0 = globaltimer_ns();
       while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -1556,7 +1556,6 @@ constexpr int FEW_TMEM_COLS = BM;
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_few_tiles_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
-  allow_next_launch();
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sW = smem;
   unsigned char* sX = smem + (size_t)FEW_STAGES * A_STAGE_BYTES;
@@ -1635,6 +1634,7 @@ remote_gemm_few_tiles_kernel(const __grid_constant__ CUtensorMap map_x, const __
           if (++s == FEW_STAGES) s = 0, ph ^= 1u;
         }
       }
+      allow_next_launch();
       if (*abort && lane == 0) {  // let copies that are still in flight land before shared memory is used for the sum
         const uint64_t t0 = globaltimer_ns();
         while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -1782,7 +1782,6 @@ __global__ void __launch_bounds__(GEMM8P_THREADS, 1)
 remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                             const __grid_constant__ CUtensorMap map_y, GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
-  allow_next_launch();
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA = smem;
   unsigned char* sB = smem + (size_t)STAGES8P * A_STAGE_BYTES;
@@ -1914,6 +1913,7 @@ remote_gemm_fp8_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       }
       if (k < k_blocks) break;
     }
+    allow_next_launch();
     if (*abort && lane == 0) {  // loads in flight still write shared memory: give them time to land
       const uint64_t t0 = globaltimer_ns();
       while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -2104,8 +2104,8 @@ struct ClusterLaunch {
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    // A GEMM may be launched while the kernel before it in the stream still runs: a CTA sets up its barriers and TMEM on an
-    // SM that has become free and waits there (128 x 8192 x 8192 bf16 32.8 us per call without and 30.4 with, fp8 20.5 and 18.6).
+    // A GEMM may be launched while the kernel before it in the stream ends: a CTA sets up its barriers and TMEM on an SM that
+    // has become free and waits there.
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;

@@ -346,3 +346,33 @@ def test_block_scaled_fp8_shares_give_up(cuda_device, m, n, k):
     """K shared by two, four and eight CTAs, one of whose warps finds that X never arrives: what it says has reached the
     thread that tells the other CTAs, and none of them writes."""
     test_a_wait_that_runs_out(cuda_device, "fp8_block", m, n, k)
+
+
+def test_what_follows_a_gemm_leaves_room_for_other_streams(cuda_device):
+    """A long GEMM with a large push behind it in its stream, and a small push in another stream: the large one, whose turn
+    has not come, does not take the room beside the GEMM that the small one needs."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    from execution_ucx_b200.ops.remote_gemm import RemoteGemm
+    n = 8192
+    x = torch.randn(n, n, device=cuda_device).to(torch.bfloat16)
+    g, y = RemoteGemm(x, n), torch.empty_like(x)
+    big, small = torch.zeros(1 << 26, device=cuda_device), torch.zeros(1 << 20, device=cuda_device)
+    big_to, small_to = (torch.empty_like(t, dtype=torch.bfloat16) for t in (big, small))
+    one, other = torch.cuda.Stream(), torch.cuda.Stream()
+    start, end, small_end = (torch.cuda.Event(enable_timing=True) for _ in range(3))
+    for follow in (True, False, True):  # the first time round sets up what a stream keeps
+        torch.cuda.synchronize()
+        with torch.cuda.stream(one):
+            start.record()
+            g(x.data_ptr(), n, y.data_ptr(), x_is_local=True)
+            if follow:
+                tx.push(big, big_to)
+            else:
+                end.record()
+        with torch.cuda.stream(other):
+            tx.push(small, small_to)
+            small_end.record()
+        torch.cuda.synchronize()
+        if not follow:
+            alone = start.elapsed_time(end)
+    assert start.elapsed_time(small_end) < 0.5 * alone
