@@ -59,12 +59,6 @@ struct PackT<16> {
   using type = uint4;
 };
 
-// The first thing a transfer kernel does.
-__device__ __forceinline__ void xfer_begin(const eux_xfer_desc& d) {
-  if (d.wait_flag == nullptr) allow_next_launch();
-  wait_for_launch_before();
-}
-
 // Wait (bounded) for the arrival flag; every thread of the CTA learns the outcome.
 __device__ __forceinline__ bool cta_wait_arrival(const eux_xfer_desc& d) {
   if (d.wait_flag == nullptr) return true;
@@ -104,6 +98,22 @@ __device__ __forceinline__ void cta_publish(const eux_xfer_desc& d, uint32_t* co
   if (last) fence_sys();  // what all CTAs wrote, the others before they counted themselves, comes before the flags
   if (last && ok && d.flag) st_relaxed_sys(d.flag, d.flag_value);
   if (last && ok && d.flag2) st_relaxed_sys(d.flag2, d.flag2_value);
+}
+
+// The first and the last thing a transfer kernel does. What follows in the stream may be launched when a CTA has issued its
+// last stores, and from the start where the whole takes a few microseconds (a source of up to 32 MiB). It sits on the SMs
+// until the transfer ends: let in at the start, a GEMM behind a push of 1 GiB held up a small GEMM of another stream for as long as
+// the push and itself took, 0.98 ms instead of 0.34, and large transfers in a loop were no faster for it (4096 x 7168 fp32 to
+// e4m3 23.8 us and 23.3 from the end on, 8192 x 8192 bf16 transposed 45.4 and 45.0). A push of 640 x 1024 with a
+// GEMM of 640 x 4096 x 1024 behind it takes 11.8 us with the GEMM let in at the start and 12.9 at the end, pushes of 16 MiB
+// 4.48 and 4.62 (graph replays).
+__device__ __forceinline__ void xfer_begin(const eux_xfer_desc& d) {
+  if (d.wait_flag == nullptr && d.n_elems * (uint64_t)dtype_size(d.src_dtype) <= (32u << 20)) allow_next_launch();
+  wait_for_launch_before();
+}
+__device__ __forceinline__ void xfer_end(const eux_xfer_desc& d, uint32_t* counter, bool ok) {
+  if (d.wait_flag == nullptr) allow_next_launch();
+  cta_publish(d, counter, ok);
 }
 
 // Dense byte copy. A CTA works on one contiguous block at a time and the blocks are dealt
@@ -173,7 +183,7 @@ __global__ void __launch_bounds__(kXferThreads) xfer_bytes_kernel(XferArgs a) {
     copy_bytes_grid<V32>(reinterpret_cast<const unsigned char*>(d.src), reinterpret_cast<unsigned char*>(d.dst), nbytes,
                          blockIdx.x, gridDim.x);
   }
-  cta_publish(d, a.counter, ok);
+  xfer_end(d, a.counter, ok);
 }
 
 // Dense byte copy on the bulk-copy engine: two threads per CTA drive a ring of shared-memory
@@ -312,7 +322,7 @@ __global__ void __launch_bounds__(kXferThreads, sizeof(S) == 4 ? 2 : 4) xfer_typ
   xfer_begin(d);
   bool ok = cta_wait_arrival(d);
   if (ok) typed_body<S, D>(d);
-  cta_publish(d, a.counter, ok);
+  xfer_end(d, a.counter, ok);
 }
 
 // One tensor-RPC echo step of a rank in a single launch: push the request into the partner's arena and
@@ -510,7 +520,7 @@ __global__ void __launch_bounds__(kXferThreads) xfer_gather_kernel(const __grid_
       dst[e] = Convert<S, D, RAW>::one(src[row + (int64_t)c * inner], op, arg);
     }
   }
-  cta_publish(d, a.x.counter, ok);
+  xfer_end(d, a.x.counter, ok);
 }
 
 // Small tensors (a step for every thread of the device, or less), and single bytes in rows of less than a chunk: one
@@ -548,7 +558,7 @@ __global__ void __launch_bounds__(kXferThreads) xfer_element_kernel(const __grid
       }
     }
   }
-  cta_publish(d, a.x.counter, ok);
+  xfer_end(d, a.x.counter, ok);
 }
 
 // Transposes. A tile is `tp` steps of the dimension with stride 1 in the source (P) times `tq` of the innermost
@@ -756,7 +766,7 @@ __global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_co
       __syncthreads();
     }
   }
-  cta_publish(d, t.x.counter, ok);
+  xfer_end(d, t.x.counter, ok);
 }
 
 // Transposes of a dense matrix with few columns (P below 64, rows of the source next to one another): the source of a
@@ -826,7 +836,7 @@ __global__ void __launch_bounds__(kTileThreads) xfer_narrow_kernel(const __grid_
       __syncthreads();
     }
   }
-  cta_publish(d, t.x.counter, ok);
+  xfer_end(d, t.x.counter, ok);
 }
 
 // One CTA per descriptor; meant for many small messages per launch.
@@ -976,8 +986,8 @@ static int num_sms() {
   return sms[dev];
 }
 
-// Transfers are launched while the kernel before them runs (calls in a loop: 4096 x 7168 fp32 to e4m3 24.9 -> 23.6 us,
-// 4096 x 4096 bf16 to e4m3 8.2 -> 6.8, a push and a GEMM by turns 20.4 -> 15.8). One that waits for an arrival is launched when
+// Transfers are launched while the kernel before them ends (calls in a loop, without that and with it: 4096 x 7168 fp32 to
+// e4m3 24.9 and 23.4 us, 4096 x 4096 bf16 to e4m3 8.2 and 7.0). One that waits for an arrival is launched when
 // its turn has come: until then it would hold its SMs for nothing.
 template <typename A>
 static void launch_xfer(void (*kernel)(A), int grid, int threads, cudaStream_t st, const A& a, const eux_xfer_desc& d) {

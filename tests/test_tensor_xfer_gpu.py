@@ -397,3 +397,34 @@ def test_pushes_behind_one_another(cuda_device, rows, cols):
         run()
         torch.cuda.synchronize()
         assert torch.equal(g, want)
+
+
+def test_what_follows_a_push_leaves_room_for_other_streams(cuda_device):
+    """A large push with a large GEMM behind it in its stream, and a small GEMM in another stream: the large one, whose turn
+    has not come, does not take the shared memory that the small one needs."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    from execution_ucx_b200.ops.remote_gemm import RemoteGemm
+    n = 8192
+    x = torch.randn(n, n, device=cuda_device).to(torch.bfloat16)
+    g, y = RemoteGemm(x, n), torch.empty_like(x)
+    small, out = RemoteGemm(x[:512, :512].contiguous(), 128), torch.empty(128, 512, dtype=torch.bfloat16, device=cuda_device)
+    src = torch.zeros(1 << 30, dtype=torch.uint8, device=cuda_device)
+    dst = torch.empty_like(src)
+    one, other = torch.cuda.Stream(), torch.cuda.Stream()
+    start, pushed, end, small_end = (torch.cuda.Event(enable_timing=True) for _ in range(4))
+    for apart in (True, True, False):  # the first time round sets up what a stream keeps
+        torch.cuda.synchronize()
+        with torch.cuda.stream(one):
+            start.record()
+            tx.push(src, dst)
+            if apart:
+                pushed.record()
+            g(x.data_ptr(), n, y.data_ptr(), x_is_local=True)
+            end.record()
+        with torch.cuda.stream(other):
+            small(x.data_ptr(), 128, out.data_ptr(), x_is_local=True)
+            small_end.record()
+        torch.cuda.synchronize()
+        if apart:
+            push, gemm = start.elapsed_time(pushed), pushed.elapsed_time(end)
+    assert start.elapsed_time(small_end) < push + 0.5 * gemm
