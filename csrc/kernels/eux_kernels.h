@@ -203,7 +203,8 @@ typedef struct eux_gemm_desc {
   int32_t copy_ctas;     /* CTAs that stream X from the peer; 0 when x_stage == x_src */
   int32_t flags;         /* EUX_GEMM_FLAG_* */
 } eux_gemm_desc;
-/* bf16: tiles of 256 x 256 computed by pairs of CTAs (cta_group::2) where there are enough of them */
+/* bf16: tiles computed by pairs of CTAs (cta_group::2): of 256 x 256 where there are enough of them, of 128 x 256 with up
+   to one pair of SMs for each. Without the flag a tile is one CTA's, or shared over K by a cluster of single CTAs. */
 #define EUX_GEMM_FLAG_CTA_PAIRS 1
 /* With a remote X: two spare warps of every CTA copy X (and its scales) beside the GEMM's warps, instead of
    copy_ctas CTAs that copy first and compute afterwards. */

@@ -603,6 +603,7 @@ __device__ __forceinline__ void split_sum(const GemmParams& p, uint32_t tmem_bas
   split_write(p, parts, p.y + ((size_t)mb * BM * p.N + (size_t)nb * BN) * 2, warp, lane);
 }
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_y, GemmParams p) {
@@ -664,7 +665,11 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   const int m_blocks = p.M / BM, n_blocks = p.N / BN;
   const int total = m_blocks * n_blocks;
-  const int k_iters = p.K * p.elem_bytes / BKB;
+  const int k_all = p.K * p.elem_bytes / BKB;
+  const int rank = SPLIT ? (int)cluster_cta_rank() : 0;
+  const int tile0 = SPLIT ? (int)blockIdx.x / p.split : 0;  // past the last tile: this cluster only helps to copy X
+  const int k_begin = SPLIT ? k_all * rank / p.split : 0;   // this CTA's share of K
+  const int k_iters = (SPLIT ? k_all * (rank + 1) / p.split : k_all) - k_begin;
   const int kelems = BKB / p.elem_bytes;  // elements of K per stage
   volatile int* abort = &s_abort;
   // the next tile as the consumer roles see it: bounded wait on the ring slot, then its content
@@ -686,9 +691,9 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     int s = 0;
     uint32_t ph = 0;
     for (int it = 0;; ++it) {
-      int tile = total;
+      int tile = it == 0 ? tile0 : total;  // SPLIT: one tile per cluster
       if (lane == 0) {
-        tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
+        if (!SPLIT) tile = *abort ? total : (int)atomicAdd(p.sched + 2, 1u);
         s_tiles[it & (TILE_RING - 1)] = tile;
         mbar_arrive(tile_bar(it & (TILE_RING - 1)));
       }
@@ -701,8 +706,8 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (; k < k_iters; ++k) {
         if (!mbar_wait_warp(empty_bar(s), ph ^ 1u, abort, p.timeout_ns)) break;
         mbar_expect_tx(issue, full_bar(s), A_STAGE_BYTES + B_STAGE_BYTES);
-        tma_load_2d(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_bar(s), k * kelems, mb * BM);
-        tma_load_2d(issue, b0 + (uint32_t)s * B_STAGE_BYTES, &map_b, full_bar(s), k * kelems, nb * BN);
+        tma_load_2d(issue, a0 + (uint32_t)s * A_STAGE_BYTES, &map_a, full_bar(s), (k_begin + k) * kelems, mb * BM);
+        tma_load_2d(issue, b0 + (uint32_t)s * B_STAGE_BYTES, &map_b, full_bar(s), (k_begin + k) * kelems, nb * BN);
         if (++s == STAGES) s = 0, ph ^= 1u;
       }
       if (k < k_iters) break;
@@ -762,6 +767,7 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const uint32_t tph = (uint32_t)(it >> 1) & 1u;
       const bool got = mbar_wait(tfull_bar(buf), tph, abort, p.timeout_ns);
       if (epi_vote_any(1, !got)) break;  // all four warps or none: the slab barriers below need everyone
+      if (SPLIT) break;                  // summed over the cluster below
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)buf * BN;
 #pragma unroll 1
@@ -806,6 +812,14 @@ remote_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   tc_fence_before();
   __syncthreads();
+  if (SPLIT && tile0 < total) {
+    tc_fence_after();
+    int mb, nb;
+    tile_coords(tile0, m_blocks, n_blocks, p.head_blocks, mb, nb);
+    split_sum(p, tmem_base, smem_u32(smem), mb, nb, rank, 0, 1, &s_abort);
+    tc_fence_before();
+    __syncthreads();
+  }
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS)
@@ -2213,8 +2227,8 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   const int waves = (tiles + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
   // Few tiles: the K of a tile is shared out over a cluster of CTAs (or CTA pairs), which add their sums up through
   // distributed shared memory. All clusters have to fit at once: a second wave costs more.
-  // bf16: wherever there is a pair of SMs for each 128 x 256 tile, and several pairs per tile from eight K steps on, four or
-  // more for each. Against single CTAs that shared K from 24 steps on, eight or more for each (calls in a loop):
+  // bf16 on CTA pairs: wherever there is a pair of SMs for each 128 x 256 tile, and several pairs per tile from eight K steps
+  // on, four or more for each. Against single CTAs, which share K from 24 steps on, eight or more for each (calls in a loop):
   // 128 x 8192 x 8192 30.1 -> 27.8 us, 128 x 512 x 8192 12.8 -> 11.2, 256 x 8192 x 8192 40.5 -> 37.5, 128 x 8192 x 1024
   // 10.1 -> 8.1 (8.7 without sharing K), 128 x 512 x 512 7.3 -> 6.5, 1152 x 2048 x 1024 (72 tiles) 10.3 -> 9.1.
   // 256 x 256 tiles whose K is shared: 256 x 8192 x 2048 13.7 against 11.7 us, 256 x 8192 x 8192 35.2 against 35.5.
@@ -2236,7 +2250,7 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
         return launch_clusters<remote_gemm_2cta_kernel<true, true>>(dev, 2 * s, 2 * clusters * s, GEMM_THREADS, PairCfg<true>::SMEM, st, ma, mb2,
                                my, msa, msb, p);
       }
-    } else if (!d->fp8) {
+    } else if (!d->fp8 && (d->flags & EUX_GEMM_FLAG_CTA_PAIRS)) {
       clusters = sms / 2;
       const int s = choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, tiles, 2, k_iters, 8, 4, &clusters);
       if (tiles <= clusters) {
@@ -2250,13 +2264,15 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
         return launch_clusters<remote_gemm_few_tiles_kernel>(dev, 2 * s, 2 * clusters * s, GEMM_THREADS, FEW_SMEM, st, mx2, mb2, p);
       }
     } else {
-      const int s = choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters, 24, 8, &clusters);
+      const int s = d->fp8 ? choose_split<remote_gemm_fp8_kernel<true>>(dev, GEMM8_THREADS, GEMM8_SMEM, tiles, 1, k_iters, 24, 8, &clusters)
+                           : choose_split<remote_gemm_kernel<true>>(dev, GEMM_THREADS, GEMM_SMEM, tiles, 1, k_iters, 24, 8, &clusters);
       if (s > 1) {
         if (!pull) clusters = tiles;
         p.split = s, p.copy_ctas = 0;
         p.copy_warps = pull ? 2 * clusters * s : 0;
         p.panel_target = pull ? warp_target(p.copy_warps) : 0;
-        return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, clusters * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
+        if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<true>>(dev, s, clusters * s, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
+        return launch_clusters<remote_gemm_kernel<true>>(dev, s, clusters * s, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
       }
     }
   }
@@ -2306,7 +2322,7 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
     p.panel_target = warp_target(p.copy_warps);
   }
   if (d->fp8) return launch_clusters<remote_gemm_fp8_kernel<false>>(dev, 1, grid, GEMM8_THREADS, GEMM8_SMEM, st, ma, mb, my, p);
-  return launch_clusters<remote_gemm_kernel>(dev, 1, grid, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
+  return launch_clusters<remote_gemm_kernel<false>>(dev, 1, grid, GEMM_THREADS, GEMM_SMEM, st, ma, mb, my, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -2321,12 +2337,12 @@ static __device__ __align__(256) uint32_t g_noalloc_gemm_scratch[EUX_NOALLOC_GEM
 
 // Everything that a first launch of one of the bf16 kernels would set up: which of them a call takes depends on its shape.
 static int prepare_bf16(int dev) {
-  const void* kernels[] = {(const void*)remote_gemm_kernel, (const void*)remote_gemm_few_tiles_kernel,
+  const void* kernels[] = {(const void*)remote_gemm_kernel<false>, (const void*)remote_gemm_few_tiles_kernel,
                            (const void*)remote_gemm_2cta_kernel<false, false>};
   cudaFuncAttributes attr;
   for (const void* k : kernels)
     if (cudaError_t e = cudaFuncGetAttributes(&attr, k); e != cudaSuccess) return (int)e;
-  cudaError_t e = allow_smem<remote_gemm_kernel>(dev, GEMM_SMEM);
+  cudaError_t e = allow_smem<remote_gemm_kernel<false>>(dev, GEMM_SMEM);
   if (e == cudaSuccess) e = allow_smem<remote_gemm_2cta_kernel<false, false>>(dev, PairCfg<false>::SMEM);
   int clusters = 0;  // one tile and a long K: every size of cluster is asked about
   if (e == cudaSuccess) e = allow_smem<remote_gemm_few_tiles_kernel>(dev, FEW_SMEM);
@@ -2383,7 +2399,8 @@ extern "C" int eux_gemm_bf16_noalloc(const void* x, const void* w_t, void* y, in
 // that loads): a service that launches on behalf of a peer calls this when it is set up.
 extern "C" int eux_gemm_preload(void) {
   cudaFuncAttributes attr;
-  const void* kernels[] = {(const void*)remote_gemm_kernel,                  (const void*)remote_gemm_few_tiles_kernel,
+  const void* kernels[] = {(const void*)remote_gemm_kernel<false>,           (const void*)remote_gemm_kernel<true>,
+                           (const void*)remote_gemm_few_tiles_kernel,
                            (const void*)remote_gemm_fp8_kernel<false>,       (const void*)remote_gemm_fp8_kernel<true>,
                            (const void*)remote_gemm_2cta_kernel<false, false>, (const void*)remote_gemm_2cta_kernel<true, false>,
                            (const void*)remote_gemm_2cta_kernel<true, true>, (const void*)remote_gemm_fp8_2cta_kernel};

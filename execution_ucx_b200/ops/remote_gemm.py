@@ -51,13 +51,14 @@ class RemoteGemm:
                  cta_pairs: bool = True, head_blocks: Optional[int] = None,
                  copy_warps: Optional[bool] = None) -> None:
         """Y[m,N] (at ``y_ptr``) = X[m,K] (at ``x_ptr``) @ W. Both addresses may be peer memory.
-        ``cta_pairs`` selects the kernel that computes 256 x 256 tiles on pairs of CTAs
-        (tcgen05 cta_group::2); shapes that half a tile of padding would cost a wave, and
-        ``cta_pairs=False``, run the kernel with one CTA per 128 x 256 tile. With few tiles a cluster
-        of CTAs shares the K of each. Its sums are added up in an order that is fixed for a shape, so a
-        call repeats itself bit by bit, but the low bits of a row can differ between calls with other
-        numbers of rows, whose tiles are shared by more CTAs or fewer. ``head_blocks``
-        overrides the height (in row blocks) of the first group of tiles when X is remote.
+        ``cta_pairs`` has tiles computed by pairs of CTAs (tcgen05 cta_group::2), of 128 x 256 where
+        there are at most as many as pairs of SMs and of 256 x 256 otherwise; shapes that half a tile
+        of padding would cost a wave, and ``cta_pairs=False``, run the kernel with one CTA per
+        128 x 256 tile. With few tiles a cluster of pairs, or of CTAs, shares the K of each. Its sums
+        are added up in an order that is fixed for a shape, so a call repeats itself bit by bit, but
+        the low bits of a row can differ between calls with other numbers of rows, whose tiles are
+        shared by more CTAs or fewer, and with and without pairs. ``head_blocks`` overrides the height
+        (in row blocks) of the first group of tiles when X is remote.
         A remote X is copied into the staging buffer by two spare warps of every CTA while the
         other warps compute (``copy_warps``, the default), or, when ``copy_ctas`` > 0 is given, by
         that many CTAs that copy first and compute afterwards."""
@@ -230,22 +231,24 @@ class RemoteGemmMx:
 
 
 def smoke(device) -> None:
-    """The pair kernel (bf16) with X pulled by the copy warps, the one-CTA kernel, and the MXFP8 kernel, on tiny shapes."""
-    x = torch.randn(256, 256, device=device).to(torch.bfloat16)
-    w = (torch.randn(256, 512, device=device) * 0.05).to(torch.bfloat16)
-    g = RemoteGemm(w, 256)
-    y = torch.empty(256, 512, dtype=torch.bfloat16, device=device)
-    for kw in (dict(x_is_local=True), dict(x_is_local=False), dict(x_is_local=True, cta_pairs=False)):
-        y.zero_()
-        g(x.data_ptr(), 256, y.data_ptr(), **kw)
+    """Every bf16 kernel on a tiny shape (pairs of CTAs with few tiles, X pulled by the copy warps; pairs with many; one CTA
+    per tile), and the MXFP8 kernel."""
+    y = torch.empty(2560 * 1024, dtype=torch.bfloat16, device=device)
+    for m, n, k, kw in ((256, 512, 256, dict(x_is_local=False)), (2560, 1024, 64, dict(x_is_local=True)),
+                        (256, 512, 256, dict(x_is_local=True, cta_pairs=False))):
+        x = torch.randn(m, k, device=device).to(torch.bfloat16)
+        w = (torch.randn(k, n, device=device) * 0.05).to(torch.bfloat16)
+        g = RemoteGemm(w, m)
+        out = y[:m * n].view(m, n).zero_()
+        g(x.data_ptr(), m, out.data_ptr(), **kw)
         torch.cuda.synchronize()
         g.check_status()
-        torch.testing.assert_close(y.float(), x.float() @ w.float(), rtol=2e-2, atol=2e-2)
+        torch.testing.assert_close(out.float(), x.float() @ w.float(), rtol=2e-2, atol=2e-2)
     gx = RemoteGemmMx(w.float(), 256)
     xq, xsf = quantize_mx(x.float())
     chunks = mx_scale_chunks(xsf, False)
-    y.zero_()
-    gx(xq.data_ptr(), chunks.data_ptr(), 256, y.data_ptr(), x_is_local=True)
+    out.zero_()
+    gx(xq.data_ptr(), chunks.data_ptr(), 256, out.data_ptr(), x_is_local=True)
     torch.cuda.synchronize()
     gx.check_status()
-    torch.testing.assert_close(y.float(), mx_dequantized_reference(xq, xsf, gx.w_q_t, gx.w_sf), rtol=2e-2, atol=2e-2)
+    torch.testing.assert_close(out.float(), mx_dequantized_reference(xq, xsf, gx.w_q_t, gx.w_sf), rtol=2e-2, atol=2e-2)

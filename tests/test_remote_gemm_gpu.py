@@ -376,3 +376,47 @@ def test_what_follows_a_gemm_leaves_room_for_other_streams(cuda_device):
         if not follow:
             alone = start.elapsed_time(end)
     assert start.elapsed_time(small_end) < 0.5 * alone
+
+
+@pytest.mark.parametrize("pull", [False, True])
+@pytest.mark.parametrize("cta_pairs", [False, True])
+def test_cta_pairs_is_what_the_caller_says(cuda_device, cta_pairs, pull):
+    """With few tiles too. The order of the sums tells: 2^24 + 1 + 1 - 2^24, each in an eighth of K, is 0 where eight CTAs have
+    an eighth each, and 1 where four pairs have a quarter (2^24 + 1 rounds to 2^24, 1 - 2^24 is exact)."""
+    from execution_ucx_b200.ops.remote_gemm import RemoteGemm
+    m, n, k = 128, 512, 8192
+    x, w = torch.zeros(m, k, device=cuda_device), torch.zeros(k, n, device=cuda_device)
+    for part, value in enumerate((4096.0, 1.0, 1.0, -4096.0)):
+        x[:, part * k // 8] = value
+        w[part * k // 8] = abs(value)
+    x, g = x.to(torch.bfloat16), RemoteGemm(w.to(torch.bfloat16), m)
+    y = torch.full((m, n), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    g(x.data_ptr(), m, y.data_ptr(), x_is_local=not pull, cta_pairs=cta_pairs)
+    torch.cuda.synchronize()
+    g.check_status()
+    assert bool((y == (1 if cta_pairs else 0)).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 256, 1536), (128, 512, 8192), (384, 2048, 4096 + 64), (256, 4096, 1536 + 192), (640, 768, 2048)])
+@pytest.mark.parametrize("pull", [False, True])
+def test_few_tiles_on_single_ctas(cuda_device, m, n, k, pull):
+    """K shared by clusters of single CTAs, in two, four and eight shares, of unequal length too; twice, the same bits; and a
+    wait that runs out. The tolerance of test_few_tiles."""
+    g, (args,), (ref,) = _operands("bf16", m, n, k, 1, cuda_device)
+    x, buf, first = args[0], torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device=cuda_device), None
+    for _ in range(2):
+        g(x.data_ptr(), m, buf.data_ptr(), x_is_local=not pull, cta_pairs=False)
+        torch.cuda.synchronize()
+        g.check_status()
+        y = buf[:m].double()
+        assert bool(((y - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
+        assert bool((buf[m] == 7).all())
+        assert first is None or torch.equal(buf, first)
+        first = buf.clone()
+    if pull:
+        buf.fill_(7)
+        g.sched[3] = 0x7fffffff  # nothing of X arrives
+        g(x.data_ptr(), m, buf.data_ptr(), x_is_local=False, cta_pairs=False, timeout_ns=20_000_000)
+        torch.cuda.synchronize()
+        assert int(g.status) & 0xff == 1 and bool((buf == 7).all())
+        assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
