@@ -420,3 +420,61 @@ def test_few_tiles_on_single_ctas(cuda_device, m, n, k, pull):
         torch.cuda.synchronize()
         assert int(g.status) & 0xff == 1 and bool((buf == 7).all())
         assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+
+
+def test_early_launches_over_two_streams(cuda_device):
+    """Pushes and GEMMs on two streams that hand their results to one another over events, with a copy and a memset of the
+    runtime in between: every launch that may come early has something else than a kernel of its own stream in front of it.
+    Long pushes in front of the events, so that a launch that did not wait would read the zeros of before. The sums are
+    of small whole numbers, exact in any order: what torch computes, from plain calls and from a captured graph."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    from execution_ucx_b200.ops.remote_gemm import RemoteGemm
+    rows, k = 16384, 1024
+    x = torch.randint(-2, 3, (rows, k), device=cuda_device).float()
+    w = torch.randint(-1, 2, (k, k), device=cuda_device).to(torch.bfloat16)
+    w[32:] = 0
+    g, h = RemoteGemm(w, 2048), RemoteGemm(w, 2048)
+    a, b, c, p = (torch.empty(rows, k, dtype=torch.bfloat16, device=cuda_device) for _ in range(4))
+    q, r, s = (torch.empty(2048, k, dtype=torch.bfloat16, device=cuda_device) for _ in range(3))
+    other = torch.cuda.Stream()
+    bufs = (a, b, c, p, q, r, s)
+
+    def chain():
+        here = torch.cuda.current_stream()
+        other.wait_stream(here)
+        tx.push(x, a)                                                         # one: long
+        with torch.cuda.stream(other):
+            tx.push(x, p, op=tx.OP_ADD, op_arg=1.0)                           # two: long, of its own
+            other.wait_stream(here)
+            tx.push(a, b, op=tx.OP_MUL, op_arg=0.5)                           # behind an event of one
+            h(p[-2048:].data_ptr(), 2048, q.data_ptr(), x_is_local=True)      # behind a kernel
+        here.wait_stream(other)
+        g(b[-2048:].data_ptr(), 2048, r.data_ptr(), x_is_local=False)         # behind an event of two
+        c.copy_(b)                                                            # a copy of the runtime
+        tx.push(c[-2048:], s, op=tx.OP_ADD, op_arg=1.0)                       # behind the copy
+        c.zero_()
+        g(s.data_ptr(), 2048, c.data_ptr(), x_is_local=True)                  # behind the memset
+
+    tail = x[-2048:].to(torch.bfloat16).double()
+    want_q, want_r = (tail + 1) @ w.double(), (tail * 0.5) @ w.double()
+    want_s = tail * 0.5 + 1
+    want_c = want_s @ w.double()
+
+    def check(run):
+        for buf in bufs:
+            buf.zero_()
+        torch.cuda.synchronize()
+        run()
+        torch.cuda.synchronize()
+        g.check_status()
+        for got, want in ((q, want_q), (r, want_r), (s, want_s), (c[:2048], want_c)):
+            assert torch.equal(got.double(), want)
+        assert not bool(c[2048:].any())
+
+    for _ in range(3):
+        check(chain)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    for _ in range(3):
+        check(graph.replay)
