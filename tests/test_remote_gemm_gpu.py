@@ -103,8 +103,9 @@ def test_few_tiles(cuda_device, fmt, m, n, k, pull):
 @pytest.mark.parametrize("m,n,k", [(1920, 2688, 2048), (1664, 3200, 2176), (3968, 1280, 2432)])
 @pytest.mark.parametrize("pull", [False, "warps"])
 def test_block_scaled_fp8_pairs(cuda_device, m, n, k, pull):
-    """More than one wave of 128 x 128 tiles: the kernel on CTA pairs, with half tiles at the end of M and of N, K-blocks
-    that are not whole batches of scales, and every row's scale different. fp32 sums in another order and one rounding to
+    """More than two waves of 128 x 128 tiles, on single CTAs where pairs would need more than 5 / 8 of the waves (as here) and
+    on pairs otherwise: half tiles at the end of M and of N, K-blocks that are not whole batches of scales, and every row's
+    scale different. fp32 sums in another order and one rounding to
     bf16: half a unit in the last of 8 bits of the result, and 1e-5 of the product's scale for the sums."""
     from execution_ucx_b200.ops import remote_gemm as rg
     torch.manual_seed(m + n + k)
@@ -129,8 +130,8 @@ def test_block_scaled_fp8_pairs(cuda_device, m, n, k, pull):
 @pytest.mark.parametrize("pull", [False, True, "warps"])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 768, 1024), (1024, 512, 2048), (5120, 512, 128)])
 def test_bf16_cta_pairs(cuda_device, m, n, k, pull):
-    """The kernel that computes 256 x 256 tiles on pairs of CTAs (tcgen05 cta_group::2) against fp32 PyTorch,
-    with X read in place, with X streamed in by copying pairs that then join the GEMM, and with X
+    """CTA pairs (tcgen05 cta_group::2), on 128 x 256 tiles where there are few and on 256 x 256 otherwise, against fp32
+    PyTorch, with X read in place, with X streamed in by copying pairs that then join the GEMM, and with X
     streamed in by two warps of every CTA."""
     from execution_ucx_b200.ops.remote_gemm import RemoteGemm
     torch.manual_seed(m + n + k)
@@ -478,3 +479,37 @@ def test_early_launches_over_two_streams(cuda_device):
         chain()
     for _ in range(3):
         check(graph.replay)
+
+
+@pytest.mark.parametrize("pull", [False, True, "warps"])
+@pytest.mark.parametrize("m,n,k", [(2560, 1024, 64), (2560, 2304, 1088), (5120, 1024, 2112), (1536, 1792, 4096)])
+def test_bf16_cta_pairs_of_many_tiles(cuda_device, m, n, k, pull):
+    """More than 74 tiles of 128 x 256, so tiles of 256 x 256: one tile per pair and two, K of one step, of fewer steps than
+    there are stages times tiles, and of many, not a multiple of the stages."""
+    test_bf16_cta_pairs(cuda_device, m, n, k, pull)
+
+
+@pytest.mark.parametrize("pull", [False, "warps"])
+@pytest.mark.parametrize("m,n,k,cta_pairs", [(640, 4096, 1024, True), (1152, 4352, 512, True), (640, 4096, 64, True),
+                                             (2048, 4096, 320, False), (2048, 2560, 4160, False)])
+def test_bf16_one_cta_per_tile(cuda_device, m, n, k, cta_pairs, pull):
+    """More tiles than pairs of SMs on single CTAs: an odd number of row blocks with a short K, or as the caller says. One
+    tile per CTA and two, K of one step and of more than there are stages. The tolerance of test_few_tiles."""
+    g, (args,), (ref,) = _operands("bf16", m, n, k, 1, cuda_device)
+    buf = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    done = torch.zeros(1, dtype=torch.int64, device=cuda_device)
+    for call in range(2):
+        buf[:m].zero_()
+        g(args[0].data_ptr(), m, buf.data_ptr(), x_is_local=not pull, cta_pairs=cta_pairs, done_flag_ptr=done.data_ptr(), done_value=call + 1)
+        torch.cuda.synchronize()
+        g.check_status()
+        assert int(done) == call + 1
+        assert bool(((buf[:m].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
+        assert bool((buf[m] == 7).all())
+        assert int(g.panel_flags.sum()) == 0 and int(g.sched.sum()) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(640, 4096, 1024), (1152, 4352, 512), (2560, 2304, 2048)])
+def test_bf16_of_many_tiles_gives_up(cuda_device, m, n, k):
+    """X never arrives: one CTA per tile, in one wave and in two, and pairs."""
+    test_a_wait_that_runs_out(cuda_device, "bf16", m, n, k)

@@ -13,7 +13,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m", [512, 384])   # 512: the CTA-pair kernel (M % 256 == 0); 384: one CTA per tile
+# 512 and 384: few tiles; 3328: 256 x 256 tiles on CTA pairs; 3200 (an odd number of row blocks, a short K): one CTA per tile
+@pytest.mark.parametrize("m", [512, 384, 3328, 3200])
 def test_noalloc_gemm_matches_regular_entry_point(cuda_device, m):
     from execution_ucx_b200.ops import _native
     from execution_ucx_b200.ops.remote_gemm import RemoteGemm
