@@ -2227,12 +2227,18 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   const int waves = (tiles + sms - 1) / sms, waves2 = (tiles2 + sms / 2 - 1) / (sms / 2);
   // Few tiles: the K of a tile is shared out over a cluster of CTAs (or CTA pairs), which add their sums up through
   // distributed shared memory. All clusters have to fit at once: a second wave costs more.
-  // bf16 on CTA pairs: wherever there is a pair of SMs for each 128 x 256 tile, and several pairs per tile from eight K steps
-  // on, four or more for each. Against single CTAs, which share K from 24 steps on, eight or more for each (calls in a loop):
-  // 128 x 8192 x 8192 30.1 -> 27.8 us, 128 x 512 x 8192 12.8 -> 11.2, 256 x 8192 x 8192 40.5 -> 37.5, 128 x 8192 x 1024
-  // 10.1 -> 8.1 (8.7 without sharing K), 128 x 512 x 512 7.3 -> 6.5, 1152 x 2048 x 1024 (72 tiles) 10.3 -> 9.1.
+  // bf16 on CTA pairs: where there is a pair of SMs for each 128 x 256 tile, from twelve K steps on, with several pairs per
+  // tile where they fit, four steps or more for each. Against single CTAs, which share K from 24 steps on, eight or more for
+  // each (calls in a loop): 128 x 8192 x 8192 30.1 -> 27.8 us, 128 x 512 x 8192 12.8 -> 11.2, 256 x 8192 x 8192 40.5 -> 37.5,
+  // 128 x 8192 x 1024 10.1 -> 8.1 (8.7 without sharing K), 1152 x 2048 x 1024 (72 tiles) 10.3 -> 9.1.
   // 256 x 256 tiles whose K is shared: 256 x 8192 x 2048 13.7 against 11.7 us, 256 x 8192 x 8192 35.2 against 35.5.
+  // A shorter K goes to single CTAs, which have no cluster to set up: with X in place pairs are ahead from eight steps on, with
+  // X copied from about fourteen (pairs and single CTAs, graph replays; 512 x 1024, K = 512 6.9 and 8.1 us, copied 10.1 and 8.9;
+  // 768 7.4 and 9.3, 10.4 and 10.2; 1024 7.8 and 10.3, 10.7 and 11.5), and the line is the same for both, so that a call has the
+  // same bits either way. Tiles whose K is not shared have the same bits on both, and with X copied they keep to single CTAs
+  // up to twenty steps (1152 x 2048, copied: K = 1024 13.0 and 12.6, 1280 14.4 and 14.8).
   // fp8 and MXFP8, whose partial sums are twice as large for a CTA's operand bytes: from 24 steps on, eight for each.
+  bool few_tiles = false;  // bf16: as many pairs of SMs as tiles
   if (!pull || copy_by_warps) {
     int clusters = 0;
     if (mx) {
@@ -2252,8 +2258,9 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
       }
     } else if (!d->fp8 && (d->flags & EUX_GEMM_FLAG_CTA_PAIRS)) {
       clusters = sms / 2;
-      const int s = choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, tiles, 2, k_iters, 8, 4, &clusters);
-      if (tiles <= clusters) {
+      const int s = choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, tiles, 2, k_iters, 12, 4, &clusters);
+      few_tiles = tiles <= clusters;
+      if (few_tiles && k_iters >= (pull && s == 1 ? 20 : 12)) {
         if (!pull) clusters = tiles;
         CUtensorMap mx2, mb2;  // a CTA's half of either operand
         if (int rc = make_map(&mx2, d->x_stage, eb, (uint64_t)d->M, (uint64_t)d->K, BM / 2)) return rc;
@@ -2278,9 +2285,9 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   }
   // bf16 on CTA pairs (bit 0 of the descriptor's flags): a K step of a 256 x 256 tile takes 0.35 us, one of a single
   // CTA's 128 x 256 tile 0.40, so pairs are taken unless half a tile of padding (M an odd number of 128-row blocks)
-  // costs them a wave or K is short (calls in a loop: 640 x 8192 x 8192 90 us against 102, 640 x 4096 x 1024 16.3 against
+  // costs them a wave, K is short or there are few tiles (calls in a loop: 640 x 8192 x 8192 90 us against 102, 640 x 4096 x 1024 16.3 against
   // 14.6). CTAs that copy X before they compute keep to whole tiles.
-  const bool pairs_bf16 = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) && !d->fp8 &&
+  const bool pairs_bf16 = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) && !d->fp8 && !few_tiles &&
                           (d->M % (2 * BM) == 0 || ((!pull || copy_by_warps) && waves2 <= waves && k_iters >= 24));
   // Block-scaled fp8 on CTA pairs: a K-block takes 0.54 us of a pair's 256 x 256 tile and 0.35 us of a CTA's 128 x 128
   // tile, so the pairs are taken when they need at most 5 / 8 of the waves and K is not short (calls in a loop, pairs and
@@ -2346,7 +2353,7 @@ static int prepare_bf16(int dev) {
   if (e == cudaSuccess) e = allow_smem<remote_gemm_2cta_kernel<false, false>>(dev, PairCfg<false>::SMEM);
   int clusters = 0;  // one tile and a long K: every size of cluster is asked about
   if (e == cudaSuccess) e = allow_smem<remote_gemm_few_tiles_kernel>(dev, FEW_SMEM);
-  choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, 1, 2, 64, 8, 4, &clusters);
+  choose_split<remote_gemm_few_tiles_kernel>(dev, GEMM_THREADS, FEW_SMEM, 1, 2, 64, 12, 4, &clusters);
   return (int)e;
 }
 

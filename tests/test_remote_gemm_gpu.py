@@ -295,8 +295,9 @@ def test_calls_behind_one_another(cuda_device, m, k, pull):
                                    (128, 4096, 16 * 64)])
 @pytest.mark.parametrize("pull", [False, True])
 def test_few_tiles_of_any_k(cuda_device, m, n, k, pull):
-    """A pair of SMs for each tile: one K step and more than there are stages, one, two and four shares of K of unequal
-    length, one tile, and as many as there are pairs. The tolerance of test_few_tiles."""
+    """At most a pair of SMs for each tile: a K of less than twelve steps, which is a single CTA's, of one step and of more
+    than there are stages; and on pairs one and four shares of K, of unequal length, one tile, and about as many as there are
+    pairs. The tolerance of test_few_tiles."""
     test_few_tiles(cuda_device, "bf16", m, n, k, pull)
 
 
@@ -513,3 +514,37 @@ def test_bf16_one_cta_per_tile(cuda_device, m, n, k, cta_pairs, pull):
 def test_bf16_of_many_tiles_gives_up(cuda_device, m, n, k):
     """X never arrives: one CTA per tile, in one wave and in two, and pairs."""
     test_a_wait_that_runs_out(cuda_device, "bf16", m, n, k)
+
+
+@pytest.mark.parametrize("pull", [False, True])
+@pytest.mark.parametrize("k,paired", [(512, False), (704, False), (768, True), (1024, True)])
+def test_short_k_with_few_tiles(cuda_device, k, paired, pull):
+    """K of less than twelve steps stays on single CTAs, wherever X is. The order of the sums tells, as in
+    test_cta_pairs_is_what_the_caller_says: 2^24 + 1 in the first half of K, 1 - 2^24 at the start of the second."""
+    from execution_ucx_b200.ops.remote_gemm import RemoteGemm
+    m, n = 256, 512
+    x, w = torch.zeros(m, k, device=cuda_device), torch.zeros(k, n, device=cuda_device)
+    for at, value in ((0, 4096.0), (64, 1.0), (k // 128 * 64, 1.0), (k // 128 * 64 + 64, -4096.0)):
+        x[:, at] = value
+        w[at] = abs(value)
+    x, g = x.to(torch.bfloat16), RemoteGemm(w.to(torch.bfloat16), m)
+    y = torch.full((m, n), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    g(x.data_ptr(), m, y.data_ptr(), x_is_local=not pull)
+    torch.cuda.synchronize()
+    g.check_status()
+    assert bool((y == (1 if paired else 0)).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 512, 512), (512, 1024, 768), (128, 8192, 960), (768, 1536, 1024), (1152, 2048, 768),
+                                   (256, 9472, 1216), (640, 2048, 1280)])
+def test_few_tiles_the_same_bits_wherever_x_is(cuda_device, m, n, k):
+    """On both sides of the lengths of K from which few tiles are computed by pairs, K shared and not, where a call whose X is
+    streamed in may take another kernel than one whose X is in place."""
+    g, (args,), (ref,) = _operands("bf16", m, n, k, 1, cuda_device)
+    here, there = (torch.zeros(m, n, dtype=torch.bfloat16, device=cuda_device) for _ in range(2))
+    g(args[0].data_ptr(), m, here.data_ptr(), x_is_local=True)
+    g(args[0].data_ptr(), m, there.data_ptr(), x_is_local=False)
+    torch.cuda.synchronize()
+    g.check_status()
+    assert torch.equal(here, there)
+    assert bool(((here.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5 * ref.abs().amax(1, keepdim=True)).all())
