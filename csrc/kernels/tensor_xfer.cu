@@ -102,11 +102,13 @@ __device__ __forceinline__ void cta_publish(const eux_xfer_desc& d, uint32_t* co
 
 // The first and the last thing a transfer kernel does. What follows in the stream may be launched when a CTA has issued its
 // last stores, and from the start where the whole takes a few microseconds (a source of up to 32 MiB). It sits on the SMs
-// until the transfer ends: let in at the start, a GEMM behind a push of 1 GiB held up a small GEMM of another stream for as long as
-// the push and itself took, 0.98 ms instead of 0.34, and large transfers in a loop were no faster for it (4096 x 7168 fp32 to
-// e4m3 23.8 us and 23.3 from the end on, 8192 x 8192 bf16 transposed 45.4 and 45.0). A push of 640 x 1024 with a
-// GEMM of 640 x 4096 x 1024 behind it takes 11.8 us with the GEMM let in at the start and 12.9 at the end, pushes of 16 MiB
-// 4.48 and 4.62 (graph replays).
+// until the transfer ends: let in at the start, a GEMM behind a push of 1 GiB held up a small GEMM of another stream for as
+// long as the push and itself took, 0.98 ms instead of 0.34, and large transfers in a loop were no faster for it (4096 x 7168
+// fp32 to e4m3 23.8 us and 23.4 from the end on). A push of 640 x 1024 with a GEMM of 640 x 4096 x 1024 behind it takes 11.8 us
+// with the GEMM let in at the start and 13.1 at the end, pushes of 16 MiB 4.42 and 4.55 (graph replays).
+// Tiles let it in at the end only: several small launches were on the SMs at a time and the later ones of them found room on
+// some SMs more than on others (2048 x 2048 e4m3 to bf16 transposed, graph replays, 6.5 us, 4.1 so, 4.5 without early launches;
+// bytes 5.3, 3.2 and 3.6).
 __device__ __forceinline__ void xfer_begin(const eux_xfer_desc& d) {
   if (d.wait_flag == nullptr && d.n_elems * (uint64_t)dtype_size(d.src_dtype) <= (32u << 20)) allow_next_launch();
   wait_for_launch_before();
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(kTileThreads) xfer_tile_kernel(const __grid_co
   constexpr uint32_t PITCH = QW + 1;
   __shared__ uint32_t sm[TP * PITCH > kTileWords ? TP * PITCH : kTileWords];
   const eux_xfer_desc& d = t.x.d;
-  xfer_begin(d);
+  wait_for_launch_before();
   const bool ok = cta_wait_arrival(d);
   if (ok) {
     const int op = d.op;
@@ -777,7 +779,7 @@ template <typename S, typename D, bool RAW>
 __global__ void __launch_bounds__(kTileThreads) xfer_narrow_kernel(const __grid_constant__ TileArgs t) {
   __shared__ __align__(16) unsigned char sm[kNarrowBytes];
   const eux_xfer_desc& d = t.x.d;
-  xfer_begin(d);
+  wait_for_launch_before();
   const bool ok = cta_wait_arrival(d);
   if (ok) {
     constexpr uint32_t E = 16 / sizeof(D);

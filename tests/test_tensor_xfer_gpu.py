@@ -428,3 +428,34 @@ def test_what_follows_a_push_leaves_room_for_other_streams(cuda_device):
         if apart:
             push, gemm = start.elapsed_time(pushed), pushed.elapsed_time(end)
     assert start.elapsed_time(small_end) < push + 0.5 * gemm
+
+
+def test_small_transposes_in_a_graph(cuda_device):
+    """Transposes of 4 MiB behind one another in a graph, each of 128 tiles. Launched early they may not take longer than with
+    a memset of the runtime, which keeps the next launch back, between each two of them."""
+    from execution_ucx_b200.ops import tensor_xfer as tx
+    x = torch.randint(0, 256, (2048, 2048), dtype=torch.uint8, device=cuda_device)
+    ys = [torch.empty_like(x) for _ in range(6)]
+    word = torch.zeros(1, dtype=torch.int32, device=cuda_device)
+
+    def graph(apart):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for i in range(48):
+                tx.push(x.t(), ys[i % 6])
+                if apart:
+                    word.zero_()
+        return g
+
+    tx.push(x.t(), ys[0])
+    graphs, best = (graph(False), graph(True)), [float("inf")] * 2
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for _ in range(20):
+        for i, g in enumerate(graphs):
+            start.record()
+            g.replay()
+            end.record()
+            torch.cuda.synchronize()
+            best[i] = min(best[i], start.elapsed_time(end))
+    assert all(torch.equal(y, x.t()) for y in ys)
+    assert best[0] < best[1]
