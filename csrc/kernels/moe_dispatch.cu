@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(kMoeThreads, 2) moe_dispatch_fp8_kernel(eux_mo
 // ---- dispatch, e4m3 rows, two tokens per CTA and more: row images in shared memory, moved by bulk copies -------------------
 // Twelve warps quantise units of (token, 1024 elements) into images of whole rows (values, scales, padding) in a ring of
 // slots; four warps send the finished images to their top-k rows, a bulk copy each. The kernel above has what its registers
-// hold in flight and a barrier in front of the scales: 43 % of the DRAM's rate at 4096 tokens of 7168. Dispatches in a
-// loop, above and here: 4096 x 7168 75.1 and 65.0 us, 4096 x 2048 32.6 and 25.9, 1024 x 7168 25.7 and 23.0, 300 x 7168 16.0
+// hold in flight and a barrier in front of the scales: 4096 tokens of 7168 keep the DRAM at 43 % of its peak (ncu, part of
+// the rows still in L2 at the end). Dispatches in a loop, above and here: 4096 x 7168 75.1 and 65.0 us, 4096 x 2048 32.6 and 25.9, 1024 x 7168 25.7 and 23.0, 300 x 7168 16.0
 // and 15.9, 128 x 7168 13.3 and 14.1 (with one sending warp 65.4, 34.0, 22.8, 15.8: its look-ups are a trip to L2 per token).
 // Token tl of the CTA: slot tl % slots, barriers tl % 32, sending warp tl % 4. The number of slots is a multiple of four
 // too, so everything about a token belongs to one of four classes, each of which one warp sends in order. A quantising warp

@@ -1559,7 +1559,8 @@ remote_gemm_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 //   * a K step brings 24 KiB into a CTA: eight stages.
 // K is shared out over p.split pairs of a cluster (1, 2 or 4), which add their sums up in the order of the shares.
 // One tile per cluster; clusters past the last tile only help to copy X.
-// 128 x 8192 x 8192 takes 27.5 us a call (30.1 with four single CTAs to a tile), 20.5 of them W at the rate of HBM.
+// Calls in a loop, and with single CTAs that share K (cta_pairs=False): 128 x 7168 x 7168 23.2 and 25.7 us, 128 x 8192 x 8192, of
+// which W at the rate of HBM is 20.5, 30.3 and 31.0.
 // ---------------------------------------------------------------------------
 constexpr int FEW_STAGES = 8;
 constexpr int FEW_X_BYTES = (BM / 2) * BKB;
@@ -1760,8 +1761,9 @@ remote_gemm_few_tiles_kernel(const __grid_constant__ CUtensorMap map_x, const __
 //     warp's chain (waiting, TMEM loads, the arrive) is latency, which four warps per scheduler hide better than two.
 //   * The loading warp multiplies and stages the scales, eight K-blocks at a time, so that a fold reads one word. Staged by
 //     the folding warps they cost each of them 200 cycles per K-block. It holds a batch in registers while it issues loads.
-// 1920 x 4608 x 7168: 74.9 us with eight folding warps that staged their scales, 64.6 now (calls in a loop). Tried: the two
-// halves of the columns as products of their own, four in flight (66.5 to 74: the MMA warp waits and commits more often).
+// 1920 x 4608 x 7168: 74.9 us with eight folding warps that staged their scales, 64.6 so (graph replays at full clocks; under
+// the power cap up to 79). Tried: the two halves of the columns as products of their own, four in flight (66.5 to 74: the
+// MMA warp waits and commits more often).
 // Twenty warps of 96 registers fill the register file; a twenty-first would leave each 80.
 // Rows and columns past M and N (both are multiples of 128, a tile is 256) are zero-filled loads, and nothing is stored
 // for them.
@@ -2229,8 +2231,9 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   // distributed shared memory. All clusters have to fit at once: a second wave costs more.
   // bf16 on CTA pairs: where there is a pair of SMs for each 128 x 256 tile, from twelve K steps on, with several pairs per
   // tile where they fit, four steps or more for each. Against single CTAs, which share K from 24 steps on, eight or more for
-  // each (calls in a loop): 128 x 8192 x 8192 30.1 -> 27.8 us, 128 x 512 x 8192 12.8 -> 11.2, 256 x 8192 x 8192 40.5 -> 37.5,
-  // 128 x 8192 x 1024 10.1 -> 8.1 (8.7 without sharing K), 1152 x 2048 x 1024 (72 tiles) 10.3 -> 9.1.
+  // each (calls in a loop, single CTAs and pairs): 128 x 8192 x 8192 31.0 and 30.3 us, 128 x 8192 x 4096 15.4 and 13.3,
+  // 128 x 512 x 8192 14.0 and 12.1, 256 x 8192 x 8192 42 and 38, 128 x 8192 x 1024 11.3 and 9.6, 1152 x 2048 x 1024 (72 tiles)
+  // 11.5 and 10.9.
   // 256 x 256 tiles whose K is shared: 256 x 8192 x 2048 13.7 against 11.7 us, 256 x 8192 x 8192 35.2 against 35.5.
   // A shorter K goes to single CTAs, which have no cluster to set up: with X in place pairs are ahead from eight steps on, with
   // X copied from about fourteen (pairs and single CTAs, graph replays; 512 x 1024, K = 512 6.9 and 8.1 us, copied 10.1 and 8.9;
@@ -2290,9 +2293,9 @@ extern "C" int eux_gemm_launch(const eux_gemm_desc* d, void* stream) {
   const bool pairs_bf16 = (d->flags & EUX_GEMM_FLAG_CTA_PAIRS) && !d->fp8 && !few_tiles &&
                           (d->M % (2 * BM) == 0 || ((!pull || copy_by_warps) && waves2 <= waves && k_iters >= 24));
   // Block-scaled fp8 on CTA pairs: a K-block takes 0.54 us of a pair's 256 x 256 tile and 0.35 us of a CTA's 128 x 128
-  // tile, so the pairs are taken when they need at most 5 / 8 of the waves and K is not short (calls in a loop, pairs and
-  // single CTAs: 1920 x 4608 x 7168, two waves of four, 65 and 84 us; 2560 x 4096 x 4096, three of five, 58 and 62;
-  // 1536 x 4096 x 2048, two of three, 27 and 24; 4096 x 4096 x 512 23 and 23).
+  // tile, so the pairs are taken when they need at most 5 / 8 of the waves and K is not short (graph replays at full
+  // clocks, pairs and single CTAs: 1920 x 4608 x 7168, two waves of four, 65 and 84 us; 2560 x 4096 x 4096, three of five,
+  // 58 and 62; 1536 x 4096 x 2048, two of three, 27 and 24; 4096 x 4096 x 512 23 and 23).
   const bool pairs_fp8 = d->fp8 && !mx && (!pull || copy_by_warps) && waves2 * 8 <= waves * 5 && k_iters >= 16;
   if (mx || pairs_bf16 || pairs_fp8) {
     CUtensorMap mb2;  // this CTA's half of a Wt tile: 128 rows

@@ -1,6 +1,6 @@
 """Small, self-ending cases of each data-plane kernel, for profiler captures.
 
-    python -m execution_ucx_b200.models.profile_case --kernel gemm        (CTA pairs; gemm_1cta: one CTA per tile)
+    python -m execution_ucx_b200.models.profile_case --kernel gemm        (CTA pairs; gemm_1cta: one CTA per tile; gemm_few: few tiles)
     python -m execution_ucx_b200.models.profile_case --kernel gemm_fp8   (or gemm_mx)
     python -m execution_ucx_b200.models.profile_case --kernel xfer
     python -m execution_ucx_b200.models.profile_case --kernel moe
@@ -22,19 +22,20 @@ import torch
 
 def main() -> None:
     ap = argparse.ArgumentParser()
-    ap.add_argument("--kernel", choices=["gemm", "gemm_1cta", "gemm_fp8", "gemm_mx", "xfer", "pull_batch", "moe", "moe_fp8", "gemm_pull", "gemm_mx_pull", "gemm_fp8_pull", "xfer_peer", "xfer_gather"], required=True)
+    ap.add_argument("--kernel", choices=["gemm", "gemm_1cta", "gemm_few", "gemm_fp8", "gemm_mx", "xfer", "pull_batch", "moe", "moe_fp8", "gemm_pull", "gemm_mx_pull", "gemm_fp8_pull", "xfer_peer", "xfer_gather"], required=True)
     ap.add_argument("--iters", type=int, default=3)
     args = ap.parse_args()
     dev = torch.device("cuda", 0)
-    if args.kernel in ("gemm", "gemm_1cta"):
+    if args.kernel in ("gemm", "gemm_1cta", "gemm_few"):
         from ..ops.remote_gemm import RemoteGemm
-        m, n, k = 4096, 4096, 4096  # 3 x 32 MiB operands/result: > L2 in total, milliseconds per launch
+        # 3 x 32 MiB operands/result, a tenth of a millisecond per launch; or one row block against a weight larger than L2
+        m, n, k = (128, 8192, 8192) if args.kernel == "gemm_few" else (4096, 4096, 4096)
         x = torch.randn(m, k, device=dev).to(torch.bfloat16)
         w = (torch.randn(k, n, device=dev) * 0.02).to(torch.bfloat16)
         g = RemoteGemm(w, m)
         y = torch.empty(m, n, dtype=torch.bfloat16, device=dev)
         for _ in range(args.iters):
-            g(x.data_ptr(), m, y.data_ptr(), x_is_local=True, cta_pairs=args.kernel == "gemm")
+            g(x.data_ptr(), m, y.data_ptr(), x_is_local=True, cta_pairs=args.kernel != "gemm_1cta")
         torch.cuda.synchronize()
         g.check_status()
     elif args.kernel in ("gemm_pull", "gemm_mx_pull", "gemm_fp8_pull", "xfer_peer"):
