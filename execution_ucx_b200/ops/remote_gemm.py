@@ -234,7 +234,7 @@ def smoke(device) -> None:
     """Every bf16 kernel on a tiny shape (pairs of CTAs with few tiles, X pulled by the copy warps; pairs with many; one CTA
     per tile), and the MXFP8 kernel."""
     y = torch.empty(2560 * 1024, dtype=torch.bfloat16, device=device)
-    for m, n, k, kw in ((256, 512, 256, dict(x_is_local=False)), (2560, 1024, 64, dict(x_is_local=True)),
+    for m, n, k, kw in ((256, 512, 768, dict(x_is_local=False)), (2560, 1024, 64, dict(x_is_local=True)),
                         (256, 512, 256, dict(x_is_local=True, cta_pairs=False))):
         x = torch.randn(m, k, device=device).to(torch.bfloat16)
         w = (torch.randn(k, n, device=device) * 0.05).to(torch.bfloat16)

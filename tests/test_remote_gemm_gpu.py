@@ -130,9 +130,9 @@ def test_block_scaled_fp8_pairs(cuda_device, m, n, k, pull):
 @pytest.mark.parametrize("pull", [False, True, "warps"])
 @pytest.mark.parametrize("m,n,k", [(256, 256, 64), (512, 768, 1024), (1024, 512, 2048), (5120, 512, 128)])
 def test_bf16_cta_pairs(cuda_device, m, n, k, pull):
-    """CTA pairs (tcgen05 cta_group::2), on 128 x 256 tiles where there are few and on 256 x 256 otherwise, against fp32
-    PyTorch, with X read in place, with X streamed in by copying pairs that then join the GEMM, and with X
-    streamed in by two warps of every CTA."""
+    """CTA pairs (tcgen05 cta_group::2), on 128 x 256 tiles where there are few (whose K, of one step, is a single CTA's in the
+    first shape unless CTAs copy X) and on 256 x 256 otherwise, against fp32 PyTorch, with X read in place, with X streamed in
+    by copying pairs that then join the GEMM, and with X streamed in by two warps of every CTA."""
     from execution_ucx_b200.ops.remote_gemm import RemoteGemm
     torch.manual_seed(m + n + k)
     x = torch.randn(m, k, device=cuda_device).to(torch.bfloat16)

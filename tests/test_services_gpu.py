@@ -32,7 +32,7 @@ def test_remote_gemm_and_moe_through_the_runtime_one_gpu(cuda_device):
                 # block-scaled product but the same numbers, up to the order of the fp32 additions
                 assert w.max_abs_err(256) < 2e-2, w.max_abs_err(256)
         assert api.server.gemm_launches() == 8
-        # M that is not a multiple of 256: one CTA per tile with many tiles, and a few tiles on pairs
+        # M that is not a multiple of 256: one CTA per tile, with many tiles and with few
         w = RemoteGemmAxon(api, 4992, 512, 512, fmt="bf16", weight_id=8)
         await w.step()
         assert w.max_abs_err(128) < 0.25
