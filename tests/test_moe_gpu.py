@@ -382,7 +382,7 @@ def test_dispatches_of_several_threads(cuda_device):
     import threading
     from execution_ucx_b200.ops import _native, moe
     t, launch = 4, _native.load().eux_moe_dispatch_launch
-    start, refused, work = threading.Barrier(4), [], []
+    start, refused, work = threading.Barrier(4, timeout=60), [], []
     for hidden, ne in [(12928, 4096), (7168, 8), (12928, 4096), (11008, 8)]:
         (rk,) = moe.MoeAllToAll.emulated(1, t, hidden, 2, ne, fp8=True)
         work.append((rk, torch.randn(t, hidden, device=cuda_device).to(torch.bfloat16), *_routing(t, 2, ne, cuda_device, hidden)))
